@@ -226,9 +226,9 @@ int fh_h_batch_set_u(fh_h_batch *b, const double *U);
 int fh_h_batch_restart(fh_h_batch *b, int i, const fh_h_params *p, const double *U0_host);
 /* Small batches (at most 32 instances of at most 2046 interior nodes, FP64
  * history, no space-fractional instances) run all the steps of one
- * fh_h_batch_step call in one launch: a cluster of eight CTAs per instance
- * shares the history sum (distributed shared memory) and one of them solves
- * the line, step after step, with cluster barriers between.  On by default;
+ * fh_h_batch_step call in one launch: a cluster of four to sixteen CTAs per
+ * instance, one of which solves the line of a step while the others prepare
+ * the weights and history sums of the next one.  On by default;
  * enable = 0 steps such batches kernel by kernel like larger ones (the same
  * sums within FP64 rounding: the history splits differ).  No reference
  * counterpart. */

@@ -2,9 +2,9 @@
 // mt_psi_caputo.cpp:369-1507 with gamma = 1): per step
 //   1. k_h_weights      per-instance history weights and current weight
 //   2. k_hist_tiles     history sum per instance segment (split-K partials)
-//   3. k_h_line_warp    one warp per instance: coefficients, right part,
-//                       Thomas sweep as warp scans, back substitution,
-//                       history append
+//   3. k_h_line         one CTA per instance: coefficients, right part,
+//                       elimination and substitutions as scans, history
+//                       append (fh_hline.cuh)
 //
 // All instances advance in lock step.  The concatenated state holds each
 // instance's N_i+2 nodes in a segment padded to an even length; the history
@@ -22,6 +22,7 @@
 #include "fh_df.cuh"
 #include "fh_slices.cuh"
 #include "fh_weights.cuh"
+#include "fh_hline.cuh"
 
 // batched far contraction on the tensor cores (fh_blocked.cu)
 struct fh_hblk;
@@ -36,21 +37,6 @@ __nv_bfloat16 *fh_hblk_wplanes(fh_hblk &b);
 int8_t *fh_hblk_wexp(fh_hblk &b);
 int fh_hblk_kcap(const fh_hblk &b);
 size_t fh_hblk_bytes(const fh_hblk &b);
-
-struct fh_h_dev_inst {
-  int N, weights, kmodel, gravity;
-  int fixed;  // coefficients independent of u and of the step: factor once
-  // the instance's own clock (fh_h_batch_restart): its step is tstep - tb and
-  // its saved-layer count nsaved - ob; history slots below ob belong to an
-  // earlier occupant and are never read
-  int tb, ob;
-  long long off;  // segment start in the concatenated state
-  double dL, Dg, Da, tau, alpha, beta, kc, kgam, cinv, al_left, bt_left, u_right;
-  // space-fractional derivative in z (fh_h_batch_set_space_order): order
-  // spg, spA = 1 - spg (0: classical second derivative), kbf = the
-  // mt_psi_caputo factor kb(gamma, i-1, i, i) of A, B, R
-  double spg, spA, kbf;
-};
 
 struct fh_h_tile {
   int inst;
@@ -69,14 +55,12 @@ struct fh_h_batch {
   long long Ptot = 0;
   std::vector<fh_h_params> hp;
   std::vector<long long> off;
-  fh_dbuf inst, U, D, W, Lb, ibt, lgt, wc, part, Al, Bt, sA, sB, sR, sOm;
+  fh_dbuf inst, U, D, W, Lb, ibt, lgt, wc, part, Al, Bt, fF, fG;  // fF, fG: factors of fixed instances
   fh_graph_cache graph;
   bool use_graph = true;
   int mode = FH_H_FP64;  // FH_H_DF64: history as (hi, lo) FP32 pairs; FH_H_BLOCKED: below
-  // Al of the variable-coefficient instances serially in the reference order
-  // (h_alpha_serial); varcoef: the batch has such instances
-  bool serial_al = true, varcoef = false;
   bool persistent = true;  // small FP64 batches: one launch per call (k_h_persistent)
+  int pers_ctas = 4;       // CTAs per instance there
   std::vector<fh_h_dev_inst> di;  // host copy of inst
   std::vector<int> cap;           // nodes a restarted occupant of each instance may have (segment - 2)
   // space-fractional instances: Toeplitz weights wsp and the sums sV per
@@ -110,7 +94,7 @@ struct fh_h_batch {
 static constexpr int kTileThreads = 512;  // largest tile CTA (1024 nodes)
 static constexpr int kTileShapes[3] = {128, 256, 512};  // candidate tile CTAs
 static inline int tile_shape_index(int threads) { return threads == 128 ? 0 : threads == 256 ? 1 : 2; }
-static constexpr int kLineCtaMaxInst = 152;  // batches below this many instances solve one CTA per instance
+static constexpr int kLineCtaMaxInst = 152;  // batches below this many instances: eight warps per line, weights ahead on the side stream
 static constexpr int kSpaceMaxN = 2048;  // nodes of a space-fractional instance (shared-memory sums)
 static constexpr int kHWeightThreads = 128;                 // slots per weights CTA
 // per psi instance: Lc[kIbTerms] | Uc[kIbTerms] | B(a, b) | kIbLowMax^(1/beta) |
@@ -361,286 +345,70 @@ __global__ void __launch_bounds__(256) k_h_space_v(const fh_h_dev_inst *__restri
   if (threadIdx.x == 0) V[I.off] = 0.0;
 }
 
-__device__ __forceinline__ double fh_h_K(const fh_h_dev_inst &I, double u) {
-  return I.kmodel == FH_K_CONST ? I.kc : I.kc * exp(I.kgam * u);
-}
-
-// New history entry: FP64, or a (hi, lo) FP32 pair in the double-float mode.
-__device__ __forceinline__ void fh_h_store_diff(double *D, long long i, double d, int dfstore) {
-  if (dfstore)
-    reinterpret_cast<float2 *>(D)[i] = fh_df_pair(fh_df_from_double(d));
-  else
-    D[i] = d;
-}
-
-// H_solver::U1 with one warp per instance (al1, Om1, bt1, bottom Dirichlet,
-// back substitution, history append).  The serial recurrences become warp
-// scans over per-lane chunks of consecutive equations:
-//   Al[i+1] = B_i / (R_i - A_i Al[i])            Moebius maps (matrix scan)
-//   Bt[i+1] = (Al[i+1]/B_i)(A_i Bt[i] - Om_i)    affine maps
-//   u_i     = Al[i+1] u_{i+1} + Bt[i+1]           affine maps, reverse order
-// after which every lane re-walks its chunk from the scanned start value with
-// one reciprocal per equation (Al[i+1] = B_i g, g = 1 / (R_i - A_i Al[i])).  The coefficients are kept in the scratch
-// arrays sA, sB, sR (reused for Al[i+1]/B_i) and sOm at the equation's node.
-// Scans and syncs of one instance's group of threads: one warp (NW = 1) or
-// the whole CTA (NW warps, named barrier 1).
-template <int NW>
-struct HGroup {
-  static __device__ __forceinline__ fh_mob mob(fh_mob f, fh_mob *sm) { return fh_group_exclusive_mob<NW>(f, sm, 1); }
-  static __device__ __forceinline__ fh_aff aff(fh_aff f, fh_aff *sm) { return fh_group_exclusive_affine<NW>(f, sm, 1); }
-  static __device__ __forceinline__ fh_aff aff_rev(fh_aff f, fh_aff *sm) {
-    return fh_group_exclusive_affine_rev<NW>(f, sm, 1);
-  }
-  static __device__ __forceinline__ void sync() { __syncthreads(); }
-};
-template <>
-struct HGroup<1> {
-  static __device__ __forceinline__ fh_mob mob(fh_mob f, fh_mob *) { return fh_warp_exclusive_mob(f); }
-  static __device__ __forceinline__ fh_aff aff(fh_aff f, fh_aff *) { return fh_warp_exclusive_affine(f); }
-  static __device__ __forceinline__ fh_aff aff_rev(fh_aff f, fh_aff *) { return fh_warp_exclusive_affine_rev(f); }
-  static __device__ __forceinline__ void sync() { __syncwarp(); }
-};
-
-// Parts of the line solve one launch runs: everything (kLineAll), the
-// coefficients and right parts only (kLineCoef), or the sweeps from an Al
-// already in memory (kLineSolve; k_h_alpha_lanes writes it in between).
-enum { kLineAll = 0, kLineCoef = 1, kLineSolve = 2 };
-
-// Al[i+1] = B_i / (R_i - A_i Al[i]) for i = 1..N-1 from Al[1], serially in the
-// order and arithmetic of H_solver::al1 (mt_psi_caputo.cpp:1262-1292,
-// mt_minimal.cpp:829-858): the product, the difference and the quotient are
-// each rounded once (no contraction), so the factors are those of the
-// reference for the same coefficients.  The Thomas factors of a diffusion line
-// are a weakly contracting recurrence: any re-association of it (a parallel
-// scan) changes every factor by a few ulps, and over hundreds of steps of a
-// 1000-node line those changes grew to 1e-10 of the solution.
-__device__ __forceinline__ void h_alpha_serial(int N, double al_left, const double *__restrict__ A,
-                                               const double *__restrict__ B, const double *__restrict__ R,
-                                               double *__restrict__ Al) {
-  double a = al_left;
-  Al[1] = a;
-  int i = 1;
-  for (; i + 4 <= N; i += 4) {  // coefficient loads ahead of the dependent chain
-    double Aq[4], Bq[4], Rq[4];
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      Aq[k] = A[i + k];
-      Bq[k] = B[i + k];
-      Rq[k] = R[i + k];
-    }
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      a = __ddiv_rn(Bq[k], __dsub_rn(Rq[k], __dmul_rn(Aq[k], a)));
-      Al[i + k + 1] = a;
-    }
-  }
-  for (; i < N; ++i) {
-    a = __ddiv_rn(B[i], __dsub_rn(R[i], __dmul_rn(A[i], a)));
-    Al[i + 1] = a;
-  }
-}
-
-// One instance by a group of 32 NW threads; `lane` is the thread's index in
-// the group (its chunk of consecutive equations).  serial: Al of the
-// variable-coefficient instances serially (h_alpha_serial, by lane 0 in
-// kLineAll launches); otherwise by the Moebius scan (kLineAll only).
-template <int NW, bool SPACE, int PH>
-__device__ __forceinline__ void h_line(const fh_h_dev_inst &I, int b, int lane, double *__restrict__ U,
-                                       const double *__restrict__ wc, const double *__restrict__ part,
-                                       long long ldpart, int splits, double *__restrict__ Al,
-                                       double *__restrict__ Bt, double *__restrict__ sA, double *__restrict__ sB,
-                                       double *__restrict__ sR, double *__restrict__ sOm, double *__restrict__ Dnew,
-                                       int append, int os, int dfstore, const double *__restrict__ sV,
-                                       fh_mob *smm, fh_aff *sma, int serial) {
-  constexpr int TG = 32 * NW;
-  const bool first = os == I.ob;  // the instance's first step (saved-layer count os)
-  const long long o = I.off;
-  double *u = U + o;
-  const int N = I.N;
-  const double DaW = I.Da * wc[b];
-  // ---- pass 1: coefficients of equations i in [f0, f1), chunk Moebius map;
-  // the products and sums in the reference's order, each rounded once
-  const int chf = (N - 1 + TG - 1) / TG;
-  const int f0 = 1 + lane * chf, f1 = min(N, f0 + chf);
-  fh_mob T{1.0, 0.0, 0.0, 1.0};
-  if (PH != kLineSolve && f0 < f1) {
-    double Km = fh_h_K(I, u[f0 - 1]), Kc = fh_h_K(I, u[f0]);
-    for (int i = f0; i < f1; ++i) {
-      const double Kp = fh_h_K(I, u[i + 1]);
-      double A = I.Dg * Km * I.cinv;
-      double B = I.Dg * Kp * I.cinv;
-      double R = I.cinv * (Kp + Km) * I.Dg;
-      double om = -DaW * u[i];
-      if (SPACE && I.spA != 0.0) {  // space-fractional derivative (k_h_space_v)
-        if (I.weights == FH_W_PSI) {
-          A = A * I.kbf * I.spA;
-          B = B * I.kbf * I.spA;
-          R = R * I.kbf * I.spA;
-        }
-        const double flux = __dsub_rn(__dmul_rn(Kc, sV[o + i]), __dmul_rn(Km, sV[o + i - 1]));
-        om = __dsub_rn(-I.Dg * I.cinv * flux, DaW * u[i]);
-      }
-      R = __dadd_rn(R, DaW);
-      if (I.gravity) om = __dadd_rn(om, __ddiv_rn(Kc - Km, I.dL));
-      double ts = 0.0;
-      for (int s = 0; s < splits; ++s) ts += part[(long long)s * ldpart + o + i];
-      om = __dadd_rn(om, __dmul_rn(I.Da, ts));
-      sOm[o + i] = om;
-      if (!I.fixed || first) {
-        sA[o + i] = A;
-        sB[o + i] = B;
-        sR[o + i] = R;
-      }
-      if (!I.fixed && !serial) {
-        T = fh_mob_compose(fh_mob{0.0, B, -A, R}, T);
-        if (((i - f0) & 7) == 7) T = fh_mob_normalise(T);
-      }
-      Km = Kc;
-      Kc = Kp;
-    }
-  }
-  if (PH == kLineCoef) return;
-  fh_aff F{1.0, 0.0};
-  if (I.fixed || serial) {
-    // Al serially in the reference order (h_alpha_serial): once for constant
-    // coefficients (kept for later steps), every step otherwise; then
-    // sR[i] = Al[i+1] / B_i, the reference's factor of the Bt recurrence
-    const bool need = I.fixed ? first : PH == kLineAll;
-    if (need) {
-      HGroup<NW>::sync();
-      if (lane == 0) h_alpha_serial(N, I.al_left, sA + o, sB + o, sR + o, Al + o);
-      HGroup<NW>::sync();
-    }
-    if (!I.fixed || first)
-      for (int i = f0; i < f1; ++i) sR[o + i] = __ddiv_rn(Al[o + i + 1], sB[o + i]);
-    for (int i = f0; i < f1; ++i) {
-      const double gq = sR[o + i];
-      F = fh_aff_compose(fh_aff{gq * sA[o + i], -(gq * sOm[o + i])}, F);
-    }
-  } else {
-    // ---- Al: Moebius scan, re-walk with the reference arithmetic, chunk affine map of Bt
-    const fh_mob PT = HGroup<NW>::mob(T, smm);
-    double alv = (lane == 0) ? I.al_left : fma(PT.m00, I.al_left, PT.m01) / fma(PT.m10, I.al_left, PT.m11);
-    for (int i = f0; i < f1; ++i) {
-      const double A = sA[o + i], B = sB[o + i], R = sR[o + i], om = sOm[o + i];
-      const double gq = 1.0 / (R - A * alv);  // Al[i+1] / B_i
-      const double aln = B * gq;
-      Al[o + i + 1] = aln;
-      sR[o + i] = gq;
-      F = fh_aff_compose(fh_aff{gq * A, -(gq * om)}, F);
-      alv = aln;
-    }
-    if (lane == 0) Al[o + 1] = I.al_left;
-  }
-  // ---- Bt: scan, re-walk Bt[i+1] = (Al[i+1]/B)(A Bt[i] - Om)
-  const fh_aff PF = HGroup<NW>::aff(F, sma);
-  double btv = (lane == 0) ? I.bt_left : fma(PF.a, I.bt_left, PF.b);
-  for (int i = f0; i < f1; ++i) {
-    btv = sR[o + i] * (sA[o + i] * btv - sOm[o + i]);
-    Bt[o + i + 1] = btv;
-  }
-  if (lane == 0) Bt[o + 1] = I.bt_left;
-  HGroup<NW>::sync();
-  // ---- back substitution u_i = Al[i+1] u_{i+1} + Bt[i+1], i = N-1..0; u_N = u_right
-  const double uN = I.u_right;
-  const int chb = (N + TG - 1) / TG;
-  const int b0 = lane * chb, b1 = min(N, b0 + chb);
-  fh_aff G{1.0, 0.0};
-  for (int i = b1 - 1; i >= b0; --i) G = fh_aff_compose(fh_aff{Al[o + i + 1], Bt[o + i + 1]}, G);
-  const fh_aff PG = HGroup<NW>::aff_rev(G, sma);
-  double un = fma(PG.a, uN, PG.b);  // u at node b1
-  // every lane reads the old values of its own nodes before writing them
-  for (int i = b1 - 1; i >= b0; --i) {
-    un = Al[o + i + 1] * un + Bt[o + i + 1];
-    const double old = u[i];
-    u[i] = un;
-    if (append) fh_h_store_diff(Dnew, o + i, un - old, dfstore);
-  }
-  if (lane == 0) {
-    const double oldN = u[N], oldG = u[N + 1];
-    u[N] = uN;
-    u[N + 1] = uN;
-    if (append) {
-      fh_h_store_diff(Dnew, o + N, uN - oldN, dfstore);
-      fh_h_store_diff(Dnew, o + N + 1, uN - oldG, dfstore);
-    }
-  }
-}
-
-// SPACE: the batch has space-fractional instances (a separate instantiation
-// keeps the registers of the classical path).  PH: the part of the line solve
-// (kLineAll with the Moebius scan for Al, or kLineCoef / kLineSolve around
-// k_h_alpha_lanes).  Seven resident CTAs per SM (registers <= 73) keep 4096
-// instances (1024 CTAs) in one wave on 152 SMs.
-template <bool SPACE, int PH>
-__global__ void __launch_bounds__(128, 7) k_h_line_warp(const fh_h_dev_inst *__restrict__ inst, int n,
-                                                     double *__restrict__ U, const double *__restrict__ wc,
-                                                     const double *__restrict__ part, long long ldpart, int splits,
-                                                     double *__restrict__ Al, double *__restrict__ Bt,
-                                                     double *__restrict__ sA, double *__restrict__ sB,
-                                                     double *__restrict__ sR, double *__restrict__ sOm,
-                                                     double *__restrict__ Dnew, int append, int os,
-                                                     int dfstore, const double *__restrict__ sV) {
-  const int b = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  if (b >= n) return;  // whole warp
-  h_line<1, SPACE, PH>(inst[b], b, threadIdx.x & 31, U, wc, part, ldpart, splits, Al, Bt, sA, sB, sR, sOm, Dnew,
-                       append, os, dfstore, sV, nullptr, nullptr, PH != kLineAll);
-}
-
-// Al of every variable-coefficient instance (h_alpha_serial), one lane per
-// instance: the chain is FP64 latency (~650 cycles per equation on GB300), so
-// 32 instances share each warp instruction, and one warp per CTA spreads the
-// chains over the SMs.
-__global__ void __launch_bounds__(32) k_h_alpha_lanes(const fh_h_dev_inst *__restrict__ inst, int n,
-                                                      const double *__restrict__ sA, const double *__restrict__ sB,
-                                                      const double *__restrict__ sR, double *__restrict__ Al) {
-  const int b = blockIdx.x * 32 + threadIdx.x;
-  if (b >= n) return;
-  const fh_h_dev_inst I = inst[b];
-  if (I.fixed) return;
-  h_alpha_serial(I.N, I.al_left, sA + I.off, sB + I.off, sR + I.off, Al + I.off);
-}
-
-// Small batches (fewer instances than SMs): one CTA of kLineCtaWarps warps per
-// instance, so that each thread walks ~N/256 equations instead of ~N/32; Al
-// serially by thread 0 (serial != 0) or by the Moebius scan.
-static constexpr int kLineCtaWarps = 8;
-template <bool SPACE>
-__global__ void __launch_bounds__(32 * kLineCtaWarps) k_h_line_cta(
+// The line solves of one step (fh_hline), one CTA of NW warps per instance.
+// Four warps at 152 instances or more, where the FP64 pipe is shared by
+// several CTAs per SM and fewer, longer chunks cost less in scans; eight
+// below, where each instance has an SM to itself.
+template <int NW, bool SPACE>
+__global__ void __launch_bounds__(32 * NW, NW == 4 ? 3 : 1) k_h_line(
     const fh_h_dev_inst *__restrict__ inst, double *__restrict__ U, const double *__restrict__ wc,
     const double *__restrict__ part, long long ldpart, int splits, double *__restrict__ Al, double *__restrict__ Bt,
-    double *__restrict__ sA, double *__restrict__ sB, double *__restrict__ sR, double *__restrict__ sOm,
-    double *__restrict__ Dnew, int append, int os, int dfstore, const double *__restrict__ sV, int serial) {
-  __shared__ fh_mob smm[kLineCtaWarps];
-  __shared__ fh_aff sma[kLineCtaWarps];
-  h_line<kLineCtaWarps, SPACE, kLineAll>(inst[blockIdx.x], blockIdx.x, threadIdx.x, U, wc, part, ldpart, splits, Al,
-                                         Bt, sA, sB, sR, sOm, Dnew, append, os, dfstore, sV, smm, sma, serial);
+    double *__restrict__ fF, double *__restrict__ fG, double *__restrict__ Dnew, int os, int dfstore,
+    const double *__restrict__ sV) {
+  extern __shared__ double hsm[];
+  __shared__ fh_hline_scan<NW> sc;
+  const fh_h_dev_inst I = inst[blockIdx.x];
+  const double *pp = part + I.off;
+  auto ts = [&](int i) {  // split order
+    double a = 0.0;
+    for (int s = 0; s < splits; ++s) a += pp[(long long)s * ldpart + i];
+    return a;
+  };
+  fh_hline<NW, SPACE, false>(I, I.Da * wc[blockIdx.x], ts, U, Al, Bt, fF, fG, Dnew, os == I.ob, dfstore, sV, hsm, sc,
+                             fh_hline_keep{});
 }
+static constexpr int kLineWarps = 4, kLineWarpsSmall = 8;
 
 // ------------------------------------------- persistent solves of small batches
 // Batches of few instances run all the steps of a call in one launch: one
-// cluster of kPersCtas CTAs per instance.  Per step CTA r computes the
-// weights of its share of the instance's history slots and their sum over the
-// instance's nodes into its shared memory; after a cluster barrier CTA 0 adds
-// the CTAs' partial sums in rank order (distributed shared memory), solves the
-// line (h_line on eight warps, as k_h_line_cta) and appends the new layer; a
-// second cluster barrier publishes the layer (and frees the partial sums) for
-// the next step.  No kernel boundary and no grid-wide synchronisation: the
-// instances are independent, and a cluster barrier is a hardware barrier that
-// every CTA of the cluster reaches the same number of times.
-constexpr int kPersCtas = 8;
-constexpr int kPersThreads = 32 * kLineCtaWarps;
+// cluster of C CTAs per instance.  CTA 0 solves the line of step s (fh_hline,
+// state, newest layer and constant factors resident in shared memory) while
+// CTAs 1 .. C - 1 prepare step s + 1: everything in it that does not depend on
+// step s, that is all its weights (they depend on the step number only) and
+// the sums over all its history slots but the newest, each CTA its share of
+// the slots for all nodes.  CTA 0 reads those partial sums, the newest slot's
+// weight and the current slot's through distributed shared memory, adds them
+// in rank order and the newest layer last.  One hardware cluster barrier per
+// step publishes the new layer and the partial sums (double-buffered by the
+// parity of the step); the instances are independent, and every CTA of a
+// cluster reaches the barrier the same number of times.
+// The sums of a step are split by its slot count alone, so a solve does not
+// depend on how its steps are spread over calls.
+// Measured against the form that summed and solved one after the other (two
+// barriers a step, eight CTAs for any batch, serial factors): one L1 instance
+// of N = 200 over 1000 steps 13.6 -> 6.6 ms, 32 psi instances of N = 512 over
+// 250 steps 60.8 -> 8.3 ms.
+constexpr int kPersThreads = 32 * kLineWarpsSmall;
 constexpr int kPersMaxNodes = 2048;  // nodes of an instance (N + 2) in the partial sums
 constexpr int kPersMaxInst = 32;     // larger batches step kernel by kernel
-constexpr int kPersMaxChunk = 3800;  // history slots of one CTA (weights in shared memory, < 48 KiB in all)
+constexpr int kPersMaxSteps = 30400;
+constexpr int kPersStage = 1024;     // slots of a CTA whose weights are staged at a time
+constexpr int kPersMaxCtas = 16;
+constexpr int kPersNodes = kPersMaxNodes / kPersThreads;  // nodes per thread at most
+// dynamic shared memory: CTA 0 the resident line, the others the partial sums
+// of two steps and the staged weights; all of them the two weights of a step
+constexpr size_t kPersSmem = fh_hline_res_smem(kPersThreads) > sizeof(double) * (2 * kPersMaxNodes + kPersStage)
+                                 ? fh_hline_res_smem(kPersThreads)
+                                 : sizeof(double) * (2 * kPersMaxNodes + kPersStage);
 
 // Phase stamps of the persistent solve for profiling builds (-DFH_H_STAMPS):
-// %clock64 at the phase boundaries of the first 1024 steps of CTA 0 of
-// instance 0, read with fh_h_stamps_read.  Empty otherwise.
+// %clock64 of CTA 0 (phases 0, 1) and CTA 1 (2, 3) at the start and the end of
+// their part of the first 1024 steps of instance 0, read with
+// fh_h_stamps_read.  Empty otherwise.
 #ifdef FH_H_STAMPS
 __device__ long long g_h_stamps[1024 * 8];
 #define H_STAMP(p)                                                              \
-  if (b == 0 && r == 0 && threadIdx.x == 0 && s < 1024) g_h_stamps[s * 8 + (p)] = clock64();
+  if (b == 0 && threadIdx.x == 0 && s >= 0 && s < 1024) g_h_stamps[s * 8 + (p)] = clock64();
 extern "C" int fh_h_stamps_read(long long *h) {
   return (int)cudaMemcpyFromSymbol(h, g_h_stamps, sizeof(g_h_stamps));
 }
@@ -648,70 +416,124 @@ extern "C" int fh_h_stamps_read(long long *h) {
 #define H_STAMP(p)
 #endif
 
-__global__ void __cluster_dims__(kPersCtas, 1, 1) __launch_bounds__(kPersThreads)
-    k_h_persistent(const fh_h_dev_inst *__restrict__ inst, int tstep0, int os0, int nsteps, double *D,
-                   long long ldd, int ldw, double *wc, const double *__restrict__ Lb,
-                   const double *__restrict__ ibt, const double2 *__restrict__ lgt, double *U, double *part,
-                   double *Al, double *Bt, double *sA, double *sB, double *sR, double *sOm, int serial) {
+__global__ void __launch_bounds__(kPersThreads, 1)
+    k_h_persistent(const fh_h_dev_inst *__restrict__ inst, int tstep0, int os0, int nsteps, double *D, long long ldd,
+                   int ldw, const double *__restrict__ Lb, const double *__restrict__ ibt,
+                   const double2 *__restrict__ lgt, double *U, double *Al, double *Bt, double *fF, double *fG) {
   namespace cg = cooperative_groups;
   cg::cluster_group cl = cg::this_cluster();
-  extern __shared__ double wsh[];  // this CTA's weights of the step (kPersMaxChunk at most)
-  __shared__ double psum[kPersMaxNodes];
-  __shared__ fh_mob smm[kLineCtaWarps];
-  __shared__ fh_aff sma[kLineCtaWarps];
-  const int b = blockIdx.x / kPersCtas;
-  const int r = (int)cl.block_rank();
+  extern __shared__ double psm[];
+  __shared__ fh_hline_scan<kLineWarpsSmall> sc;
+  __shared__ double wstep[2][2];  // newest slot's and current slot's weight of a step (rank C - 1)
+  const int C = (int)cl.num_blocks(), r = (int)cl.block_rank();
+  const int b = blockIdx.x / C, t = threadIdx.x;
   const fh_h_dev_inst I = inst[b];
   const int np = I.N + 2;
-  for (int s = 0; s < nsteps; ++s) {
-    const int os_g = os0 + s;
-    const int tstep = tstep0 + s - I.tb, os = os_g - I.ob;
-    const int K = os >= 2 ? os - 1 : 0;  // history slots
-    const double invX = 1.0 / (double)(tstep + 1);
-    const int kch = (K + kPersCtas - 1) / kPersCtas;
-    const int k0 = min(K, r * kch), k1 = min(K, k0 + kch), nk = k1 - k0;
-    H_STAMP(0);
-    for (int k = (int)threadIdx.x; k < nk; k += blockDim.x)
-      wsh[k] = h_slot_weight(I, b, k0 + k, false, tstep, os, invX, ldw, Lb, ibt, lgt);
-    if (r == 0 && threadIdx.x == 0)
-      wc[b] = h_slot_weight(I, b, os > 1 ? os - 1 : 0, true, tstep, os, invX, ldw, Lb, ibt, lgt);
-    __syncthreads();
-    H_STAMP(1);
-    // slots of the instance's occupant start at global slot I.ob; eight
-    // independent loads ahead of the multiply-adds
-    for (int p = threadIdx.x; p < np; p += blockDim.x) {
-      double acc = 0.0;
-      const double *d = D + (long long)(I.ob + k0) * ldd + I.off + p;
-      int k = 0;
-      for (; k + 8 <= nk; k += 8, d += 8 * ldd) {
-        double v[8];
-#pragma unroll
-        for (int u = 0; u < 8; ++u) v[u] = __ldcg(d + u * ldd);
-#pragma unroll
-        for (int u = 0; u < 8; ++u) acc = fma(wsh[k + u], v[u], acc);
-      }
-      for (; k < nk; ++k, d += ldd) acc = fma(wsh[k], __ldcg(d), acc);
-      psum[p] = acc;
+  // history slots of the occupant before the newest one, at step s of the call
+  auto older = [&](int s) { return max(os0 + s - I.ob - 2, 0); };
+  if (r == 0) {
+    constexpr int L = fh_hline_len(kPersThreads);
+    fh_hline_keep keep;
+    keep.dn = psm + 3 * L;
+    keep.f = psm + 4 * L;
+    keep.g = psm + 5 * L;
+    keep.al = psm + 6 * L;
+    keep.pf = psm + 7 * L;
+    keep.pb = psm + 8 * L;
+    keep.lv = psm + 9 * L;
+    {  // the newest layer before the call
+      const bool has = os0 - I.ob >= 2;
+      const double *d = D + (long long)(has ? os0 - 2 : 0) * ldd + I.off;
+      for (int p = t; p < np; p += kPersThreads) keep.dn[fh_hsk(p)] = has ? __ldcg(d + p) : 0.0;
     }
+    cl.sync();  // step 0 is prepared
+    for (int s = 0; s < nsteps; ++s) {
+      H_STAMP(0);
+      const int os_g = os0 + s, os = os_g - I.ob, par = s & 1;
+      const double *ws = cl.map_shared_rank(&wstep[par][0], C - 1);
+      const double wnew = ws[0], DaW = I.Da * ws[1];
+      const double *pq = psm + par * kPersMaxNodes;
+      auto ts = [&](int i) {
+        double a = 0.0;
+        if (os >= 2) {
+          double v[kPersMaxCtas - 1];
+#pragma unroll
+          for (int q = 0; q < kPersMaxCtas - 1; ++q) v[q] = q + 1 < C ? cl.map_shared_rank(pq, q + 1)[i] : 0.0;
+          // pairwise in a fixed order
+          a = (v[0] + v[1]) + v[2];
+          if (C > 4) a = a + ((v[3] + v[4]) + (v[5] + v[6]));
+          if (C > 8) a = a + (((v[7] + v[8]) + (v[9] + v[10])) + ((v[11] + v[12]) + (v[13] + v[14])));
+          a = fma(wnew, keep.dn[fh_hsk(i)], a);
+        }
+        return a;
+      };
+      keep.load = s == 0;
+      keep.last = s == nsteps - 1;
+      fh_hline<kLineWarpsSmall, false, true>(I, DaW, ts, U, Al, Bt, fF, fG,
+                                             os_g >= 1 ? D + (long long)(os_g - 1) * ldd : nullptr, os == 0, 0, nullptr,
+                                             psm, sc, keep);
+      H_STAMP(1);
+      cl.sync();
+    }
+    return;
+  }
+  double *wsh = psm + 2 * kPersMaxNodes;
+  for (int s = -1; s < nsteps; ++s) {  // while CTA 0 solves step s: step s + 1
+    const int sn = s + 1, par = sn & 1;
     H_STAMP(2);
-    cl.sync();
-    H_STAMP(3);
-    if (r == 0) {
-      for (int p = threadIdx.x; p < np; p += blockDim.x) {
-        double t = 0.0;
-        for (int q = 0; q < kPersCtas; ++q) t += cl.map_shared_rank(psum, q)[p];
-        part[I.off + p] = t;
+    if (sn < nsteps) {
+      const int tstep = tstep0 + sn - I.tb, os = os0 + sn - I.ob;
+      const int K = older(sn), kch = (K + C - 2) / (C - 1);
+      const int k0 = min(K, (r - 1) * kch), nk = min(K, k0 + kch) - k0;
+      const double invX = I.weights == FH_W_PSI ? 1.0 / (double)(tstep + 1) : 0.0;
+      // the newest slot's and the current slot's weight on the last CTA's last two warps
+      if (r == C - 1 && (t == kPersThreads - 32 || t == kPersThreads - 64)) {
+        const int j = t == kPersThreads - 32;
+        const int slot = j ? (os > 1 ? os - 1 : 0) : os - 2;
+        wstep[par][j] =
+            j || os >= 2 ? h_slot_weight(I, b, slot, j != 0, tstep, os, invX, ldw, Lb, ibt, lgt) : 0.0;
       }
-      __syncthreads();
-      H_STAMP(4);
-      const int append = os_g >= 1;
-      double *Dnew = append ? D + (long long)(os_g - 1) * ldd : nullptr;
-      h_line<kLineCtaWarps, false, kLineAll>(I, b, threadIdx.x, U, wc, part, 0, 1, Al, Bt, sA, sB, sR, sOm, Dnew,
-                                             append, os_g, 0, nullptr, smm, sma, serial);
-      H_STAMP(5);
+      double acc[kPersNodes];
+#pragma unroll
+      for (int q = 0; q < kPersNodes; ++q) acc[q] = 0.0;
+      for (int kb = 0; kb < nk; kb += kPersStage) {
+        const int ns = min(kPersStage, nk - kb);
+        if (kb > 0) __syncthreads();
+        for (int k = t; k < ns; k += kPersThreads)
+          wsh[k] = h_slot_weight(I, b, k0 + kb + k, false, tstep, os, invX, ldw, Lb, ibt, lgt);
+        __syncthreads();
+#pragma unroll
+        for (int q = 0; q < kPersNodes; ++q) {
+          const int p = t + q * kPersThreads;
+          if (p < np) {
+            // slots of the instance's occupant start at global slot I.ob; 16
+            // independent loads ahead of the multiply-adds
+            const double *d = D + (long long)(I.ob + k0 + kb) * ldd + I.off + p;
+            double a = acc[q];
+            int k = 0;
+            for (; k + 16 <= ns; k += 16, d += 16 * ldd) {
+              double v[16];
+#pragma unroll
+              for (int w = 0; w < 16; ++w) v[w] = __ldcg(d + w * ldd);
+#pragma unroll
+              for (int w = 0; w < 16; ++w) a = fma(wsh[k + w], v[w], a);
+            }
+            double v[16];
+#pragma unroll
+            for (int w = 0; w < 16; ++w) v[w] = k + w < ns ? __ldcg(d + w * ldd) : 0.0;
+#pragma unroll
+            for (int w = 0; w < 16; ++w)
+              if (k + w < ns) a = fma(wsh[k + w], v[w], a);
+            acc[q] = a;
+          }
+        }
+      }
+#pragma unroll
+      for (int q = 0; q < kPersNodes; ++q)
+        if (t + q * kPersThreads < np) psm[par * kPersMaxNodes + t + q * kPersThreads] = acc[q];
     }
+    H_STAMP(3);
     cl.sync();
-    H_STAMP(6);
   }
 }
 
@@ -1214,14 +1036,6 @@ static int h_one_step(fh_h_batch *B, bool next) {
     rc = h_hist(B, ti, K, splits, kchunk, B->Wp(par), ctx->stream);
     fh_prof_mark(ctx, FH_PROF_HISTORY, true);
     if (rc) return rc;
-    // fold the partial sums into split 0 (in split order) for the warp-per-
-    // instance lines; the CTA-per-instance lines of small batches read all
-    // splits themselves (one launch less per step)
-    if (splits > 2 && B->n >= kLineCtaMaxInst) {
-      if ((rc = fh_launch_reduce_splits(ctx, splits, B->Ptot, B->part.as<double>(), B->Ptot, B->part.as<double>())))
-        return rc;
-      splits = 1;
-    }
   }
   fh_prof_mark(ctx, FH_PROF_SWEEP, false);  // right parts (incl. the space-fractional sums) and line solves
   if (B->space) {
@@ -1229,53 +1043,25 @@ static int h_one_step(fh_h_batch *B, bool next) {
                                                                    B->wsp.as<double>(), B->sV.as<double>());
     if ((rc = fh_after_launch(ctx, "k_h_space_v"))) return rc;
   }
-  const int append = os >= 1;
-  double *Dnew = !append ? nullptr
+  double *Dnew = os < 1 ? nullptr
                  : blk   ? reinterpret_cast<double *>(B->ring.as<float2>() + (long long)((os - 1) & 127) * B->Ptot)
                          : B->D.as<double>() + (long long)(os - 1) * B->Ptot;
   {
-    const int fst = os, dfs = (B->mode == FH_H_DF64 || blk) ? 1 : 0;  // first step per instance: os == its base
-    const dim3 gc((unsigned)B->n), gw((unsigned)fh_ceil_div(B->n, 4));
-    const fh_h_dev_inst *in = B->inst.as<fh_h_dev_inst>();
-    double *Al = B->Al.as<double>(), *Bt = B->Bt.as<double>(), *sA = B->sA.as<double>(), *sB = B->sB.as<double>();
-    double *sR = B->sR.as<double>(), *sOm = B->sOm.as<double>(), *U = B->U.as<double>();
-    const double *part = B->part.as<double>(), *wcp = B->wcp(par), *sV = B->sV.as<double>();
-    const int serial = B->serial_al ? 1 : 0;
-    if (B->n < kLineCtaMaxInst) {
-      if (B->space)
-        k_h_line_cta<true><<<gc, 32 * kLineCtaWarps, 0, ctx->stream>>>(in, U, wcp, part, B->Ptot, splits, Al, Bt, sA, sB,
-                                                                      sR, sOm, Dnew, append, fst, dfs, sV, serial);
-      else
-        k_h_line_cta<false><<<gc, 32 * kLineCtaWarps, 0, ctx->stream>>>(in, U, wcp, part, B->Ptot, splits, Al, Bt, sA,
-                                                                       sB, sR, sOm, Dnew, append, fst, dfs, sV, serial);
-    } else if (!serial || !B->varcoef) {
-      if (B->space)
-        k_h_line_warp<true, kLineAll><<<gw, 128, 0, ctx->stream>>>(in, B->n, U, wcp, part, B->Ptot, splits, Al, Bt, sA,
-                                                                   sB, sR, sOm, Dnew, append, fst, dfs, sV);
-      else
-        k_h_line_warp<false, kLineAll><<<gw, 128, 0, ctx->stream>>>(in, B->n, U, wcp, part, B->Ptot, splits, Al, Bt,
-                                                                    sA, sB, sR, sOm, Dnew, append, fst, dfs, sV);
-    } else {
-      // coefficients, serial Al one lane per instance, sweeps
-      if (B->space)
-        k_h_line_warp<true, kLineCoef><<<gw, 128, 0, ctx->stream>>>(in, B->n, U, wcp, part, B->Ptot, splits, Al, Bt,
-                                                                    sA, sB, sR, sOm, Dnew, append, fst, dfs, sV);
-      else
-        k_h_line_warp<false, kLineCoef><<<gw, 128, 0, ctx->stream>>>(in, B->n, U, wcp, part, B->Ptot, splits, Al, Bt,
-                                                                     sA, sB, sR, sOm, Dnew, append, fst, dfs, sV);
-      if ((rc = fh_after_launch(ctx, "k_h_line_warp"))) return rc;
-      k_h_alpha_lanes<<<(unsigned)fh_ceil_div(B->n, 32), 32, 0, ctx->stream>>>(in, B->n, sA, sB, sR, Al);
-      if ((rc = fh_after_launch(ctx, "k_h_alpha_lanes"))) return rc;
-      if (B->space)
-        k_h_line_warp<true, kLineSolve><<<gw, 128, 0, ctx->stream>>>(in, B->n, U, wcp, part, B->Ptot, splits, Al, Bt,
-                                                                     sA, sB, sR, sOm, Dnew, append, fst, dfs, sV);
-      else
-        k_h_line_warp<false, kLineSolve><<<gw, 128, 0, ctx->stream>>>(in, B->n, U, wcp, part, B->Ptot, splits, Al,
-                                                                      Bt, sA, sB, sR, sOm, Dnew, append, fst, dfs, sV);
-    }
+    const int dfs = (B->mode == FH_H_DF64 || blk) ? 1 : 0;
+    auto line = [&](auto kern, int nw) {
+      kern<<<(unsigned)B->n, 32 * nw, fh_hline_smem(32 * nw), ctx->stream>>>(
+          B->inst.as<fh_h_dev_inst>(), B->U.as<double>(), B->wcp(par), B->part.as<double>(), B->Ptot, splits,
+          B->Al.as<double>(), B->Bt.as<double>(), B->fF.as<double>(), B->fG.as<double>(), Dnew, os, dfs,
+          B->sV.as<double>());
+    };
+    if (B->n < kLineCtaMaxInst)
+      B->space ? line(k_h_line<kLineWarpsSmall, true>, kLineWarpsSmall)
+               : line(k_h_line<kLineWarpsSmall, false>, kLineWarpsSmall);
+    else
+      B->space ? line(k_h_line<kLineWarps, true>, kLineWarps) : line(k_h_line<kLineWarps, false>, kLineWarps);
   }
   fh_prof_mark(ctx, FH_PROF_SWEEP, true);
-  if ((rc = fh_after_launch(ctx, "k_h_line_warp"))) return rc;
+  if ((rc = fh_after_launch(ctx, "k_h_line"))) return rc;
   B->nsaved++;
   B->tstep++;
   return FH_OK;
@@ -1315,6 +1101,7 @@ static void h_fill_inst(const fh_h_params &p, long long off, fh_h_dev_inst &I) {
   I.ob = 0;
   I.off = off;
   I.dL = p.L / p.N;
+  I.rdL = 1.0 / I.dL;
   I.Dg = pow(I.dL, -2.0);
   I.Da = p.weights == FH_W_L1 ? pow(p.tau, -p.alpha) / tgamma(2.0 - p.alpha) : pow(p.tau, -1.0) / tgamma(2.0 - p.alpha);
   I.tau = p.tau;
@@ -1331,12 +1118,50 @@ static void h_fill_inst(const fh_h_params &p, long long off, fh_h_dev_inst &I) {
   I.kbf = 1.0;
 }
 
+// Shared memory above 48 KiB: the eight-warp line solve and the persistent
+// solve (their largest size, the same for every batch).
+static int h_set_smem_attrs(fh_ctx *ctx) {
+  constexpr auto at = cudaFuncAttributeMaxDynamicSharedMemorySize;
+  const int sl = (int)fh_hline_smem(32 * kLineWarpsSmall);
+  FH_CUDA_TRY(ctx, cudaFuncSetAttribute(k_h_line<kLineWarpsSmall, false>, at, sl));
+  FH_CUDA_TRY(ctx, cudaFuncSetAttribute(k_h_line<kLineWarpsSmall, true>, at, sl));
+  FH_CUDA_TRY(ctx, cudaFuncSetAttribute(k_h_persistent, at, (int)kPersSmem));
+  FH_CUDA_TRY(ctx, cudaFuncSetAttribute(k_h_persistent, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+  return FH_OK;
+}
+
+// CTAs per instance of the persistent solve: the largest cluster of which the
+// device holds all n at once (a second wave would double the step time; with
+// few instances more CTAs share the history sums), at least four.
+static int h_pers_ctas(int n) {
+  for (int c = kPersMaxCtas; c > 4; c /= 2) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(n * c));
+    cfg.blockDim = dim3(kPersThreads);
+    cfg.dynamicSmemBytes = kPersSmem;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = (unsigned)c;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    int active = 0;
+    if (cudaOccupancyMaxActiveClusters(&active, k_h_persistent, &cfg) == cudaSuccess && active >= n) return c;
+    cudaGetLastError();
+  }
+  return 4;
+}
+
 extern "C" {
 
 int fh_h_batch_create(fh_ctx *ctx, int ninst, const fh_h_params *params_host, int max_steps, fh_h_batch **out) {
   FH_REQUIRE(ctx, ctx && params_host && out, FH_EINVAL, "fh_h_batch_create: null argument");
   *out = nullptr;
   FH_REQUIRE(ctx, ninst >= 1 && max_steps >= 1, FH_EINVAL, "fh_h_batch_create: need ninst >= 1, max_steps >= 1");
+  {
+    const int rc0 = h_set_smem_attrs(ctx);
+    if (rc0) return rc0;
+  }
   fh_h_batch *B = new fh_h_batch();
   B->ctx = ctx;
   B->n = ninst;
@@ -1353,7 +1178,6 @@ int fh_h_batch_create(fh_ctx *ctx, int ninst, const fh_h_params *params_host, in
     }
     fh_h_dev_inst &I = di[b];
     h_fill_inst(p, off, I);
-    if (!I.fixed) B->varcoef = true;
     if (I.weights == FH_W_L1) B->has_l1 = true;
     B->off.push_back(off);
     const int seg = ((p.N + 2) + 1) & ~1;
@@ -1365,14 +1189,15 @@ int fh_h_batch_create(fh_ctx *ctx, int ninst, const fh_h_params *params_host, in
     off += seg;
   }
   B->Ptot = off;
+  if (ninst <= kPersMaxInst) B->pers_ctas = h_pers_ctas(ninst);
   int rc;
   const size_t st = sizeof(double) * (size_t)B->Ptot;
   if ((rc = fh_alloc(ctx, B->inst, sizeof(fh_h_dev_inst) * ninst, false)) ||
       (rc = fh_alloc(ctx, B->tl_by[0], sizeof(fh_h_tile) * B->tiles_by[0].size(), false)) ||
       (rc = fh_alloc(ctx, B->tl_by[1], sizeof(fh_h_tile) * B->tiles_by[1].size(), false)) ||
       (rc = fh_alloc(ctx, B->tl_by[2], sizeof(fh_h_tile) * B->tiles_by[2].size(), false)) || (rc = fh_alloc(ctx, B->U, st)) ||
-      (rc = fh_alloc(ctx, B->Al, st)) || (rc = fh_alloc(ctx, B->Bt, st)) || (rc = fh_alloc(ctx, B->sA, st)) ||
-      (rc = fh_alloc(ctx, B->sB, st)) || (rc = fh_alloc(ctx, B->sR, st)) || (rc = fh_alloc(ctx, B->sOm, st)) ||
+      (rc = fh_alloc(ctx, B->Al, st)) || (rc = fh_alloc(ctx, B->Bt, st)) || (rc = fh_alloc(ctx, B->fF, st)) ||
+      (rc = fh_alloc(ctx, B->fG, st)) ||
       (rc = fh_alloc(ctx, B->D, st * (size_t)max_steps)) ||
       (rc = fh_alloc(ctx, B->W, sizeof(double) * 2 * (size_t)ninst * B->max_weights)) ||
       (rc = fh_alloc(ctx, B->Lb, sizeof(double) * (size_t)ninst * B->max_weights, false)) ||
@@ -1442,7 +1267,7 @@ int fh_h_batch_destroy(fh_h_batch *b) {
 long long fh_h_batch_device_bytes(const fh_h_batch *b) {
   if (!b) return -1;
   const fh_dbuf *bufs[] = {&b->inst, &b->U, &b->D, &b->W, &b->Lb, &b->ibt, &b->lgt, &b->wc, &b->part, &b->Al,
-                           &b->Bt, &b->sA, &b->sB, &b->sR, &b->sOm, &b->wsp, &b->sV, &b->ring, &b->far, &b->cheb,
+                           &b->Bt, &b->fF, &b->fG, &b->wsp, &b->sV, &b->ring, &b->far, &b->cheb,
                            &b->tl_by[0], &b->tl_by[1], &b->tl_by[2]};
   size_t s = 0;
   for (const fh_dbuf *d : bufs) s += d->bytes;
@@ -1491,7 +1316,6 @@ int fh_h_batch_restart(fh_h_batch *b, int i, const fh_h_params *p, const double 
   I.ob = b->nsaved;
   b->di[i] = I;
   b->hp[i] = *p;
-  if (!I.fixed) b->varcoef = true;
   if (I.weights == FH_W_L1) b->has_l1 = true;
   FH_CUDA_TRY(ctx, cudaMemcpyAsync(b->U.as<double>() + b->off[i], U0_host, sizeof(double) * ((size_t)p->N + 2),
                                    cudaMemcpyHostToDevice, ctx->stream));
@@ -1562,7 +1386,7 @@ int fh_h_batch_get_u_range_host(fh_h_batch *b, int first, int count, double *U_h
 // instances of at most kPersMaxNodes nodes each.
 static bool h_persistent_ok(const fh_h_batch *b) {
   if (!b->persistent || b->mode != FH_H_FP64 || b->space || b->n > kPersMaxInst) return false;
-  if ((b->max_steps + kPersCtas - 1) / kPersCtas > kPersMaxChunk) return false;
+  if (b->max_steps > kPersMaxSteps) return false;
   for (const auto &p : b->hp)
     if (p.N + 2 > kPersMaxNodes) return false;
   return true;
@@ -1571,13 +1395,23 @@ static bool h_persistent_ok(const fh_h_batch *b) {
 static int h_persistent_run(fh_h_batch *b, int nsteps) {
   fh_ctx *ctx = b->ctx;
   b->w_ready = -1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(b->n * b->pers_ctas));
+  cfg.blockDim = dim3(kPersThreads);
+  cfg.dynamicSmemBytes = kPersSmem;
+  cfg.stream = ctx->stream;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = (unsigned)b->pers_ctas;
+  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
   fh_prof_mark(ctx, FH_PROF_HISTORY, false);
-  const size_t smem = sizeof(double) * (size_t)((b->max_steps + kPersCtas - 1) / kPersCtas);
-  k_h_persistent<<<(unsigned)(b->n * kPersCtas), kPersThreads, smem, ctx->stream>>>(
-      b->inst.as<fh_h_dev_inst>(), b->tstep, b->nsaved, nsteps, b->D.as<double>(), b->Ptot, b->max_weights,
-      b->wcp(0), b->Lb.as<double>(), b->ibt.as<double>(), b->lgt.as<double2>(), b->U.as<double>(),
-      b->part.as<double>(), b->Al.as<double>(), b->Bt.as<double>(), b->sA.as<double>(), b->sB.as<double>(),
-      b->sR.as<double>(), b->sOm.as<double>(), b->serial_al ? 1 : 0);
+  FH_CUDA_TRY(ctx, cudaLaunchKernelEx(&cfg, k_h_persistent, (const fh_h_dev_inst *)b->inst.as<fh_h_dev_inst>(), b->tstep,
+                                      b->nsaved, nsteps, b->D.as<double>(), b->Ptot, b->max_weights,
+                                      (const double *)b->Lb.as<double>(), (const double *)b->ibt.as<double>(),
+                                      (const double2 *)b->lgt.as<double2>(), b->U.as<double>(), b->Al.as<double>(),
+                                      b->Bt.as<double>(), b->fF.as<double>(), b->fG.as<double>()));
   fh_prof_mark(ctx, FH_PROF_HISTORY, true);
   int rc = fh_after_launch(ctx, "k_h_persistent");
   if (rc) return rc;
@@ -1800,9 +1634,6 @@ int fh_h_batch_set_mode(fh_h_batch *b, int mode) {
     if ((rc = fh_alloc(ctx, b->D, sizeof(double) * (size_t)b->Ptot * (size_t)b->max_steps))) return rc;
   }
   b->mode = mode;
-  // the blocked mode's bound is 1e-9: Al by the parallel Moebius scan (within
-  // ~1e-10), not by the serial reference-order chain the 1e-12 modes need
-  b->serial_al = mode != FH_H_BLOCKED;
   b->graph.reset();
   return FH_OK;
 }
