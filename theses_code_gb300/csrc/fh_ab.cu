@@ -6,6 +6,9 @@
 // history stores dC_t/tau = (C^{t+1}-C^t)/tau per node.  The matrix is the same
 // every step, so its elimination coefficients are built once and every step
 // runs the two affine recurrences with one warp (see fh_linescan.cuh).
+#include <cooperative_groups.h>
+
+#include <algorithm>
 #include <cmath>
 
 #include "fh_internal.h"
@@ -36,12 +39,12 @@ struct fh_ab_solver {
   fh_dbuf far;            // far rows ((hi, lo) pairs) of the steps T0+1 .. T0+128
   long long ldfar = 0;
   int T0 = 0;
-  // blocked mode with the line in shared memory: 8-step launches of
-  // k_ab_line_fused in double-float; history entries, lag weights, source rows
-  // and elimination tables as (hi, lo) FP32 pairs
-  bool fused = false;
-  fh_dbuf mid;            // history rows of the current 8-step sub-block (pairs)
-  fh_dbuf w2, src2, tab2; // pairs: lag weights, source rows, tables sl, pf, -al, pb, inv
+  // blocked mode, lines of at most 2560 nodes: all steps up to the next block
+  // boundary in one launch of k_ab_resident in double-float; history entries,
+  // lag weights, source rows and elimination tables as (hi, lo) FP32 pairs
+  bool resident = false;
+  double Ii = 0;          // current-step coefficient (host copy of ii)
+  fh_dbuf w2, src2, tab2; // pairs: lag weights, source rows, tables sl, -al, inv
   ~fh_ab_solver() {
     if (blk) fh_blk_delete(blk);
   }
@@ -178,209 +181,354 @@ __global__ void __launch_bounds__(kAbThreads) k_ab_line(int m, double oma, const
   }
 }
 
-// ------------------------------------------------ blocked mode: 8-step sub-blocks
-// The history of step i (entries tt < K = i - 1) splits into the far rows of
-// the current 128-step block (tt < T0, tensor cores), the sub-block rows
-// (T0 <= tt < K8, k_ab_mid, once per 8 steps) and the at most 7 entries of the
-// sub-block itself (K8 <= tt < K), which k_ab_line_fused adds while it runs
-// the 8 steps of the sub-block in one launch.
-static constexpr int kAbSub = 8;
-static constexpr int kAbFuseThreads = 512;
-static constexpr int kAbFuseMaxNodes = 5;  // nodes per thread: m + 1 <= 2560
-
-// mid[r][j] = far row of step K8 + r + sum_{T0 <= tt < K8} w[K8 + r + 1 - tt] D[tt][j], r < nr,
-// in double-float (D and w as (hi, lo) pairs, TwoSum accumulation as in
-// k_hist_sum_df), one node and one row per thread.
-__global__ void k_ab_mid(int m, long long P, int T0, int K8, int nr, const float2 *__restrict__ w2,
-                         const float2 *__restrict__ D, const float2 *__restrict__ far, long long ldfar,
-                         float2 *__restrict__ mid) {
-  const int j = blockIdx.x * blockDim.x + threadIdx.x;
-  const int r = blockIdx.y;
-  if (j > m || r >= nr) return;
-  const int i = K8 + r + 1;  // reference step index of row r
-  fh_df acc{0.f, 0.f};
-  if (far) acc = fh_df_from_pair(far[(long long)(K8 + r - T0) * ldfar + j]);
-  float sh = acc.h, sl = acc.l;
-  for (int tt = T0; tt < K8; ++tt) {
-    const float2 w = __ldg(w2 + i - tt);
-    const float2 d = D[(long long)tt * P + j];
-    const float ph = w.x * d.x;
-    float pl = fmaf(w.x, d.x, -ph);
-    pl = fmaf(w.x, d.y, pl);
-    pl = fmaf(w.y, d.x, pl);
-    const float t = sh + ph;
-    const float bb = t - sh;
-    const float e = (sh - (t - bb)) + (ph - bb);
-    sh = t;
-    sl += e + pl;
-    if ((tt & 15) == 15) {  // renormalise
-      const float u = sh + sl;
-      sl = sl - (u - sh);
-      sh = u;
-    }
+// ------------------------------------------------ resident solve of a block
+// All steps of a call up to the next block boundary in one launch of one
+// cluster.  The entries older than the block (tt < T0) come as far rows from
+// the tensor cores; the block's own entries are summed here.
+//   CTA 0 solves the line, step after step: field, elimination tables, prefix
+//     products and the slopes of both scans stay in registers and shared
+//     memory.  The right part needs one history term from it, the newest
+//     entry; the rest of the history sum arrives in distributed shared memory.
+//   CTAs 1 .. C - 1 own a range of the line's threads each and sum, while
+//     CTA 0 solves step s, the history of step s + 1 for the nodes of those
+//     threads: far row plus every entry of the block but the newest.  They keep
+//     their nodes' entries in shared memory, fetched from CTA 0 one step after
+//     they are made.
+// One hardware cluster barrier per step; newest entries and sums are
+// double-buffered by the parity of the step.  Every CTA reaches the barrier
+// the same number of times.
+//
+// The matrix is fixed, so the slopes of both substitutions are too: a thread
+// owns E consecutive equations, walks them from a zero start and adds prefix
+// product x start value, and the scans move offsets only (one multiply-add and
+// one shuffle of a value per level).  What bounds a step is the dependent chain
+// on CTA 0: right part, 4-5 equations, 5 + 4 scan levels, the same backwards.
+// Arithmetic A: double-float on the FP32 pipe (blocked mode).
+struct fh_ab_df {
+  using S = float2;  // stored
+  using V = fh_df;   // computed with
+  static __device__ __forceinline__ V ld(S s) { return fh_df_from_pair(s); }
+  static __device__ __forceinline__ S st(V v) { return fh_df_pair(v); }
+  static __device__ __forceinline__ V of(double x) { return fh_df_from_double(x); }
+  static __device__ __forceinline__ double to(V v) { return fh_df_to_double(v); }
+  static __device__ __forceinline__ V fma(V a, V b, V c) { return fh_df_fma(a, b, c); }
+  static __device__ __forceinline__ V mul(V a, V b) { return fh_df_mul(a, b); }
+  static __device__ __forceinline__ V add(V a, V b) { return fh_df_add(a, b); }
+  static __device__ __forceinline__ V sub(V a, V b) { return fh_df_sub(a, b); }
+  static __device__ __forceinline__ V shfl(V v, int lane) {
+    return fh_df{__shfl_sync(0xffffffffu, v.h, lane), __shfl_sync(0xffffffffu, v.l, lane)};
   }
-  const float h = sh + sl;
-  mid[(long long)r * P + j] = make_float2(h, sl - (h - sh));
+};
+
+constexpr int kAbResThreads = 512;
+constexpr int kAbResMaxCtas = 16;
+constexpr int kAbResMaxSteps = 128;  // entries of a block
+constexpr int kAbResLv = 12;         // scan constants per thread: 5 levels and the exclusive prefix, both ways
+
+struct fh_ab_res_args {
+  int m, nrows, T0, K0, ns;    // history entries older than T0 in the far rows; steps K0 .. K0 + ns - 1
+  long long P, ldfar;
+  const void *sl, *nal, *inv;  // forward slopes, -al and 1/den (S per node)
+  const void *src;             // source rows (S), m + 1 per row
+  const double *bl, *br;       // boundary values per row
+  const void *w;               // lag weights (S)
+  const void *far;             // far row of step T0 + r at far + r ldfar (S), null: none
+  void *D;                     // entry tt at D + tt P (S)
+  double *C;
+  double cI, nioma, itau;      // Ii/(1-a), -1/(1-a), 1/tau
+};
+
+// Shared memory: CTA 0 the tables [5][E][T], scan constants [12][T], newest
+// entries [2][E][T]; the others their nodes' sums [2][E][TW], partial sums and
+// entries [128][E TW].
+__host__ __device__ inline int ab_res_tw(int nw, int ctas) { return (32 * nw + ctas - 2) / (ctas - 1); }
+static size_t ab_res_smem(int nw, int E, int ctas) {
+  const int T = 32 * nw, nn = E * ab_res_tw(nw, ctas);
+  const size_t line = 8 * ((size_t)7 * E * T + (size_t)kAbResLv * T);
+  const size_t work = 8 * ((size_t)2 * nn + kAbResThreads + (size_t)kAbResMaxSteps * nn);
+  return line > work ? line : work;
 }
 
-// Steps K8 + s0 .. K8 + s0 + ns - 1 of one sub-block in one CTA, in
-// double-float: the elimination tables and the field stay in shared memory
-// for the whole launch; per step the right parts (source row, sub-block row or
-// far row, the sub-block's own entries), the solve of k_ab_line
-// (kAbSolveWarps warps, double-float group scans) and the new history entry
-// dC/tau.  FP64 only
-// converts the field at the start and the end of the launch.  Every thread
-// keeps the right-part loads of all its nodes (j = tid + 512 k) in flight at
-// once, the sub-block's entries two per round trip.
-__global__ void __launch_bounds__(kAbFuseThreads, 1)
-    k_ab_line_fused(int m, double oma, const double *__restrict__ ii, const float2 *__restrict__ tab,
-                    long long ldt, const float2 *__restrict__ src2, int nrows, const double *__restrict__ blp,
-                    const double *__restrict__ brp, double *C, float2 *D, long long P,
-                    const float2 *__restrict__ w2, const float2 *__restrict__ mid, const float2 *__restrict__ far8,
-                    long long ldfar, int K8, int s0, int ns, double tau) {
-  constexpr int NMAX = kAbFuseMaxNodes;  // nodes per thread
-  extern __shared__ float2 smf[];
-  const int ch = (m + kAbSolveThreads - 1) / kAbSolveThreads;
-  const int Lm = m + 2 + m / ch + 1;
-  float2 *rb = smf, *sl = rb + Lm, *pf = sl + Lm, *nal = pf + Lm, *pb = nal + Lm, *bt = pb + Lm, *cv = bt + Lm,
-         *inv = cv + Lm, *Cs = inv + Lm;
-  auto sk = [ch](int j) { return j + j / ch; };
-  __shared__ float2 cst[3], wts[kAbSub][kAbSub], bnd[kAbSub][2];
-  for (int j = threadIdx.x; j <= m; j += kAbFuseThreads) {
-    sl[sk(j)] = tab[j];
-    pf[sk(j)] = tab[ldt + j];
-    nal[sk(j)] = tab[2 * ldt + j];
-    pb[sk(j)] = tab[3 * ldt + j];
-    inv[j] = tab[4 * ldt + j];
-    Cs[j] = fh_df_pair(fh_df_from_double(C[j]));
+// Scan of the chunk maps' offsets over 32 NW threads with recorded slopes lv
+// (and lw: the same for the NW warp totals, [5][32]); v: value at the line's
+// first (REV: last) end; returns the value at the thread's chunk.
+template <class A, int NW, bool REV>
+__device__ __forceinline__ typename A::V ab_scan(typename A::V g, typename A::V v, typename A::S *tot,
+                                                 const typename A::S *lv, const typename A::S *lw) {
+  using V = typename A::V;
+  constexpr int T = 32 * NW;
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+#pragma unroll
+  for (int k = 0; k < 5; ++k) {
+    const int d = 1 << k;
+    const V p = A::shfl(g, REV ? lane + d : lane - d);
+    if (REV ? lane + d < 32 : lane >= d) g = A::fma(A::ld(lv[k * T + t]), p, g);
   }
-  // step constants (one FP64 conversion per thread), the weights of the
-  // sub-block's entries wts[s][t] = w[(K8 + s + 1) - (K8 + t)] and the
-  // boundary values of every step
-  if (threadIdx.x == 0) cst[0] = fh_df_pair(fh_df_from_double(ii[0] / oma));  // Ii/(1-a)
-  if (threadIdx.x == 1) cst[1] = fh_df_pair(fh_df_from_double(-1.0 / oma));
-  if (threadIdx.x == 2) cst[2] = fh_df_pair(fh_df_from_double(1.0 / tau));
-  if (threadIdx.x >= 32 && threadIdx.x < 32 + kAbSub * kAbSub) {
-    const int v = threadIdx.x - 32, ss = v / kAbSub, t = v % kAbSub;
-    wts[ss][t] = t < ss ? w2[ss + 1 - t] : make_float2(0.f, 0.f);
+  if (lane == (REV ? 0 : 31)) tot[warp] = A::st(g);
+  V e = A::shfl(g, REV ? lane + 1 : lane - 1);
+  if (lane == (REV ? 31 : 0)) e = A::of(0.0);
+  fh_group_bar(1, T);
+  // warp totals: lane l holds warp l's (REV: warp NW-1-l's)
+  const int wl = lane < NW ? (REV ? NW - 1 - lane : lane) : 0;
+  V q = A::ld(tot[wl]);
+#pragma unroll
+  for (int k = 0; (1 << k) < NW; ++k) {
+    const int d = 1 << k;
+    const V p = A::shfl(q, lane - d);
+    if (lane >= d) q = A::fma(A::ld(lw[k * 32 + lane]), p, q);
   }
-  if (threadIdx.x >= 128 && threadIdx.x < 128 + 2 * kAbSub) {
-    const int v = threadIdx.x - 128, ss = v >> 1;
-    if (ss >= s0 && ss < s0 + ns) {
-      const int K = K8 + ss, row = K < nrows - 1 ? K : nrows - 1;
-      bnd[ss][v & 1] = fh_df_pair(fh_df_from_double((v & 1) ? brp[row] : blp[row]));
+  // start of this warp: the inclusive scan up to the warp before it
+  const int wi = REV ? NW - 1 - warp : warp;
+  const V off = A::shfl(q, wi > 0 ? wi - 1 : 0);
+  if (wi > 0) v = A::fma(A::ld(lw[4 * 32 + wi - 1]), v, off);
+  return A::fma(A::ld(lv[5 * T + t]), v, e);
+}
+
+// The constants of ab_scan from the chunks' slopes a (once per launch).
+template <class A, int NW, bool REV>
+__device__ __forceinline__ void ab_scan_setup(typename A::V a, typename A::S *tot, typename A::S *lv,
+                                              typename A::S *lw) {
+  using V = typename A::V;
+  constexpr int T = 32 * NW;
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+#pragma unroll
+  for (int k = 0; k < 5; ++k) {
+    const int d = 1 << k;
+    lv[k * T + t] = A::st(a);
+    const V p = A::shfl(a, REV ? lane + d : lane - d);
+    if (REV ? lane + d < 32 : lane >= d) a = A::mul(a, p);
+  }
+  if (lane == (REV ? 0 : 31)) tot[warp] = A::st(a);
+  V e = A::shfl(a, REV ? lane + 1 : lane - 1);
+  if (lane == (REV ? 31 : 0)) e = A::of(1.0);
+  lv[5 * T + t] = A::st(e);
+  fh_group_bar(1, T);
+  if (warp == 0) {
+    V q = lane < NW ? A::ld(tot[REV ? NW - 1 - lane : lane]) : A::of(1.0);
+#pragma unroll
+    for (int k = 0; (1 << k) < NW; ++k) {
+      const int d = 1 << k;
+      lw[k * 32 + lane] = A::st(q);
+      const V p = A::shfl(q, lane - d);
+      if (lane >= d) q = A::mul(q, p);
     }
+    lw[4 * 32 + lane] = A::st(q);
   }
-  __syncthreads();
-  const fh_df cI = fh_df_from_pair(cst[0]), nioma = fh_df_from_pair(cst[1]), itau = fh_df_from_pair(cst[2]);
-  const fh_daff I{fh_df{1.f, 0.f}, fh_df{0.f, 0.f}};
-  __shared__ fh_daff scan_sm[kAbSolveWarps];
-  for (int s = s0; s < s0 + ns; ++s) {
-    const int K = K8 + s;  // history entries of this step (reference step i = K + 1)
-    const int row = K < nrows - 1 ? K : nrows - 1;
-    const float2 *srow = src2 + (long long)row * (m + 1);
-    const float2 *mrow = mid ? mid + (long long)s * P : nullptr;
-    const float2 *frow = far8 ? far8 + (long long)s * ldfar : nullptr;
-    const bool hist = mrow || frow || s > 0;
-    {
-      // right parts: all of the thread's loads in flight together
-      float2 sr[NMAX], hv[NMAX];
+  fh_group_bar(1, T);
+}
+
+template <class A, int NW, int EM>
+__global__ void __launch_bounds__(kAbResThreads, 1) k_ab_resident(const fh_ab_res_args a) {
+  namespace cg = cooperative_groups;
+  using S = typename A::S;
+  using V = typename A::V;
+  constexpr int T = 32 * NW;  // threads of the line solve
+  cg::cluster_group cl = cg::this_cluster();
+  extern __shared__ double2 ab_sm2[];
+  S *sm = reinterpret_cast<S *>(ab_sm2);
+  __shared__ S tot[2][NW], lw[2][5 * 32], wl[kAbResMaxSteps + 2];
+  const int C = (int)cl.num_blocks(), r = (int)cl.block_rank(), t = threadIdx.x;
+  const int m = a.m, n = m - 1;  // equations 1 .. m - 1
+  const int E = (n + T - 1) / T;
+  const int TW = ab_res_tw(NW, C);
+  S *D = reinterpret_cast<S *>(a.D);
+  const S *w = reinterpret_cast<const S *>(a.w);
+  if (r == 0) {
+    S *tf = sm, *ti = tf + E * T, *tn = ti + E * T, *pf = tn + E * T, *pb = pf + E * T;
+    S *lvf = pb + E * T, *lvb = lvf + 6 * T, *dn = lvf + kAbResLv * T;  // dn: [2][E][T]
+    const bool solving = t < T;  // whole warps; the others only keep the cluster barriers
+    const int j0 = 1 + t * E;    // the thread's first equation
+    const int c = solving ? max(0, min(E, m - j0)) : 0;
+    V Cv[EM], dv[EM], sv[EM];
+    V zero = A::of(0.0), one = A::of(1.0);
+    if (solving) {
+      V pa = one;
 #pragma unroll
-      for (int k = 0; k < NMAX; ++k) {
-        const int j = threadIdx.x + k * kAbFuseThreads;
-        if (j <= m) {
-          sr[k] = srow[j];
-          hv[k] = mrow ? mrow[j] : (frow ? frow[j] : make_float2(0.f, 0.f));
-        }
-      }
-      fh_df hs[NMAX];
-#pragma unroll
-      for (int k = 0; k < NMAX; ++k) hs[k] = fh_df_from_pair(hv[k]);
-      if (mrow && frow) {
-#pragma unroll
-        for (int k = 0; k < NMAX; ++k) {
-          const int j = threadIdx.x + k * kAbFuseThreads;
-          if (j <= m) hs[k] = fh_df_add(fh_df_from_pair(mrow[j]), fh_df_from_pair(frow[j]));
-        }
-      }
-      for (int t0 = 0; t0 < s; t0 += 2) {  // the sub-block's own entries, two per round trip
-        float2 d[2][NMAX];
-#pragma unroll
-        for (int u = 0; u < 2; ++u)
-#pragma unroll
-          for (int k = 0; k < NMAX; ++k) {
-            const int j = threadIdx.x + k * kAbFuseThreads;
-            if (t0 + u < s && j <= m) d[u][k] = __ldcg(D + (long long)(K8 + t0 + u) * P + j);
+      for (int e = 0; e < EM; ++e)
+        if (e < E) {
+          const bool in = e < c;
+          const int q = e * T + t, j = in ? j0 + e : 0;
+          const V f = in ? A::ld(reinterpret_cast<const S *>(a.sl)[j]) : zero;
+          tf[q] = A::st(f);
+          ti[q] = in ? reinterpret_cast<const S *>(a.inv)[j] : A::st(zero);
+          tn[q] = in ? reinterpret_cast<const S *>(a.nal)[j] : A::st(one);
+          pa = A::mul(pa, f);
+          pf[q] = A::st(pa);
+          Cv[e] = in ? A::of(a.C[j]) : zero;
+          dv[e] = zero;
+          if (in && a.K0 > a.T0) {  // the newest entry before the call
+            const S d = D[(long long)(a.K0 - 1) * a.P + j];
+            dv[e] = A::ld(d);
           }
+          sv[e] = zero;
+        }
+      V pq = one;
 #pragma unroll
-        for (int u = 0; u < 2; ++u)
-          if (t0 + u < s) {
-            const fh_df w = fh_df_from_pair(wts[s][t0 + u]);
+      for (int e = EM - 1; e >= 0; --e)
+        if (e < E) {
+          const int q = e * T + t;
+          pq = A::mul(pq, A::ld(tn[q]));
+          pb[q] = A::st(pq);
+        }
+      ab_scan_setup<A, NW, false>(pa, tot[0], lvf, lw[0]);
+      ab_scan_setup<A, NW, true>(pq, tot[1], lvb, lw[1]);
+    }
+    V c0 = A::of(a.C[0]), cm = A::of(a.C[m]);  // the boundary nodes (thread 0 keeps them)
+    const V cI = A::of(a.cI), nioma = A::of(a.nioma), itau = A::of(a.itau);
+    const V w2 = A::ld(w[2]);  // the newest entry's weight
+    int row = -1;
+    V bl = zero, br = zero;
+    auto load_row = [&](int K) {  // source row and boundary values of the step with K entries
+      const int nr = K < a.nrows - 1 ? K : a.nrows - 1;
+      if (!solving || nr == row) return;
+      row = nr;
+      bl = A::of(a.bl[row]);
+      br = A::of(a.br[row]);
+      const S *src = reinterpret_cast<const S *>(a.src) + (long long)row * (m + 1);
 #pragma unroll
-            for (int k = 0; k < NMAX; ++k) hs[k] = fh_df_fma(w, fh_df_from_pair(d[u][k]), hs[k]);
+      for (int e = 0; e < EM; ++e)
+        if (e < c) sv[e] = A::ld(src[j0 + e]);
+    };
+    load_row(a.K0);
+    cl.sync();  // step K0 is prepared
+    for (int s = 0; s < a.ns; ++s) {
+      const int K = a.K0 + s, par = s & 1;
+      if (solving) {
+        V bt[EM];
+        {
+          // sums of the thread's nodes from the CTA that owns the thread
+          const S *hs = cl.map_shared_rank(sm + par * E * TW, 1 + t / TW) + t % TW;
+          const bool newest = K > a.T0;
+          S h[EM];
+#pragma unroll
+          for (int e = 0; e < EM; ++e)
+            if (e < E) h[e] = hs[e * TW];
+          V v = zero;
+#pragma unroll
+          for (int e = 0; e < EM; ++e)
+            if (e < E) {
+              const int q = e * T + t;
+              V x = A::fma(cI, Cv[e], sv[e]);
+              V y = A::ld(h[e]);
+              if (newest) y = A::fma(w2, dv[e], y);
+              x = A::fma(nioma, y, x);  // MF_intF_simple returns ret/(1-a)
+              v = A::fma(A::ld(tf[q]), v, A::mul(x, A::ld(ti[q])));
+              bt[e] = v;
+            }
+          const V st = ab_scan<A, NW, false>(v, bl, tot[0], lvf, lw[0]);  // bt before the thread's equations
+#pragma unroll
+          for (int e = 0; e < EM; ++e)
+            if (e < E) bt[e] = A::fma(A::ld(pf[e * T + t]), st, bt[e]);
+        }
+        V v = zero;
+#pragma unroll
+        for (int e = EM - 1; e >= 0; --e)
+          if (e < E) {
+            v = A::fma(A::ld(tn[e * T + t]), v, e < c ? bt[e] : zero);
+            bt[e] = v;
           }
-      }
+        const V st = ab_scan<A, NW, true>(v, br, tot[1], lvb, lw[1]);  // C after the thread's equations
 #pragma unroll
-      for (int k = 0; k < NMAX; ++k) {
-        const int j = threadIdx.x + k * kAbFuseThreads;
-        if (j <= m) {
-          fh_df r = fh_df_fma(cI, fh_df_from_pair(Cs[j]), fh_df_from_pair(sr[k]));
-          if (hist) r = fh_df_fma(nioma, hs[k], r);  // MF_intF_simple returns ret/(1-a)
-          rb[sk(j)] = fh_df_pair(fh_df_mul(r, fh_df_from_pair(inv[j])));
+        for (int e = 0; e < EM; ++e)
+          if (e < E) {
+            const V x = A::fma(A::ld(pb[e * T + t]), st, bt[e]);
+            dv[e] = A::mul(A::sub(x, Cv[e]), itau);
+            if (e < c) Cv[e] = x;
+            dn[(par * E + e) * T + t] = A::st(dv[e]);
+          }
+        if (t == 0) {
+          S *Dk = D + (long long)K * a.P;
+          Dk[0] = A::st(A::mul(A::sub(bl, c0), itau));
+          Dk[m] = A::st(A::mul(A::sub(br, cm), itau));
+          c0 = bl;
+          cm = br;
+        }
+        if (s + 1 < a.ns) load_row(K + 1);
+      }
+      cl.sync();
+    }
+    if (solving) {
+#pragma unroll
+      for (int e = 0; e < EM; ++e)
+        if (e < c) a.C[j0 + e] = A::to(Cv[e]);
+      if (t == 0) {
+        a.C[0] = A::to(c0);
+        a.C[m] = A::to(cm);
+      }
+    }
+    cl.sync();  // the last entries have been fetched
+    return;
+  }
+  // ---- history of the nodes of threads [t0, t0 + TW): item i = e TW + (thread - t0)
+  const int t0 = (r - 1) * TW, nn = E * TW;
+  S *hs = sm, *pt = hs + 2 * nn, *ent = pt + kAbResThreads;
+  auto node = [&](int i) { return 1 + (t0 + i % TW) * E + i / TW; };
+  auto live = [&](int i) { return t0 + i % TW < T && node(i) < m; };
+  for (int k = t; k < kAbResMaxSteps + 2; k += kAbResThreads) wl[k] = k < a.K0 - a.T0 + a.ns + 2 ? w[k] : A::st(A::of(0.0));
+  const int K0 = a.K0, T0 = a.T0;
+  for (int x = t; x < (K0 - T0) * nn; x += kAbResThreads) {
+    const int tt = x / nn, i = x - tt * nn;
+    ent[x] = live(i) ? D[(long long)(T0 + tt) * a.P + node(i)] : A::st(A::of(0.0));
+  }
+  // the block's entries in up to `parts` runs per item, summed side by side
+  const int parts = max(1, kAbResThreads / nn);
+  for (int s = -1; s <= a.ns; ++s) {
+    // entry K0 + s - 1 (made by CTA 0 in the phase before): own copy and the stored history
+    if (s >= 1) {
+      const int K = K0 + s - 1, par = (s - 1) & 1;
+      const S *dn = cl.map_shared_rank(sm + (size_t)5 * E * T + (size_t)kAbResLv * T, 0) + (size_t)par * E * T;
+      for (int i = t; i < nn; i += kAbResThreads) {
+        S d = A::st(A::of(0.0));
+        if (live(i)) {
+          d = dn[(i / TW) * T + t0 + i % TW];
+          D[(long long)K * a.P + node(i)] = d;
+        }
+        ent[(K - T0) * nn + i] = d;
+      }
+    }
+    __syncthreads();
+    const int sn = s + 1;  // the step to prepare
+    if (sn < a.ns) {
+      const int K = K0 + sn, no = max(K - 1 - T0, 0);  // entries T0 .. K - 2
+      const S *far = a.far ? reinterpret_cast<const S *>(a.far) + (long long)(K - T0) * a.ldfar : nullptr;
+      S *out = hs + (sn & 1) * nn;
+      const int per = (no + parts - 1) / parts;
+      for (int i0 = 0; i0 < nn; i0 += kAbResThreads) {  // one round unless nn > 512
+        const int i = i0 + t % min(nn, kAbResThreads), p = t / min(nn, kAbResThreads);
+        V s0 = A::of(0.0);
+        if (i < nn && p < parts) {
+          const int b = min(no, p * per), e = min(no, b + per);
+          if (p == 0 && far && live(i)) s0 = A::ld(far[node(i)]);
+          V s1 = A::of(0.0);
+          int tt = b;
+          for (; tt + 2 <= e; tt += 2) {  // entry tt has lag K + 1 - (T0 + tt)
+            s0 = A::fma(A::ld(wl[K + 1 - T0 - tt]), A::ld(ent[tt * nn + i]), s0);
+            s1 = A::fma(A::ld(wl[K - T0 - tt]), A::ld(ent[(tt + 1) * nn + i]), s1);
+          }
+          if (tt < e) s0 = A::fma(A::ld(wl[K + 1 - T0 - tt]), A::ld(ent[tt * nn + i]), s0);
+          s0 = A::add(s0, s1);
+        }
+        if (parts > 1) {
+          if (p < parts) pt[t] = A::st(s0);
+          __syncthreads();
+          if (p == 0 && i < nn) {
+            for (int q = 1; q < parts; ++q) s0 = A::add(s0, A::ld(pt[q * nn + i]));
+            out[i] = A::st(s0);
+          }
+        } else if (i < nn) {
+          out[i] = A::st(s0);
         }
       }
     }
-    __syncthreads();
-    if (threadIdx.x < kAbSolveThreads) {
-      const int t = threadIdx.x;
-      const fh_df bl = fh_df_from_pair(bnd[s][0]), br = fh_df_from_pair(bnd[s][1]);
-      const int f0 = 1 + t * ch, f1 = min(m + 1, f0 + ch);
-      fh_df b{0.f, 0.f};
-      for (int j = f0; j < f1; ++j) {
-        b = fh_df_fma(fh_df_from_pair(sl[sk(j)]), b, fh_df_from_pair(rb[sk(j)]));
-        bt[sk(j)] = fh_df_pair(b);
-      }
-      const fh_daff Pf = fh_group_exclusive_daff<kAbSolveWarps>(
-          f1 > f0 ? fh_daff{fh_df_from_pair(pf[sk(f1 - 1)]), b} : I, scan_sm, 1);
-      const fh_df s0v = fh_df_fma(Pf.a, bl, Pf.b);  // bt[f0 - 1]
-      for (int j = f0; j < f1; ++j)
-        bt[sk(j)] = fh_df_pair(fh_df_fma(fh_df_from_pair(pf[sk(j)]), s0v, fh_df_from_pair(bt[sk(j)])));
-      if (t == 0) bt[sk(0)] = fh_df_pair(bl);
-      fh_group_bar(1, kAbSolveThreads);
-      const int b0 = t * ch, b1 = min(m, b0 + ch);
-      fh_df c{0.f, 0.f};
-      for (int j = b1 - 1; j >= b0; --j) {
-        c = fh_df_fma(fh_df_from_pair(nal[sk(j)]), c, fh_df_from_pair(bt[sk(j)]));
-        cv[sk(j)] = fh_df_pair(c);
-      }
-      const fh_daff Pb = fh_group_exclusive_daff_rev<kAbSolveWarps>(
-          b1 > b0 ? fh_daff{fh_df_from_pair(pb[sk(b0)]), c} : I, scan_sm, 1);
-      const fh_df tv = fh_df_fma(Pb.a, br, Pb.b);  // C[b1]
-      for (int j = b0; j < b1; ++j)
-        cv[sk(j)] = fh_df_pair(fh_df_fma(fh_df_from_pair(pb[sk(j)]), tv, fh_df_from_pair(cv[sk(j)])));
-      if (t == 0) cv[sk(m)] = fh_df_pair(br);
-    }
-    __syncthreads();
-    float2 *Dk = D + (long long)K * P;
-    for (int j = threadIdx.x; j <= m; j += kAbFuseThreads) {
-      const fh_df v = fh_df_from_pair(cv[sk(j)]);
-      Dk[j] = fh_df_pair(fh_df_mul(fh_df_sub(v, fh_df_from_pair(Cs[j])), itau));
-      Cs[j] = fh_df_pair(v);
-    }
-    __syncthreads();
+    if (s < a.ns) cl.sync();
   }
-  for (int j = threadIdx.x; j <= m; j += kAbFuseThreads) C[j] = fh_df_to_double(fh_df_from_pair(Cs[j]));
+  cl.sync();
 }
 
 // (hi, lo) pairs of n doubles; neg: of their negatives
 __global__ void k_ab_pairs(const double *__restrict__ x, float2 *__restrict__ y, long long n, int neg) {
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) y[i] = fh_df_pair(fh_df_from_double(neg ? -x[i] : x[i]));
-}
-
-static size_t ab_fused_smem(int m) {
-  const int ch = (m + kAbSolveThreads - 1) / kAbSolveThreads;
-  return sizeof(float2) * (8 * (size_t)(m + 2 + m / ch + 1) + (size_t)m + 1);
 }
 
 // Pair copies for the double-float launches: elimination tables (after every
@@ -390,19 +538,17 @@ static int ab_pairs(fh_ctx *ctx, const double *x, float2 *y, long long n, int ne
   return fh_after_launch(ctx, "k_ab_pairs");
 }
 static int ab_table_pairs(fh_ab_solver *s) {
-  if (!s->fused) return FH_OK;
+  if (!s->resident) return FH_OK;
   const long long n = s->m + 1;
   float2 *t = s->tab2.as<float2>();
   int rc;
-  if ((rc = ab_pairs(s->ctx, s->sl.as<double>(), t, n, 0)) || (rc = ab_pairs(s->ctx, s->pf.as<double>(), t + s->P, n, 0)) ||
-      (rc = ab_pairs(s->ctx, s->al.as<double>(), t + 2 * s->P, n, 1)) ||
-      (rc = ab_pairs(s->ctx, s->pb.as<double>(), t + 3 * s->P, n, 0)) ||
-      (rc = ab_pairs(s->ctx, s->inv.as<double>(), t + 4 * s->P, n, 0)))
+  if ((rc = ab_pairs(s->ctx, s->sl.as<double>(), t, n, 0)) || (rc = ab_pairs(s->ctx, s->al.as<double>(), t + s->P, n, 1)) ||
+      (rc = ab_pairs(s->ctx, s->inv.as<double>(), t + 2 * s->P, n, 0)))
     return rc;
   return FH_OK;
 }
 static int ab_src_pairs(fh_ab_solver *s) {
-  if (!s->fused || s->nrows < 1) return FH_OK;
+  if (!s->resident || s->nrows < 1) return FH_OK;
   int rc = fh_alloc(s->ctx, s->src2, sizeof(float2) * (size_t)s->nrows * (s->m + 1), false);
   if (rc) return rc;
   return ab_pairs(s->ctx, s->src.as<double>(), s->src2.as<float2>(), (long long)s->nrows * (s->m + 1), 0);
@@ -413,7 +559,7 @@ static size_t ab_line_smem(int m) {
   return sizeof(double) * 7 * (size_t)(m + 2 + m / ch + 1);
 }
 
-static int ab_fused_steps(fh_ab_solver *s, int max_n, int *done);
+static int ab_res_steps(fh_ab_solver *s, int max_n, int *done);
 
 static int ab_one_step(fh_ab_solver *s, int max_n, int *done) {
   *done = 1;
@@ -425,7 +571,7 @@ static int ab_one_step(fh_ab_solver *s, int max_n, int *done) {
   if (s->blk && K > 0 && K % kAbBlock == 0) {
     // new block: entries [K-128, K) into the slice planes, Toeplitz rows of the
     // next 128 steps, far rows S_far[r] = sum_{tt<K} w[K+1+r-tt] dC_tt
-    const int dfh = s->fused ? 1 : 0;  // fused launches store the entries as (hi, lo) pairs
+    const int dfh = s->resident ? 1 : 0;  // the resident solve stores the entries as (hi, lo) pairs
     if ((rc = fh_blk_convert(ctx, *s->blk, s->D.as<double>(), s->P, K - kAbBlock, dfh)) ||
         (rc = fh_blk_convert(ctx, *s->blk, s->D.as<double>(), s->P, K - kAbBlock / 2, dfh)))
       return rc;
@@ -434,7 +580,7 @@ static int ab_one_step(fh_ab_solver *s, int max_n, int *done) {
     if ((rc = fh_blk_gemm(ctx, *s->blk, K, s->far.as<float2>(), s->ldfar))) return rc;
     s->T0 = K;
   }
-  if (s->fused) return ab_fused_steps(s, max_n, done);
+  if (s->resident) return ab_res_steps(s, max_n, done);
   const int k0 = s->blk ? s->T0 : 0;  // entries summed on the CUDA cores this step
   const int kn = K - k0;
   const float2 *far = (s->blk && s->T0 > 0) ? s->far.as<float2>() + (long long)(K - s->T0) * s->ldfar : nullptr;
@@ -464,33 +610,85 @@ static int ab_one_step(fh_ab_solver *s, int max_n, int *done) {
   return FH_OK;
 }
 
-// Blocked mode: the block-start work of step K is already enqueued; runs up to
-// max_n steps of the current 8-step sub-block (k_ab_mid first at its start).
-static int ab_fused_steps(fh_ab_solver *s, int max_n, int *done) {
+template <class A, int NW, int EM>
+static int ab_res_launch(fh_ab_solver *s, const fh_ab_res_args &a) {
   fh_ctx *ctx = s->ctx;
-  const int K = s->step;
-  const int T0 = s->blk ? s->T0 : 0;
-  const int K8 = (K / kAbSub) * kAbSub;  // >= T0: blocks are whole sub-blocks
-  int rc;
-  if (K == K8 && K8 > T0) {
-    const int nr = min(kAbSub, s->max_steps - K8);
-    fh_prof_mark(ctx, FH_PROF_HISTORY, false);
-    k_ab_mid<<<dim3((unsigned)fh_ceil_div(s->m + 1, 128), (unsigned)nr), 128, 0, ctx->stream>>>(
-        s->m, s->P, T0, K8, nr, s->w2.as<float2>(), reinterpret_cast<const float2 *>(s->D.as<double>()),
-        (s->blk && T0 > 0) ? s->far.as<float2>() : nullptr, s->ldfar, s->mid.as<float2>());
-    fh_prof_mark(ctx, FH_PROF_HISTORY, true);
-    if ((rc = fh_after_launch(ctx, "k_ab_mid"))) return rc;
-  }
-  const float2 *mid = K8 > T0 ? s->mid.as<float2>() : nullptr;
-  const float2 *far8 = (!mid && s->blk && T0 > 0) ? s->far.as<float2>() + (long long)(K8 - T0) * s->ldfar : nullptr;
-  const int ns = min(max_n, kAbSub - (K - K8));
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(kAbResMaxCtas);
+  cfg.blockDim = dim3(kAbResThreads);
+  cfg.dynamicSmemBytes = ab_res_smem(NW, (s->m - 1 + 32 * NW - 1) / (32 * NW), kAbResMaxCtas);
+  cfg.stream = ctx->stream;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = kAbResMaxCtas;
+  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
   fh_prof_mark(ctx, FH_PROF_SWEEP, false);
-  k_ab_line_fused<<<1, kAbFuseThreads, ab_fused_smem(s->m), ctx->stream>>>(
-      s->m, 1.0 - s->alpha, s->ii.as<double>(), s->tab2.as<float2>(), s->P, s->src2.as<float2>(), s->nrows,
-      s->bl.as<double>(), s->br.as<double>(), s->C.as<double>(), reinterpret_cast<float2 *>(s->D.as<double>()),
-      s->P, s->w2.as<float2>(), mid, far8, s->ldfar, K8, K - K8, ns, s->tau);
+  FH_CUDA_TRY(ctx, cudaLaunchKernelEx(&cfg, k_ab_resident<A, NW, EM>, a));
   fh_prof_mark(ctx, FH_PROF_SWEEP, true);
-  if ((rc = fh_after_launch(ctx, "k_ab_line_fused"))) return rc;
+  return fh_after_launch(ctx, "k_ab_resident");
+}
+
+// Whether the device takes the resident solve's clusters (sixteen CTAs with
+// this much shared memory); sets the kernel's attributes.
+template <class A, int NW, int EM>
+static bool ab_res_ok(int m) {
+  const int E = (m - 1 + 32 * NW - 1) / (32 * NW);
+  if (E > EM) return false;
+  auto kern = k_ab_resident<A, NW, EM>;
+  const int smem = (int)ab_res_smem(NW, EM, kAbResMaxCtas);  // the largest size: solvers share the attribute
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(kAbResMaxCtas);
+  cfg.blockDim = dim3(kAbResThreads);
+  cfg.dynamicSmemBytes = (size_t)smem;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = kAbResMaxCtas;
+  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  int active = 0;
+  const bool ok = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) == cudaSuccess &&
+                  cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
+                  cudaOccupancyMaxActiveClusters(&active, kern, &cfg) == cudaSuccess && active >= 1;
+  cudaGetLastError();
+  return ok;
+}
+
+// Blocked mode: the block-start work of step K is already enqueued; runs up to
+// max_n steps, to the end of the block at most.  Four solving warps where they
+// take the line at five equations a thread (fewer barriers and warp totals),
+// sixteen above.
+constexpr int kAbResEq = 5, kAbResSmall = 4 * 32 * kAbResEq;
+static int ab_res_steps(fh_ab_solver *s, int max_n, int *done) {
+  const int K = s->step, T0 = s->blk ? s->T0 : 0;
+  const int ns = std::min(max_n, T0 + kAbResMaxSteps - K);
+  fh_ab_res_args a;
+  a.m = s->m;
+  a.nrows = s->nrows;
+  a.T0 = T0;
+  a.K0 = K;
+  a.ns = ns;
+  a.P = s->P;
+  a.ldfar = s->ldfar;
+  const float2 *tab = s->tab2.as<float2>();
+  a.sl = tab;
+  a.nal = tab + s->P;
+  a.inv = tab + 2 * s->P;
+  a.src = s->src2.p;
+  a.bl = s->bl.as<double>();
+  a.br = s->br.as<double>();
+  a.w = s->w2.p;
+  a.far = s->blk && T0 > 0 ? s->far.p : nullptr;
+  a.D = s->D.p;
+  a.C = s->C.as<double>();
+  a.cI = s->Ii / (1.0 - s->alpha);
+  a.nioma = -1.0 / (1.0 - s->alpha);
+  a.itau = 1.0 / s->tau;
+  const int rc = s->m - 1 <= kAbResSmall ? ab_res_launch<fh_ab_df, 4, kAbResEq>(s, a)
+                                         : ab_res_launch<fh_ab_df, 16, kAbResEq>(s, a);
+  if (rc) return rc;
   s->step += ns;
   *done = ns;
   return FH_OK;
@@ -507,7 +705,6 @@ int fh_ab_create(fh_ctx *ctx, int m, int max_steps, double tau, double alpha, fh
     const size_t sm = ab_line_smem(m);
     FH_REQUIRE(ctx, sm <= 200 * 1024, FH_EINVAL, "fh_ab_create: m too large for the staged line (m <= 3500)");
     FH_CUDA_TRY(ctx, cudaFuncSetAttribute(k_ab_line, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-    FH_CUDA_TRY(ctx, cudaFuncSetAttribute(k_ab_line_fused, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
   }
   fh_ab_solver *s = new fh_ab_solver();
   s->ctx = ctx;
@@ -540,6 +737,7 @@ int fh_ab_create(fh_ctx *ctx, int m, int max_steps, double tau, double alpha, fh
   double ii_h = 0.0;
   FH_CUDA_TRY(ctx, cudaMemcpyAsync(&ii_h, s->w.p, sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
   FH_CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));
+  s->Ii = ii_h;
   s->Bd = (ii_h / (1.0 - alpha)) + (2.0 / (h * h));
   k_ab_factor<<<1, 1, 0, ctx->stream>>>(m, s->A, s->Bd, s->Cc, s->al.as<double>(), s->den.as<double>(),
                                         s->inv.as<double>(), s->sl.as<double>(), s->pf.as<double>(),
@@ -574,6 +772,7 @@ int fh_ab_set_source_host(fh_ab_solver *s, int nrows, const double *src_host, co
   FH_CUDA_TRY(ctx, cudaMemcpyAsync(s->bl.p, bl_host, sizeof(double) * nrows, cudaMemcpyHostToDevice, ctx->stream));
   FH_CUDA_TRY(ctx, cudaMemcpyAsync(s->br.p, br_host, sizeof(double) * nrows, cudaMemcpyHostToDevice, ctx->stream));
   s->nrows = nrows;
+  s->graph.reset();  // the rows' addresses and count are in the captured launches
   if ((rc = ab_src_pairs(s))) return rc;
   FH_CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));
   return FH_OK;
@@ -606,10 +805,12 @@ int fh_ab_set_current_coef(fh_ab_solver *s, double Ii) {
   FH_CUDA_TRY(ctx, cudaMemcpyAsync(s->ii.p, &Ii, sizeof(double), cudaMemcpyHostToDevice, ctx->stream));
   FH_CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));
   const double h = 1.0 / s->m;
+  s->Ii = Ii;
   s->Bd = (Ii / (1.0 - s->alpha)) + (2.0 / (h * h));
   k_ab_factor<<<1, 1, 0, ctx->stream>>>(s->m, s->A, s->Bd, s->Cc, s->al.as<double>(), s->den.as<double>(),
                                         s->inv.as<double>(), s->sl.as<double>(), s->pf.as<double>(),
                                         s->pb.as<double>());
+  s->graph.reset();  // the coefficient is an argument of the captured launches
   const int rc = fh_after_launch(ctx, "k_ab_factor");
   return rc ? rc : ab_table_pairs(s);
 }
@@ -655,13 +856,11 @@ int fh_ab_set_mode(fh_ab_solver *s, int mode) {
     fh_blk_delete(s->blk);
     s->blk = nullptr;
   }
-  // 8-step launches when the tables and the field fit in shared memory
-  s->fused = mode == FH_AB_BLOCKED && ab_fused_smem(s->m) <= 200 * 1024 &&
-             s->m + 1 <= kAbFuseThreads * kAbFuseMaxNodes;
-  if (s->fused) {
+  s->resident = mode == FH_AB_BLOCKED && (s->m - 1 <= kAbResSmall ? ab_res_ok<fh_ab_df, 4, kAbResEq>(s->m)
+                                                                  : ab_res_ok<fh_ab_df, 16, kAbResEq>(s->m));
+  if (s->resident) {
     int rc;
-    if (!s->mid.p && (rc = fh_alloc(ctx, s->mid, sizeof(float2) * kAbSub * (size_t)s->P))) return rc;
-    if (!s->tab2.p && (rc = fh_alloc(ctx, s->tab2, sizeof(float2) * 5 * (size_t)s->P))) return rc;
+    if (!s->tab2.p && (rc = fh_alloc(ctx, s->tab2, sizeof(float2) * 3 * (size_t)s->P))) return rc;
     if (!s->w2.p) {
       if ((rc = fh_alloc(ctx, s->w2, sizeof(float2) * (size_t)(s->max_steps + 2)))) return rc;
       if ((rc = ab_pairs(ctx, s->w.as<double>(), s->w2.as<float2>(), s->max_steps + 2, 0))) return rc;
