@@ -1,8 +1,7 @@
 """The resident Atangana-Baleanu solve (k_ab_resident) at the edges of its
-tiling: one equation, partly filled chunks, the limits of four and of sixteen
-solving warps at five equations a thread, a block boundary, several source
-rows with boundary values, one captured call and uneven calls, against the
-oracle.
+tiling: one equation, partly filled chunks, the limits of four, eight and
+sixteen solving warps, a block boundary, several source rows with boundary
+values, one captured call and uneven calls, against the oracle.
 
 Tolerance: the blocked mode's bound, 1e-9 of the largest value; the two call
 patterns run the same sums on the same entries, so they agree to the roundings
@@ -17,7 +16,7 @@ pytestmark = pytest.mark.gpu
 STEPS = 150  # block boundary at 128
 
 
-@pytest.mark.parametrize("m", [2, 3, 33, 129, 130, 640, 641, 642, 1025, 2559])
+@pytest.mark.parametrize("m", [2, 3, 33, 129, 130, 513, 514, 1025, 1026, 2049, 2559])
 def test_resident_tiling(m):
     from theses_code_gb300 import workloads
     from theses_code_gb300._lib import FH_AB_BLOCKED, Context

@@ -10,11 +10,13 @@
 
 #include <algorithm>
 #include <cmath>
+#include <type_traits>
 
 #include "fh_internal.h"
 #include "fh_common.cuh"
 #include "fh_linescan.cuh"
 #include "fh_df.cuh"
+#include "fh_cluster.cuh"
 
 // blocked contraction helpers (fh_blocked.cu)
 struct fh_blk;
@@ -44,7 +46,8 @@ struct fh_ab_solver {
   // lag weights, source rows and elimination tables as (hi, lo) FP32 pairs
   bool resident = false;
   double Ii = 0;          // current-step coefficient (host copy of ii)
-  fh_dbuf w2, src2, tab2; // pairs: lag weights, source rows, tables sl, -al, inv
+  fh_dbuf w2, src2, tab2, dx;  // pairs: lag weights, source rows, tables sl, -al, inv, last change of C
+  fh_dbuf derr;           // set when a device wait ran out
   ~fh_ab_solver() {
     if (blk) fh_blk_delete(blk);
   }
@@ -187,22 +190,30 @@ __global__ void __launch_bounds__(kAbThreads) k_ab_line(int m, double oma, const
 // the tensor cores; the block's own entries are summed here.
 //   CTA 0 solves the line, step after step: field, elimination tables, prefix
 //     products and the slopes of both scans stay in registers and shared
-//     memory.  The right part needs one history term from it, the newest
-//     entry; the rest of the history sum arrives in distributed shared memory.
-//   CTAs 1 .. C - 1 own a range of the line's threads each and sum, while
-//     CTA 0 solves step s, the history of step s + 1 for the nodes of those
-//     threads: far row plus every entry of the block but the newest.  They keep
-//     their nodes' entries in shared memory, fetched from CTA 0 one step after
-//     they are made.
-// One hardware cluster barrier per step; newest entries and sums are
-// double-buffered by the parity of the step.  Every CTA reaches the barrier
-// the same number of times.
+//     memory.  Of the right part times 1/den it adds only what needs the last
+//     step, Ii/(1-a) C and the newest entry.
+//   CTAs 1 .. 15 own a range of the line's threads each and prepare the rest
+//     for the nodes of those threads: source, far row and every entry of the
+//     block but the newest, times 1/den.  They keep their nodes' entries in
+//     shared memory, made from the field differences CTA 0 sends, and store
+//     them for the block's contraction.
+// Both directions are one-sided (fh_cluster.cuh): the difference of step s goes
+// out when it is solved, the right parts of step s + 2 come back while CTA 0
+// solves step s + 1.  Buffers alternate with the parity of the step: CTA 0
+// sends the difference of step s after it has the right parts of step s, which
+// their owner sent after it had read the difference of step s - 2; and an
+// owner sends right parts of step s + 2 after it has the difference of step s,
+// sent when CTA 0 had read the right parts of step s.  A cluster barrier before
+// the first and after the last message; waits are bounded (*err on expiry).
+// With one cluster barrier a step instead, reading each other's shared memory,
+// 2048 nodes took 4.4-5.4 us a step, of which a 200-node line still took 2.9.
 //
 // The matrix is fixed, so the slopes of both substitutions are too: a thread
 // owns E consecutive equations, walks them from a zero start and adds prefix
 // product x start value, and the scans move offsets only (one multiply-add and
-// one shuffle of a value per level).  What bounds a step is the dependent chain
-// on CTA 0: right part, 4-5 equations, 5 + 4 scan levels, the same backwards.
+// one shuffle of a value per level).  What bounds a step is CTA 0: ~100 FP32
+// instructions per equation and ~20 per scan level and warp, and their
+// dependent chain.
 // Arithmetic A: double-float on the FP32 pipe (blocked mode).
 struct fh_ab_df {
   using S = float2;  // stored
@@ -229,22 +240,24 @@ struct fh_ab_res_args {
   int m, nrows, T0, K0, ns;    // history entries older than T0 in the far rows; steps K0 .. K0 + ns - 1
   long long P, ldfar;
   const void *sl, *nal, *inv;  // forward slopes, -al and 1/den (S per node)
+  void *dx;                    // C minus C of the step before at the end of a call (S per node)
   const void *src;             // source rows (S), m + 1 per row
   const double *bl, *br;       // boundary values per row
   const void *w;               // lag weights (S)
+  int *err;
   const void *far;             // far row of step T0 + r at far + r ldfar (S), null: none
   void *D;                     // entry tt at D + tt P (S)
   double *C;
   double cI, nioma, itau;      // Ii/(1-a), -1/(1-a), 1/tau
 };
 
-// Shared memory: CTA 0 the tables [5][E][T], scan constants [12][T], newest
-// entries [2][E][T]; the others their nodes' sums [2][E][TW], partial sums and
-// entries [128][E TW].
+// Shared memory: CTA 0 the tables [6][E][T], scan constants [12][T], prepared
+// right parts [2][E][T]; the others their nodes' differences [2][E][TW],
+// partial sums and entries [128][E TW].
 __host__ __device__ inline int ab_res_tw(int nw, int ctas) { return (32 * nw + ctas - 2) / (ctas - 1); }
 static size_t ab_res_smem(int nw, int E, int ctas) {
   const int T = 32 * nw, nn = E * ab_res_tw(nw, ctas);
-  const size_t line = 8 * ((size_t)7 * E * T + (size_t)kAbResLv * T);
+  const size_t line = 8 * ((size_t)8 * E * T + (size_t)kAbResLv * T);
   const size_t work = 8 * ((size_t)2 * nn + kAbResThreads + (size_t)kAbResMaxSteps * nn);
   return line > work ? line : work;
 }
@@ -327,21 +340,33 @@ __global__ void __launch_bounds__(kAbResThreads, 1) k_ab_resident(const fh_ab_re
   extern __shared__ double2 ab_sm2[];
   S *sm = reinterpret_cast<S *>(ab_sm2);
   __shared__ S tot[2][NW], lw[2][5 * 32], wl[kAbResMaxSteps + 2];
+  __shared__ uint64_t bars[2];  // CTA 0: right parts here; the others: differences here
   const int C = (int)cl.num_blocks(), r = (int)cl.block_rank(), t = threadIdx.x;
   const int m = a.m, n = m - 1;  // equations 1 .. m - 1
   const int E = (n + T - 1) / T;
   const int TW = ab_res_tw(NW, C);
   S *D = reinterpret_cast<S *>(a.D);
   const S *w = reinterpret_cast<const S *>(a.w);
+  const uint32_t bar = fh_smem_u32(bars), smb = fh_smem_u32(sm);
+  if (t == 0) {
+    fh_mbar_init(bar, 1);
+    fh_mbar_init(bar + 8, 1);
+    fh_fence_mbar_init();
+  }
+  bool ok = true;
   if (r == 0) {
-    S *tf = sm, *ti = tf + E * T, *tn = ti + E * T, *pf = tn + E * T, *pb = pf + E * T;
-    S *lvf = pb + E * T, *lvb = lvf + 6 * T, *dn = lvf + kAbResLv * T;  // dn: [2][E][T]
+    // forward slope, Ii/(1-a)/den, newest entry's factor, -al, prefix products
+    S *tf = sm, *tc = tf + E * T, *tw = tc + E * T, *tn = tw + E * T, *pf = tn + E * T, *pb = pf + E * T;
+    S *lvf = pb + E * T, *lvb = lvf + 6 * T, *rp = lvf + kAbResLv * T;  // rp: [2][E][T]
     const bool solving = t < T;  // whole warps; the others only keep the cluster barriers
     const int j0 = 1 + t * E;    // the thread's first equation
     const int c = solving ? max(0, min(E, m - j0)) : 0;
-    V Cv[EM], dv[EM], sv[EM];
-    V zero = A::of(0.0), one = A::of(1.0);
+    V Cv[EM], dv[EM];  // field, its last change
+    const V zero = A::of(0.0), one = A::of(1.0);
     if (solving) {
+      const V cI = A::of(a.cI);
+      // the newest entry, lag 2: -1/(1-a) w dC / tau
+      const V cw = A::mul(A::ld(w[2]), A::of(a.nioma * a.itau));
       V pa = one;
 #pragma unroll
       for (int e = 0; e < EM; ++e)
@@ -350,17 +375,14 @@ __global__ void __launch_bounds__(kAbResThreads, 1) k_ab_resident(const fh_ab_re
           const int q = e * T + t, j = in ? j0 + e : 0;
           const V f = in ? A::ld(reinterpret_cast<const S *>(a.sl)[j]) : zero;
           tf[q] = A::st(f);
-          ti[q] = in ? reinterpret_cast<const S *>(a.inv)[j] : A::st(zero);
+          const V iv = in ? A::ld(reinterpret_cast<const S *>(a.inv)[j]) : zero;
+          tc[q] = A::st(A::mul(cI, iv));
+          tw[q] = A::st(A::mul(cw, iv));
           tn[q] = in ? reinterpret_cast<const S *>(a.nal)[j] : A::st(one);
           pa = A::mul(pa, f);
           pf[q] = A::st(pa);
           Cv[e] = in ? A::of(a.C[j]) : zero;
-          dv[e] = zero;
-          if (in && a.K0 > a.T0) {  // the newest entry before the call
-            const S d = D[(long long)(a.K0 - 1) * a.P + j];
-            dv[e] = A::ld(d);
-          }
-          sv[e] = zero;
+          dv[e] = in && a.K0 > a.T0 ? A::ld(reinterpret_cast<const S *>(a.dx)[j]) : zero;
         }
       V pq = one;
 #pragma unroll
@@ -374,45 +396,37 @@ __global__ void __launch_bounds__(kAbResThreads, 1) k_ab_resident(const fh_ab_re
       ab_scan_setup<A, NW, true>(pq, tot[1], lvb, lw[1]);
     }
     V c0 = A::of(a.C[0]), cm = A::of(a.C[m]);  // the boundary nodes (thread 0 keeps them)
-    const V cI = A::of(a.cI), nioma = A::of(a.nioma), itau = A::of(a.itau);
-    const V w2 = A::ld(w[2]);  // the newest entry's weight
+    const V itau = A::of(a.itau);
     int row = -1;
     V bl = zero, br = zero;
-    auto load_row = [&](int K) {  // source row and boundary values of the step with K entries
+    auto load_row = [&](int K) {  // boundary values of the step with K entries
       const int nr = K < a.nrows - 1 ? K : a.nrows - 1;
       if (!solving || nr == row) return;
       row = nr;
       bl = A::of(a.bl[row]);
       br = A::of(a.br[row]);
-      const S *src = reinterpret_cast<const S *>(a.src) + (long long)row * (m + 1);
-#pragma unroll
-      for (int e = 0; e < EM; ++e)
-        if (e < c) sv[e] = A::ld(src[j0 + e]);
     };
     load_row(a.K0);
-    cl.sync();  // step K0 is prepared
+    // the thread's differences in its owner's buffer
+    const uint32_t own = 1 + t / TW, obar = fh_mapa(bar, own), odst = fh_mapa(smb, own) + 8 * (t % TW);
+    cl.sync();
     for (int s = 0; s < a.ns; ++s) {
       const int K = a.K0 + s, par = s & 1;
       if (solving) {
+        if (t == 0) fh_mbar_arrive_expect_tx(bar + 8 * par, 8 * E * T);
+        ok = fh_group_and(1, T, fh_mbar_wait(bar + 8 * par, (s >> 1) & 1));
+        if (!ok) break;
         V bt[EM];
         {
-          // sums of the thread's nodes from the CTA that owns the thread
-          const S *hs = cl.map_shared_rank(sm + par * E * TW, 1 + t / TW) + t % TW;
           const bool newest = K > a.T0;
-          S h[EM];
-#pragma unroll
-          for (int e = 0; e < EM; ++e)
-            if (e < E) h[e] = hs[e * TW];
           V v = zero;
 #pragma unroll
           for (int e = 0; e < EM; ++e)
             if (e < E) {
               const int q = e * T + t;
-              V x = A::fma(cI, Cv[e], sv[e]);
-              V y = A::ld(h[e]);
-              if (newest) y = A::fma(w2, dv[e], y);
-              x = A::fma(nioma, y, x);  // MF_intF_simple returns ret/(1-a)
-              v = A::fma(A::ld(tf[q]), v, A::mul(x, A::ld(ti[q])));
+              V x = A::fma(A::ld(tc[q]), Cv[e], A::ld(rp[par * E * T + q]));
+              if (newest) x = A::fma(A::ld(tw[q]), dv[e], x);
+              v = A::fma(A::ld(tf[q]), v, x);
               bt[e] = v;
             }
           const V st = ab_scan<A, NW, false>(v, bl, tot[0], lvf, lw[0]);  // bt before the thread's equations
@@ -432,9 +446,9 @@ __global__ void __launch_bounds__(kAbResThreads, 1) k_ab_resident(const fh_ab_re
         for (int e = 0; e < EM; ++e)
           if (e < E) {
             const V x = A::fma(A::ld(pb[e * T + t]), st, bt[e]);
-            dv[e] = A::mul(A::sub(x, Cv[e]), itau);
+            dv[e] = A::sub(x, Cv[e]);
             if (e < c) Cv[e] = x;
-            dn[(par * E + e) * T + t] = A::st(dv[e]);
+            fh_st_async8(odst + 8 * (par * E + e) * TW, A::st(dv[e]), obar + 8 * par);
           }
         if (t == 0) {
           S *Dk = D + (long long)K * a.P;
@@ -445,83 +459,90 @@ __global__ void __launch_bounds__(kAbResThreads, 1) k_ab_resident(const fh_ab_re
         }
         if (s + 1 < a.ns) load_row(K + 1);
       }
-      cl.sync();
     }
+    if (!ok) atomicOr(a.err, 1);
     if (solving) {
 #pragma unroll
       for (int e = 0; e < EM; ++e)
-        if (e < c) a.C[j0 + e] = A::to(Cv[e]);
+        if (e < c) {
+          a.C[j0 + e] = A::to(Cv[e]);
+          reinterpret_cast<S *>(a.dx)[j0 + e] = A::st(dv[e]);
+        }
       if (t == 0) {
         a.C[0] = A::to(c0);
         a.C[m] = A::to(cm);
       }
     }
-    cl.sync();  // the last entries have been fetched
+    cl.sync();
     return;
   }
   // ---- history of the nodes of threads [t0, t0 + TW): item i = e TW + (thread - t0)
-  const int t0 = (r - 1) * TW, nn = E * TW;
-  S *hs = sm, *pt = hs + 2 * nn, *ent = pt + kAbResThreads;
-  auto node = [&](int i) { return 1 + (t0 + i % TW) * E + i / TW; };
-  auto live = [&](int i) { return t0 + i % TW < T && node(i) < m; };
-  for (int k = t; k < kAbResMaxSteps + 2; k += kAbResThreads) wl[k] = k < a.K0 - a.T0 + a.ns + 2 ? w[k] : A::st(A::of(0.0));
+  const int t0 = (r - 1) * TW, nn = E * TW, tw = max(0, min(TW, T - t0));
+  S *dxb = sm, *pt = dxb + 2 * nn, *ent = pt + kAbResThreads;
+  // thread t sums run p of the block's entries for item i; run 0 also fetches,
+  // stores and sends
+  const int i = t % nn, p = t / nn, parts = kAbResThreads / nn;
+  const int ti = t0 + i % TW, node = 1 + ti * E + i / TW;
+  const bool mine = ti < T, live = mine && node < m;
   const int K0 = a.K0, T0 = a.T0;
-  for (int x = t; x < (K0 - T0) * nn; x += kAbResThreads) {
-    const int tt = x / nn, i = x - tt * nn;
-    ent[x] = live(i) ? D[(long long)(T0 + tt) * a.P + node(i)] : A::st(A::of(0.0));
-  }
-  // the block's entries in up to `parts` runs per item, summed side by side
-  const int parts = max(1, kAbResThreads / nn);
-  for (int s = -1; s <= a.ns; ++s) {
-    // entry K0 + s - 1 (made by CTA 0 in the phase before): own copy and the stored history
-    if (s >= 1) {
-      const int K = K0 + s - 1, par = (s - 1) & 1;
-      const S *dn = cl.map_shared_rank(sm + (size_t)5 * E * T + (size_t)kAbResLv * T, 0) + (size_t)par * E * T;
-      for (int i = t; i < nn; i += kAbResThreads) {
+  for (int k = t; k < kAbResMaxSteps + 2; k += kAbResThreads) wl[k] = k < K0 - T0 + a.ns + 2 ? w[k] : A::st(A::of(0.0));
+  if (p < parts)
+    for (int tt = p; tt < K0 - T0; tt += parts)
+      ent[tt * nn + i] = live ? D[(long long)(T0 + tt) * a.P + node] : A::st(A::of(0.0));
+  const V itau = A::of(a.itau);
+  const V iv = live ? A::ld(reinterpret_cast<const S *>(a.inv)[node]) : A::of(0.0);
+  const V ni = A::mul(A::of(a.nioma), iv);  // MF_intF_simple returns ret/(1-a)
+  const uint32_t rbar = fh_mapa(bar, 0);
+  const uint32_t rdst = fh_mapa(smb, 0) + 8 * ((6 * E + kAbResLv) * T + (i / TW) * T + ti);
+  int row = -1;
+  V sr = A::of(0.0);  // source times 1/den
+  cl.sync();
+  for (int s = -2; s < a.ns; ++s) {
+    if (s >= 0) {  // the difference of step s: own copy and the stored history
+      const int K = K0 + s;
+      if (t == 0) fh_mbar_arrive_expect_tx(bar + 8 * (s & 1), 8 * E * tw);
+      if (tw > 0) ok = fh_mbar_wait(bar + 8 * (s & 1), (s >> 1) & 1);
+      if (p == 0) {
         S d = A::st(A::of(0.0));
-        if (live(i)) {
-          d = dn[(i / TW) * T + t0 + i % TW];
-          D[(long long)K * a.P + node(i)] = d;
+        if (live) {
+          d = A::st(A::mul(A::ld(dxb[(s & 1) * nn + i]), itau));
+          D[(long long)K * a.P + node] = d;
         }
         ent[(K - T0) * nn + i] = d;
       }
     }
-    __syncthreads();
-    const int sn = s + 1;  // the step to prepare
+    ok = __syncthreads_and(ok);
+    if (!ok) break;
+    const int sn = s + 2;  // the step to prepare
     if (sn < a.ns) {
       const int K = K0 + sn, no = max(K - 1 - T0, 0);  // entries T0 .. K - 2
-      const S *far = a.far ? reinterpret_cast<const S *>(a.far) + (long long)(K - T0) * a.ldfar : nullptr;
-      S *out = hs + (sn & 1) * nn;
-      const int per = (no + parts - 1) / parts;
-      for (int i0 = 0; i0 < nn; i0 += kAbResThreads) {  // one round unless nn > 512
-        const int i = i0 + t % min(nn, kAbResThreads), p = t / min(nn, kAbResThreads);
-        V s0 = A::of(0.0);
-        if (i < nn && p < parts) {
-          const int b = min(no, p * per), e = min(no, b + per);
-          if (p == 0 && far && live(i)) s0 = A::ld(far[node(i)]);
-          V s1 = A::of(0.0);
-          int tt = b;
-          for (; tt + 2 <= e; tt += 2) {  // entry tt has lag K + 1 - (T0 + tt)
-            s0 = A::fma(A::ld(wl[K + 1 - T0 - tt]), A::ld(ent[tt * nn + i]), s0);
-            s1 = A::fma(A::ld(wl[K - T0 - tt]), A::ld(ent[(tt + 1) * nn + i]), s1);
-          }
-          if (tt < e) s0 = A::fma(A::ld(wl[K + 1 - T0 - tt]), A::ld(ent[tt * nn + i]), s0);
-          s0 = A::add(s0, s1);
-        }
-        if (parts > 1) {
-          if (p < parts) pt[t] = A::st(s0);
-          __syncthreads();
-          if (p == 0 && i < nn) {
-            for (int q = 1; q < parts; ++q) s0 = A::add(s0, A::ld(pt[q * nn + i]));
-            out[i] = A::st(s0);
-          }
-        } else if (i < nn) {
-          out[i] = A::st(s0);
-        }
+      const int nr = K < a.nrows - 1 ? K : a.nrows - 1;
+      if (nr != row) {
+        row = nr;
+        if (live) sr = A::mul(A::ld(reinterpret_cast<const S *>(a.src)[(long long)row * (m + 1) + node]), iv);
       }
+      const int per = (no + parts - 1) / parts;
+      const int b = min(no, p * per), e = p < parts ? min(no, b + per) : b;
+      V s0 = A::of(0.0), s1 = A::of(0.0);
+      if (p == 0 && a.far && live) s0 = A::ld(reinterpret_cast<const S *>(a.far)[(long long)(K - T0) * a.ldfar + node]);
+      int tt = b;
+      for (; tt + 2 <= e; tt += 2) {  // entry tt has lag K + 1 - (T0 + tt)
+        s0 = A::fma(A::ld(wl[K + 1 - T0 - tt]), A::ld(ent[tt * nn + i]), s0);
+        s1 = A::fma(A::ld(wl[K - T0 - tt]), A::ld(ent[(tt + 1) * nn + i]), s1);
+      }
+      if (tt < e) s0 = A::fma(A::ld(wl[K + 1 - T0 - tt]), A::ld(ent[tt * nn + i]), s0);
+      s0 = A::add(s0, s1);
+      if (parts > 1) {
+        if (p > 0 && p < parts) pt[t] = A::st(s0);
+        __syncthreads();
+        if (p == 0)
+          for (int q = 1; q < parts; ++q) s0 = A::add(s0, A::ld(pt[q * nn + i]));
+      }
+      if (p == 0 && mine)
+        fh_st_async8(rdst + 8 * (sn & 1) * E * T, A::st(A::fma(ni, s0, sr)), rbar + 8 * (sn & 1));
     }
-    if (s < a.ns) cl.sync();
   }
+  if (!ok) atomicOr(a.err, 1);
   cl.sync();
 }
 
@@ -657,10 +678,14 @@ static bool ab_res_ok(int m) {
 }
 
 // Blocked mode: the block-start work of step K is already enqueued; runs up to
-// max_n steps, to the end of the block at most.  Four solving warps where they
-// take the line at five equations a thread (fewer barriers and warp totals),
-// sixteen above.
-constexpr int kAbResEq = 5, kAbResSmall = 4 * 32 * kAbResEq;
+// max_n steps, to the end of the block at most.  Solving warps: the fewest that
+// take the line at four equations a thread, sixteen (five) for the longest.
+template <class F>
+static auto ab_res_pick(int m, F f) {
+  if (m - 1 <= 4 * 32 * 4) return f(std::integral_constant<int, 4>(), std::integral_constant<int, 4>());
+  if (m - 1 <= 8 * 32 * 4) return f(std::integral_constant<int, 8>(), std::integral_constant<int, 4>());
+  return f(std::integral_constant<int, 16>(), std::integral_constant<int, 5>());
+}
 static int ab_res_steps(fh_ab_solver *s, int max_n, int *done) {
   const int K = s->step, T0 = s->blk ? s->T0 : 0;
   const int ns = std::min(max_n, T0 + kAbResMaxSteps - K);
@@ -677,6 +702,8 @@ static int ab_res_steps(fh_ab_solver *s, int max_n, int *done) {
   a.nal = tab + s->P;
   a.inv = tab + 2 * s->P;
   a.src = s->src2.p;
+  a.dx = s->dx.p;
+  a.err = s->derr.as<int>();
   a.bl = s->bl.as<double>();
   a.br = s->br.as<double>();
   a.w = s->w2.p;
@@ -686,8 +713,7 @@ static int ab_res_steps(fh_ab_solver *s, int max_n, int *done) {
   a.cI = s->Ii / (1.0 - s->alpha);
   a.nioma = -1.0 / (1.0 - s->alpha);
   a.itau = 1.0 / s->tau;
-  const int rc = s->m - 1 <= kAbResSmall ? ab_res_launch<fh_ab_df, 4, kAbResEq>(s, a)
-                                         : ab_res_launch<fh_ab_df, 16, kAbResEq>(s, a);
+  const int rc = ab_res_pick(s->m, [&](auto nw, auto em) { return ab_res_launch<fh_ab_df, nw(), em()>(s, a); });
   if (rc) return rc;
   s->step += ns;
   *done = ns;
@@ -856,11 +882,13 @@ int fh_ab_set_mode(fh_ab_solver *s, int mode) {
     fh_blk_delete(s->blk);
     s->blk = nullptr;
   }
-  s->resident = mode == FH_AB_BLOCKED && (s->m - 1 <= kAbResSmall ? ab_res_ok<fh_ab_df, 4, kAbResEq>(s->m)
-                                                                  : ab_res_ok<fh_ab_df, 16, kAbResEq>(s->m));
+  s->resident = mode == FH_AB_BLOCKED &&
+                ab_res_pick(s->m, [&](auto nw, auto em) { return ab_res_ok<fh_ab_df, nw(), em()>(s->m); });
   if (s->resident) {
     int rc;
     if (!s->tab2.p && (rc = fh_alloc(ctx, s->tab2, sizeof(float2) * 3 * (size_t)s->P))) return rc;
+    if (!s->derr.p && (rc = fh_alloc(ctx, s->derr, sizeof(int)))) return rc;
+    if (!s->dx.p && (rc = fh_alloc(ctx, s->dx, sizeof(float2) * (size_t)s->P))) return rc;
     if (!s->w2.p) {
       if ((rc = fh_alloc(ctx, s->w2, sizeof(float2) * (size_t)(s->max_steps + 2)))) return rc;
       if ((rc = ab_pairs(ctx, s->w.as<double>(), s->w2.as<float2>(), s->max_steps + 2, 0))) return rc;
@@ -900,7 +928,10 @@ int fh_ab_get_c_host(fh_ab_solver *s, double *C_host) {
   fh_ctx *ctx = s->ctx;
   FH_REQUIRE(ctx, C_host, FH_EINVAL, "fh_ab_get_c_host: null pointer");
   FH_CUDA_TRY(ctx, cudaMemcpyAsync(C_host, s->C.p, sizeof(double) * (s->m + 1), cudaMemcpyDeviceToHost, ctx->stream));
+  int err = 0;
+  if (s->derr.p) FH_CUDA_TRY(ctx, cudaMemcpyAsync(&err, s->derr.p, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
   FH_CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));
+  FH_REQUIRE(ctx, err == 0, FH_ETIMEOUT, "fh_ab_step: a wait of the resident solve ran out");
   return FH_OK;
 }
 

@@ -232,6 +232,17 @@ __device__ __forceinline__ void fh_group_bar(int bar, int nthreads) {
   asm volatile("bar.sync %0, %1;" ::"r"(bar), "r"(nthreads) : "memory");
 }
 
+// Whether every thread of the group says so.
+__device__ __forceinline__ bool fh_group_and(int bar, int nthreads, bool mine) {
+  int all;
+  asm volatile(
+      "{\n .reg .pred p, q;\n setp.ne.s32 p, %1, 0;\n barrier.cta.red.and.pred q, %2, %3, p;\n selp.s32 %0, 1, 0, q;\n}\n"
+      : "=r"(all)
+      : "r"((int)mine), "r"(bar), "r"(nthreads)
+      : "memory");
+  return all != 0;
+}
+
 // Thread t receives f_{t-1} o ... o f_0 (identity for thread 0).
 template <int NW>
 __device__ __forceinline__ fh_aff fh_group_exclusive_affine(fh_aff f, fh_aff *sm, int bar) {
