@@ -279,9 +279,15 @@ typedef struct {
   double dL, dLx;   /* steps of the x sweep (along i) and y sweep (along j) */
 } fh_tg_params;
 
-#define FH_TG_FP64 0      /* FP64 history, FP64 FMA sums (bit-faithful arithmetic)        */
+#define FH_TG_FP64 0      /* FP64 history, sums and line solves                          */
 #define FH_TG_BLOCKED 1   /* far history on the tensor cores (exact bf16 slices), near in DF64 */
 #define FH_TG_DF64 2      /* history as (hi, lo) FP32 pairs, double-float sums on the FP32 pipe */
+/* FH_TG_FP64 and FH_TG_DF64, full history, up to 4096 steps: the layers before
+ * the current 32-step block are contracted for the whole block on the tensor
+ * cores in exact base-256 digits (seven per value, 2^-55 of a 128-layer group's
+ * largest; results as near to a 64-bit sum as the FP64 pipe's); the rest of the
+ * sums and all line solves as named.  64 rows of the field more memory; without
+ * it every layer is summed every step. */
 
 typedef struct fh_tg_solver fh_tg_solver;
 
@@ -387,8 +393,10 @@ int fh_ab_set_current_coef(fh_ab_solver *s, double Ii);
 int fh_ab_set_lag_weights_host(fh_ab_solver *s, int n, const double *w_host);
 /* History mode, before the first step: FH_AB_FP64 (default, FP64 sums) or
  * FH_AB_BLOCKED (entries older than the current 128-step block contracted on
- * the tensor cores with exact bf16 slices, the rest in FP64; ~2x the history
- * memory).  No counterpart in the reference. */
+ * the tensor cores with exact bf16 slices, the rest in double-float; ~2x the
+ * history memory).  FH_AB_FP64 contracts the entries before the current
+ * 64-step block in exact digits at FP64 accuracy (as FH_TG_FP64) on lines of at
+ * most 2049 nodes.  No counterpart in the reference. */
 #define FH_AB_FP64 0
 #define FH_AB_BLOCKED 1
 int fh_ab_set_mode(fh_ab_solver *s, int mode);

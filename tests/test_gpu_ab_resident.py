@@ -3,9 +3,9 @@ tiling: one equation, partly filled chunks, the limits of four, eight and
 sixteen solving warps, a block boundary, several source rows with boundary
 values, one captured call and uneven calls, against the oracle.
 
-Tolerance: the blocked mode's bound, 1e-9 of the largest value; the two call
-patterns run the same sums on the same entries, so they agree to the roundings
-of the field's round trip through FP64 (none) and must be equal."""
+Tolerances: the modes' bounds, 1e-9 (blocked) and 1e-12 (FP64) of the largest
+value; the call patterns run the same sums on the same entries, so they agree to
+the roundings of the field's round trip through FP64 (none) and must be equal."""
 import numpy as np
 import pytest
 
@@ -13,13 +13,14 @@ from oracle import oracle as O
 
 pytestmark = pytest.mark.gpu
 
-STEPS = 150  # block boundary at 128
+STEPS = 150  # block boundaries at 64 (FP64) and 128
 
 
+@pytest.mark.parametrize("mode,tol", [("FH_AB_BLOCKED", 1e-9), ("FH_AB_FP64", 1e-12)])
 @pytest.mark.parametrize("m", [2, 3, 33, 129, 130, 513, 514, 1025, 1026, 2049, 2559])
-def test_resident_tiling(m):
-    from theses_code_gb300 import workloads
-    from theses_code_gb300._lib import FH_AB_BLOCKED, Context
+def test_resident_tiling(m, mode, tol):
+    from theses_code_gb300 import _lib, workloads
+    from theses_code_gb300._lib import Context
     from theses_code_gb300.solvers import ABSolver
     cfg, src, _, _, C0 = workloads.ab_1d(m=m, alpha=0.7, tau=1e-3, seed=m)
     rows = 5
@@ -30,16 +31,17 @@ def test_resident_tiling(m):
     ref, _ = O.ab_solve(m, STEPS, cfg["tau"], cfg["alpha"], w, src[at], bl[at], br[at], C0)
     ctx = Context(0)
     got = []
-    for calls in ((STEPS,), (1, 60, 80, 9), (64, 64, 22)):
-        s = ABSolver(ctx, m, STEPS, cfg["tau"], cfg["alpha"], FH_AB_BLOCKED)
+    for solves in (((STEPS,),), ((1, 60, 80, 9),), ((64, 64, 22),), ((140,), (140, 10))):
+        s = ABSolver(ctx, m, STEPS, cfg["tau"], cfg["alpha"], getattr(_lib, mode))
         s.set_source(src, bl, br)
-        s.set_c(C0)
-        for n in calls:
-            s.calc_step(n)
+        for calls in solves:  # the second solve replays the first one's steps, then goes on
+            s.set_c(C0)
+            for n in calls:
+                s.calc_step(n)
         got.append(s.get_c())
         s.close()
     ctx.close()
-    assert float(np.max(np.abs(got[0] - ref)) / np.max(np.abs(ref))) <= 1e-9
+    assert float(np.max(np.abs(got[0] - ref)) / np.max(np.abs(ref))) <= tol
     for g in got[1:]:
         assert np.array_equal(g, got[0])
 

@@ -5,7 +5,7 @@
 // The lag weights I(.) are computed once on the device (fh_weights_ab); the
 // history stores dC_t/tau = (C^{t+1}-C^t)/tau per node.  The matrix is the same
 // every step, so its elimination coefficients are built once and every step
-// runs the two affine recurrences with one warp (see fh_linescan.cuh).
+// runs the two affine recurrences (see fh_linescan.cuh).
 #include <cooperative_groups.h>
 
 #include <algorithm>
@@ -17,6 +17,7 @@
 #include "fh_linescan.cuh"
 #include "fh_df.cuh"
 #include "fh_cluster.cuh"
+#include "fh_far64.h"
 
 // blocked contraction helpers (fh_blocked.cu)
 struct fh_blk;
@@ -34,7 +35,7 @@ struct fh_ab_solver {
   int m = 0, max_steps = 0, step = 0, nrows = 0, max_splits = 1024;
   long long P = 0;  // m+1 rounded up to even
   double tau = 0, alpha = 0, A = 0, Bd = 0, Cc = 0;
-  fh_dbuf w, ii, al, den, inv, sl, pf, pb, C, D, W, part, S, src, bl, br;
+  fh_dbuf w, ii, al, nal, den, inv, sl, pf, pb, C, D, W, part, S, src, bl, br;
   fh_graph_cache graph;
   int mode = FH_AB_FP64;
   fh_blk *blk = nullptr;  // blocked mode: bf16 slice planes of the history entries older than T0
@@ -44,12 +45,16 @@ struct fh_ab_solver {
   // blocked mode, lines of at most 2560 nodes: all steps up to the next block
   // boundary in one launch of k_ab_resident in double-float; history entries,
   // lag weights, source rows and elimination tables as (hi, lo) FP32 pairs
+  // FP64 mode, lines of at most 2049 nodes: the same in FP64, the entries
+  // before the current 64-step block contracted at FP64 accuracy (f64)
   bool resident = false;
+  fh_far64 *f64 = nullptr;
   double Ii = 0;          // current-step coefficient (host copy of ii)
   fh_dbuf w2, src2, tab2, dx;  // pairs: lag weights, source rows, tables sl, -al, inv, last change of C
   fh_dbuf derr;           // set when a device wait ran out
   ~fh_ab_solver() {
     if (blk) fh_blk_delete(blk);
+    if (f64) fh_far64_delete(f64);
   }
 };
 
@@ -62,31 +67,43 @@ constexpr int kAbSolveThreads = 32 * kAbSolveWarps;
 // tabulated here once: inv[j] = 1/den[j], the forward slope sl[j] = -A inv[j],
 // and the per-lane chunk prefix products of the forward slopes (pf) and of the
 // backward slopes -al[j] (pb) in the chunking of k_ab_line.
-__global__ void k_ab_factor(int m, double A, double Bd, double Cc, double *__restrict__ al, double *__restrict__ den,
-                            double *__restrict__ inv, double *__restrict__ sl, double *__restrict__ pf,
-                            double *__restrict__ pb) {
-  if (blockIdx.x != 0 || threadIdx.x != 0) return;
-  double a = 0.0;
-  al[0] = 0.0;
-  den[0] = 1.0;
-  for (int j = 1; j <= m; ++j) {
-    const double d = Bd - A * a;
-    a = Cc / d;
-    al[j] = a;
-    den[j] = d;
-    inv[j] = 1.0 / d;
+// The pivots are a serial chain of FP64 divisions (thread 0); everything that
+// follows from them runs over the threads of one CTA (1.4 -> 0.6 ms at 2048 nodes).
+__global__ void __launch_bounds__(kAbSolveThreads) k_ab_factor(int m, double A, double Bd, double Cc,
+                                                               double *__restrict__ al, double *__restrict__ den,
+                                                               double *__restrict__ inv, double *__restrict__ sl,
+                                                               double *__restrict__ pf, double *__restrict__ pb,
+                                                               double *__restrict__ nal) {
+  const int t = threadIdx.x;
+  if (t == 0) {
+    double a = 0.0;
+    al[0] = 0.0;
+    den[0] = 1.0;
+    for (int j = 1; j <= m; ++j) {
+      const double d = Bd - A * a;
+      a = Cc / d;
+      al[j] = a;
+      den[j] = d;
+    }
+  }
+  __syncthreads();
+  for (int j = t; j <= m; j += kAbSolveThreads) {
+    nal[j] = -al[j];
+    if (j == 0) continue;
+    inv[j] = 1.0 / den[j];
     sl[j] = -A * inv[j];
   }
+  __syncthreads();
   const int ch = (m + kAbSolveThreads - 1) / kAbSolveThreads;
   double p = 1.0;
-  for (int j = 1; j <= m; ++j) {
-    p = ((j - 1) % ch == 0) ? sl[j] : p * sl[j];
+  for (int j = 1 + t * ch; j <= min(m, (t + 1) * ch); ++j) {
+    p = j == 1 + t * ch ? sl[j] : p * sl[j];
     pf[j] = p;
   }
   double q = 1.0;
-  for (int j = m - 1; j >= 0; --j) {
-    const int b1 = min(m, (j / ch + 1) * ch);
-    q = (j == b1 - 1) ? -al[j] : q * -al[j];
+  const int b1 = min(m, (t + 1) * ch);
+  for (int j = b1 - 1; j >= t * ch; --j) {
+    q = j == b1 - 1 ? -al[j] : q * -al[j];
     pb[j] = q;
   }
 }
@@ -214,7 +231,8 @@ __global__ void __launch_bounds__(kAbThreads) k_ab_line(int m, double oma, const
 // one shuffle of a value per level).  What bounds a step is CTA 0: ~100 FP32
 // instructions per equation and ~20 per scan level and warp, and their
 // dependent chain.
-// Arithmetic A: double-float on the FP32 pipe (blocked mode).
+// Arithmetic A: double-float on the FP32 pipe (blocked mode) or FP64 (fh_ab_f64).
+//
 struct fh_ab_df {
   using S = float2;  // stored
   using V = fh_df;   // computed with
@@ -229,6 +247,21 @@ struct fh_ab_df {
   static __device__ __forceinline__ V shfl(V v, int lane) {
     return fh_df{__shfl_sync(0xffffffffu, v.h, lane), __shfl_sync(0xffffffffu, v.l, lane)};
   }
+};
+
+// FP64 (FP64 mode).
+struct fh_ab_f64 {
+  using S = double;
+  using V = double;
+  static __device__ __forceinline__ V ld(S s) { return s; }
+  static __device__ __forceinline__ S st(V v) { return v; }
+  static __device__ __forceinline__ V of(double x) { return x; }
+  static __device__ __forceinline__ double to(V v) { return v; }
+  static __device__ __forceinline__ V fma(V a, V b, V c) { return ::fma(a, b, c); }
+  static __device__ __forceinline__ V mul(V a, V b) { return a * b; }
+  static __device__ __forceinline__ V add(V a, V b) { return a + b; }
+  static __device__ __forceinline__ V sub(V a, V b) { return a - b; }
+  static __device__ __forceinline__ V shfl(V v, int lane) { return __shfl_sync(0xffffffffu, v, lane); }
 };
 
 constexpr int kAbResThreads = 512;
@@ -559,7 +592,7 @@ static int ab_pairs(fh_ctx *ctx, const double *x, float2 *y, long long n, int ne
   return fh_after_launch(ctx, "k_ab_pairs");
 }
 static int ab_table_pairs(fh_ab_solver *s) {
-  if (!s->resident) return FH_OK;
+  if (!s->resident || s->mode != FH_AB_BLOCKED) return FH_OK;
   const long long n = s->m + 1;
   float2 *t = s->tab2.as<float2>();
   int rc;
@@ -569,7 +602,7 @@ static int ab_table_pairs(fh_ab_solver *s) {
   return FH_OK;
 }
 static int ab_src_pairs(fh_ab_solver *s) {
-  if (!s->resident || s->nrows < 1) return FH_OK;
+  if (!s->resident || s->mode != FH_AB_BLOCKED || s->nrows < 1) return FH_OK;
   int rc = fh_alloc(s->ctx, s->src2, sizeof(float2) * (size_t)s->nrows * (s->m + 1), false);
   if (rc) return rc;
   return ab_pairs(s->ctx, s->src.as<double>(), s->src2.as<float2>(), (long long)s->nrows * (s->m + 1), 0);
@@ -599,6 +632,17 @@ static int ab_one_step(fh_ab_solver *s, int max_n, int *done) {
     const int mrows = s->max_steps - K < kAbBlock ? s->max_steps - K : kAbBlock;
     if ((rc = fh_blk_toeplitz_weights(ctx, *s->blk, s->w.as<double>(), K + 1, K, mrows))) return rc;
     if ((rc = fh_blk_gemm(ctx, *s->blk, K, s->far.as<float2>(), s->ldfar))) return rc;
+    s->T0 = K;
+  }
+  if (s->f64 && K > 0 && K % kF64Rows == 0) {
+    // new block: the newest 64 entries join the exponents, then the rows of the
+    // next 64 steps, S_far[r] = sum_{tt<K} w[K+1+r-tt] dC_tt
+    const int nrows = std::min(kF64Rows, s->max_steps - K);
+    if ((rc = fh_far64_append(ctx, *s->f64, s->D.p, s->P, K - 2 * kF64Block)) ||
+        (rc = fh_far64_append(ctx, *s->f64, s->D.p, s->P, K - kF64Block)) ||
+        (rc = fh_far64_weights_lag(ctx, *s->f64, K, s->w.as<double>(), K + 1, nrows)) ||
+        (rc = fh_far64_run(ctx, *s->f64, s->D.p, s->P, K)))
+      return rc;
     s->T0 = K;
   }
   if (s->resident) return ab_res_steps(s, max_n, done);
@@ -677,18 +721,62 @@ static bool ab_res_ok(int m) {
   return ok;
 }
 
-// Blocked mode: the block-start work of step K is already enqueued; runs up to
-// max_n steps, to the end of the block at most.  Solving warps: the fewest that
+// The block-start work of step K is already enqueued; runs up to max_n steps, to
+// the end of the block at most.  Solving warps, double-float: the fewest that
 // take the line at four equations a thread, sixteen (five) for the longest.
+// FP64 (one warp instruction per 19 cycles and SM: fewer warps, fewer scans):
+// eight equations a thread, up to 2049 nodes.
 template <class F>
-static auto ab_res_pick(int m, F f) {
-  if (m - 1 <= 4 * 32 * 4) return f(std::integral_constant<int, 4>(), std::integral_constant<int, 4>());
-  if (m - 1 <= 8 * 32 * 4) return f(std::integral_constant<int, 8>(), std::integral_constant<int, 4>());
-  return f(std::integral_constant<int, 16>(), std::integral_constant<int, 5>());
+static auto ab_res_pick(const fh_ab_solver *s, F f) {
+  const int n = s->m - 1;
+  if (s->mode == FH_AB_BLOCKED) {
+    if (n <= 4 * 32 * 4) return f(k_ab_resident<fh_ab_df, 4, 4>, 4, 4);
+    if (n <= 8 * 32 * 4) return f(k_ab_resident<fh_ab_df, 8, 4>, 8, 4);
+    return f(k_ab_resident<fh_ab_df, 16, 5>, 16, 5);
+  }
+  if (n <= 4 * 32 * 8) return f(k_ab_resident<fh_ab_f64, 4, 8>, 4, 8);
+  return f(k_ab_resident<fh_ab_f64, 8, 8>, 8, 8);
 }
+
+static cudaLaunchConfig_t ab_res_config(cudaLaunchAttribute *at, size_t smem, cudaStream_t st) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(kAbResMaxCtas);
+  cfg.blockDim = dim3(kAbResThreads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = kAbResMaxCtas;
+  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  return cfg;
+}
+
+// Whether the solver's mode and line run the resident solve, on a device that
+// takes its clusters (sixteen CTAs with this much shared memory); sets the
+// kernel's attributes (to the kernel's largest size: solvers share them).
+static bool ab_res_ok(const fh_ab_solver *s) {
+  return ab_res_pick(s, [&](auto kern, int nw, int em) {
+    if (s->m - 1 > 32 * nw * em) return false;
+    const int smem = (int)ab_res_smem(nw, em, kAbResMaxCtas);
+    cudaLaunchAttribute at[1];
+    const cudaLaunchConfig_t cfg = ab_res_config(at, (size_t)smem, nullptr);
+    int active = 0;
+    const bool ok = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) == cudaSuccess &&
+                    cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
+                    cudaOccupancyMaxActiveClusters(&active, kern, &cfg) == cudaSuccess && active >= 1;
+    cudaGetLastError();
+    return ok;
+  });
+}
+
+static int ab_block(const fh_ab_solver *s) { return s->f64 ? kF64Rows : kAbBlock; }
+
 static int ab_res_steps(fh_ab_solver *s, int max_n, int *done) {
-  const int K = s->step, T0 = s->blk ? s->T0 : 0;
-  const int ns = std::min(max_n, T0 + kAbResMaxSteps - K);
+  fh_ctx *ctx = s->ctx;
+  const bool df = s->mode == FH_AB_BLOCKED;
+  const int K = s->step, T0 = s->T0, ns = std::min(max_n, T0 + ab_block(s) - K);
+  FH_REQUIRE(ctx, K >= T0 && ns >= 1, FH_EINVAL, "fh_ab_step: step %d outside its block at %d", K, T0);
   fh_ab_res_args a;
   a.m = s->m;
   a.nrows = s->nrows;
@@ -696,28 +784,64 @@ static int ab_res_steps(fh_ab_solver *s, int max_n, int *done) {
   a.K0 = K;
   a.ns = ns;
   a.P = s->P;
-  a.ldfar = s->ldfar;
   const float2 *tab = s->tab2.as<float2>();
-  a.sl = tab;
-  a.nal = tab + s->P;
-  a.inv = tab + 2 * s->P;
-  a.src = s->src2.p;
+  a.sl = df ? (const void *)tab : s->sl.p;
+  a.nal = df ? (const void *)(tab + s->P) : s->nal.p;
+  a.inv = df ? (const void *)(tab + 2 * s->P) : s->inv.p;
+  a.src = df ? s->src2.p : s->src.p;
+  a.w = df ? s->w2.p : s->w.p;
   a.dx = s->dx.p;
   a.err = s->derr.as<int>();
   a.bl = s->bl.as<double>();
   a.br = s->br.as<double>();
-  a.w = s->w2.p;
-  a.far = s->blk && T0 > 0 ? s->far.p : nullptr;
+  a.far = T0 == 0 ? nullptr : s->f64 ? fh_far64_rows(*s->f64) : s->far.p;
+  a.ldfar = s->f64 ? fh_far64_pitch(*s->f64) : s->ldfar;
   a.D = s->D.p;
   a.C = s->C.as<double>();
   a.cI = s->Ii / (1.0 - s->alpha);
   a.nioma = -1.0 / (1.0 - s->alpha);
   a.itau = 1.0 / s->tau;
-  const int rc = ab_res_pick(s->m, [&](auto nw, auto em) { return ab_res_launch<fh_ab_df, nw(), em()>(s, a); });
+  fh_prof_mark(ctx, FH_PROF_SWEEP, false);
+  const cudaError_t e = ab_res_pick(s, [&](auto kern, int nw, int) {
+    cudaLaunchAttribute at[1];
+    const cudaLaunchConfig_t cfg =
+        ab_res_config(at, ab_res_smem(nw, (s->m - 1 + 32 * nw - 1) / (32 * nw), kAbResMaxCtas), ctx->stream);
+    return cudaLaunchKernelEx(&cfg, kern, a);
+  });
+  fh_prof_mark(ctx, FH_PROF_SWEEP, true);
+  if (e != cudaSuccess) return fh_set_error(ctx, FH_ECUDA, "k_ab_resident: %s", cudaGetErrorString(e));
+  const int rc = fh_after_launch(ctx, "k_ab_resident");
   if (rc) return rc;
   s->step += ns;
   *done = ns;
   return FH_OK;
+}
+
+// The resident solve's buffers and, in the FP64 mode, the contraction of older
+// entries (without memory for it every step sums every entry).
+static int ab_res_setup(fh_ab_solver *s) {
+  fh_ctx *ctx = s->ctx;
+  int rc;
+  s->graph.reset();
+  if (s->f64) fh_far64_delete(s->f64);
+  s->f64 = nullptr;
+  s->resident = ab_res_ok(s);
+  if (s->resident && s->mode == FH_AB_FP64 && s->max_steps > kF64Rows &&
+      fh_far64_create(ctx, s->P, (int)fh_ceil_div(s->max_steps, kF64Rows) * kF64Rows, false, &s->f64)) {
+    s->resident = false;
+    cudaGetLastError();
+  }
+  if (!s->resident) return FH_OK;
+  if (!s->derr.p && (rc = fh_alloc(ctx, s->derr, sizeof(int)))) return rc;
+  if (!s->dx.p && (rc = fh_alloc(ctx, s->dx, sizeof(double) * (size_t)s->P))) return rc;
+  if (s->mode != FH_AB_BLOCKED) return FH_OK;
+  if (!s->tab2.p && (rc = fh_alloc(ctx, s->tab2, sizeof(float2) * 3 * (size_t)s->P))) return rc;
+  if (!s->w2.p) {
+    if ((rc = fh_alloc(ctx, s->w2, sizeof(float2) * (size_t)(s->max_steps + 2)))) return rc;
+    if ((rc = ab_pairs(ctx, s->w.as<double>(), s->w2.as<float2>(), s->max_steps + 2, 0))) return rc;
+  }
+  if ((rc = ab_table_pairs(s))) return rc;
+  return ab_src_pairs(s);
 }
 
 extern "C" {
@@ -745,7 +869,7 @@ int fh_ab_create(fh_ctx *ctx, int m, int max_steps, double tau, double alpha, fh
   int rc;
   const size_t fld = sizeof(double) * (size_t)s->P;
   if ((rc = fh_alloc(ctx, s->w, sizeof(double) * (size_t)(max_steps + 2))) || (rc = fh_alloc(ctx, s->ii, 16)) ||
-      (rc = fh_alloc(ctx, s->al, fld)) || (rc = fh_alloc(ctx, s->den, fld)) || (rc = fh_alloc(ctx, s->inv, fld)) ||
+      (rc = fh_alloc(ctx, s->al, fld)) || (rc = fh_alloc(ctx, s->nal, fld)) || (rc = fh_alloc(ctx, s->den, fld)) || (rc = fh_alloc(ctx, s->inv, fld)) ||
       (rc = fh_alloc(ctx, s->sl, fld)) || (rc = fh_alloc(ctx, s->pf, fld)) || (rc = fh_alloc(ctx, s->pb, fld)) ||
       (rc = fh_alloc(ctx, s->C, fld)) ||
       (rc = fh_alloc(ctx, s->D, fld * (size_t)max_steps)) ||
@@ -765,10 +889,10 @@ int fh_ab_create(fh_ctx *ctx, int m, int max_steps, double tau, double alpha, fh
   FH_CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));
   s->Ii = ii_h;
   s->Bd = (ii_h / (1.0 - alpha)) + (2.0 / (h * h));
-  k_ab_factor<<<1, 1, 0, ctx->stream>>>(m, s->A, s->Bd, s->Cc, s->al.as<double>(), s->den.as<double>(),
+  k_ab_factor<<<1, kAbSolveThreads, 0, ctx->stream>>>(m, s->A, s->Bd, s->Cc, s->al.as<double>(), s->den.as<double>(),
                                         s->inv.as<double>(), s->sl.as<double>(), s->pf.as<double>(),
-                                        s->pb.as<double>());
-  if ((rc = fh_after_launch(ctx, "k_ab_factor"))) {
+                                        s->pb.as<double>(), s->nal.as<double>());
+  if ((rc = fh_after_launch(ctx, "k_ab_factor")) || (rc = ab_res_setup(s))) {
     delete s;
     return rc;
   }
@@ -833,9 +957,9 @@ int fh_ab_set_current_coef(fh_ab_solver *s, double Ii) {
   const double h = 1.0 / s->m;
   s->Ii = Ii;
   s->Bd = (Ii / (1.0 - s->alpha)) + (2.0 / (h * h));
-  k_ab_factor<<<1, 1, 0, ctx->stream>>>(s->m, s->A, s->Bd, s->Cc, s->al.as<double>(), s->den.as<double>(),
+  k_ab_factor<<<1, kAbSolveThreads, 0, ctx->stream>>>(s->m, s->A, s->Bd, s->Cc, s->al.as<double>(), s->den.as<double>(),
                                         s->inv.as<double>(), s->sl.as<double>(), s->pf.as<double>(),
-                                        s->pb.as<double>());
+                                        s->pb.as<double>(), s->nal.as<double>());
   s->graph.reset();  // the coefficient is an argument of the captured launches
   const int rc = fh_after_launch(ctx, "k_ab_factor");
   return rc ? rc : ab_table_pairs(s);
@@ -882,21 +1006,7 @@ int fh_ab_set_mode(fh_ab_solver *s, int mode) {
     fh_blk_delete(s->blk);
     s->blk = nullptr;
   }
-  s->resident = mode == FH_AB_BLOCKED &&
-                ab_res_pick(s->m, [&](auto nw, auto em) { return ab_res_ok<fh_ab_df, nw(), em()>(s->m); });
-  if (s->resident) {
-    int rc;
-    if (!s->tab2.p && (rc = fh_alloc(ctx, s->tab2, sizeof(float2) * 3 * (size_t)s->P))) return rc;
-    if (!s->derr.p && (rc = fh_alloc(ctx, s->derr, sizeof(int)))) return rc;
-    if (!s->dx.p && (rc = fh_alloc(ctx, s->dx, sizeof(float2) * (size_t)s->P))) return rc;
-    if (!s->w2.p) {
-      if ((rc = fh_alloc(ctx, s->w2, sizeof(float2) * (size_t)(s->max_steps + 2)))) return rc;
-      if ((rc = ab_pairs(ctx, s->w.as<double>(), s->w2.as<float2>(), s->max_steps + 2, 0))) return rc;
-    }
-    if ((rc = ab_table_pairs(s)) || (rc = ab_src_pairs(s))) return rc;
-  }
-  s->graph.reset();
-  return FH_OK;
+  return ab_res_setup(s);
 }
 
 int fh_ab_step(fh_ab_solver *s, int nsteps) {
@@ -914,6 +1024,7 @@ int fh_ab_step(fh_ab_solver *s, int nsteps) {
     });
     if (rc) return rc;
     s->step = nsteps;
+    s->T0 = s->blk || s->f64 ? ((nsteps - 1) / ab_block(s)) * ab_block(s) : 0;  // where the replayed steps left it
     return FH_OK;
   }
   for (int n = 0, d = 1; n < nsteps; n += d) {
@@ -932,7 +1043,7 @@ int fh_ab_get_c_host(fh_ab_solver *s, double *C_host) {
   if (s->derr.p) FH_CUDA_TRY(ctx, cudaMemcpyAsync(&err, s->derr.p, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
   FH_CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));
   FH_REQUIRE(ctx, err == 0, FH_ETIMEOUT, "fh_ab_step: a wait of the resident solve ran out");
-  return FH_OK;
+  return s->f64 ? fh_far64_check(ctx, *s->f64) : (int)FH_OK;
 }
 
 }  // extern "C"

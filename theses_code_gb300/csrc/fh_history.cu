@@ -23,7 +23,8 @@ static constexpr int kHistStage = 2048;
 template <int M>
 __global__ void __launch_bounds__(kHistThreads) k_hist_sum(const double *__restrict__ D, long long ldd, long long P,
                                                            int K, const double *__restrict__ W, int ldw, int kchunk,
-                                                           double *__restrict__ part, long long ldpart) {
+                                                           double *__restrict__ part, long long ldpart,
+                                                           const double *__restrict__ far, long long ldfar) {
   extern __shared__ double ws[];  // [M][min(kchunk, kHistStage)]
   const int s = blockIdx.y;
   const int k0 = s * kchunk;
@@ -33,7 +34,14 @@ __global__ void __launch_bounds__(kHistThreads) k_hist_sum(const double *__restr
   const bool live = p < P;
   double acc0[M], acc1[M];
 #pragma unroll
-  for (int m = 0; m < M; ++m) acc0[m] = acc1[m] = 0.0;
+  for (int m = 0; m < M; ++m) {
+    acc0[m] = acc1[m] = 0.0;
+    if (far && s == 0 && live) {  // split 0 starts from the older layers' row m
+      const double2 f = *reinterpret_cast<const double2 *>(far + (long long)m * ldfar + p);
+      acc0[m] = f.x;
+      acc1[m] = f.y;
+    }
+  }
   const double *d = D + (long long)k0 * ldd + (live ? p : 0);
   for (int kb = 0; kb < nk; kb += ldws) {
     const int ns = min(ldws, nk - kb);
@@ -287,16 +295,17 @@ void fh_hist_plan(long long P, int K, int max_splits, int *splits, int *kchunk) 
 }
 
 int fh_launch_hist_sum_partials(fh_ctx *ctx, int M, int K, long long P, const double *W, int ldw, const double *D,
-                                long long ldd, int splits, int kchunk, double *part, long long ldpart) {
+                                long long ldd, int splits, int kchunk, double *part, long long ldpart,
+                                const double *far, long long ldfar) {
   if (K <= 0 || P <= 0) return FH_OK;
   dim3 grid((unsigned)fh_ceil_div(P, 2LL * kHistThreads), (unsigned)splits);
   FH_REQUIRE(ctx, kchunk >= 1, FH_EINVAL, "history chunk of %d layers", kchunk);
   const size_t smem = sizeof(double) * (size_t)M * (size_t)(kchunk < kHistStage ? kchunk : kHistStage);
   fh_prof_mark(ctx, FH_PROF_HISTORY, false);
   if (M == 1)
-    k_hist_sum<1><<<grid, kHistThreads, smem, ctx->stream>>>(D, ldd, P, K, W, ldw, kchunk, part, ldpart);
+    k_hist_sum<1><<<grid, kHistThreads, smem, ctx->stream>>>(D, ldd, P, K, W, ldw, kchunk, part, ldpart, far, ldfar);
   else
-    k_hist_sum<2><<<grid, kHistThreads, smem, ctx->stream>>>(D, ldd, P, K, W, ldw, kchunk, part, ldpart);
+    k_hist_sum<2><<<grid, kHistThreads, smem, ctx->stream>>>(D, ldd, P, K, W, ldw, kchunk, part, ldpart, far, ldfar);
   fh_prof_mark(ctx, FH_PROF_HISTORY, true);
   return fh_after_launch(ctx, "k_hist_sum");
 }

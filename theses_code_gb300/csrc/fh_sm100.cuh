@@ -66,6 +66,14 @@ __device__ __forceinline__ void fh_tma_load_3d(uint32_t dst, const CUtensorMap *
       : "memory");
 }
 
+// Bulk copy of `bytes` (16-byte aligned addresses and size) into shared memory,
+// completion counted on `bar`.
+__device__ __forceinline__ void fh_bulk_load(uint32_t dst, const void *src, uint32_t bytes, uint32_t bar) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
+               "l"(reinterpret_cast<uint64_t>(src)), "r"(bytes), "r"(bar)
+               : "memory");
+}
+
 // ---------------------------------------------------------------- tcgen05
 __device__ __forceinline__ void fh_tmem_alloc(uint32_t dst_smem, uint32_t ncols) {
   asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(dst_smem), "r"(ncols)

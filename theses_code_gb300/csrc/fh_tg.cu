@@ -6,8 +6,10 @@
 //                     weights (a per-solve table when it fits, else per step)
 //   2. history sum    S_x, S_y over the stored full-step differences, one pass
 //                     (the reference reads the layers once per half step);
-//                     in blocked mode only the layers of the current 64-step
-//                     block, the older ones come from the tensor-core rows
+//                     only over the layers of the current block where the older
+//                     ones come from tensor-core rows: blocks of 64 steps and
+//                     four digits in blocked mode (fh_blocked.cu), of 32 steps
+//                     and FP64 accuracy in the other two (fh_far64.cu)
 //   3. k_tg_xsweep    one CTA per x line (j = 1..M-1), unknowns along i; writes
 //                     the half-step field Ch
 //   4. k_tg_ysweep    four y lines per CTA (i = 1..sN-1), unknowns along j;
@@ -34,6 +36,7 @@
 #include "fh_slices.cuh"
 #include "fh_weights.cuh"
 #include "fh_two_series.h"
+#include "fh_far64.h"
 
 // blocked contraction helpers (fh_blocked.cu)
 struct fh_blk;
@@ -99,6 +102,9 @@ struct fh_tg_solver {
   fh_dbuf mws, mwe;
   bool wtab = false;      // Wall/cwall hold every step's weights (computed at step 0)
   fh_blk *blk = nullptr;  // blocked mode: bf16 slice planes and tensor maps
+  // FP64 and DF64 modes: the layers before the current 32-step block at FP64
+  // accuracy on the tensor cores (null: every layer summed every step)
+  fh_far64 *f64 = nullptr;
   int j0 = 0;             // first step of the current block (far rows valid when j0 > 0)
   long long ldfar = 0;
   fh_graph_cache graph;
@@ -122,6 +128,7 @@ struct fh_tg_solver {
   ~fh_tg_solver() {
     if (two) fh_ta_delete(two);
     if (blk) fh_blk_delete(blk);
+    if (f64) fh_far64_delete(f64);
   }
 };
 
@@ -1890,9 +1897,21 @@ static int tg_one_step(fh_tg_solver *s, int max_n, int *done) {
     if ((rc = fh_blk_gemm(ctx, *s->blk, j, s->far.as<float2>(), s->ldfar, gbeg))) return rc;
     s->j0 = j;
   }
+  if (s->f64 && j > 0 && j % kF64Block == 0) {
+    // new block: the layers [j - 32, j) join the exponents, then the rows of
+    // steps j .. j + 31 over every layer so far
+    const int nrows = 2 * std::min(kF64Block, s->max_steps - j);
+    fh_prof_mark(ctx, FH_PROF_WEIGHTS, false);
+    if ((rc = fh_far64_append(ctx, *s->f64, s->D.p, g.P, j - kF64Block)) ||
+        (rc = fh_far64_weights(ctx, *s->f64, j, s->W.as<double>() + (long long)j * 2 * ldw, 2LL * ldw, ldw, nrows)))
+      return rc;
+    fh_prof_mark(ctx, FH_PROF_WEIGHTS, true);
+    if ((rc = fh_far64_run(ctx, *s->f64, s->D.p, g.P, j))) return rc;
+    s->j0 = j;
+  }
   // history layers summed in FP64 this step: the current block in blocked
-  // mode; with restricted summing and psi = t, the layers within the cut lag
-  int kstart = blocked ? s->j0 : 0;
+  // mode and where the older layers are contracted; with restricted summing and psi = t, the layers within the cut lag
+  int kstart = blocked || s->f64 ? s->j0 : 0;
   if (!blocked && s->rs_lag >= 0 && j > s->rs_lag) kstart = j - s->rs_lag;
   if (s->one_layer()) kstart = j;  // series expansions: no layer sums
   const int knear = j - kstart;
@@ -1924,9 +1943,19 @@ static int tg_one_step(fh_tg_solver *s, int max_n, int *done) {
   if (!s->factor_fixed || j == 0)
     if ((rc = tg_factor(s, cwj))) return rc;
   if (s->dfsweep) return tg_step_df(s, Wj, cwj, max_n, done);
-  // far-history rows of this step ((hi, lo) pairs, x row 2r, y row 2r+1)
+  // far-history rows of this step (x row 2r, y row 2r + 1): (hi, lo) pairs in
+  // the DF64 mode, FP64 in the FP64 mode
   const float2 *far = nullptr;
-  if (blocked && s->j0 > 0) far = s->far.as<float2>() + 2LL * (j - s->j0) * s->ldfar;
+  const double *far64 = nullptr;
+  long long ldfar = 0;
+  if (s->f64 && s->j0 > 0) {
+    ldfar = fh_far64_pitch(*s->f64);
+    const long long o = 2LL * (j - s->j0) * ldfar;
+    if (s->df)
+      far = static_cast<const float2 *>(fh_far64_rows(*s->f64)) + o;
+    else
+      far64 = static_cast<const double *>(fh_far64_rows(*s->f64)) + o;
+  }
   int splits = 0, kchunk = 0;
   if (s->ser_J && j >= 1) {
     fh_prof_mark(ctx, FH_PROF_HISTORY, false);
@@ -1951,18 +1980,25 @@ static int tg_one_step(fh_tg_solver *s, int max_n, int *done) {
     if (s->df)
       rc = fh_launch_hist_sum_df_partials(ctx, 2, knear, g.P, Wj + kstart, ldw,
                                           reinterpret_cast<const float2 *>(s->D.as<double>()) + (long long)kstart * g.P,
-                                          g.P, splits, kchunk, s->part.as<double>(), g.P, far, s->ldfar, 0);
+                                          g.P, splits, kchunk, s->part.as<double>(), g.P, far, ldfar, 0);
     else
       rc = fh_launch_hist_sum_partials(ctx, 2, knear, g.P, Wj + kstart, ldw,
                                        s->D.as<double>() + (long long)kstart * g.P, g.P, splits, kchunk,
-                                       s->part.as<double>(), g.P);
+                                       s->part.as<double>(), g.P, far64, ldfar);
     if (rc) return rc;
   }
   // the near kernel has folded the far rows in; otherwise the sweeps add them
   const float2 *farx = nullptr, *fary = nullptr;
   if (far && !(knear >= 1 && s->df)) {
     farx = far;
-    fary = far + s->ldfar;
+    fary = far + ldfar;
+  }
+  const double *sums = s->part.as<double>();
+  long long ldsums = g.P;
+  if (far64 && knear < 1) {  // a block's first step: its far rows are the sums
+    sums = far64;
+    ldsums = ldfar;
+    splits = 1;
   }
   fh_prof_mark(ctx, FH_PROF_SWEEP, false);
   auto n1 = [&](int half) {
@@ -1976,14 +2012,14 @@ static int tg_one_step(fh_tg_solver *s, int max_n, int *done) {
   if (s->massN && (rc = n1(0))) return rc;
   const size_t smx = sizeof(double) * kXLines * 5 * (size_t)tg_line_stride(g.sN);
   k_tg_xsweep<<<(unsigned)fh_ceil_div(g.M - 1, kXLines), kXThreads, smx, ctx->stream>>>(
-      g, s->C.as<double>(), s->Ch.as<double>(), s->part.as<double>(), g.P, splits, s->fax.as<double>(),
+      g, s->C.as<double>(), s->Ch.as<double>(), sums, ldsums, splits, s->fax.as<double>(),
       s->gx.as<double>(), s->alx.as<double>(), s->pfx.as<double>(), s->pbx.as<double>(), cwj, farx, dNp);
   if ((rc = fh_after_launch(ctx, "k_tg_xsweep"))) return rc;
   if (s->massN && (rc = n1(1))) return rc;
   const size_t smy = sizeof(double) * 4 * 6 * (size_t)tg_line_stride(g.M);
   k_tg_ysweep<<<(unsigned)fh_ceil_div(g.sN - 1, 4), kYThreads, smy, ctx->stream>>>(
       g, s->C.as<double>(), s->Ch.as<double>(), s->D.as<double>() + (s->one_layer() ? 0LL : (long long)j * g.P),
-      s->part.as<double>(), g.P,
+      sums, ldsums,
       splits, s->fay.as<double>(), s->gy.as<double>(), s->aly.as<double>(), s->pfy.as<double>(),
       s->pby.as<double>(), cwj, fary, s->df ? 1 : 0, dNp);
   fh_prof_mark(ctx, FH_PROF_SWEEP, true);
@@ -2035,6 +2071,26 @@ static int tg_set_smem_attrs(fh_ctx *ctx, int sN, int M) {
     cur_y[ctx->device] = smy;
   }
   return FH_OK;
+}
+
+// Rows of the layers before a block on the tensor cores, where a step's sums
+// run over every stored layer with tabulated weights: pays from the second
+// block on (256 x 192 points, 500 steps, FP64: history 49 -> ~9 us per step).
+// Without memory for its tables (64 rows of the field) every step sums every
+// layer, as the other configurations do.
+static void tg_far64_setup(fh_tg_solver *s) {
+  const bool want = s->mode != FH_TG_BLOCKED && s->wtab && s->max_steps > kF64Block && s->dv.hcut == 0.0 && !s->one_layer();
+  if (want == (s->f64 != nullptr)) return;
+  s->graph.reset();
+  if (want) {
+    if (fh_far64_create(s->ctx, s->dv.P, (int)fh_ceil_div(s->max_steps, kF64Block) * kF64Block, s->df, &s->f64)) {
+      s->f64 = nullptr;
+      cudaGetLastError();
+    }
+  } else {
+    fh_far64_delete(s->f64);
+    s->f64 = nullptr;
+  }
 }
 
 extern "C" {
@@ -2156,6 +2212,7 @@ int fh_tg_create(fh_ctx *ctx, const fh_tg_params *p, int max_steps, int mode, fh
       return rc;
     }
   }
+  tg_far64_setup(s);
   *out = s;
   return FH_OK;
 }
@@ -2193,6 +2250,8 @@ int fh_tg_set_restricted(fh_tg_solver *s, double dt_eps) {
       }
   }
   s->graph.reset();
+  FH_CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));
+  tg_far64_setup(s);
   return FH_OK;
 }
 
@@ -2222,6 +2281,7 @@ int fh_tg_set_series(fh_tg_solver *s, int nterms) {
     s->H.release();
     s->ser_tab.release();
     s->ser_J = 0;
+    tg_far64_setup(s);
     return FH_OK;
   }
   // coefficient rows of every step j >= 1 (fr_d_t_g_2d.cpp _kb_row2 2965-3040
@@ -2265,6 +2325,7 @@ int fh_tg_set_series(fh_tg_solver *s, int nterms) {
   adopt(s->H, nH);
   adopt(s->ser_tab, ntab);
   s->ser_J = J;
+  tg_far64_setup(s);
   return FH_OK;
 }
 
@@ -2290,6 +2351,7 @@ int fh_tg_set_two_series(fh_tg_solver *s, int enable) {
   if (s->two) fh_ta_delete(s->two);
   s->two = t;
   s->graph.reset();
+  tg_far64_setup(s);
   return FH_OK;
 }
 
@@ -2391,7 +2453,9 @@ int fh_tg_step(fh_tg_solver *s, int nsteps) {
     });
     if (rc) return rc;
     s->tstep = nsteps;
-    s->j0 = (s->blk && nsteps > kTgBlock) ? ((nsteps - 1) / kTgBlock) * kTgBlock : 0;
+    s->j0 = s->blk && nsteps > kTgBlock ? ((nsteps - 1) / kTgBlock) * kTgBlock
+            : s->f64                    ? ((nsteps - 1) / kF64Block) * kF64Block
+                                        : 0;
     return FH_OK;
   }
   for (int n = 0, d = 1; n < nsteps; n += d) {
@@ -2424,7 +2488,7 @@ int fh_tg_get_c_host(fh_tg_solver *s, double *C_host) {
     FH_CUDA_TRY(ctx, cudaMemcpy(&h, s->derr.p, sizeof(int), cudaMemcpyDeviceToHost));
     if (h) return fh_set_error(ctx, FH_ETIMEOUT, "a bounded device wait expired (fused sweeps or mid rows)");
   }
-  return FH_OK;
+  return s->f64 ? fh_far64_check(ctx, *s->f64) : (int)FH_OK;
 }
 
 long long fh_tg_device_bytes(const fh_tg_solver *s) {
@@ -2437,6 +2501,7 @@ long long fh_tg_device_bytes(const fh_tg_solver *s) {
   size_t n = 0;
   for (const fh_dbuf *d : bufs) n += d->bytes;
   if (s->blk) n += fh_blk_bytes(*s->blk);
+  if (s->f64) n += fh_far64_bytes(*s->f64);
   if (s->two) n += fh_ta_bytes(s->two);
   return (long long)n;
 }
