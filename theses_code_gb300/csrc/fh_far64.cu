@@ -27,15 +27,19 @@
 // 256): per pair of layers and digit one byte permute, two logical operations
 // and one packed subtraction.
 //
-// One CTA of 256 threads per 128 points (and K split when there are few
+// One CTA of 512 threads per 128 points (and K split when there are few
 // points).  A = 128 points x 64 layers in seven K-major planes which the CTA
 // cuts itself from the stored layers, half (32 layers) by half, so that the
 // MMAs of one half run while the next is cut; B = the 64-layer image of the
 // weight digits, 7 digits x 32 rows stacked per row group, copied in bulk two
 // chunks ahead.  The MMA of data digit ia takes the first 7 - ia weight digits
 // (N = 32 (7 - ia)) and writes TMEM columns from 32 ia of its row group: the
-// product (ia, ib) lands on level ia + ib.  Thread t cuts point t & 127 and
-// holds in the epilogue the sums of that point for the 32 rows of group t >> 7.
+// product (ia, ib) lands on level ia + ib.  Thread t cuts eight layers of point
+// t & 127 and holds in the epilogue the sums of that point for 16 rows.  The
+// cutting (~45 instructions per value) and the sums (~60 per row, point and
+// group) take about as long as the MMAs; sixteen warps keep both going (eight,
+// with twice the registers: 77k cycles per tile of 256 layers at 0.31
+// instructions per cycle and scheduler).
 // Waits are bounded; on expiry *err is set and nothing is stored.
 //
 // Measured, whole solves: 2D 251 x 187, 500 steps, FP64 34.9 -> 14.3 ms (the
@@ -56,7 +60,9 @@
 namespace {
 constexpr int kSl = 7;                         // digits per value
 constexpr int kPts = 128;                      // points per CTA
-constexpr int kThr = 256;
+constexpr int kThr = 512;
+constexpr int kLay = 32 * kPts / kThr;         // layers of a half a thread cuts
+constexpr int kRows = kF64Rows * kPts / kThr;  // rows a thread sums
 constexpr int kGroup = 128;                    // layers of a group (one exponent)
 constexpr uint32_t kPlane = kPts * 128;        // one digit of 128 points x 64 layers
 constexpr uint32_t kABytes = kSl * kPlane;
@@ -67,6 +73,7 @@ constexpr uint32_t kBBytes = 2 * kBGroup;      // a chunk's weight image (56 KiB
 constexpr uint32_t kLevCols = kSl * kBRows;    // TMEM columns of a row group
 constexpr size_t kSmem = 1024 + kABytes + 2 * kBBytes + 64;
 constexpr int kNonFinite = 0x7ff;
+static_assert(kLay == 8 && kRows == 16, "one 16-byte digit store per thread and half, two threads per row group");
 }  // namespace
 
 // ------------------------------------------------------------------ digits
@@ -213,6 +220,8 @@ __global__ void __launch_bounds__(kThr, 1)
   const int pt = tid & 127, q = tid >> 7;
   const long long p = (long long)blockIdx.x * kPts + pt;
   const bool live = p < P;
+  // the thread's rows: [16 q, 16 q + 16), columns of their row group
+  const uint32_t rcol = (uint32_t)(q >> 1) * kLevCols + (uint32_t)(q & 1) * kRows;
   const int ng = (K + kGroup - 1) / kGroup;
   const int G0 = min(ng, (int)blockIdx.y * gps), G1 = min(ng, G0 + gps);
   const int h0 = 4 * G0, h1 = min(K / 32, 4 * G1);  // halves: 32 layers each
@@ -229,11 +238,11 @@ __global__ void __launch_bounds__(kThr, 1)
     fh_tmem_alloc(tslot, 512);
     fh_tmem_relinquish();
   }
-  // largest exponents of the point and (lane = row of the thread's row group) of the row
+  // largest exponents of the point and of row 16 q + lane % 16
   int eb = 1, wb = 1;
   bool bad = false;
   for (int g = G0; g < G1; ++g) {
-    const int e = live ? ed[(long long)g * lde + p] : 0, w = ew[(long long)g * kF64Rows + 32 * q + lane];
+    const int e = live ? ed[(long long)g * lde + p] : 0, w = ew[(long long)g * kF64Rows + kRows * q + lane % kRows];
     bad |= e == kNonFinite;
     eb = max(eb, e);
     wb = max(wb, w);
@@ -251,29 +260,29 @@ __global__ void __launch_bounds__(kThr, 1)
   };
   if (tid == 0)
     for (int c = 2 * G0; c < min(c1, 2 * G0 + 2); ++c) load_b(c);
-  // the thread's 16 layers of a half: [16 q, 16 q + 16)
-  S v[16];
+  // the thread's layers of a half: [8 q, 8 q + 8)
+  S v[kLay];
   auto load_v = [&](int h) {
-    const S *d = D + (long long)(32 * h + 16 * q) * ldd + (live ? p : 0);
+    const S *d = D + (long long)(32 * h + kLay * q) * ldd + (live ? p : 0);
 #pragma unroll
-    for (int i = 0; i < 16; ++i) v[i] = __ldcs(d + i * ldd);
+    for (int i = 0; i < kLay; ++i) v[i] = __ldcs(d + i * ldd);
   };
-  float s0[kBRows], s1[kBRows], s2[kBRows];
+  float s0[kRows], s1[kRows], s2[kRows];
 #pragma unroll
-  for (int n = 0; n < (int)kBRows; ++n) s0[n] = s1[n] = s2[n] = 0.f;
+  for (int n = 0; n < kRows; ++n) s0[n] = s1[n] = s2[n] = 0.f;
   // level sums of group G into the running sums
   auto epilogue = [&](int G) {
     const int e = (live ? (int)ed[(long long)G * lde + p] : 0) - eb;
-    const int w = ew[(long long)G * kF64Rows + 32 * q + lane] - wb;
-    const uint32_t cols = tmem + ((uint32_t)(32 * (warp & 3)) << 16) + (uint32_t)q * kLevCols;
+    const int w = ew[(long long)G * kF64Rows + kRows * q + lane % kRows] - wb;
+    const uint32_t cols = tmem + ((uint32_t)(32 * (warp & 3)) << 16) + rcol;
 #pragma unroll
-    for (int nb = 0; nb < (int)kBRows; nb += 8) {
-      float L[kSl][8];
+    for (int nb = 0; nb < kRows; nb += 4) {
+      float L[kSl][4];
 #pragma unroll
-      for (int l = 0; l < kSl; ++l) fh_tmem_ld8(cols + (uint32_t)(kBRows * l + nb), L[l]);
+      for (int l = 0; l < kSl; ++l) fh_tmem_ld4(cols + (uint32_t)(kBRows * l + nb), L[l]);
       fh_tmem_wait_ld();
 #pragma unroll
-      for (int i = 0; i < 8; ++i) {
+      for (int i = 0; i < 4; ++i) {
         const float sc = fh_exp2i(e + __shfl_sync(0xffffffffu, w, nb + i));
         float h, e1, m, e2, u, e3, a, b, c;
         f64_two_sum(L[0][i], L[1][i] * 0x1p-8f, h, e1);
@@ -297,12 +306,11 @@ __global__ void __launch_bounds__(kThr, 1)
     if (tid == 0 && slot == 1 && i >= 2 && (h >> 1) + 1 < c1) load_b((h >> 1) + 1);
     const int emax = live ? max((int)ed[(long long)(h >> 2) * lde + p], 1) : 1;
     const bool cut = live && emax != kNonFinite;
+    {
+      unsigned long long w[kLay];
 #pragma unroll
-    for (int o = 0; o < 2; ++o) {
-      unsigned long long w[8];
-#pragma unroll
-      for (int j = 0; j < 8; ++j) w[j] = cut ? f64_word(v[8 * o + j], emax) : 0x8080808080808080ull;
-      const uint32_t off = fh_sw128_off(pt, 32 * slot + 16 * q + 8 * o);
+      for (int j = 0; j < kLay; ++j) w[j] = cut ? f64_word(v[j], emax) : 0x8080808080808080ull;
+      const uint32_t off = fh_sw128_off(pt, 32 * slot + kLay * q);
 #pragma unroll
       for (int d = 0; d < kSl; ++d)
         *reinterpret_cast<uint4 *>(gA + d * kPlane + off) =
@@ -352,9 +360,9 @@ __global__ void __launch_bounds__(kThr, 1)
     if (last_i >= 0) fh_mbar_wait(mdone + 8 * (last_i & 1), (last_i >> 1) & 1);
   }
   if (ok) {
-    S *o = out + (long long)(32 * q) * ldo + p;
+    S *o = out + (long long)(kRows * q) * ldo + p;
 #pragma unroll
-    for (int n = 0; n < (int)kBRows; ++n) {
+    for (int n = 0; n < kRows; ++n) {
       const int w = __shfl_sync(0xffffffffu, wb, n);
       // unit of digit 0: 2^(exponent - 1028) each
       if (live) f64_store(o + n * ldo, s0[n], s1[n], s2[n], eb + w - 2 * 1028, bad || w == kNonFinite);

@@ -117,6 +117,15 @@ __device__ __forceinline__ void fh_tmem_ld16(uint32_t taddr, float (&v)[16]) {
 #pragma unroll
   for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
 }
+// 4 consecutive 32-bit columns of this thread's TMEM lane.
+__device__ __forceinline__ void fh_tmem_ld4(uint32_t taddr, float (&v)[4]) {
+  uint32_t r[4];
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"(taddr));
+#pragma unroll
+  for (int i = 0; i < 4; ++i) v[i] = __uint_as_float(r[i]);
+}
 // 8 consecutive 32-bit columns of this thread's TMEM lane.
 __device__ __forceinline__ void fh_tmem_ld8(uint32_t taddr, float (&v)[8]) {
   uint32_t r[8];
