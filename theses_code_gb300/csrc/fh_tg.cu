@@ -1255,8 +1255,9 @@ extern "C" int fh_tg_stamps_read(long long *h) {
 // Exclusive scan of the chunk maps of one line's 128 threads (four warps,
 // named barrier `bar`, warp totals in sm[4]): forward, thread t receives
 // f_{t-1} o ... o f_0; reverse, G_{t+1} o ... o G_127.
+// Only the group's first aw warps take part (the others hold no equations).
 template <bool REV>
-__device__ __forceinline__ fh_daff tg_group_scan(fh_daff f, fh_daff *sm, int bar, int w4) {
+__device__ __forceinline__ fh_daff tg_group_scan(fh_daff f, fh_daff *sm, int bar, int w4, int aw) {
   const unsigned lane = threadIdx.x & 31u;
   fh_daff g = f;
 #pragma unroll
@@ -1280,13 +1281,14 @@ __device__ __forceinline__ fh_daff tg_group_scan(fh_daff f, fh_daff *sm, int bar
     e = fh_daff{fh_df_shfl_down(g.a, 1), fh_df_shfl_down(g.b, 1)};
     if (lane == 31u) e = id;
   }
-  fh_group_bar(bar, kFuseGroup);
+  if (aw == 1) return e;
+  fh_group_bar(bar, 32 * aw);
   fh_daff P = id;
   if (!REV)
     for (int k = 0; k < w4; ++k) P = fh_daff_compose(sm[k], P);
   else
-    for (int k = 3; k > w4; --k) P = fh_daff_compose(sm[k], P);
-  fh_group_bar(bar, kFuseGroup);  // sm may be reused after this
+    for (int k = aw - 1; k > w4; --k) P = fh_daff_compose(sm[k], P);
+  fh_group_bar(bar, 32 * aw);  // sm may be reused after this
   return fh_daff_compose(e, P);
 }
 
@@ -1296,9 +1298,13 @@ __device__ __forceinline__ fh_daff tg_group_scan(fh_daff f, fh_daff *sm, int bar
 // bt_{N-1} / (1 - al_{N-1}).  Each thread walks its four equations from zero
 // (keeping the prefix slope products), the chunk maps are scanned across the
 // group, and the start value finishes each chunk.  fb (solve layout) is
-// replaced by u; ub receives u_0 and u_N.
+// replaced by u; ub receives u_0 and u_N.  Called by the group's first aw
+// warps, those that hold equations (the maps of the others would be identities,
+// which change no bit): on short lines a quarter of the warps issues a quarter
+// of the instructions.
 __device__ __forceinline__ void tg_group_solve(int N, const float2 *fa, const float2 *al, float2 *xch, float2 *ub,
-                                               fh_df al1, fh_df bt1, fh_daff *sm, fh_df *uNs, int bar, int t, int w4) {
+                                               fh_df al1, fh_df bt1, fh_daff *sm, fh_df *uNs, int bar, int t, int w4,
+                                               int aw) {
   const fh_df one{1.f, 0.f}, zero{0.f, 0.f};
   fh_df B[kFuseEq], P[kFuseEq];
   fh_df b = zero, p = one;
@@ -1314,7 +1320,7 @@ __device__ __forceinline__ void tg_group_solve(int N, const float2 *fa, const fl
     B[e] = b;
     P[e] = p;
   }
-  const fh_daff Pf = tg_group_scan<false>(fh_daff{p, b}, sm, bar, w4);
+  const fh_daff Pf = tg_group_scan<false>(fh_daff{p, b}, sm, bar, w4, aw);
   const fh_df s = fh_df_fma(Pf.a, bt1, Pf.b);  // bt at equation 4t (bt1 for t = 0)
   fh_df bt[kFuseEq];
 #pragma unroll
@@ -1327,7 +1333,7 @@ __device__ __forceinline__ void tg_group_solve(int N, const float2 *fa, const fl
       *uNs = fh_df_div(bt[e], fh_df_sub(one, aN));
     }
   }
-  fh_group_bar(bar, kFuseGroup);
+  fh_group_bar(bar, 32 * aw);
   const fh_df uN = *uNs;
   fh_df V[kFuseEq], Q[kFuseEq];
   fh_df v = zero, q = one;
@@ -1342,7 +1348,7 @@ __device__ __forceinline__ void tg_group_solve(int N, const float2 *fa, const fl
     V[e] = v;
     Q[e] = q;
   }
-  const fh_daff Pb = tg_group_scan<true>(fh_daff{q, v}, sm, bar, w4);
+  const fh_daff Pb = tg_group_scan<true>(fh_daff{q, v}, sm, bar, w4, aw);
   const fh_df u1 = fh_df_fma(Pb.a, uN, Pb.b);  // u at equation 4t + 5 (u_N past the last chunk)
 #pragma unroll
   for (int e = 0; e < kFuseEq; ++e) {
@@ -1456,6 +1462,10 @@ __global__ void __launch_bounds__(kFuseThreads, 1) k_tg_sweeps_fused(const tg_fu
   auto yid = [&](int k) { return (long long)(line0 + yc) + (long long)yq(k) * g.ld; };
   // solve mapping
   const int grp = tid / kFuseGroup, gt = tid % kFuseGroup, w4 = gt >> 5;
+  const int awx = (Nx - 1 + 127) / 128, awy = (Ny - 1 + 127) / 128;  // warps of a group with equations
+  // warps with x nodes, node slots k with y rows: the others skip the sums
+  const bool wx_live = (tid & ~31) + 1 < Nx;
+  const int yk = min(kFuseLines, (Ny - 1 + 127) / 128);
   const float2 *tiny = a.D + (long long)a.j8 * g.P;  // layers of the sub-block
   const unsigned nblk = gridDim.x;
   unsigned nb = 0;
@@ -1526,22 +1536,25 @@ __global__ void __launch_bounds__(kFuseThreads, 1) k_tg_sweeps_fused(const tg_fu
       if (t < s) {
         const fh_df w = fh_df_from_pair(wy[s][t]);
 #pragma unroll
-        for (int k = 0; k < kFuseLines; ++k) tsy[k] = fh_df_fma(w, fh_df_from_pair(d[t][k]), tsy[k]);
+        for (int k = 0; k < kFuseLines; ++k)
+          if (k < yk) tsy[k] = fh_df_fma(w, fh_df_from_pair(d[t][k]), tsy[k]);
       }
   };
 #pragma unroll
   for (int k = 0; k < kFuseLines; ++k) f[k] = ylive(k) ? __ldcg(a.Cd + yid(k)) : make_float2(0.f, 0.f);
   {
     float2 r[kFuseLines], d[kSub - 1][kFuseLines];
-    x_load(a.s0, r, d);
-    x_sum(a.s0, r, d);
+    if (wx_live) {
+      x_load(a.s0, r, d);
+      x_sum(a.s0, r, d);
+    }
   }
 
   for (int s = a.s0; s < a.s0 + a.ns; ++s) {
     const int j = a.j8 + s;
     TG_STAMP(0);
     // ---- x half step (fr_d_t_g_2d.cpp:2577-2590): field and newest layer
-    {
+    if (wx_live) {
       const fh_df kst = fh_df_from_pair(cx[s][0]), S2 = fh_df_from_pair(cx[s][1]), st = fh_df_from_pair(cx[s][2]);
       const float2 *lat = s >= 1 ? tiny + (long long)(s - 1) * g.P : nullptr;
       const fh_df wl_ = s >= 1 ? fh_df_from_pair(wx[s][s - 1]) : fh_df{0.f, 0.f};
@@ -1563,9 +1576,9 @@ __global__ void __launch_bounds__(kFuseThreads, 1) k_tg_sweeps_fused(const tg_fu
     y_prefetch(s);  // after the x loads: the copies run under the x solve
     __syncthreads();
     TG_STAMP(1);
-    if (xl_ok(grp))
+    if (xl_ok(grp) && w4 < awx)
       tg_group_solve(Nx, fa_x + grp * kFuseSL, al_x + grp * kFuseSL, xch + grp * kFuseSL, ub_sm[grp], fh_df{0.f, 0.f},
-                     fh_df_from_pair(cx[s][3]), scan_sm[grp], &uN_sm[grp], 1 + grp, gt, w4);
+                     fh_df_from_pair(cx[s][3]), scan_sm[grp], &uN_sm[grp], 1 + grp, gt, w4, awx);
     __syncthreads();
     TG_STAMP(2);
 #pragma unroll
@@ -1611,9 +1624,9 @@ __global__ void __launch_bounds__(kFuseThreads, 1) k_tg_sweeps_fused(const tg_fu
     }
     __syncthreads();
     TG_STAMP(4);
-    if (yl_ok(grp))
+    if (yl_ok(grp) && w4 < awy)
       tg_group_solve(Ny, fa_y + grp * kFuseSL, al_y + grp * kFuseSL, xch + grp * kFuseSL, ub_sm[grp], fh_df{1.f, 0.f},
-                     fh_df{0.f, 0.f}, scan_sm[grp], &uN_sm[grp], 1 + grp, gt, w4);
+                     fh_df{0.f, 0.f}, scan_sm[grp], &uN_sm[grp], 1 + grp, gt, w4, awy);
     __syncthreads();
     TG_STAMP(5);
     {
@@ -1642,8 +1655,10 @@ __global__ void __launch_bounds__(kFuseThreads, 1) k_tg_sweeps_fused(const tg_fu
       TG_STAMP(9);
       {  // the x history part of the next step overlaps the barrier (layers up to j - 1 are complete)
         float2 r[kFuseLines], d[kSub - 1][kFuseLines];
-        x_load(s + 1, r, d);
-        x_sum(s + 1, r, d);
+        if (wx_live) {
+          x_load(s + 1, r, d);
+          x_sum(s + 1, r, d);
+        }
       }
       TG_STAMP(10);
       if (!tg_grid_wait(a.bar, ++nb * nblk, a.err)) return;
