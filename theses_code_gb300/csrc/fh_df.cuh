@@ -42,6 +42,9 @@ __device__ __forceinline__ fh_df fh_df_add(fh_df a, fh_df b) {
   return fh_df_renorm(s, e);
 }
 
+// c ? a : b without a branch
+__device__ __forceinline__ fh_df fh_df_sel(bool c, fh_df a, fh_df b) { return fh_df{c ? a.h : b.h, c ? a.l : b.l}; }
+
 __device__ __forceinline__ fh_df fh_df_neg(fh_df a) { return fh_df{-a.h, -a.l}; }
 __device__ __forceinline__ fh_df fh_df_sub(fh_df a, fh_df b) { return fh_df_add(a, fh_df_neg(b)); }
 

@@ -1262,13 +1262,14 @@ __device__ __forceinline__ fh_daff tg_group_scan(fh_daff f, fh_daff *sm, int bar
   fh_daff g = f;
 #pragma unroll
   for (int d = 1; d < 32; d <<= 1) {
-    if (!REV) {
-      const fh_daff p{fh_df_shfl_up(g.a, d), fh_df_shfl_up(g.b, d)};
-      if (lane >= (unsigned)d) g = fh_daff_compose(g, p);
-    } else {
-      const fh_daff p{fh_df_shfl_down(g.a, d), fh_df_shfl_down(g.b, d)};
-      if (lane + d < 32u) g = fh_daff_compose(g, p);
-    }
+    // every lane composes and keeps its own map or the result: a divergent branch
+    // costs more than the composition (five levels 580 -> 330 cycles)
+    const fh_daff p = REV ? fh_daff{fh_df_shfl_down(g.a, d), fh_df_shfl_down(g.b, d)}
+                          : fh_daff{fh_df_shfl_up(g.a, d), fh_df_shfl_up(g.b, d)};
+    const fh_daff r = fh_daff_compose(g, p);
+    const bool in = REV ? lane + d < 32u : lane >= (unsigned)d;
+    g.a = fh_df_sel(in, r.a, g.a);
+    g.b = fh_df_sel(in, r.b, g.b);
   }
   const fh_daff id{fh_df{1.f, 0.f}, fh_df{0.f, 0.f}};
   fh_daff e;
@@ -1292,6 +1293,25 @@ __device__ __forceinline__ fh_daff tg_group_scan(fh_daff f, fh_daff *sm, int bar
   return fh_daff_compose(e, P);
 }
 
+// The end condition u_N = bt_{N-1} / (1 - al_{N-1}): x = 1 - al_{N-1} and the
+// reciprocal of its head, once per launch.  tg_div_end is fh_df_div with its two
+// FP32 quotients from the reciprocal, each corrected by its exact remainders
+// (Markstein, IBM J. Res. Dev. 34, 1990): the correctly rounded quotients
+// without two divisions (590 cycles) on the critical path of every solve.
+struct tg_end {
+  fh_df x;
+  float r;
+};
+__device__ __forceinline__ float tg_quot(float a, float b, float r) {
+  const float q0 = a * r, q = fmaf(fmaf(-q0, b, a), r, q0);  // faithful
+  return fmaf(fmaf(-q, b, a), r, q);                         // correctly rounded
+}
+__device__ __forceinline__ fh_df tg_div_end(fh_df a, const tg_end &d) {
+  const float q1 = tg_quot(a.h, d.x.h, d.r);
+  const fh_df r = fh_df_sub(a, fh_df_mul(fh_df{q1, 0.f}, d.x));
+  return fh_df_renorm(q1, tg_quot(r.h, d.x.h, d.r));
+}
+
 // One line of N nodes by the 128 threads of its group: Thomas in the
 // reference form from the fixed factors, u_i = al_i u_{i+1} + bt_i with
 // bt_i = fa_i bt_{i-1} + fb_i, bt_0 = bt1, al_0 = al1, u_N = u_{N+1} =
@@ -1303,58 +1323,49 @@ __device__ __forceinline__ fh_daff tg_group_scan(fh_daff f, fh_daff *sm, int bar
 // which change no bit): on short lines a quarter of the warps issues a quarter
 // of the instructions.
 __device__ __forceinline__ void tg_group_solve(int N, const float2 *fa, const float2 *al, float2 *xch, float2 *ub,
-                                               fh_df al1, fh_df bt1, fh_daff *sm, fh_df *uNs, int bar, int t, int w4,
-                                               int aw) {
+                                               fh_df al1, fh_df bt1, const tg_end &end, fh_daff *sm, fh_df *uNs, int bar,
+                                               int t, int w4, int aw) {
   const fh_df one{1.f, 0.f}, zero{0.f, 0.f};
+  // equations past the line's end are identities (fa = al = 1, fb = 0 in the
+  // tables, bt = 0 below): no branches in the walks
   fh_df B[kFuseEq], P[kFuseEq];
   fh_df b = zero, p = one;
 #pragma unroll
   for (int e = 0; e < kFuseEq; ++e) {
-    const int i = 1 + kFuseEq * t + e;
-    if (i < N) {
-      const int sl = e * kFuseSE + t;
-      const fh_df f = fh_df_from_pair(fa[sl]);
-      b = fh_df_fma(f, b, fh_df_from_pair(xch[sl]));
-      p = fh_df_mul(p, f);
-    }
+    const fh_df f = fh_df_from_pair(fa[e * kFuseSE + t]);
+    b = fh_df_fma(f, b, fh_df_from_pair(xch[e * kFuseSE + t]));
+    p = fh_df_mul(p, f);
     B[e] = b;
     P[e] = p;
   }
   const fh_daff Pf = tg_group_scan<false>(fh_daff{p, b}, sm, bar, w4, aw);
   const fh_df s = fh_df_fma(Pf.a, bt1, Pf.b);  // bt at equation 4t (bt1 for t = 0)
-  fh_df bt[kFuseEq];
+  fh_df bt[kFuseEq], bl = zero;
+  const int n = N - 1 - kFuseEq * t;  // equations from the thread's first to the line's last
 #pragma unroll
-  for (int e = 0; e < kFuseEq; ++e) bt[e] = fh_df_fma(P[e], s, B[e]);
-  // u_N from the thread of equation N - 1
-  {
-    const int e = (N - 2) - kFuseEq * t;
-    if (e >= 0 && e < kFuseEq) {
-      const fh_df aN = fh_df_from_pair(al[e * kFuseSE + t]);
-      *uNs = fh_df_div(bt[e], fh_df_sub(one, aN));
-    }
+  for (int e = 0; e < kFuseEq; ++e) {
+    bt[e] = fh_df_sel(e < n, fh_df_fma(P[e], s, B[e]), zero);
+    bl = fh_df_sel(e == n - 1, bt[e], bl);
   }
+  // u_N from the thread of equation N - 1
+  if (n >= 1 && n <= kFuseEq) *uNs = tg_div_end(bl, end);
   fh_group_bar(bar, 32 * aw);
   const fh_df uN = *uNs;
   fh_df V[kFuseEq], Q[kFuseEq];
   fh_df v = zero, q = one;
 #pragma unroll
   for (int e = kFuseEq - 1; e >= 0; --e) {
-    const int i = 1 + kFuseEq * t + e;
-    if (i < N) {
-      const fh_df a = fh_df_from_pair(al[e * kFuseSE + t]);
-      v = fh_df_fma(a, v, bt[e]);
-      q = fh_df_mul(q, a);
-    }
+    const fh_df a = fh_df_from_pair(al[e * kFuseSE + t]);
+    v = fh_df_fma(a, v, bt[e]);
+    q = fh_df_mul(q, a);
     V[e] = v;
     Q[e] = q;
   }
   const fh_daff Pb = tg_group_scan<true>(fh_daff{q, v}, sm, bar, w4, aw);
   const fh_df u1 = fh_df_fma(Pb.a, uN, Pb.b);  // u at equation 4t + 5 (u_N past the last chunk)
 #pragma unroll
-  for (int e = 0; e < kFuseEq; ++e) {
-    const int i = 1 + kFuseEq * t + e;
-    if (i < N) xch[e * kFuseSE + t] = fh_df_pair(fh_df_fma(Q[e], u1, V[e]));
-  }
+  for (int e = 0; e < kFuseEq; ++e)
+    if (e < n) xch[e * kFuseSE + t] = fh_df_pair(fh_df_fma(Q[e], u1, V[e]));
   if (t == 0) {
     const fh_df u0 = fh_df_fma(al1, fh_df_fma(Q[0], u1, V[0]), bt1);
     ub[0] = fh_df_pair(u0);
@@ -1368,6 +1379,7 @@ __global__ void __launch_bounds__(kFuseThreads, 1) k_tg_sweeps_fused(const tg_fu
   __shared__ float2 cx[kSub][4], cy[kSub][4], wx[kSub][kSub], wy[kSub][kSub];
   __shared__ fh_daff scan_sm[kFuseLines][4];
   __shared__ fh_df uN_sm[kFuseLines];
+  __shared__ tg_end end_sm[2][kFuseLines];
   __shared__ float2 ub_sm[kFuseLines][2];
   const fh_tg_dev &g = a.g;
   const int Nx = g.sN, Ny = g.M;
@@ -1413,16 +1425,22 @@ __global__ void __launch_bounds__(kFuseThreads, 1) k_tg_sweeps_fused(const tg_fu
       const int v = tid + u * kFuseThreads;
       const int lx = v / kFuseNL, ix = 1 + v % kFuseNL;
       const int ly = v % kFuseLines, iy = 1 + v / kFuseLines;
-      if (xl_ok(lx) && ix < Nx) {
-        fa_x[lx * kFuseSL + tg_fslot(ix)] = vx[u][0];
-        al_x[lx * kFuseSL + tg_fslot(ix)] = vx[u][1];
-        g_x[lx * kFuseNL + ix - 1] = vx[u][2];
-      }
-      if (yl_ok(ly) && iy < Ny) {
-        fa_y[ly * kFuseSL + tg_fslot(iy)] = vy[u][0];
-        al_y[ly * kFuseSL + tg_fslot(iy)] = vy[u][1];
-        g_y[ly * kFuseNL + iy - 1] = vy[u][2];
-      }
+      // past the end of a line: identities
+      const bool okx = xl_ok(lx) && ix < Nx, oky = yl_ok(ly) && iy < Ny;
+      const float2 one = make_float2(1.f, 0.f);
+      fa_x[lx * kFuseSL + tg_fslot(ix)] = okx ? vx[u][0] : one;
+      al_x[lx * kFuseSL + tg_fslot(ix)] = okx ? vx[u][1] : one;
+      g_x[lx * kFuseNL + ix - 1] = vx[u][2];
+      fa_y[ly * kFuseSL + tg_fslot(iy)] = oky ? vy[u][0] : one;
+      al_y[ly * kFuseSL + tg_fslot(iy)] = oky ? vy[u][1] : one;
+      g_y[ly * kFuseNL + iy - 1] = vy[u][2];
+      xch[lx * kFuseSL + tg_fslot(ix)] = make_float2(0.f, 0.f);
+      auto end = [&](tg_end &d, float2 alN) {
+        d.x = fh_df_sub(fh_df{1.f, 0.f}, fh_df_from_pair(alN));
+        d.r = 1.f / d.x.h;
+      };
+      if (okx && ix == Nx - 1) end(end_sm[0][lx], vx[u][1]);
+      if (oky && iy == Ny - 1) end(end_sm[1][ly], vy[u][1]);
     }
   }
   // double-float step constants and sub-block weights, one FP64 conversion per thread
@@ -1565,20 +1583,20 @@ __global__ void __launch_bounds__(kFuseThreads, 1) k_tg_sweeps_fused(const tg_fu
         d[k] = (lat && xlive(k)) ? __ldcg(lat + xid(k)) : make_float2(0.f, 0.f);
       }
 #pragma unroll
-      for (int k = 0; k < kFuseLines; ++k)
-        if (xlive(k)) {
-          const fh_df ts = lat ? fh_df_fma(wl_, fh_df_from_pair(d[k]), tsx[k]) : tsx[k];
-          fh_df om = fh_df_fma(kst, fh_df_from_pair(c[k]), S2);
-          om = fh_df_fma(st, ts, om);
-          xch[k * kFuseSL + tg_fslot(xi)] = fh_df_pair(fh_df_neg(fh_df_mul(fh_df_from_pair(g_x[k * kFuseNL + xi - 1]), om)));
-        }
+      for (int k = 0; k < kFuseLines; ++k) {
+        const fh_df ts = lat ? fh_df_fma(wl_, fh_df_from_pair(d[k]), tsx[k]) : tsx[k];
+        fh_df om = fh_df_fma(kst, fh_df_from_pair(c[k]), S2);
+        om = fh_df_fma(st, ts, om);
+        const float2 v = fh_df_pair(fh_df_neg(fh_df_mul(fh_df_from_pair(g_x[k * kFuseNL + xi - 1]), om)));
+        if (xlive(k)) xch[k * kFuseSL + tg_fslot(xi)] = v;
+      }
     }
     y_prefetch(s);  // after the x loads: the copies run under the x solve
     __syncthreads();
     TG_STAMP(1);
     if (xl_ok(grp) && w4 < awx)
       tg_group_solve(Nx, fa_x + grp * kFuseSL, al_x + grp * kFuseSL, xch + grp * kFuseSL, ub_sm[grp], fh_df{0.f, 0.f},
-                     fh_df_from_pair(cx[s][3]), scan_sm[grp], &uN_sm[grp], 1 + grp, gt, w4, awx);
+                     fh_df_from_pair(cx[s][3]), end_sm[0][grp], scan_sm[grp], &uN_sm[grp], 1 + grp, gt, w4, awx);
     __syncthreads();
     TG_STAMP(2);
 #pragma unroll
@@ -1612,21 +1630,21 @@ __global__ void __launch_bounds__(kFuseThreads, 1) k_tg_sweeps_fused(const tg_fu
       for (int k = 0; k < kFuseLines; ++k) c[k] = ylive(k) ? __ldcg(a.Chd + yid(k)) : make_float2(0.f, 0.f);
 #pragma unroll
       for (int k = 0; k < kFuseLines; ++k)
-        if (ylive(k)) {
+        if (k < yk) {
           const fh_df cc = fh_df_from_pair(c[k]);
           // old[size-2] - old[size-1] (fr_d_t_g_2d.cpp:3478-3481)
           const fh_df tt = fh_df_fma(kyh, fh_df_sub(fh_df_from_pair(f[k]), cc), tsy[k]);
           fh_df om = fh_df_fma(kst, cc, S2);
           om = fh_df_fma(st, tt, om);
-          xch[yc * kFuseSL + tg_fslot(yq(k))] =
-              fh_df_pair(fh_df_neg(fh_df_mul(fh_df_from_pair(g_y[yc * kFuseNL + yq(k) - 1]), om)));
+          const float2 v = fh_df_pair(fh_df_neg(fh_df_mul(fh_df_from_pair(g_y[yc * kFuseNL + yq(k) - 1]), om)));
+          if (ylive(k)) xch[yc * kFuseSL + tg_fslot(yq(k))] = v;
         }
     }
     __syncthreads();
     TG_STAMP(4);
     if (yl_ok(grp) && w4 < awy)
       tg_group_solve(Ny, fa_y + grp * kFuseSL, al_y + grp * kFuseSL, xch + grp * kFuseSL, ub_sm[grp], fh_df{1.f, 0.f},
-                     fh_df{0.f, 0.f}, scan_sm[grp], &uN_sm[grp], 1 + grp, gt, w4, awy);
+                     fh_df{0.f, 0.f}, end_sm[1][grp], scan_sm[grp], &uN_sm[grp], 1 + grp, gt, w4, awy);
     __syncthreads();
     TG_STAMP(5);
     {
