@@ -247,6 +247,7 @@ struct fh_ab_df {
   static __device__ __forceinline__ V shfl(V v, int lane) {
     return fh_df{__shfl_sync(0xffffffffu, v.h, lane), __shfl_sync(0xffffffffu, v.l, lane)};
   }
+  static __device__ __forceinline__ V sel(bool c, V a, V b) { return fh_df_sel(c, a, b); }
 };
 
 // FP64 (FP64 mode).
@@ -262,6 +263,7 @@ struct fh_ab_f64 {
   static __device__ __forceinline__ V add(V a, V b) { return a + b; }
   static __device__ __forceinline__ V sub(V a, V b) { return a - b; }
   static __device__ __forceinline__ V shfl(V v, int lane) { return __shfl_sync(0xffffffffu, v, lane); }
+  static __device__ __forceinline__ V sel(bool c, V a, V b) { return c ? a : b; }
 };
 
 constexpr int kAbResThreads = 512;
@@ -308,7 +310,7 @@ __device__ __forceinline__ typename A::V ab_scan(typename A::V g, typename A::V 
   for (int k = 0; k < 5; ++k) {
     const int d = 1 << k;
     const V p = A::shfl(g, REV ? lane + d : lane - d);
-    if (REV ? lane + d < 32 : lane >= d) g = A::fma(A::ld(lv[k * T + t]), p, g);
+    g = A::sel(REV ? lane + d < 32 : lane >= d, A::fma(A::ld(lv[k * T + t]), p, g), g);
   }
   if (lane == (REV ? 0 : 31)) tot[warp] = A::st(g);
   V e = A::shfl(g, REV ? lane + 1 : lane - 1);
@@ -321,7 +323,7 @@ __device__ __forceinline__ typename A::V ab_scan(typename A::V g, typename A::V 
   for (int k = 0; (1 << k) < NW; ++k) {
     const int d = 1 << k;
     const V p = A::shfl(q, lane - d);
-    if (lane >= d) q = A::fma(A::ld(lw[k * 32 + lane]), p, q);
+    q = A::sel(lane >= d, A::fma(A::ld(lw[k * 32 + lane]), p, q), q);
   }
   // start of this warp: the inclusive scan up to the warp before it
   const int wi = REV ? NW - 1 - warp : warp;

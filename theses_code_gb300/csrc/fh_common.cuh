@@ -24,6 +24,12 @@ __device__ __forceinline__ fh_aff fh_aff_compose(fh_aff f2, fh_aff f1) {
   return fh_aff{f2.a * f1.a, fma(f2.a, f1.b, f2.b)};
 }
 
+// c ? f : g without a branch: in the scans every lane composes and selects (a
+// divergent branch per level costs more than the composition).
+__device__ __forceinline__ fh_aff fh_aff_sel(bool c, fh_aff f, fh_aff g) {
+  return fh_aff{c ? f.a : g.a, c ? f.b : g.b};
+}
+
 // Exclusive scan over the warp: lane l receives f_{l-1} o ... o f_0 (identity
 // for lane 0).  All 32 lanes must participate.
 __device__ __forceinline__ fh_aff fh_warp_exclusive_affine(fh_aff f) {
@@ -34,7 +40,7 @@ __device__ __forceinline__ fh_aff fh_warp_exclusive_affine(fh_aff f) {
   for (int d = 1; d < 32; d <<= 1) {
     double pa = __shfl_up_sync(0xffffffffu, g.a, d);
     double pb = __shfl_up_sync(0xffffffffu, g.b, d);
-    if (lane >= (unsigned)d) g = fh_aff_compose(g, fh_aff{pa, pb});
+    g = fh_aff_sel(lane >= (unsigned)d, fh_aff_compose(g, fh_aff{pa, pb}), g);
   }
   double ea = __shfl_up_sync(0xffffffffu, g.a, 1);
   double eb = __shfl_up_sync(0xffffffffu, g.b, 1);

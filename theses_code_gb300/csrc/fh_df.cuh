@@ -83,6 +83,9 @@ struct fh_daff {
 __device__ __forceinline__ fh_daff fh_daff_compose(fh_daff f2, fh_daff f1) {
   return fh_daff{fh_df_mul(f2.a, f1.a), fh_df_fma(f2.a, f1.b, f2.b)};
 }
+__device__ __forceinline__ fh_daff fh_daff_sel(bool c, fh_daff f, fh_daff g) {
+  return fh_daff{fh_df_sel(c, f.a, g.a), fh_df_sel(c, f.b, g.b)};
+}
 __device__ __forceinline__ fh_df fh_df_shfl_up(fh_df v, int d) {
   return fh_df{__shfl_up_sync(0xffffffffu, v.h, d), __shfl_up_sync(0xffffffffu, v.l, d)};
 }
@@ -96,7 +99,7 @@ __device__ __forceinline__ fh_daff fh_warp_exclusive_daff(fh_daff f) {
 #pragma unroll
   for (int d = 1; d < 32; d <<= 1) {
     const fh_daff p{fh_df_shfl_up(g.a, d), fh_df_shfl_up(g.b, d)};
-    if (lane >= (unsigned)d) g = fh_daff_compose(g, p);
+    g = fh_daff_sel(lane >= (unsigned)d, fh_daff_compose(g, p), g);
   }
   fh_daff e{fh_df_shfl_up(g.a, 1), fh_df_shfl_up(g.b, 1)};
   if (lane == 0) e = fh_daff{fh_df{1.f, 0.f}, fh_df{0.f, 0.f}};
@@ -109,7 +112,7 @@ __device__ __forceinline__ fh_daff fh_warp_exclusive_daff_rev(fh_daff f) {
 #pragma unroll
   for (int d = 1; d < 32; d <<= 1) {
     const fh_daff p{fh_df_shfl_down(g.a, d), fh_df_shfl_down(g.b, d)};
-    if (lane + d < 32u) g = fh_daff_compose(g, p);
+    g = fh_daff_sel(lane + d < 32u, fh_daff_compose(g, p), g);
   }
   fh_daff e{fh_df_shfl_down(g.a, 1), fh_df_shfl_down(g.b, 1)};
   if (lane == 31u) e = fh_daff{fh_df{1.f, 0.f}, fh_df{0.f, 0.f}};

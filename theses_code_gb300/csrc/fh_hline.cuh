@@ -125,7 +125,7 @@ __device__ __forceinline__ double fh_hl_scan(fh_aff G, double v, fh_aff *tot, do
     if (lv) lv[k * T + t] = G.a;
     const double pa = REV ? __shfl_down_sync(0xffffffffu, G.a, d) : __shfl_up_sync(0xffffffffu, G.a, d);
     const double pb = REV ? __shfl_down_sync(0xffffffffu, G.b, d) : __shfl_up_sync(0xffffffffu, G.b, d);
-    if (REV ? lane + d < 32 : lane >= d) G = fh_aff_compose(G, fh_aff{pa, pb});
+    G = fh_aff_sel(REV ? lane + d < 32 : lane >= d, fh_aff_compose(G, fh_aff{pa, pb}), G);
   }
   if (lane == (REV ? 0 : 31)) tot[warp] = G;
   double ea = REV ? __shfl_down_sync(0xffffffffu, G.a, 1) : __shfl_up_sync(0xffffffffu, G.a, 1);
@@ -160,7 +160,8 @@ __device__ __forceinline__ double fh_hl_scan_fixed(double g, double v, fh_aff *t
   for (int k = 0; k < 5; ++k) {
     const int d = 1 << k;
     const double pb = REV ? __shfl_down_sync(0xffffffffu, g, d) : __shfl_up_sync(0xffffffffu, g, d);
-    if (REV ? lane + d < 32 : lane >= d) g = fma(lv[k * T + t], pb, g);
+    const double r = fma(lv[k * T + t], pb, g);
+    g = (REV ? lane + d < 32 : lane >= d) ? r : g;
   }
   if (lane == (REV ? 0 : 31)) tot[warp].b = g;
   double eb = REV ? __shfl_down_sync(0xffffffffu, g, 1) : __shfl_up_sync(0xffffffffu, g, 1);
@@ -306,7 +307,9 @@ __device__ __forceinline__ void fh_hline(const fh_h_dev_inst &I, double DaW, con
         p.m01 = __shfl_up_sync(0xffffffffu, G.m01, d);
         p.m10 = __shfl_up_sync(0xffffffffu, G.m10, d);
         p.m11 = __shfl_up_sync(0xffffffffu, G.m11, d);
-        if (lane >= d) G = fh_mob_compose(G, p);
+        const fh_mob m = fh_mob_compose(G, p);
+        const bool in = lane >= d;
+        G = fh_mob{in ? m.m00 : G.m00, in ? m.m01 : G.m01, in ? m.m10 : G.m10, in ? m.m11 : G.m11};
         if (d == 4 || d == 16) G = fh_mob_rescale(G);
       }
       if (lane == 31) sc.mob[warp] = G;

@@ -20,7 +20,7 @@ __device__ __forceinline__ fh_aff fh_warp_exclusive_affine_rev(fh_aff f) {
   for (int d = 1; d < 32; d <<= 1) {
     double pa = __shfl_down_sync(0xffffffffu, g.a, d);
     double pb = __shfl_down_sync(0xffffffffu, g.b, d);
-    if (lane + d < 32u) g = fh_aff_compose(g, fh_aff{pa, pb});
+    g = fh_aff_sel(lane + d < 32u, fh_aff_compose(g, fh_aff{pa, pb}), g);
   }
   double ea = __shfl_down_sync(0xffffffffu, g.a, 1);
   double eb = __shfl_down_sync(0xffffffffu, g.b, 1);
@@ -31,103 +31,11 @@ __device__ __forceinline__ fh_aff fh_warp_exclusive_affine_rev(fh_aff f) {
   return fh_aff{ea, eb};
 }
 
-// Line accessor contract (all lanes call with the same line):
-//   double om(int i)      right part Om_i, i = 1..N-1
-//   double A(int i)       sub-diagonal A_i
-//   double g(int i)       pivot factor g_i = Al[i+1]/B_i (or 1/(R_i - A_i Al_i) when Al[i+1] = B_i = 0)
-//   double al(int i)      Al[i+1] for i = 1..N-1
-//   void   store(int i, double u)   writes u_i, i = 0..N+1
-// buf: per-warp shared scratch of N+1 doubles.
-template <class Line>
-__device__ __forceinline__ void fh_line_solve_cached(const Line &L, int N, double al1, double bt1, double *buf) {
-  const int lane = threadIdx.x & 31;
-  // ---- forward: Bt[i+1] for i = 1..N-1, stored at buf[i]; buf[0] = Bt[1]
-  const int nf = N - 1;
-  const int chf = (nf + 31) / 32;
-  const int f0 = 1 + lane * chf, f1 = min(N, f0 + chf);
-  fh_aff F{1.0, 0.0};
-  for (int i = f0; i < f1; ++i) {
-    const double om = L.om(i), a = L.A(i), g = L.g(i);
-    buf[i] = om;
-    F = fh_aff_compose(fh_aff{g * a, -g * om}, F);
-  }
-  const fh_aff Pf = fh_warp_exclusive_affine(F);
-  double bt = fma(Pf.a, bt1, Pf.b);
-  for (int i = f0; i < f1; ++i) {
-    bt = L.g(i) * (L.A(i) * bt - buf[i]);
-    buf[i] = bt;
-  }
-  if (lane == 0) buf[0] = bt1;
-  __syncwarp();
-  // ---- u_N = Bt[N] / (1 - Al[N])
-  const double alN = (N >= 2) ? L.al(N - 1) : al1;
-  const double uN = buf[N - 1] / (1.0 - alN);
-  // ---- backward: u_i = Al[i+1] u_{i+1} + Bt[i+1], i = N-1..0
-  const int chb = (N + 31) / 32;
-  const int b0 = lane * chb, b1 = min(N, b0 + chb);
-  // chunk map G = h_{b0} o h_{b0+1} o ... o h_{b1-1} (h_{b1-1} applied first)
-  fh_aff G{1.0, 0.0};
-  for (int i = b1 - 1; i >= b0; --i) {
-    const double ali = (i >= 1) ? L.al(i) : al1;
-    G = fh_aff_compose(fh_aff{ali, buf[i]}, G);
-  }
-  const fh_aff Pb = fh_warp_exclusive_affine_rev(G);
-  double u = fma(Pb.a, uN, Pb.b);  // u at index b1
-  for (int i = b1 - 1; i >= b0; --i) {
-    const double ali = (i >= 1) ? L.al(i) : al1;
-    u = ali * u + buf[i];
-    L.store(i, u);
-  }
-  if (lane == 0) {
-    L.store(N, uN);
-    L.store(N + 1, uN);
-  }
-  __syncwarp();
-}
-
 // ------------------------------------------------------------------------
-// Staged variant: the line's coefficients already sit in shared memory.
+// The line's coefficients sit in shared memory.
 // Index skew sk(i) = i + i/16 keeps the per-lane chunks (16 consecutive
 // equations per lane for lines up to 513 nodes) on distinct bank pairs.
 __device__ __forceinline__ int fh_sk(int i) { return i + (i >> 4); }
-
-// fa/fb: forward maps Bt[i+1] = fa_i Bt[i] + fb_i (i = 1..N-1); al: Al[i+1]
-// (i = 1..N-1).  bt: scratch; u: result u_i (i = 0..N+1), may alias fa.
-__device__ __forceinline__ void fh_line_solve_staged(int N, const double *fa, const double *fb, const double *al,
-                                                     double al1, double bt1, double *bt, double *u) {
-  const int lane = threadIdx.x & 31;
-  const int nf = N - 1;
-  const int chf = (nf + 31) / 32;
-  const int f0 = 1 + lane * chf, f1 = min(N, f0 + chf);
-  fh_aff F{1.0, 0.0};
-  for (int i = f0; i < f1; ++i) F = fh_aff_compose(fh_aff{fa[fh_sk(i)], fb[fh_sk(i)]}, F);
-  const fh_aff Pf = fh_warp_exclusive_affine(F);
-  double b = fma(Pf.a, bt1, Pf.b);
-  for (int i = f0; i < f1; ++i) {
-    b = fma(fa[fh_sk(i)], b, fb[fh_sk(i)]);
-    bt[fh_sk(i)] = b;
-  }
-  if (lane == 0) bt[fh_sk(0)] = bt1;
-  __syncwarp();
-  const double alN = (N >= 2) ? al[fh_sk(N - 1)] : al1;
-  const double uN = bt[fh_sk(N - 1)] / (1.0 - alN);
-  const int chb = (N + 31) / 32;
-  const int b0 = lane * chb, b1 = min(N, b0 + chb);
-  fh_aff G{1.0, 0.0};
-  for (int i = b1 - 1; i >= b0; --i) G = fh_aff_compose(fh_aff{(i >= 1) ? al[fh_sk(i)] : al1, bt[fh_sk(i)]}, G);
-  const fh_aff Pb = fh_warp_exclusive_affine_rev(G);
-  double v = fma(Pb.a, uN, Pb.b);
-  __syncwarp();  // u may alias fa: all forward reads are done
-  for (int i = b1 - 1; i >= b0; --i) {
-    v = fma((i >= 1) ? al[fh_sk(i)] : al1, v, bt[fh_sk(i)]);
-    u[fh_sk(i)] = v;
-  }
-  if (lane == 0) {
-    u[fh_sk(N)] = uN;
-    u[fh_sk(N + 1)] = uN;
-  }
-  __syncwarp();
-}
 
 // ------------------------------------------------------------------------
 // Prefix variant for a factorization that is fixed over many solves: the
@@ -136,8 +44,7 @@ __device__ __forceinline__ void fh_line_solve_staged(int N, const double *fa, co
 // its chunk once from a zero start and then adds prefix * start value:
 //   forward   Bt[i+1] = b0_i + pf_i Bt[f0]       pf_i = fa_{f0} ... fa_i
 //   backward  u_i     = v0_i + pb_i u_{b1}       pb_i = al'_i ... al'_{b1-1}
-// Two FP64 operations per equation and phase instead of three.  Chunking as in
-// fh_line_solve_staged: lane l owns forward equations [1 + l chf, 1 + (l+1) chf)
+// Two FP64 operations per equation and phase instead of three.  Lane l owns forward equations [1 + l chf, 1 + (l+1) chf)
 // and backward nodes [l chb, (l+1) chb), chf = ceil((N-1)/32), chb = ceil(N/32).
 __host__ __device__ inline int fh_chunk_f(int N) { return (N - 1 + 31) / 32; }
 __host__ __device__ inline int fh_chunk_b(int N) { return (N + 31) / 32; }
@@ -253,7 +160,7 @@ __device__ __forceinline__ fh_aff fh_group_exclusive_affine(fh_aff f, fh_aff *sm
   for (int d = 1; d < 32; d <<= 1) {
     const double pa = __shfl_up_sync(0xffffffffu, g.a, d);
     const double pb = __shfl_up_sync(0xffffffffu, g.b, d);
-    if (lane >= (unsigned)d) g = fh_aff_compose(g, fh_aff{pa, pb});
+    g = fh_aff_sel(lane >= (unsigned)d, fh_aff_compose(g, fh_aff{pa, pb}), g);
   }
   if (lane == 31u) sm[w] = g;
   double ea = __shfl_up_sync(0xffffffffu, g.a, 1);
@@ -279,7 +186,7 @@ __device__ __forceinline__ fh_aff fh_group_exclusive_affine_rev(fh_aff f, fh_aff
   for (int d = 1; d < 32; d <<= 1) {
     const double pa = __shfl_down_sync(0xffffffffu, g.a, d);
     const double pb = __shfl_down_sync(0xffffffffu, g.b, d);
-    if (lane + d < 32u) g = fh_aff_compose(g, fh_aff{pa, pb});
+    g = fh_aff_sel(lane + d < 32u, fh_aff_compose(g, fh_aff{pa, pb}), g);
   }
   if (lane == 0u) sm[w] = g;
   double ea = __shfl_down_sync(0xffffffffu, g.a, 1);
@@ -293,48 +200,4 @@ __device__ __forceinline__ fh_aff fh_group_exclusive_affine_rev(fh_aff f, fh_aff
   for (int k = NW - 1; k > w; --k) Q = fh_aff_compose(sm[k], Q);
   fh_group_bar(bar, 32 * NW);
   return fh_aff_compose(fh_aff{ea, eb}, Q);
-}
-
-// ------------------------------------------------------------------------
-// Double-float group scans: NW warps (threads 0 .. 32 NW - 1 of the CTA) scan
-// one chain of 32 NW chunk maps in double-float; warp totals pass through
-// shared memory sm[NW] and the named barrier bar (NW warps only).
-template <int NW>
-__device__ __forceinline__ fh_daff fh_group_exclusive_daff(fh_daff f, fh_daff *sm, int bar) {
-  const unsigned lane = threadIdx.x & 31u;
-  const int w = threadIdx.x >> 5;
-  fh_daff g = f;
-#pragma unroll
-  for (int d = 1; d < 32; d <<= 1) {
-    const fh_daff p{fh_df_shfl_up(g.a, d), fh_df_shfl_up(g.b, d)};
-    if (lane >= (unsigned)d) g = fh_daff_compose(g, p);
-  }
-  if (lane == 31u) sm[w] = g;
-  fh_daff e{fh_df_shfl_up(g.a, 1), fh_df_shfl_up(g.b, 1)};
-  if (lane == 0u) e = fh_daff{fh_df{1.f, 0.f}, fh_df{0.f, 0.f}};
-  fh_group_bar(bar, 32 * NW);
-  fh_daff P{fh_df{1.f, 0.f}, fh_df{0.f, 0.f}};
-  for (int k = 0; k < w; ++k) P = fh_daff_compose(sm[k], P);
-  fh_group_bar(bar, 32 * NW);  // sm may be reused after this
-  return fh_daff_compose(e, P);
-}
-
-template <int NW>
-__device__ __forceinline__ fh_daff fh_group_exclusive_daff_rev(fh_daff f, fh_daff *sm, int bar) {
-  const unsigned lane = threadIdx.x & 31u;
-  const int w = threadIdx.x >> 5;
-  fh_daff g = f;
-#pragma unroll
-  for (int d = 1; d < 32; d <<= 1) {
-    const fh_daff p{fh_df_shfl_down(g.a, d), fh_df_shfl_down(g.b, d)};
-    if (lane + d < 32u) g = fh_daff_compose(g, p);
-  }
-  if (lane == 0u) sm[w] = g;
-  fh_daff e{fh_df_shfl_down(g.a, 1), fh_df_shfl_down(g.b, 1)};
-  if (lane == 31u) e = fh_daff{fh_df{1.f, 0.f}, fh_df{0.f, 0.f}};
-  fh_group_bar(bar, 32 * NW);
-  fh_daff Q{fh_df{1.f, 0.f}, fh_df{0.f, 0.f}};
-  for (int k = NW - 1; k > w; --k) Q = fh_daff_compose(sm[k], Q);
-  fh_group_bar(bar, 32 * NW);
-  return fh_daff_compose(e, Q);
 }

@@ -1268,8 +1268,7 @@ __device__ __forceinline__ fh_daff tg_group_scan(fh_daff f, fh_daff *sm, int bar
                           : fh_daff{fh_df_shfl_up(g.a, d), fh_df_shfl_up(g.b, d)};
     const fh_daff r = fh_daff_compose(g, p);
     const bool in = REV ? lane + d < 32u : lane >= (unsigned)d;
-    g.a = fh_df_sel(in, r.a, g.a);
-    g.b = fh_df_sel(in, r.b, g.b);
+    g = fh_daff_sel(in, r, g);
   }
   const fh_daff id{fh_df{1.f, 0.f}, fh_df{0.f, 0.f}};
   fh_daff e;
