@@ -104,3 +104,37 @@ def test_line_solve_tiling(small, kind):
         ref = _solve(p, u, steps)
         sens = _relmax(O.h_solve(dict(p, pert=2.0 ** -53), u, steps)[0], O.h_solve(p, u, steps)[0])
         assert _relmax(g, ref) <= max(1e-12, 2.0 * sens), (kind, p["N"], _relmax(g, ref), sens)
+
+
+@pytest.mark.parametrize("kind,sizes", [
+    ("psi", (2,)),                                 # one owner per node
+    ("psi", (3, 31, 200, 257, 766, 1024, 1025)),   # up to the largest line, its layers beyond shared memory
+    ("psi", (40,) * 25 + (1025,) * 7),             # three owners of up to 343 nodes
+    ("l1", (66, 255, 1025)),
+    ("dirichlet", (29, 512)),
+    ("psi", (2046, 70)),                           # lines of more nodes: k_h_persistent
+])
+def test_persistent_shared_nodes(kind, sizes):
+    """k_h_pers_own (and k_h_persistent) against the kernel-by-kernel path, and the same bits
+    however the steps are spread over calls (tolerance as above)."""
+    from theses_code_gb300._lib import Context
+    from theses_code_gb300.solvers import HSolverBatch
+    steps = 90
+    jobs = [_problem(N, kind, 300 + k) for k, N in enumerate(sizes)]
+    ctx = Context(0)
+    got = []
+    for persistent, calls in ((False, (steps,)), (True, (steps,)), (True, (1, 2, 37, 50))):
+        s = HSolverBatch(ctx, [p for p, _ in jobs], steps + 1)
+        s.set_persistent(persistent)
+        s.set_u([u for _, u in jobs])
+        for n in calls:
+            s.calc_step(n)
+        got.append(s.get_u())
+        s.close()
+    ctx.close()
+    seen = {}
+    for (p, u), a, b, c in zip(jobs, *got):
+        np.testing.assert_array_equal(b, c)
+        if p["N"] not in seen:
+            seen[p["N"]] = _relmax(O.h_solve(dict(p, pert=2.0 ** -53), u, steps)[0], O.h_solve(p, u, steps)[0])
+        assert _relmax(b, a) <= max(1e-12, 2.0 * seen[p["N"]]), (kind, p["N"], _relmax(b, a), seen[p["N"]])

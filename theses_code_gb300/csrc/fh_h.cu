@@ -23,6 +23,7 @@
 #include "fh_slices.cuh"
 #include "fh_weights.cuh"
 #include "fh_hline.cuh"
+#include "fh_cluster.cuh"
 
 // batched far contraction on the tensor cores (fh_blocked.cu)
 struct fh_hblk;
@@ -61,6 +62,7 @@ struct fh_h_batch {
   int mode = FH_H_FP64;  // FH_H_DF64: history as (hi, lo) FP32 pairs; FH_H_BLOCKED: below
   bool persistent = true;  // small FP64 batches: one launch per call (k_h_persistent)
   int pers_ctas = 4;       // CTAs per instance there
+  int *perr = nullptr;     // pinned: set when a wait of the persistent solve ran out
   std::vector<fh_h_dev_inst> di;  // host copy of inst
   std::vector<int> cap;           // nodes a restarted occupant of each instance may have (segment - 2)
   // space-fractional instances: Toeplitz weights wsp and the sums sV per
@@ -88,6 +90,7 @@ struct fh_h_batch {
     if (hs) cudaStreamDestroy(hs);
     if (ev_main) cudaEventDestroy(ev_main);
     if (ev_w) cudaEventDestroy(ev_w);
+    if (perr) cudaFreeHost(perr);
   }
 };
 
@@ -535,6 +538,249 @@ __global__ void __launch_bounds__(kPersThreads, 1)
     H_STAMP(3);
     cl.sync();
   }
+}
+
+// The same for lines of at most kOwnMaxN nodes and solves of at most
+// kOwnMaxSteps steps, with the nodes instead of the slots shared out and without
+// a cluster barrier in the step:
+//   CTA 0 solves the line, step after step (fh_hline: state, newest layer and
+//     constant factors stay in shared memory).  Of a step's history sum it adds
+//     the newest layer; the rest arrives in its shared memory.
+//   CTAs 1 .. C - 1 own a range of the nodes each: they sum every slot but the
+//     newest for them (first 256 threads; the slots in runs side by side when
+//     there are fewer nodes), keep their nodes' layers in shared memory as far
+//     as it goes (the first ones; later ones are read back from the history),
+//     and store new layers to the history.  psi weights are evaluated by the
+//     owners' other 128 threads, a share of the slots each, one step ahead, and
+//     sent to every owner; L1 weights come from the lag table in shared memory.
+// Messages are one-sided (fh_cluster.cuh).  The layer of step s goes out when it
+// is solved, the sums of step s + 2 come back while CTA 0 solves step s + 1.
+// Sums and layers alternate between two buffers: CTA 0 sends layer s after it
+// has the sums of step s, which their owner sent after it had copied layer
+// s - 2; an owner sends the sums of step s + 2 after it has layer s, which CTA 0
+// sent when it had read the sums of step s.  Weights rotate through three
+// buffers: an owner that has layer s - 2 (preparing step s, sending weights of
+// s + 1) knows every owner has finished step s - 2.  A cluster barrier before the
+// first and after the last message; waits are bounded (*err on expiry).
+// The sums of a step are split by its slot count alone, so a solve does not
+// depend on how its steps are spread over calls.
+// Measured: one L1 instance of N = 200 over 1000 steps 13.6 ms with sums and
+// solves one after the other and serial factors, 6.6 ms with the solve beside the
+// next step's sums behind one cluster barrier a step, 4.5 ms in this form; 40
+// steps of N = 64 404, 266, 189 us; 32 psi instances of N = 512 over 250 steps
+// 60.6, 8.3, 6.6 ms.
+constexpr int kOwnLine = 32 * kLineWarps;     // threads of the line solve
+constexpr int kOwnSum = 256;                  // threads of the sums
+constexpr int kOwnThreads = kOwnSum + 128;    // and of the weights
+constexpr int kOwnMaxN = kOwnLine * kHLineEq + 1;  // one panel
+constexpr int kOwnMaxSteps = 4096;            // weights of three steps in shared memory; k_h_persistent above
+constexpr size_t kOwnSmem = 200 * 1024;       // dynamic shared memory
+// CTA 0: the resident line, then the sums [2][nodes]; their skewed lengths fit
+static_assert(fh_hline_res_smem(kOwnLine) + sizeof(double) * 2 * (kOwnMaxN + 2) <= kOwnSmem, "line and sums");
+
+__global__ void __launch_bounds__(kOwnThreads, 1)
+    k_h_pers_own(const fh_h_dev_inst *__restrict__ inst, int tstep0, int os0, int nsteps, double *D, long long ldd,
+                   int ldw, const double *__restrict__ Lb, const double *__restrict__ ibt,
+                   const double2 *__restrict__ lgt, double *U, double *Al, double *Bt, double *fF, double *fG,
+                   int *err) {
+  namespace cg = cooperative_groups;
+  cg::cluster_group cl = cg::this_cluster();
+  extern __shared__ double psm[];
+  __shared__ fh_hline_scan<kLineWarps> sc;
+  __shared__ double wst[3][2];  // CTA 0: psi weights of the newest and the current slot
+  __shared__ uint64_t bars[5];  // 0, 1: sums (CTA 0) or layers (owners); 2..4: psi weights
+  const int C = (int)cl.num_blocks(), r = (int)cl.block_rank();
+  const int b = blockIdx.x / C, t = threadIdx.x;
+  const fh_h_dev_inst I = inst[b];
+  const int np = I.N + 2, PW = (np + C - 2) / (C - 1);  // nodes per owner
+  const int Q = (np + PW - 1) / PW;                      // owners that have any
+  const uint32_t bar = fh_smem_u32(bars), smb = fh_smem_u32(psm);
+  if (t == 0) {
+    for (int k = 0; k < 5; ++k) fh_mbar_init(bar + 8 * k, 1);
+    fh_fence_mbar_init();
+  }
+  bool ok = true;
+  const bool psi = I.weights == FH_W_PSI;
+  if (r == 0) {
+    constexpr int L = fh_hline_len(kOwnLine);
+    fh_hline_keep keep;
+    keep.dn = psm + 3 * L;
+    keep.f = psm + 4 * L;
+    keep.g = psm + 5 * L;
+    keep.al = psm + 6 * L;
+    keep.pf = psm + 7 * L;
+    keep.pb = psm + 8 * L;
+    keep.lv = psm + 9 * L;
+    double *rp = keep.lv + kHLineLv * kOwnLine;  // sums [2][np]
+    if (t < kOwnLine) {  // the newest layer before the call
+      const bool has = os0 - I.ob >= 2;
+      const double *d = D + (long long)(has ? os0 - 2 : 0) * ldd + I.off;
+      for (int p = t; p < np; p += kOwnLine) keep.dn[fh_hsk(p)] = has ? __ldcg(d + p) : 0.0;
+    }
+    const double l1new = psi ? 0.0 : Lb[(long long)b * ldw + min(1, ldw - 1)];
+    cl.sync();
+    if (t < kOwnLine) {
+      for (int s = 0; s < nsteps; ++s) {
+        const int os = os0 + s - I.ob, par = s & 1, w3 = s % 3;
+        if (t == 0) {
+          fh_mbar_arrive_expect_tx(bar + 8 * par, 8 * np);
+          if (psi) fh_mbar_arrive_expect_tx(bar + 8 * (2 + w3), 16);
+        }
+        ok = fh_mbar_wait(bar + 8 * par, (s >> 1) & 1);
+        if (psi) ok &= fh_mbar_wait(bar + 8 * (2 + w3), (s / 3) & 1);
+        ok = fh_group_and(1, kOwnLine, ok);
+        if (!ok) break;
+        H_STAMP(0);
+        const double wnew = psi ? wst[w3][0] : l1new, DaW = I.Da * (psi ? wst[w3][1] : 1.0);
+        const double *rs = rp + par * np;
+        auto ts = [&](int i) { return os > 2 ? fma(wnew, keep.dn[fh_hsk(i)], rs[i]) : 0.0; };
+        auto sink = [&](int p, double dx) {
+          const int q = p / PW;
+          fh_st_async8(fh_mapa(smb, 1 + q) + 8 * (par * PW + p - q * PW), dx, fh_mapa(bar, 1 + q) + 8 * par);
+        };
+        keep.load = s == 0;
+        keep.last = s == nsteps - 1;
+        fh_hline<kLineWarps, false, true>(I, DaW, ts, U, Al, Bt, fF, fG, nullptr, os == 0, 0, nullptr, psm, sc, keep,
+                                          sink);
+        H_STAMP(1);
+        fh_group_bar(1, kOwnLine);  // the state is read by other threads next
+      }
+    }
+    if (!ok && t == 0) {
+      *(volatile int *)err = 1;
+      __threadfence_system();
+    }
+    cl.sync();
+    return;
+  }
+  if (r > Q) {
+    cl.sync();
+    cl.sync();
+    return;
+  }
+  // ---- owner of nodes [n0, n0 + nn)
+  const int n0 = (r - 1) * PW, nn = min(np, n0 + PW) - n0;
+  // dx [2][PW] | partial sums [256] | weights: psi [3][kw], L1 the lag table [kw] | layers [cap][PW]
+  const int kw = os0 - I.ob + nsteps + 1;
+  double *dxb = psm, *pt = dxb + 2 * PW, *wb = pt + kOwnSum, *hist = wb + (psi ? 3 : 1) * (size_t)kw;
+  const int cap = (int)((kOwnSmem / sizeof(double) - (size_t)(hist - psm)) / PW);
+  double *Dn = D + I.off + n0;
+  const int parts = max(1, kOwnSum / PW), rows = min(PW, kOwnSum);
+  const int i = t % rows, p = t / rows;  // node and run of a summing thread (nodes i, i + 256, ... when PW > 256)
+  // layers of the occupant before the call
+  const int have = max(os0 - I.ob - 1, 0);
+  for (int x = t; x < min(have, cap) * PW; x += kOwnThreads) {
+    const int k = x / PW, j = x - k * PW;
+    hist[x] = j < nn ? __ldcg(Dn + (long long)(I.ob + k) * ldd + j) : 0.0;
+  }
+  if (!psi)
+    for (int k = t; k < kw; k += kOwnThreads) wb[k] = k < ldw ? Lb[(long long)b * ldw + k] : 0.0;
+  auto older = [&](int s) { return max(os0 + s - I.ob - 2, 0); };  // slots but the newest at step s of the call
+  // in CTA 0
+  const uint32_t rbar = fh_mapa(bar, 0), rdst = fh_mapa(smb, 0) + 8 * (9 * fh_hline_len(kOwnLine) + kHLineLv * kOwnLine);
+  const uint32_t wdst = fh_mapa(fh_smem_u32(wst), 0);
+  // psi weights of step s of the call: this owner's share of the older slots to
+  // every owner, of the newest and the current one (last) to CTA 0
+  auto weights = [&](int s) {
+    const int tstep = tstep0 + s - I.tb, os = os0 + s - I.ob, K = older(s), sh = (K + 2 + Q - 1) / Q, w3 = s % 3;
+    const int k0 = (r - 1) * sh, k1 = min(K + 2, k0 + sh);
+    const double invX = 1.0 / (double)(tstep + 1);
+    for (int k = k0 + t - kOwnSum; k < k1; k += kOwnThreads - kOwnSum) {
+      const bool cur = k == K + 1;
+      const int slot = cur ? max(os - 1, 0) : k == K ? max(os - 2, 0) : k;
+      const double w = h_slot_weight(I, b, slot, cur, tstep, os, invX, ldw, Lb, ibt, lgt);
+      if (k < K) {
+        const uint32_t off = (uint32_t)(8 * ((wb - psm) + (size_t)w3 * kw + k));
+        for (int q = 1; q <= Q; ++q) fh_st_async8(fh_mapa(smb, q) + off, w, fh_mapa(bar, q) + 8 * (2 + w3));
+      } else {
+        fh_st_async8(wdst + 8 * (2 * w3 + k - K), w, rbar + 8 * (2 + w3));
+      }
+    }
+  };
+  cl.sync();
+  if (psi && t >= kOwnSum) weights(0);
+  for (int s = -2; s < nsteps; ++s) {
+    if (s >= 0) {  // the layer of step s: slot os0 + s - 1
+      H_STAMP(2);
+      if (t == 0) fh_mbar_arrive_expect_tx(bar + 8 * (s & 1), 8 * nn);
+      ok = fh_mbar_wait(bar + 8 * (s & 1), (s >> 1) & 1);
+      const int slot = os0 + s - 1;
+      if (ok && slot >= 0)
+        for (int j = t; j < nn; j += kOwnThreads) {
+          const double d = dxb[(s & 1) * PW + j];
+          if (slot - I.ob >= 0 && slot - I.ob < cap) hist[(slot - I.ob) * PW + j] = d;
+          Dn[(long long)slot * ldd + j] = d;
+        }
+    }
+    const int sn = s + 2;  // the step to prepare
+    if (psi && sn < nsteps) {
+      if (t == 0) fh_mbar_arrive_expect_tx(bar + 8 * (2 + sn % 3), 8 * older(sn));
+      ok &= fh_mbar_wait(bar + 8 * (2 + sn % 3), (sn / 3) & 1);
+    }
+    ok = __syncthreads_and(ok);
+    if (!ok) break;
+    if (sn >= nsteps) continue;
+    const int os = os0 + sn - I.ob, K = older(sn), per = (K + parts - 1) / parts;
+    if (t >= kOwnSum) {
+      if (psi && sn + 1 < nsteps) weights(sn + 1);
+    } else {
+      const double *w = wb + (psi ? (size_t)(sn % 3) * kw : 0);
+      auto wt = [&](int k) { return psi ? w[k] : w[os - 1 - k]; };  // L1: by the lag
+      for (int j = i; j < PW; j += rows) {  // one round unless PW > 256
+        double a0 = 0.0, a1 = 0.0;
+        if (p < parts && j < nn) {
+          // slot 0 carries no weight; even places from k to a0, odd ones to a1
+          int k = max(1, p * per);
+          const int k1 = min(K, (p + 1) * per), kc = k1 <= cap ? k1 : k + (max(cap - k, 0) & ~1);
+          for (; k + 2 <= kc; k += 2) {
+            a0 = fma(wt(k), hist[k * PW + j], a0);
+            a1 = fma(wt(k + 1), hist[(k + 1) * PW + j], a1);
+          }
+          if (k < kc) {
+            a0 = fma(wt(k), hist[k * PW + j], a0);
+            ++k;
+          }
+          const double *d = Dn + (long long)(I.ob + k) * ldd + j;
+          for (; k + 8 <= k1; k += 8, d += 8 * ldd) {
+            double v[8];
+#pragma unroll
+            for (int u = 0; u < 8; ++u) v[u] = __ldcg(d + u * ldd);
+#pragma unroll
+            for (int u = 0; u < 8; u += 2) {
+              a0 = fma(wt(k + u), v[u], a0);
+              a1 = fma(wt(k + u + 1), v[u + 1], a1);
+            }
+          }
+          for (; k + 2 <= k1; k += 2, d += 2 * ldd) {
+            a0 = fma(wt(k), __ldcg(d), a0);
+            a1 = fma(wt(k + 1), __ldcg(d + ldd), a1);
+          }
+          if (k < k1) a0 = fma(wt(k), __ldcg(d), a0);
+        }
+        double a = a0 + a1;
+        if (parts > 1) {
+          pt[t] = a;
+          fh_group_bar(2, kOwnSum);
+          if (p == 0) {
+            double v = 0.0;
+            for (int q = 1; q + 1 < parts; q += 2) {
+              a += pt[q * rows + j];
+              v += pt[(q + 1) * rows + j];
+            }
+            if (!(parts & 1)) a += pt[(parts - 1) * rows + j];
+            a += v;
+          }
+        }
+        if (p == 0 && j < nn) fh_st_async8(rdst + 8 * ((sn & 1) * np + n0 + j), a, rbar + 8 * (sn & 1));
+      }
+    }
+    H_STAMP(3);
+  }
+  if (!ok && t == 0) {
+    *(volatile int *)err = 1;
+    __threadfence_system();
+  }
+  cl.sync();
 }
 
 // ---------------------------------------------------- blocked history mode
@@ -1127,6 +1373,8 @@ static int h_set_smem_attrs(fh_ctx *ctx) {
   FH_CUDA_TRY(ctx, cudaFuncSetAttribute(k_h_line<kLineWarpsSmall, true>, at, sl));
   FH_CUDA_TRY(ctx, cudaFuncSetAttribute(k_h_persistent, at, (int)kPersSmem));
   FH_CUDA_TRY(ctx, cudaFuncSetAttribute(k_h_persistent, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+  FH_CUDA_TRY(ctx, cudaFuncSetAttribute(k_h_pers_own, at, (int)kOwnSmem));
+  FH_CUDA_TRY(ctx, cudaFuncSetAttribute(k_h_pers_own, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
   return FH_OK;
 }
 
@@ -1189,8 +1437,16 @@ int fh_h_batch_create(fh_ctx *ctx, int ninst, const fh_h_params *params_host, in
     off += seg;
   }
   B->Ptot = off;
-  if (ninst <= kPersMaxInst) B->pers_ctas = h_pers_ctas(ninst);
   int rc;
+  if (ninst <= kPersMaxInst) {
+    B->pers_ctas = h_pers_ctas(ninst);
+    if (cudaHostAlloc(&B->perr, sizeof(int), cudaHostAllocMapped) != cudaSuccess) {
+      cudaGetLastError();
+      delete B;
+      return fh_set_error(ctx, FH_ENOMEM, "fh_h_batch_create: no pinned memory");
+    }
+    *B->perr = 0;
+  }
   const size_t st = sizeof(double) * (size_t)B->Ptot;
   if ((rc = fh_alloc(ctx, B->inst, sizeof(fh_h_dev_inst) * ninst, false)) ||
       (rc = fh_alloc(ctx, B->tl_by[0], sizeof(fh_h_tile) * B->tiles_by[0].size(), false)) ||
@@ -1351,6 +1607,14 @@ int fh_h_batch_set_u(fh_h_batch *b, const double *U) {
   return h_reset_clocks(b);
 }
 
+// Waits for the stream; FH_ETIMEOUT once a wait of the persistent solve ran out.
+static int h_sync_check(fh_h_batch *b) {
+  fh_ctx *ctx = b->ctx;
+  FH_CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));
+  FH_REQUIRE(ctx, !b->perr || *(volatile int *)b->perr == 0, FH_ETIMEOUT, "fh_h_batch_step: a wait of the persistent solve ran out");
+  return FH_OK;
+}
+
 int fh_h_batch_get_u_host(fh_h_batch *b, double *U_host) {
   FH_REQUIRE(nullptr, b, FH_EINVAL, "null batch");
   fh_ctx *ctx = b->ctx;
@@ -1362,8 +1626,7 @@ int fh_h_batch_get_u_host(fh_h_batch *b, double *U_host) {
                                      cudaMemcpyDeviceToHost, ctx->stream));
     dst += (long long)cnt;
   }
-  FH_CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));
-  return FH_OK;
+  return h_sync_check(b);
 }
 
 int fh_h_batch_get_u_range_host(fh_h_batch *b, int first, int count, double *U_host) {
@@ -1378,8 +1641,7 @@ int fh_h_batch_get_u_range_host(fh_h_batch *b, int first, int count, double *U_h
                                      cudaMemcpyDeviceToHost, ctx->stream));
     dst += (long long)cnt;
   }
-  FH_CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));
-  return FH_OK;
+  return h_sync_check(b);
 }
 
 // The persistent path: FP64 history, no space-fractional instances, few
@@ -1406,12 +1668,22 @@ static int h_persistent_run(fh_h_batch *b, int nsteps) {
   at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
   cfg.attrs = at;
   cfg.numAttrs = 1;
+  // nodes or slots shared out (see the kernels)
+  bool own = b->max_steps <= kOwnMaxSteps;
+  for (const auto &p : b->hp) own = own && p.N <= kOwnMaxN;
+  if (own) {
+    cfg.blockDim = dim3(kOwnThreads);
+    cfg.dynamicSmemBytes = kOwnSmem;
+  }
   fh_prof_mark(ctx, FH_PROF_HISTORY, false);
-  FH_CUDA_TRY(ctx, cudaLaunchKernelEx(&cfg, k_h_persistent, (const fh_h_dev_inst *)b->inst.as<fh_h_dev_inst>(), b->tstep,
-                                      b->nsaved, nsteps, b->D.as<double>(), b->Ptot, b->max_weights,
-                                      (const double *)b->Lb.as<double>(), (const double *)b->ibt.as<double>(),
-                                      (const double2 *)b->lgt.as<double2>(), b->U.as<double>(), b->Al.as<double>(),
-                                      b->Bt.as<double>(), b->fF.as<double>(), b->fG.as<double>()));
+  auto launch = [&](auto kern, auto... last) {
+    return cudaLaunchKernelEx(&cfg, kern, (const fh_h_dev_inst *)b->inst.as<fh_h_dev_inst>(), b->tstep, b->nsaved,
+                              nsteps, b->D.as<double>(), b->Ptot, b->max_weights, (const double *)b->Lb.as<double>(),
+                              (const double *)b->ibt.as<double>(), (const double2 *)b->lgt.as<double2>(),
+                              b->U.as<double>(), b->Al.as<double>(), b->Bt.as<double>(), b->fF.as<double>(),
+                              b->fG.as<double>(), last...);
+  };
+  FH_CUDA_TRY(ctx, own ? launch(k_h_pers_own, b->perr) : launch(k_h_persistent));
   fh_prof_mark(ctx, FH_PROF_HISTORY, true);
   int rc = fh_after_launch(ctx, "k_h_persistent");
   if (rc) return rc;

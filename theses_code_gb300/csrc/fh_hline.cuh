@@ -135,7 +135,7 @@ __device__ __forceinline__ double fh_hl_scan(fh_aff G, double v, fh_aff *tot, do
     eb = 0.0;
   }
   if (lv) lv[5 * T + t] = ea;
-  __syncthreads();
+  fh_group_bar(1, T);
   double vw = v;
 #pragma unroll
   for (int j = 0; j < NW; ++j) {
@@ -166,7 +166,7 @@ __device__ __forceinline__ double fh_hl_scan_fixed(double g, double v, fh_aff *t
   if (lane == (REV ? 0 : 31)) tot[warp].b = g;
   double eb = REV ? __shfl_down_sync(0xffffffffu, g, 1) : __shfl_up_sync(0xffffffffu, g, 1);
   if (lane == (REV ? 31 : 0)) eb = 0.0;
-  __syncthreads();
+  fh_group_bar(1, T);
 #pragma unroll
   for (int j = 0; j < NW; ++j) {
     const int k = REV ? NW - 1 - j : j;
@@ -182,11 +182,14 @@ __device__ __forceinline__ double fh_hl_scan_fixed(double g, double v, fh_aff *t
 __host__ __device__ constexpr size_t fh_hline_res_smem(int threads) {
   return sizeof(double) * (9 * (size_t)fh_hline_len(threads) + (size_t)kHLineLv * threads);
 }
-// What fh_hline keeps there (RES): sDn skewed by node.
+// What fh_hline keeps there (RES): dn skewed by node.
 struct fh_hline_keep {
   double *dn, *f, *g, *al, *pf, *pb, *lv;
   bool load;  // state and factors from global memory (the call's first step)
   bool last;  // state to global memory (its last)
+};
+struct fh_hline_no_sink {
+  __device__ void operator()(int, double) const {}
 };
 
 // One step of instance I by the CTA (32 NW threads): DaW = Da wc, the weight
@@ -194,15 +197,17 @@ struct fh_hline_keep {
 // Al, f = g A and g of the constant-coefficient instances, written on the
 // instance's first step; Al and Bt scratch of lines of several panels share
 // fac_al and fac_bt.  sm: fh_hline_smem(32 NW) bytes.
+// Only the CTA's first 32 NW threads call (named barrier 1).
 // RES: a line of one panel whose state stays in shared memory between the
 // steps of a launch (keep); a constant-coefficient line keeps its factors, the
-// prefix products and the slopes of its scans there too.
-template <int NW, bool SPACE, bool RES, class TS>
+// prefix products and the slopes of its scans there too.  The new differences
+// go to keep.dn and sink(node, difference) instead of Dnew.
+template <int NW, bool SPACE, bool RES, class TS, class SINK = fh_hline_no_sink>
 __device__ __forceinline__ void fh_hline(const fh_h_dev_inst &I, double DaW, const TS &ts, double *__restrict__ U,
                                          double *__restrict__ fac_al, double *__restrict__ fac_bt,
                                          double *__restrict__ fac_f, double *__restrict__ fac_g, double *Dnew,
                                          bool first, int dfstore, const double *__restrict__ sV, double *sm,
-                                         fh_hline_scan<NW> &sc, const fh_hline_keep &keep) {
+                                         fh_hline_scan<NW> &sc, const fh_hline_keep &keep, const SINK &sink = SINK()) {
   constexpr int T = 32 * NW;
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
   double *sK = sm, *sO = sK + fh_hline_len(T), *sU = sO + fh_hline_len(T);
@@ -221,7 +226,7 @@ __device__ __forceinline__ void fh_hline(const fh_h_dev_inst &I, double DaW, con
   for (int pan = 0; pan < npan; ++pan) {
     i0 = 1 + pan * T * E;
     cnt = min(N - i0, T * E);
-    if (pan > 0) __syncthreads();
+    if (pan > 0) fh_group_bar(1, T);
     // ---- state and K(u) of nodes i0 - 1 .. i0 + cnt
     for (int k = t; k < cnt + 2; k += T) {
       double x;
@@ -234,7 +239,7 @@ __device__ __forceinline__ void fh_hline(const fh_h_dev_inst &I, double DaW, con
       sK[fh_hsk(k)] = fh_h_K(I, x);
     }
     if (RES && keep.load && t == 0) sU[fh_hsk(N + 1)] = u[N + 1];
-    __syncthreads();
+    fh_group_bar(1, T);
     // ---- right parts, in the reference's order, each operation rounded once
     for (int k = t; k < cnt; k += T) {
       const double x = sU[fh_hsk(k + 1)];
@@ -249,7 +254,7 @@ __device__ __forceinline__ void fh_hline(const fh_h_dev_inst &I, double DaW, con
       }
       sO[fh_hsk(k)] = __dadd_rn(om, __dmul_rn(I.Da, ts(i0 + k)));
     }
-    __syncthreads();
+    fh_group_bar(1, T);
     const int s0 = t * E;
     c = max(0, min(E, cnt - s0));
     const int i1 = i0 + s0;  // the thread's first equation
@@ -319,7 +324,7 @@ __device__ __forceinline__ void fh_hline(const fh_h_dev_inst &I, double DaW, con
       X.m10 = __shfl_up_sync(0xffffffffu, G.m10, 1);
       X.m11 = __shfl_up_sync(0xffffffffu, G.m11, 1);
       if (lane == 0) X = fh_mob{1.0, 0.0, 0.0, 1.0};
-      __syncthreads();
+      fh_group_bar(1, T);
       double dw = d0, qw = q0;  // (d : q) at the warp's first equation
       double dl = d0, ql = q0;
 #pragma unroll
@@ -414,7 +419,7 @@ __device__ __forceinline__ void fh_hline(const fh_h_dev_inst &I, double DaW, con
   double un = I.u_right;
   for (int pan = npan - 1; pan >= 0; --pan) {
     if (npan > 1) {
-      __syncthreads();
+      fh_group_bar(1, T);
       i0 = 1 + pan * T * E;
       cnt = min(N - i0, T * E);
       c = max(0, min(E, cnt - t * E));
@@ -447,7 +452,7 @@ __device__ __forceinline__ void fh_hline(const fh_h_dev_inst &I, double DaW, con
 #pragma unroll
     for (int e = 0; e < kHLineEq; ++e)
       if (e < c) sO[fh_hsk(s0 + e)] = fma(al[e], S, bt[e]);
-    __syncthreads();
+    fh_group_bar(1, T);
     // ---- the new state and history entry, coalesced; the ends of the line
     for (int k = t; k < cnt; k += T) {
       const double x = sO[fh_hsk(k)], dx = x - sU[fh_hsk(k + 1)];
@@ -455,6 +460,7 @@ __device__ __forceinline__ void fh_hline(const fh_h_dev_inst &I, double DaW, con
       if (RES) {
         sU[fh_hsk(k + 1)] = x;
         keep.dn[fh_hsk(k + 1)] = dx;
+        sink(i0 + k, dx);
       }
       if (Dnew) fh_h_store_diff(Dnew, o + i0 + k, dx, dfstore);
     }
@@ -464,6 +470,7 @@ __device__ __forceinline__ void fh_hline(const fh_h_dev_inst &I, double DaW, con
       if (RES) {
         sU[0] = x;
         keep.dn[0] = dx;
+        sink(0, dx);
       }
       if (Dnew) fh_h_store_diff(Dnew, o, dx, dfstore);
     }
@@ -479,6 +486,8 @@ __device__ __forceinline__ void fh_hline(const fh_h_dev_inst &I, double DaW, con
       sU[fh_hsk(N)] = sU[fh_hsk(N + 1)] = uN;
       keep.dn[fh_hsk(N)] = dN;
       keep.dn[fh_hsk(N + 1)] = dG;
+      sink(N, dN);
+      sink(N + 1, dG);
     }
     if (Dnew) {
       fh_h_store_diff(Dnew, o + N, dN, dfstore);
