@@ -486,15 +486,21 @@ static constexpr int kXThreads = kXGroup * kXLines;
 static constexpr int kYThreads = 512;  // four adjacent y lines per CTA
 static constexpr int kUnroll = 4;      // equations staged per thread per round
 
-// x half-step (fr_d_t_g_2d.cpp:2577-2590): four lines j per CTA.  A group of
-// 128 threads per line stages its forward maps into shared memory with
-// independent, coalesced loads (all four lines in one round trip), then warp
-// w solves line w (the four solving warps sit on the SM's four
-// sub-partitions, so the solves run in parallel), then the groups write the
-// half-step field Ch.  The boundary
-// nodes i = 0, N, N+1 are also written into C, which otherwise keeps the
-// full-step field.
-__global__ void __launch_bounds__(kXThreads) k_tg_xsweep(fh_tg_dev g, double *C, double *__restrict__ Ch,
+// Lines per CTA of the FP64 sweeps: four fill an SM's sub-partitions, but FP64
+// instructions of all of them share one pipe (19 cycles each), so where the lines
+// leave SMs idle fewer per CTA finish sooner.  251 x 187 (186 and 250 lines): x
+// 10.2 -> 9.4, y 10.8 -> 9.7 us with two instead of four, 500 steps 14.0 -> 12.9 ms.
+static inline int tg_lines(int lines) { return lines <= 152 ? 1 : lines <= 2 * 152 ? 2 : 4; }
+
+// x half-step (fr_d_t_g_2d.cpp:2577-2590): LINES lines j per CTA (tg_lines).  A
+// group of 128 threads per line stages its forward maps into shared memory with
+// independent, coalesced loads (all lines in one round trip), then warp
+// w solves line w (the solving warps sit on the SM's sub-partitions, so the
+// solves run in parallel), then the groups write the half-step field Ch.  The
+// boundary nodes i = 0, N, N+1 are also written into C, which otherwise keeps
+// the full-step field.
+template <int LINES>
+__global__ void __launch_bounds__(kXGroup *LINES) k_tg_xsweep(fh_tg_dev g, double *C, double *__restrict__ Ch,
                                                         const double *__restrict__ part, long long ldp, int splits,
                                                         const double *__restrict__ fax,
                                                         const double *__restrict__ gx,
@@ -506,7 +512,7 @@ __global__ void __launch_bounds__(kXThreads) k_tg_xsweep(fh_tg_dev g, double *C,
                                                         const double *__restrict__ dN) {
   extern __shared__ double sbuf[];
   const int warp = threadIdx.x >> 5;
-  const int line0 = 1 + blockIdx.x * kXLines;
+  const int line0 = 1 + blockIdx.x * LINES;
   const int N = g.sN;
   const int L = tg_line_stride(N);
   const double kst = -g.st * (cw[0] + 0.0), S2 = g.S * 0.5, st = g.st;
@@ -559,7 +565,7 @@ __global__ void __launch_bounds__(kXThreads) k_tg_xsweep(fh_tg_dev g, double *C,
     if (tg == 0 && line < g.M) pb[fh_sk(0)] = pbx[base];
   }
   __syncthreads();
-  if (warp < kXLines && line0 + warp < g.M) {
+  if (warp < LINES && line0 + warp < g.M) {
     double *fa = sbuf + (size_t)warp * 5 * L;
     // bt scratch reuses pf's slots only after pf is consumed: use a separate
     // region, the fb array, which the forward walk overwrites in place
@@ -579,12 +585,13 @@ __global__ void __launch_bounds__(kXThreads) k_tg_xsweep(fh_tg_dev g, double *C,
   }
 }
 
-// y half-step (fr_d_t_g_2d.cpp:2634-2648): four adjacent lines i per CTA so
-// that the strided column loads share 32-byte sectors; 128 threads stage each
+// y half-step (fr_d_t_g_2d.cpp:2634-2648): LINES adjacent lines i per CTA (four:
+// the strided column loads share 32-byte sectors); 128 threads stage each
 // line (kUnroll rows per thread in flight), warp w solves line w.  Reads the
 // half-step field Ch and the full-step field C, writes the new full-step field
 // into C and appends the difference D_j = C^{j+1} - C^j.
-__global__ void __launch_bounds__(kYThreads) k_tg_ysweep(fh_tg_dev g, double *C, const double *__restrict__ Ch,
+template <int LINES>
+__global__ void __launch_bounds__(kXGroup *LINES) k_tg_ysweep(fh_tg_dev g, double *C, const double *__restrict__ Ch,
                                                         double *__restrict__ Dj, const double *__restrict__ part,
                                                         long long ldp, int splits, const double *__restrict__ fay,
                                                         const double *__restrict__ gy,
@@ -598,11 +605,11 @@ __global__ void __launch_bounds__(kYThreads) k_tg_ysweep(fh_tg_dev g, double *C,
   const int warp = threadIdx.x >> 5;
   const int N = g.M;
   const int L = tg_line_stride(N);
-  const int i0 = 1 + blockIdx.x * 4;
+  const int i0 = 1 + blockIdx.x * LINES;
   const double kst = -g.st * (cw[1] + 0.0), kyh = cw[2], S2 = g.S * 0.5, st = g.st;
-  const int col = threadIdx.x & 3;
-  const int rg = threadIdx.x >> 2;  // row group 0..127
-  constexpr int kRows = kYThreads / 4;
+  const int col = threadIdx.x % LINES;
+  const int rg = threadIdx.x / LINES;  // row group 0..127
+  constexpr int kRows = kXGroup;
   const int line = i0 + col;
   const bool live = line < g.sN;
   double *fa = sbuf + (size_t)col * 6 * L, *fb = fa + L, *al = fb + L, *pf = al + L, *pb = pf + L, *cf = pb + L;
@@ -652,7 +659,7 @@ __global__ void __launch_bounds__(kYThreads) k_tg_ysweep(fh_tg_dev g, double *C,
   }
   if (live && rg == 0) pb[fh_sk(0)] = pby[line];  // node 0: lane 0's backward chunk
   __syncthreads();
-  if (warp < 4 && i0 + warp < g.sN) {
+  if (warp < LINES && i0 + warp < g.sN) {
     double *wfa = sbuf + (size_t)warp * 6 * L;
     fh_line_solve_prefix(N, wfa, wfa + L, wfa + 2 * L, wfa + 3 * L, wfa + 4 * L, 1.0, 0.0, wfa + L, wfa);
   }
@@ -2042,14 +2049,17 @@ static int tg_one_step(fh_tg_solver *s, int max_n, int *done) {
   };
   const double *dNp = s->massN ? s->dN.as<double>() : nullptr;
   if (s->massN && (rc = n1(0))) return rc;
-  const size_t smx = sizeof(double) * kXLines * 5 * (size_t)tg_line_stride(g.sN);
-  k_tg_xsweep<<<(unsigned)fh_ceil_div(g.M - 1, kXLines), kXThreads, smx, ctx->stream>>>(
+  const int lx = tg_lines(g.M - 1), ly = tg_lines(g.sN - 1);
+  const size_t smx = sizeof(double) * lx * 5 * (size_t)tg_line_stride(g.sN);
+  auto kx = lx == 1 ? k_tg_xsweep<1> : lx == 2 ? k_tg_xsweep<2> : k_tg_xsweep<4>;
+  kx<<<(unsigned)fh_ceil_div(g.M - 1, lx), kXGroup * lx, smx, ctx->stream>>>(
       g, s->C.as<double>(), s->Ch.as<double>(), sums, ldsums, splits, s->fax.as<double>(),
       s->gx.as<double>(), s->alx.as<double>(), s->pfx.as<double>(), s->pbx.as<double>(), cwj, farx, dNp);
   if ((rc = fh_after_launch(ctx, "k_tg_xsweep"))) return rc;
   if (s->massN && (rc = n1(1))) return rc;
-  const size_t smy = sizeof(double) * 4 * 6 * (size_t)tg_line_stride(g.M);
-  k_tg_ysweep<<<(unsigned)fh_ceil_div(g.sN - 1, 4), kYThreads, smy, ctx->stream>>>(
+  const size_t smy = sizeof(double) * ly * 6 * (size_t)tg_line_stride(g.M);
+  auto ky = ly == 1 ? k_tg_ysweep<1> : ly == 2 ? k_tg_ysweep<2> : k_tg_ysweep<4>;
+  ky<<<(unsigned)fh_ceil_div(g.sN - 1, ly), kXGroup * ly, smy, ctx->stream>>>(
       g, s->C.as<double>(), s->Ch.as<double>(), s->D.as<double>() + (s->one_layer() ? 0LL : (long long)j * g.P),
       sums, ldsums,
       splits, s->fay.as<double>(), s->gy.as<double>(), s->aly.as<double>(), s->pfy.as<double>(),
@@ -2084,7 +2094,8 @@ static int tg_set_smem_attrs(fh_ctx *ctx, int sN, int M) {
   FH_REQUIRE(ctx, ctx->device >= 0 && ctx->device < 64, FH_EINVAL, "fh_tg_create: device index");
   std::lock_guard<std::mutex> lk(mu);
   if (smx > cur_x[ctx->device]) {
-    FH_CUDA_TRY(ctx, cudaFuncSetAttribute(k_tg_xsweep, cudaFuncAttributeMaxDynamicSharedMemorySize, smx));
+    for (auto k : {k_tg_xsweep<1>, k_tg_xsweep<2>, k_tg_xsweep<4>})
+      FH_CUDA_TRY(ctx, cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smx));
     FH_CUDA_TRY(ctx, cudaFuncSetAttribute(k_tg_xsweep_df, cudaFuncAttributeMaxDynamicSharedMemorySize, smx));
     cur_x[ctx->device] = smx;
   }
@@ -2098,7 +2109,8 @@ static int tg_set_smem_attrs(fh_ctx *ctx, int sN, int M) {
     }
   }
   if (smy > cur_y[ctx->device]) {
-    FH_CUDA_TRY(ctx, cudaFuncSetAttribute(k_tg_ysweep, cudaFuncAttributeMaxDynamicSharedMemorySize, smy));
+    for (auto k : {k_tg_ysweep<1>, k_tg_ysweep<2>, k_tg_ysweep<4>})
+      FH_CUDA_TRY(ctx, cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smy));
     FH_CUDA_TRY(ctx, cudaFuncSetAttribute(k_tg_ysweep_df, cudaFuncAttributeMaxDynamicSharedMemorySize, smy));
     cur_y[ctx->device] = smy;
   }
