@@ -59,3 +59,12 @@ def test_far_rows_scale_free(mode, k):
     got, _ = _solve(33, 40, 100, mode, scale=2.0 ** k)
     keep = np.abs(base) > 1e-6 * np.max(np.abs(base))  # clear of the FP32 pairs' smallest numbers
     assert np.array_equal(np.ldexp(got, -k)[keep], base[keep])
+
+
+@pytest.mark.parametrize("mode", ["FH_TG_FP64", "FH_TG_DF64"])
+@pytest.mark.parametrize("sN,M", [(153, 154), (154, 153), (305, 306), (306, 305)])
+def test_sweep_lines_vs_oracle(sN, M, mode):
+    """One, two and four lines per CTA, the sums ahead among their idle warps."""
+    got, (p, V2, C0) = _solve(sN, M, 36, mode)
+    ref = np.asarray(O.tg_solve(p, V2, C0, 36)[0]).ravel()
+    assert float(np.max(np.abs(got - ref)) / np.max(np.abs(ref))) <= 1e-12

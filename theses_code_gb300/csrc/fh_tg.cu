@@ -105,6 +105,7 @@ struct fh_tg_solver {
   // FP64 and DF64 modes: the layers before the current 32-step block at FP64
   // accuracy on the tensor cores (null: every layer summed every step)
   fh_far64 *f64 = nullptr;
+  int ahead = -1;         // step whose sums the last sweeps have prepared (tg_ahead)
   int j0 = 0;             // first step of the current block (far rows valid when j0 > 0)
   long long ldfar = 0;
   fh_graph_cache graph;
@@ -492,6 +493,180 @@ static constexpr int kUnroll = 4;      // equations staged per thread per round
 // 10.2 -> 9.4, y 10.8 -> 9.7 us with two instead of four, 500 steps 14.0 -> 12.9 ms.
 static inline int tg_lines(int lines) { return lines <= 152 ? 1 : lines <= 2 * 152 ? 2 : 4; }
 
+// CTAs of a sweep: the lines', and beside sums ahead of four lines per CTA the
+// SMs those leave idle (512 x 512, DF64, 500 steps: 25.9 -> 25.1 ms; two lines per
+// CTA leave their own threads enough: 251 x 187 11.8 against 11.9 ms).
+static inline unsigned tg_sweep_ctas(int lines, int per, bool sums) {
+  const int n = (int)fh_ceil_div(lines, per);
+  return (unsigned)(sums && per == 4 && n < 152 ? 152 : n);
+}
+
+// Sums over the current block's layers in the block form (fh_far64.cu), one step
+// ahead: the sweeps of step j leave the sums of step j + 1 over the layers
+// [j0, j) (far rows included) to the warps that have no line to solve, half of
+// the points to each sweep, and add the newest layer to the sums of their own
+// step while they stage it.  A kernel of its own for the sums took 9.4 us of a
+// step's 28 at 251 x 187 (FP64) and 12.3 of 54 at 512 x 512 (DF64); 500 steps
+// 12.9 -> 12.1 and 27.0 -> 25.1 ms.  FP64:
+// the additions and their order are those of k_hist_sum; DF64: of k_hist_sum_df,
+// the newest layer last in both.
+constexpr int kAheadMax = kF64Block - 1;
+struct tg_ahead {
+  // newest layer of this step's sums (null: none) and its weights (x row; y row at ldw)
+  const double *dn = nullptr, *wn = nullptr;
+  // the next step's sums: K layers of D, weight rows W and W + ldw, starting from its far rows; rows out and out + P
+  int K = 0, ldw = 0, df = 0;
+  const double *D = nullptr, *W = nullptr, *far = nullptr;
+  long long P = 0, ldfar = 0;
+  double *out = nullptr;
+};
+
+// Double-float s += w d (the step of k_hist_sum_df).
+__device__ __forceinline__ void tg_acc(float2 w, float dh, float dl, float &sh, float &sl) {
+  const float ph = w.x * dh;
+  float pl = fmaf(w.x, dh, -ph);
+  pl = fmaf(w.x, dl, pl);
+  pl = fmaf(w.y, dh, pl);
+  const float t = sh + ph;
+  const float bb = t - sh;
+  const float e = (sh - (t - bb)) + (ph - bb);
+  sh = t;
+  sl += e + pl;
+}
+__device__ __forceinline__ float2 tg_wpair(double w) {
+  const float h = __double2float_rn(w);
+  return make_float2(h, __double2float_rn(w - (double)h));
+}
+// (double)x on the integer pipe (a conversion takes the FP64 pipe 19 cycles).
+__device__ __forceinline__ double tg_f2d(float x) {
+  const unsigned b = __float_as_uint(x), e = b & 0x7f800000u;
+  if (e == 0 && (b << 1) != 0) return (double)x;  // below the normal range
+  unsigned hi = ((b & 0x7fffffffu) >> 3) + 0x38000000u;
+  hi = e == 0 ? 0u : e == 0x7f800000u ? hi | 0x7ff00000u : hi;
+  return __hiloint2double((int)(hi | (b & 0x80000000u)), (int)(b << 29));
+}
+__device__ __forceinline__ double tg_pair(float2 v) { return tg_f2d(v.x) + tg_f2d(v.y); }
+
+// Weights of the sums ahead into shared memory (double, or pairs).
+__device__ __forceinline__ void tg_ahead_stage(const tg_ahead &a, double *wsm) {
+  const int t = threadIdx.x;
+  if (t < 2 * kAheadMax) {
+    const int m = t >= kAheadMax, k = t - m * kAheadMax;
+    if (k < a.K) {
+      const double w = a.W[(long long)m * a.ldw + k];
+      if (a.df)
+        reinterpret_cast<float2 *>(wsm)[t] = tg_wpair(w);
+      else
+        wsm[t] = w;
+    }
+  }
+}
+// This thread's share of half `half` of the points: nline CTAs have lines to
+// solve and sum with their threads from 32 LINES on, the others with all
+// threads and twice the points each.
+template <int LINES>
+__device__ __forceinline__ void tg_ahead_sums(const tg_ahead &a, int half, int nline, const double *wsm) {
+  const long long np = a.P / 2, hb = (np + 1) / 2, p0 = half ? hb : 0, p1 = half ? np : hb;
+  constexpr int T = kXGroup * LINES, TS = T - 32 * LINES;
+  const int solo = (int)blockIdx.x - nline, slots = nline * TS + ((int)gridDim.x - nline) * 2 * T;
+  const int slot = solo < 0 ? (int)blockIdx.x * TS + (int)threadIdx.x - 32 * LINES : nline * TS + solo * 2 * T + (int)threadIdx.x;
+  int r = 0;
+  for (long long q = p0 + slot; q < p1; r ^= 1, q += solo < 0 ? slots : r ? T : slots - T) {
+    const long long p = 2 * q;
+    if (!a.df) {
+      double s[2][2] = {};
+      if (a.far) {
+#pragma unroll
+        for (int m = 0; m < 2; ++m) {
+          const double2 f = *reinterpret_cast<const double2 *>(a.far + m * a.ldfar + p);
+          s[m][0] = f.x;
+          s[m][1] = f.y;
+        }
+      }
+      const double *d = a.D + p;
+      int k = 0;
+      auto add = [&](int k, double2 v) {
+#pragma unroll
+        for (int m = 0; m < 2; ++m) {
+          s[m][0] = fma(wsm[m * kAheadMax + k], v.x, s[m][0]);
+          s[m][1] = fma(wsm[m * kAheadMax + k], v.y, s[m][1]);
+        }
+      };
+      for (; k + 8 <= a.K; k += 8, d += 8 * a.P) {
+        double2 v[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) v[u] = __ldcg(reinterpret_cast<const double2 *>(d + u * a.P));
+#pragma unroll
+        for (int u = 0; u < 8; ++u) add(k + u, v[u]);
+      }
+      double2 v[8];
+#pragma unroll
+      for (int u = 0; u < 7; ++u)
+        v[u] = k + u < a.K ? __ldcg(reinterpret_cast<const double2 *>(d + u * a.P)) : make_double2(0.0, 0.0);
+#pragma unroll
+      for (int u = 0; u < 7; ++u)
+        if (k + u < a.K) add(k + u, v[u]);
+#pragma unroll
+      for (int m = 0; m < 2; ++m) *reinterpret_cast<double2 *>(a.out + m * a.P + p) = make_double2(s[m][0], s[m][1]);
+    } else {
+      const float2 *w = reinterpret_cast<const float2 *>(wsm);
+      float h[2][2] = {}, l[2][2] = {};
+      if (a.far) {
+#pragma unroll
+        for (int m = 0; m < 2; ++m) {
+          const float4 f = *reinterpret_cast<const float4 *>(a.far + m * a.ldfar + p);
+          h[m][0] = f.x;
+          l[m][0] = f.y;
+          h[m][1] = f.z;
+          l[m][1] = f.w;
+        }
+      }
+      const double *d = a.D + p;
+      auto add = [&](int k, float4 v) {
+#pragma unroll
+        for (int m = 0; m < 2; ++m) {
+          tg_acc(w[m * kAheadMax + k], v.x, v.y, h[m][0], l[m][0]);
+          tg_acc(w[m * kAheadMax + k], v.z, v.w, h[m][1], l[m][1]);
+        }
+      };
+      int k = 0;
+      for (; k + 8 <= a.K; k += 8, d += 8 * a.P) {
+        float4 v[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) v[u] = __ldcg(reinterpret_cast<const float4 *>(d + u * a.P));
+#pragma unroll
+        for (int u = 0; u < 8; ++u) add(k + u, v[u]);
+        if ((k & 15) == 8) {
+#pragma unroll
+          for (int m = 0; m < 2; ++m)
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {  // renormalise (fast two-sum)
+              const float x = h[m][e] + l[m][e];
+              l[m][e] = l[m][e] - (x - h[m][e]);
+              h[m][e] = x;
+            }
+        }
+      }
+      float4 v[8];
+#pragma unroll
+      for (int u = 0; u < 7; ++u)
+        v[u] = k + u < a.K ? __ldcg(reinterpret_cast<const float4 *>(d + u * a.P)) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+      for (int u = 0; u < 7; ++u)
+        if (k + u < a.K) add(k + u, v[u]);
+#pragma unroll
+      for (int m = 0; m < 2; ++m) {
+        float4 o;
+        o.x = h[m][0] + l[m][0];
+        o.y = l[m][0] - (o.x - h[m][0]);
+        o.z = h[m][1] + l[m][1];
+        o.w = l[m][1] - (o.z - h[m][1]);
+        *reinterpret_cast<float4 *>(a.out + m * a.P + p) = o;
+      }
+    }
+  }
+}
+
 // x half-step (fr_d_t_g_2d.cpp:2577-2590): LINES lines j per CTA (tg_lines).  A
 // group of 128 threads per line stages its forward maps into shared memory with
 // independent, coalesced loads (all lines in one round trip), then warp
@@ -509,20 +684,30 @@ __global__ void __launch_bounds__(kXGroup *LINES) k_tg_xsweep(fh_tg_dev g, doubl
                                                         const double *__restrict__ pbx,
                                                         const double *__restrict__ cw,
                                                         const float2 *__restrict__ far,
-                                                        const double *__restrict__ dN) {
+                                                        const double *__restrict__ dN, const tg_ahead ah) {
   extern __shared__ double sbuf[];
+  __shared__ double wsm[2 * kAheadMax];
   const int warp = threadIdx.x >> 5;
   const int line0 = 1 + blockIdx.x * LINES;
   const int N = g.sN;
   const int L = tg_line_stride(N);
   const double kst = -g.st * (cw[0] + 0.0), S2 = g.S * 0.5, st = g.st;
+  const double wn = ah.dn ? ah.wn[0] : 0.0;
+  const float2 wnp = tg_wpair(wn);
+  tg_ahead_stage(ah, wsm);
+  const int nline = (g.M - 2 + LINES) / LINES;
+  if ((int)blockIdx.x >= nline) {
+    __syncthreads();
+    tg_ahead_sums<LINES>(ah, 0, nline, wsm);
+    return;
+  }
   {
     const int ln = threadIdx.x / kXGroup, tg = threadIdx.x % kXGroup;
     const int line = line0 + ln;
     double *fa = sbuf + (size_t)ln * 5 * L, *fb = fa + L, *al = fb + L, *pf = al + L, *pb = pf + L;
     const long long base = (long long)line * g.ld;
     for (int r0 = 1; line < g.M && r0 < N; r0 += kXGroup * kUnroll) {
-      double ts[kUnroll], c[kUnroll], a[kUnroll], gi[kUnroll], l[kUnroll], qf[kUnroll], qb[kUnroll];
+      double ts[kUnroll], c[kUnroll], a[kUnroll], gi[kUnroll], l[kUnroll], qf[kUnroll], qb[kUnroll], nv[kUnroll];
 #pragma unroll
       for (int e = 0; e < kUnroll; ++e) {
         const int i = r0 + tg + e * kXGroup;
@@ -533,10 +718,18 @@ __global__ void __launch_bounds__(kXGroup *LINES) k_tg_xsweep(fh_tg_dev g, doubl
         l[e] = alx[id];
         qf[e] = pfx[id];
         qb[e] = pbx[id];
-        ts[e] = 0.0;
-        if (far) {
-          const float2 fp = far[id];
-          ts[e] = (double)fp.x + (double)fp.y;
+        ts[e] = far ? reinterpret_cast<const double *>(far)[id] : 0.0;  // a pair where there are far rows
+        nv[e] = ah.dn ? ah.dn[id] : 0.0;
+      }
+      if (far || ah.df) {
+#pragma unroll
+        for (int e = 0; e < kUnroll; ++e) {
+          float2 v = *reinterpret_cast<const float2 *>(&ts[e]);
+          if (ah.dn && ah.df) {
+            const float2 d = *reinterpret_cast<const float2 *>(&nv[e]);
+            tg_acc(wnp, d.x, d.y, v.x, v.y);
+          }
+          ts[e] = tg_pair(v);
         }
       }
       for (int s = 0; s < splits; ++s)
@@ -545,6 +738,9 @@ __global__ void __launch_bounds__(kXGroup *LINES) k_tg_xsweep(fh_tg_dev g, doubl
           const int i = r0 + tg + e * kXGroup;
           ts[e] += part[(long long)(2 * s) * ldp + base + (i < N ? i : 1)];
         }
+      if (ah.dn && !ah.df)
+#pragma unroll
+        for (int e = 0; e < kUnroll; ++e) ts[e] = fma(wn, nv[e], ts[e]);
 #pragma unroll
       for (int e = 0; e < kUnroll; ++e) {
         const int i = r0 + tg + e * kXGroup;
@@ -570,6 +766,8 @@ __global__ void __launch_bounds__(kXGroup *LINES) k_tg_xsweep(fh_tg_dev g, doubl
     // bt scratch reuses pf's slots only after pf is consumed: use a separate
     // region, the fb array, which the forward walk overwrites in place
     fh_line_solve_prefix(N, fa, fa + L, fa + 2 * L, fa + 3 * L, fa + 4 * L, 0.0, g.C1, fa + L, fa);
+  } else if (warp >= LINES && ah.K > 0) {
+    tg_ahead_sums<LINES>(ah, 0, nline, wsm);
   }
   __syncthreads();
   {
@@ -600,13 +798,23 @@ __global__ void __launch_bounds__(kXGroup *LINES) k_tg_ysweep(fh_tg_dev g, doubl
                                                         const double *__restrict__ pby,
                                                         const double *__restrict__ cw,
                                                         const float2 *__restrict__ far, int dfstore,
-                                                        const double *__restrict__ dN) {
+                                                        const double *__restrict__ dN, const tg_ahead ah) {
   extern __shared__ double sbuf[];
+  __shared__ double wsm[2 * kAheadMax];
   const int warp = threadIdx.x >> 5;
   const int N = g.M;
   const int L = tg_line_stride(N);
   const int i0 = 1 + blockIdx.x * LINES;
   const double kst = -g.st * (cw[1] + 0.0), kyh = cw[2], S2 = g.S * 0.5, st = g.st;
+  const double wn = ah.dn ? ah.wn[ah.ldw] : 0.0;
+  const float2 wnp = tg_wpair(wn);
+  tg_ahead_stage(ah, wsm);
+  const int nline = (g.sN - 2 + LINES) / LINES;
+  if ((int)blockIdx.x >= nline) {
+    __syncthreads();
+    tg_ahead_sums<LINES>(ah, 1, nline, wsm);
+    return;
+  }
   const int col = threadIdx.x % LINES;
   const int rg = threadIdx.x / LINES;  // row group 0..127
   constexpr int kRows = kXGroup;
@@ -614,7 +822,7 @@ __global__ void __launch_bounds__(kXGroup *LINES) k_tg_ysweep(fh_tg_dev g, doubl
   const bool live = line < g.sN;
   double *fa = sbuf + (size_t)col * 6 * L, *fb = fa + L, *al = fb + L, *pf = al + L, *pb = pf + L, *cf = pb + L;
   for (int r0 = 1; r0 < N; r0 += kRows * kUnroll) {
-    double ts[kUnroll], c[kUnroll], f[kUnroll], a[kUnroll], gi[kUnroll], l[kUnroll], qf[kUnroll], qb[kUnroll];
+    double ts[kUnroll], c[kUnroll], f[kUnroll], a[kUnroll], gi[kUnroll], l[kUnroll], qf[kUnroll], qb[kUnroll], nv[kUnroll];
 #pragma unroll
     for (int e = 0; e < kUnroll; ++e) {
       const int q = r0 + rg + e * kRows;
@@ -626,10 +834,18 @@ __global__ void __launch_bounds__(kXGroup *LINES) k_tg_ysweep(fh_tg_dev g, doubl
       l[e] = aly[id];
       qf[e] = pfy[id];
       qb[e] = pby[id];
-      ts[e] = 0.0;
-      if (far) {
-        const float2 fp = far[id];
-        ts[e] = (double)fp.x + (double)fp.y;
+      ts[e] = far ? reinterpret_cast<const double *>(far)[id] : 0.0;  // a pair where there are far rows
+      nv[e] = ah.dn ? ah.dn[id] : 0.0;
+    }
+    if (far || ah.df) {
+#pragma unroll
+      for (int e = 0; e < kUnroll; ++e) {
+        float2 v = *reinterpret_cast<const float2 *>(&ts[e]);
+        if (ah.dn && ah.df) {
+          const float2 d = *reinterpret_cast<const float2 *>(&nv[e]);
+          tg_acc(wnp, d.x, d.y, v.x, v.y);
+        }
+        ts[e] = tg_pair(v);
       }
     }
     for (int s = 0; s < splits; ++s)
@@ -638,6 +854,9 @@ __global__ void __launch_bounds__(kXGroup *LINES) k_tg_ysweep(fh_tg_dev g, doubl
         const int q = r0 + rg + e * kRows;
         ts[e] += part[(long long)(2 * s + 1) * ldp + (live ? line : 1) + (long long)(q < N ? q : 1) * g.ld];
       }
+    if (ah.dn && !ah.df)
+#pragma unroll
+      for (int e = 0; e < kUnroll; ++e) ts[e] = fma(wn, nv[e], ts[e]);
 #pragma unroll
     for (int e = 0; e < kUnroll; ++e) {
       const int q = r0 + rg + e * kRows;
@@ -662,6 +881,8 @@ __global__ void __launch_bounds__(kXGroup *LINES) k_tg_ysweep(fh_tg_dev g, doubl
   if (warp < LINES && i0 + warp < g.sN) {
     double *wfa = sbuf + (size_t)warp * 6 * L;
     fh_line_solve_prefix(N, wfa, wfa + L, wfa + 2 * L, wfa + 3 * L, wfa + 4 * L, 1.0, 0.0, wfa + L, wfa);
+  } else if (warp >= LINES && ah.K > 0) {
+    tg_ahead_sums<LINES>(ah, 1, nline, wsm);
   }
   __syncthreads();
   if (live) {
@@ -673,7 +894,7 @@ __global__ void __launch_bounds__(kXGroup *LINES) k_tg_ysweep(fh_tg_dev g, doubl
         const double dd = u - cf[fh_sk(q)];
         if (dfstore) {  // (hi, lo) FP32 pair, 2^-48 relative
           const float h = __double2float_rn(dd);
-          reinterpret_cast<float2 *>(Dj)[id] = make_float2(h, __double2float_rn(dd - (double)h));
+          reinterpret_cast<float2 *>(Dj)[id] = make_float2(h, __double2float_rn(dd - tg_f2d(h)));
         } else {
           Dj[id] = dd;
         }
@@ -1982,19 +2203,6 @@ static int tg_one_step(fh_tg_solver *s, int max_n, int *done) {
   if (!s->factor_fixed || j == 0)
     if ((rc = tg_factor(s, cwj))) return rc;
   if (s->dfsweep) return tg_step_df(s, Wj, cwj, max_n, done);
-  // far-history rows of this step (x row 2r, y row 2r + 1): (hi, lo) pairs in
-  // the DF64 mode, FP64 in the FP64 mode
-  const float2 *far = nullptr;
-  const double *far64 = nullptr;
-  long long ldfar = 0;
-  if (s->f64 && s->j0 > 0) {
-    ldfar = fh_far64_pitch(*s->f64);
-    const long long o = 2LL * (j - s->j0) * ldfar;
-    if (s->df)
-      far = static_cast<const float2 *>(fh_far64_rows(*s->f64)) + o;
-    else
-      far64 = static_cast<const double *>(fh_far64_rows(*s->f64)) + o;
-  }
   int splits = 0, kchunk = 0;
   if (s->ser_J && j >= 1) {
     fh_prof_mark(ctx, FH_PROF_HISTORY, false);
@@ -2014,30 +2222,69 @@ static int tg_one_step(fh_tg_solver *s, int max_n, int *done) {
     if (rc) return rc;
     splits = 1;
   }
-  if (knear >= 1) {
+  // rows of sums for the sweeps: FP64 (sums, splits) or, in the DF64 mode's block
+  // form, (hi, lo) pairs (farx, fary)
+  const double *sums = s->part.as<double>();
+  long long ldsums = g.P;
+  const float2 *farx = nullptr, *fary = nullptr;
+  tg_ahead ah;
+  ah.df = s->f64 && s->df;
+  ah.ldw = ldw;
+  ah.P = g.P;
+  if (s->f64) {
+    auto far = [&](int jj) -> const double * {  // far rows of step jj of this block (x row 2r, y row 2r + 1)
+      return s->j0 > 0 ? static_cast<const double *>(fh_far64_rows(*s->f64)) + 2LL * (jj - s->j0) * fh_far64_pitch(*s->f64)
+                       : nullptr;
+    };
+    auto rows = [&](int jj) { return s->part.as<double>() + (jj & 1) * 2 * g.P; };  // sums ahead of step jj
+    const double *base = far(j);
+    ldsums = fh_far64_pitch(*s->f64);
+    if (knear >= 2) {
+      if (s->ahead != j) {  // first step of a call
+        rc = s->df ? fh_launch_hist_sum_df_partials(
+                         ctx, 2, knear - 1, g.P, Wj + kstart, ldw,
+                         reinterpret_cast<const float2 *>(s->D.as<double>()) + (long long)kstart * g.P, g.P, 1,
+                         kAheadMax + 1, rows(j), g.P, reinterpret_cast<const float2 *>(base), ldsums, 1)
+                   : fh_launch_hist_sum_partials(ctx, 2, knear - 1, g.P, Wj + kstart, ldw,
+                                                 s->D.as<double>() + (long long)kstart * g.P, g.P, 1, kAheadMax + 1,
+                                                 rows(j), g.P, base, ldsums);
+        if (rc) return rc;
+      }
+      base = rows(j);
+      ldsums = g.P;
+    }
+    if (knear >= 1) {
+      ah.dn = s->D.as<double>() + (long long)(j - 1) * g.P;
+      ah.wn = Wj + j - 1;
+    }
+    if (s->df) {
+      farx = reinterpret_cast<const float2 *>(base);
+      fary = base ? farx + ldsums : nullptr;
+    } else if (base) {
+      sums = base;
+      splits = 1;
+    }
+    s->ahead = -1;
+    if (max_n > 1 && knear >= 1 && (j + 1) % kF64Block != 0) {
+      ah.K = knear;
+      ah.W = Wj + 2 * ldw + kstart;
+      ah.D = s->D.as<double>() + (long long)kstart * g.P;
+      ah.far = far(j + 1);
+      ah.ldfar = fh_far64_pitch(*s->f64);
+      ah.out = rows(j + 1);
+      s->ahead = j + 1;
+    }
+  } else if (knear >= 1) {
     fh_hist_plan(g.P, knear, s->max_splits, &splits, &kchunk);
     if (s->df)
       rc = fh_launch_hist_sum_df_partials(ctx, 2, knear, g.P, Wj + kstart, ldw,
                                           reinterpret_cast<const float2 *>(s->D.as<double>()) + (long long)kstart * g.P,
-                                          g.P, splits, kchunk, s->part.as<double>(), g.P, far, ldfar, 0);
+                                          g.P, splits, kchunk, s->part.as<double>(), g.P, nullptr, 0, 0);
     else
       rc = fh_launch_hist_sum_partials(ctx, 2, knear, g.P, Wj + kstart, ldw,
                                        s->D.as<double>() + (long long)kstart * g.P, g.P, splits, kchunk,
-                                       s->part.as<double>(), g.P, far64, ldfar);
+                                       s->part.as<double>(), g.P, nullptr, 0);
     if (rc) return rc;
-  }
-  // the near kernel has folded the far rows in; otherwise the sweeps add them
-  const float2 *farx = nullptr, *fary = nullptr;
-  if (far && !(knear >= 1 && s->df)) {
-    farx = far;
-    fary = far + ldfar;
-  }
-  const double *sums = s->part.as<double>();
-  long long ldsums = g.P;
-  if (far64 && knear < 1) {  // a block's first step: its far rows are the sums
-    sums = far64;
-    ldsums = ldfar;
-    splits = 1;
   }
   fh_prof_mark(ctx, FH_PROF_SWEEP, false);
   auto n1 = [&](int half) {
@@ -2052,18 +2299,18 @@ static int tg_one_step(fh_tg_solver *s, int max_n, int *done) {
   const int lx = tg_lines(g.M - 1), ly = tg_lines(g.sN - 1);
   const size_t smx = sizeof(double) * lx * 5 * (size_t)tg_line_stride(g.sN);
   auto kx = lx == 1 ? k_tg_xsweep<1> : lx == 2 ? k_tg_xsweep<2> : k_tg_xsweep<4>;
-  kx<<<(unsigned)fh_ceil_div(g.M - 1, lx), kXGroup * lx, smx, ctx->stream>>>(
+  kx<<<tg_sweep_ctas(g.M - 1, lx, ah.K > 0), kXGroup * lx, smx, ctx->stream>>>(
       g, s->C.as<double>(), s->Ch.as<double>(), sums, ldsums, splits, s->fax.as<double>(),
-      s->gx.as<double>(), s->alx.as<double>(), s->pfx.as<double>(), s->pbx.as<double>(), cwj, farx, dNp);
+      s->gx.as<double>(), s->alx.as<double>(), s->pfx.as<double>(), s->pbx.as<double>(), cwj, farx, dNp, ah);
   if ((rc = fh_after_launch(ctx, "k_tg_xsweep"))) return rc;
   if (s->massN && (rc = n1(1))) return rc;
   const size_t smy = sizeof(double) * ly * 6 * (size_t)tg_line_stride(g.M);
   auto ky = ly == 1 ? k_tg_ysweep<1> : ly == 2 ? k_tg_ysweep<2> : k_tg_ysweep<4>;
-  ky<<<(unsigned)fh_ceil_div(g.sN - 1, ly), kXGroup * ly, smy, ctx->stream>>>(
+  ky<<<tg_sweep_ctas(g.sN - 1, ly, ah.K > 0), kXGroup * ly, smy, ctx->stream>>>(
       g, s->C.as<double>(), s->Ch.as<double>(), s->D.as<double>() + (s->one_layer() ? 0LL : (long long)j * g.P),
       sums, ldsums,
       splits, s->fay.as<double>(), s->gy.as<double>(), s->aly.as<double>(), s->pfy.as<double>(),
-      s->pby.as<double>(), cwj, fary, s->df ? 1 : 0, dNp);
+      s->pby.as<double>(), cwj, fary, s->df ? 1 : 0, dNp, ah);
   fh_prof_mark(ctx, FH_PROF_SWEEP, true);
   if ((rc = fh_after_launch(ctx, "k_tg_ysweep"))) return rc;
   s->tstep++;
@@ -2487,6 +2734,7 @@ int fh_tg_step(fh_tg_solver *s, int nsteps) {
   FH_REQUIRE(ctx, nsteps >= 0, FH_EINVAL, "fh_tg_step: nsteps < 0");
   FH_REQUIRE(ctx, s->tstep + nsteps <= s->max_steps, FH_ENOMEM, "fh_tg_step: history full (%d + %d > %d)", s->tstep,
              nsteps, s->max_steps);
+  s->ahead = -1;
   if (ctx->graphs && s->tstep == 0 && nsteps > 1) {
     int rc = fh_graph_run(ctx, s->graph, nsteps, [&]() {
       for (int n = 0, d = 1; n < nsteps; n += d) {
