@@ -23,6 +23,7 @@
 #include "fh_slices.cuh"
 #include "fh_weights.cuh"
 #include "fh_hline.cuh"
+#include "fh_hline_df.cuh"
 #include "fh_cluster.cuh"
 
 // batched far contraction on the tensor cores (fh_blocked.cu)
@@ -82,6 +83,8 @@ struct fh_h_batch {
   // ring (slot t in row t mod 128)
   fh_hblk *hb = nullptr;
   fh_dbuf ring, far, cheb;  // cheb: interpolation tables of k_hb_wcheb
+  fh_dbuf wb, wcb;          // the block's near and current weights (k_h_weights_block)
+  int max_n = 0;            // the longest instance's N
   bool has_l1 = false;      // some instance has L1 weights (k_hb_weights covers every group)
   double *Wp(int par) const { return W.as<double>() + (long long)par * n * max_weights; }
   double *wcp(int par) const { return wc.as<double>() + (long long)par * n; }
@@ -110,8 +113,8 @@ static constexpr int kIbStride = 2 * kIbTerms + 4;
 // and wc[b], the weight of the current slot [tstep, tstep + 1].  The
 // reference's t = 0 term multiplies layer1 - layer1 (its layer pointer starts
 // at old[1], mt_minimal.cpp:913-917), so slot 0 carries weight 0.
-// Thread i of CTA (x, b) owns slot i = t_lo + x*128 + threadIdx.x (slots below
-// t_lo are not computed); i = max(os - 1, 0) is the current slot.
+// Thread i of CTA (x, b) owns slot i = x*128 + threadIdx.x; i = max(os - 1, 0)
+// is the current slot.
 // Weight of slot i of instance b at its step tstep with os saved layers
 // (cur: the current slot's weight, the factor of the newest difference);
 // invX = 1 / (tstep + 1).  The arithmetic of every weight kind as described
@@ -161,7 +164,7 @@ __device__ __forceinline__ double h_slot_weight(const fh_h_dev_inst &I, int b, i
   return fh_psi_int_t((double)t, (double)t + 1.0, (double)(tstep + 1), I.tau, I.alpha) * (1 - I.alpha);
 }
 
-__global__ void k_h_weights(const fh_h_dev_inst *__restrict__ inst, int n, int tstep_g, int os_g, int t_lo,
+__global__ void k_h_weights(const fh_h_dev_inst *__restrict__ inst, int n, int tstep_g, int os_g,
                             double *__restrict__ W_g, int ldw, double *__restrict__ wc, const double *__restrict__ Lb,
                             const double *__restrict__ ibt, const double2 *__restrict__ lgt, double invX_g) {
   const int b = blockIdx.y;
@@ -170,7 +173,7 @@ __global__ void k_h_weights(const fh_h_dev_inst *__restrict__ inst, int n, int t
   const int tstep = tstep_g - I.tb, os = os_g - I.ob;
   double *W = W_g + I.ob;
   const double invX = I.tb == 0 ? invX_g : 1.0 / (double)(tstep + 1);
-  const int i = t_lo + blockIdx.x * kHWeightThreads + threadIdx.x;
+  const int i = blockIdx.x * kHWeightThreads + threadIdx.x;
   const int nh = os > 1 ? os - 1 : 0;  // history slots
   if (i > nh) return;
   const bool cur = i == nh;
@@ -179,6 +182,33 @@ __global__ void k_h_weights(const fh_h_dev_inst *__restrict__ inst, int n, int t
     wc[b] = w;
   else
     W[(long long)b * ldw + i] = w;
+}
+
+// Blocked mode: the near weights of every step of the block whose older slots
+// are [0, K0), in one launch (2145 weights per instance; a launch per step held
+// at most 64 and took 19 us of its latency).  Row q is step os_first + q,
+// os_first = K0 + 1, or 0 in the first block, whose steps 0 and 1 both have no
+// slot: its history slots from K0 at wb[inst][q][.], its current weight at
+// wcb[q][inst].
+constexpr int kNearRows = 65, kNearLd = 64;
+__global__ void __launch_bounds__(kHWeightThreads) k_h_weights_block(
+    const fh_h_dev_inst *__restrict__ inst, int n, int K0, int max_steps, double *__restrict__ wb,
+    double *__restrict__ wcb, const double *__restrict__ Lb, int ldw, const double *__restrict__ ibt,
+    const double2 *__restrict__ lgt) {
+  const int b = blockIdx.y, x = blockIdx.x * kHWeightThreads + threadIdx.x;
+  int q = (int)((sqrtf(8.0f * x + 1.0f) - 1.0f) * 0.5f);  // x = q (q + 1) / 2 + r, r <= q
+  if (q * (q + 1) / 2 > x) --q;
+  if ((q + 1) * (q + 2) / 2 <= x) ++q;
+  const int r = x - q * (q + 1) / 2, os = (K0 > 0 ? K0 + 1 : 0) + q, K = max(os - 1, 0);
+  if (q >= kNearRows || os >= max_steps || K - K0 >= kNearLd || r > K - K0) return;
+  const fh_h_dev_inst I = inst[b];
+  const int tstep = os + 1;
+  const bool cur = r == K - K0;
+  const double w = h_slot_weight(I, b, K0 + r, cur, tstep, os, 1.0 / (double)(tstep + 1), ldw, Lb, ibt, lgt);
+  if (cur)
+    wcb[(long long)q * n + b] = w;
+  else
+    wb[((long long)b * kNearRows + q) * kNearLd + r] = w;
 }
 
 // Incomplete-beta series coefficients of every psi instance (fh_ib_tables).
@@ -395,6 +425,28 @@ __global__ void __launch_bounds__(32 * NW, NW == 4 ? 3 : 1) k_h_line(
                              fh_hline_keep{});
 }
 static constexpr int kLineWarps = 4, kLineWarpsSmall = 8;
+
+// The same in double-float, for the blocked mode: history sums and the new
+// layer as pairs.  A line out of its range runs the FP64 solve (its factors
+// are never kept here, so it always makes them).
+template <int NW>
+__global__ void __launch_bounds__(32 * NW, NW == 4 ? 4 : 2) k_h_line_df(
+    const fh_h_dev_inst *__restrict__ inst, double *__restrict__ U, const double *__restrict__ wc,
+    const float2 *__restrict__ part, double *__restrict__ Al, double *__restrict__ Bt, double *__restrict__ fF,
+    double *__restrict__ fG, float2 *__restrict__ Dnew) {
+  extern __shared__ double hsm[];
+  __shared__ union {
+    fh_hline_df_scan<NW> d;
+    fh_hline_scan<NW> f;
+  } sc;
+  const fh_h_dev_inst I = inst[blockIdx.x];
+  if (fh_hline_df<NW>(I, wc[blockIdx.x], part, U, Dnew, reinterpret_cast<float2 *>(hsm), sc.d)) return;
+  __syncthreads();
+  const float2 *pp = part + I.off;
+  fh_hline<NW, false, false>(I, I.Da * wc[blockIdx.x], [&](int i) { return fh_df_to_double(fh_df_from_pair(pp[i])); }, U,
+                             Al, Bt, fF, fG, reinterpret_cast<double *>(Dnew), true, 1, nullptr, hsm, sc.f,
+                             fh_hline_keep{});
+}
 
 // ------------------------------------------- persistent solves of small batches
 // Batches of few instances run all the steps of a call in one launch: one
@@ -1140,20 +1192,20 @@ __global__ void k_hb_weights(const fh_h_dev_inst *__restrict__ inst, int K, int 
 }
 
 // History sum of the blocked mode at one step: part[p] = far[p] + sum over
-// the near slots t in [t_lo, K) of W[inst][t] * ring[t mod 128][p], in
+// the near slots t in [t_lo, K) of W[inst][t - t_lo] * ring[t mod 128][p], in
 // double-float (the far row holds the contraction of the older slots; null
 // before the first block has one), two points per thread over the
-// per-instance tiles; written as FP64 for the line kernels.
+// per-instance tiles; written as FP64 or, for k_h_line_df, as pairs.
 __global__ void __launch_bounds__(kTileThreads) k_h_near_df(const fh_h_tile *__restrict__ tiles,
                                                             const fh_h_dev_inst *__restrict__ inst,
                                                             const float2 *__restrict__ ring, long long ldr, int t_lo,
                                                             int K, const double *__restrict__ W, int ldw,
                                                             const float2 *__restrict__ far,
-                                                            double *__restrict__ part) {
+                                                            double *__restrict__ part, bool pairs) {
   __shared__ float2 wsf2[kSlcK];
   const fh_h_tile T = tiles[blockIdx.x];
   const int nk = K - t_lo;  // < 64
-  const double *wrow = W + (long long)T.inst * ldw + t_lo;
+  const double *wrow = W + (long long)T.inst * ldw;
   for (int i = threadIdx.x; i < nk; i += blockDim.x) wsf2[i] = fh_df_pair(fh_df_from_double(wrow[i]));
   __syncthreads();
   const int q = threadIdx.x * 2;
@@ -1171,6 +1223,10 @@ __global__ void __launch_bounds__(kTileThreads) k_h_near_df(const fh_h_tile *__r
     const fh_df w = fh_df_from_pair(wsf2[k]);
     a0 = fh_df_fma(w, fh_df{v.x, v.y}, a0);
     a1 = fh_df_fma(w, fh_df{v.z, v.w}, a1);
+  }
+  if (pairs) {
+    *reinterpret_cast<float4 *>(part + p) = make_float4(a0.h, a0.l, a1.h, a1.l);
+    return;
   }
   double2 o;
   o.x = fh_df_to_double(a0);
@@ -1219,19 +1275,24 @@ static int h_hist(fh_h_batch *B, int ti, int K, int splits, int kchunk, const do
 }
 
 // Weights of step `tstep` (os saved layers) into the buffer pair `par`: the
-// history slots from t_lo on and the current weight.
-static int h_weights(fh_h_batch *B, int tstep, int os, int par, cudaStream_t st, int t_lo = 0) {
+// history slots and the current weight.
+static int h_weights(fh_h_batch *B, int tstep, int os, int par, cudaStream_t st) {
   fh_ctx *ctx = B->ctx;
   FH_REQUIRE(ctx, tstep + 1 < B->max_steps + 2, FH_EINVAL, "h_weights: step %d beyond the log table", tstep);
   const int nh = os > 1 ? os - 1 : 0;
-  if (t_lo > nh) t_lo = nh;
-  dim3 gw((unsigned)((nh - t_lo) / kHWeightThreads + 1), (unsigned)B->n);  // slots t_lo .. nh
+  dim3 gw((unsigned)(nh / kHWeightThreads + 1), (unsigned)B->n);  // slots 0 .. nh
   fh_prof_mark(ctx, FH_PROF_WEIGHTS, false, st);
-  k_h_weights<<<gw, kHWeightThreads, 0, st>>>(B->inst.as<fh_h_dev_inst>(), B->n, tstep, os, t_lo, B->Wp(par),
+  k_h_weights<<<gw, kHWeightThreads, 0, st>>>(B->inst.as<fh_h_dev_inst>(), B->n, tstep, os, B->Wp(par),
                                               B->max_weights, B->wcp(par), B->Lb.as<double>(), B->ibt.as<double>(),
                                               B->lgt.as<double2>(), 1.0 / (double)(tstep + 1));
   fh_prof_mark(ctx, FH_PROF_WEIGHTS, true, st);
   return fh_after_launch(ctx, "k_h_weights");
+}
+
+// Whether the lines are solved in double-float: the blocked mode, classical
+// derivative, lines of one panel.
+static bool h_line_in_df(const fh_h_batch *B) {
+  return B->mode == FH_H_BLOCKED && !B->space && B->max_n - 1 <= 32 * kLineWarps * kHLineEq;
 }
 
 // One step.  The weights depend on the step number only, so with `next` (and
@@ -1244,23 +1305,35 @@ static int h_one_step(fh_h_batch *B, bool next) {
   const int K = os >= 2 ? os - 1 : 0;
   const int par = B->tstep & 1;
   const bool blk = B->mode == FH_H_BLOCKED;
-  // blocked mode: slots below t_lo (whole 64-slot chunks) are in the far rows
-  auto near_lo = [&](int k) { return blk ? (k / kSlcK) * kSlcK : 0; };
-  const int t_lo = near_lo(K);
+  // blocked mode: slots below t_lo (whole 64-slot chunks) are in the far rows,
+  // this step is row q of its block's near weights
+  const int t_lo = blk ? (K / kSlcK) * kSlcK : 0, q = os - (t_lo > 0 ? t_lo + 1 : 0);
+  const double *wcur = B->wcp(par);
   int rc;
-  if (B->w_ready == B->tstep) {
+  if (blk) {
+    wcur = B->wcb.as<double>() + (long long)q * B->n;
+    if (q == 0) {
+      fh_prof_mark(ctx, FH_PROF_WEIGHTS, false);
+      k_h_weights_block<<<dim3((unsigned)fh_ceil_div(kNearRows * (kNearRows + 1) / 2, kHWeightThreads), (unsigned)B->n),
+                          kHWeightThreads, 0, ctx->stream>>>(
+          B->inst.as<fh_h_dev_inst>(), B->n, t_lo, B->max_steps, B->wb.as<double>(), B->wcb.as<double>(),
+          B->Lb.as<double>(), B->max_weights, B->ibt.as<double>(), B->lgt.as<double2>());
+      fh_prof_mark(ctx, FH_PROF_WEIGHTS, true);
+      if ((rc = fh_after_launch(ctx, "k_h_weights_block"))) return rc;
+    }
+  } else if (B->w_ready == B->tstep) {
     FH_CUDA_TRY(ctx, cudaStreamWaitEvent(ctx->stream, B->ev_w, 0));
-  } else if ((rc = h_weights(B, B->tstep, os, par, ctx->stream, t_lo))) {
+  } else if ((rc = h_weights(B, B->tstep, os, par, ctx->stream))) {
     return rc;
   }
   B->w_ready = -1;
   // only for small batches: in large ones the FP64-bound weights take SM
   // slots from the HBM-bound history sum (measured: 4096 instances, 5000
   // steps, the history sum fell from 92 % to 58 % of HBM beside them)
-  if (next && B->hs && B->n < kLineCtaMaxInst) {
+  if (!blk && next && B->hs && B->n < kLineCtaMaxInst) {
     FH_CUDA_TRY(ctx, cudaEventRecord(B->ev_main, ctx->stream));
     FH_CUDA_TRY(ctx, cudaStreamWaitEvent(B->hs, B->ev_main, 0));
-    if ((rc = h_weights(B, B->tstep + 1, os + 1, par ^ 1, B->hs, near_lo(os + 1 >= 2 ? os : 0)))) return rc;
+    if ((rc = h_weights(B, B->tstep + 1, os + 1, par ^ 1, B->hs))) return rc;
     FH_CUDA_TRY(ctx, cudaEventRecord(B->ev_w, B->hs));
     B->w_ready = B->tstep + 1;
   }
@@ -1294,8 +1367,8 @@ static int h_one_step(fh_h_batch *B, bool next) {
     const int ti = tile_shape_index(B->tile_threads);
     fh_prof_mark(ctx, FH_PROF_HISTORY, false);
     k_h_near_df<<<(unsigned)B->tiles_by[ti].size(), kTileShapes[ti], 0, ctx->stream>>>(
-        B->tl_by[ti].as<fh_h_tile>(), B->inst.as<fh_h_dev_inst>(), ring, B->Ptot, t_lo, K, B->Wp(par),
-        B->max_weights, t_lo >= kSlcK ? far + (long long)(K - t_lo) * B->Ptot : nullptr, B->part.as<double>());
+        B->tl_by[ti].as<fh_h_tile>(), B->inst.as<fh_h_dev_inst>(), ring, B->Ptot, t_lo, K,
+        B->wb.as<double>() + (long long)q * kNearLd, kNearRows * kNearLd, t_lo >= kSlcK ? far + (long long)(K - t_lo) * B->Ptot : nullptr, B->part.as<double>(), h_line_in_df(B));
     fh_prof_mark(ctx, FH_PROF_HISTORY, true);
     if ((rc = fh_after_launch(ctx, "k_h_near_df"))) return rc;
     splits = 1;
@@ -1320,11 +1393,19 @@ static int h_one_step(fh_h_batch *B, bool next) {
     const int dfs = (B->mode == FH_H_DF64 || blk) ? 1 : 0;
     auto line = [&](auto kern, int nw) {
       kern<<<(unsigned)B->n, 32 * nw, fh_hline_smem(32 * nw), ctx->stream>>>(
-          B->inst.as<fh_h_dev_inst>(), B->U.as<double>(), B->wcp(par), B->part.as<double>(), B->Ptot, splits,
+          B->inst.as<fh_h_dev_inst>(), B->U.as<double>(), wcur, B->part.as<double>(), B->Ptot, splits,
           B->Al.as<double>(), B->Bt.as<double>(), B->fF.as<double>(), B->fG.as<double>(), Dnew, os, dfs,
           B->sV.as<double>());
     };
-    if (B->n < kLineCtaMaxInst)
+    auto line_df = [&](auto kern, int nw) {
+      kern<<<(unsigned)B->n, 32 * nw, fh_hline_smem(32 * nw), ctx->stream>>>(
+          B->inst.as<fh_h_dev_inst>(), B->U.as<double>(), wcur, B->part.as<float2>(), B->Al.as<double>(),
+          B->Bt.as<double>(), B->fF.as<double>(), B->fG.as<double>(), reinterpret_cast<float2 *>(Dnew));
+    };
+    if (h_line_in_df(B))
+      B->n < kLineCtaMaxInst ? line_df(k_h_line_df<kLineWarpsSmall>, kLineWarpsSmall)
+                             : line_df(k_h_line_df<kLineWarps>, kLineWarps);
+    else if (B->n < kLineCtaMaxInst)
       B->space ? line(k_h_line<kLineWarpsSmall, true>, kLineWarpsSmall)
                : line(k_h_line<kLineWarpsSmall, false>, kLineWarpsSmall);
     else
@@ -1386,6 +1467,8 @@ static void h_fill_inst(const fh_h_params &p, long long off, fh_h_dev_inst &I) {
   I.spg = 1.0;
   I.spA = 0.0;
   I.kbf = 1.0;
+  I.dq = I.Da / (I.Dg * p.kc * p.cinv);
+  I.gq = 1.0 / (I.dL * I.Dg * p.cinv);
 }
 
 // Shared memory above 48 KiB: the eight-warp line solve and the persistent
@@ -1395,6 +1478,7 @@ static int h_set_smem_attrs(fh_ctx *ctx) {
   const int sl = (int)fh_hline_smem(32 * kLineWarpsSmall);
   FH_CUDA_TRY(ctx, cudaFuncSetAttribute(k_h_line<kLineWarpsSmall, false>, at, sl));
   FH_CUDA_TRY(ctx, cudaFuncSetAttribute(k_h_line<kLineWarpsSmall, true>, at, sl));
+  FH_CUDA_TRY(ctx, cudaFuncSetAttribute(k_h_line_df<kLineWarpsSmall>, at, sl));
   FH_CUDA_TRY(ctx, cudaFuncSetAttribute(k_h_persistent, at, (int)kPersSmem));
   FH_CUDA_TRY(ctx, cudaFuncSetAttribute(k_h_persistent, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
   FH_CUDA_TRY(ctx, cudaFuncSetAttribute(k_h_pers_own, at, (int)kOwnSmem));
@@ -1451,6 +1535,7 @@ int fh_h_batch_create(fh_ctx *ctx, int ninst, const fh_h_params *params_host, in
     fh_h_dev_inst &I = di[b];
     h_fill_inst(p, off, I);
     if (I.weights == FH_W_L1) B->has_l1 = true;
+    if (p.N > B->max_n) B->max_n = p.N;
     B->off.push_back(off);
     const int seg = ((p.N + 2) + 1) & ~1;
     B->cap.push_back(seg - 2);
@@ -1547,7 +1632,7 @@ int fh_h_batch_destroy(fh_h_batch *b) {
 long long fh_h_batch_device_bytes(const fh_h_batch *b) {
   if (!b) return -1;
   const fh_dbuf *bufs[] = {&b->inst, &b->U, &b->D, &b->W, &b->Lb, &b->ibt, &b->lgt, &b->wc, &b->part, &b->Al,
-                           &b->Bt, &b->fF, &b->fG, &b->wsp, &b->sV, &b->ring, &b->far, &b->cheb,
+                           &b->Bt, &b->fF, &b->fG, &b->wsp, &b->sV, &b->ring, &b->far, &b->cheb, &b->wb, &b->wcb,
                            &b->tl_by[0], &b->tl_by[1], &b->tl_by[2]};
   size_t s = 0;
   for (const fh_dbuf *d : bufs) s += d->bytes;
@@ -1920,6 +2005,8 @@ int fh_h_batch_set_mode(fh_h_batch *b, int mode) {
     if ((rc = fh_hblk_init(ctx, *b->hb, b->Ptot, kcap, b->n, tp0.data(), tin.data(), tnp.data(), (int)tp0.size())) ||
         (rc = fh_alloc(ctx, b->ring, sizeof(float2) * 128 * (size_t)b->Ptot)) ||
         (rc = fh_alloc(ctx, b->far, sizeof(float2) * kSlcK * (size_t)b->Ptot, false)) ||
+        (rc = fh_alloc(ctx, b->wb, sizeof(double) * kNearRows * kNearLd * (size_t)b->n, false)) ||
+        (rc = fh_alloc(ctx, b->wcb, sizeof(double) * kNearRows * (size_t)b->n, false)) ||
         (rc = fh_alloc(ctx, b->cheb, sizeof(double) * ct.size(), false)) ||
         (rc = cudaMemcpy(b->cheb.p, ct.data(), sizeof(double) * ct.size(), cudaMemcpyHostToDevice) != cudaSuccess
                   ? fh_set_error(ctx, FH_ECUDA, "fh_h_batch_set_mode: upload of the interpolation tables failed")
@@ -1929,6 +2016,8 @@ int fh_h_batch_set_mode(fh_h_batch *b, int mode) {
       b->ring.release();
       b->far.release();
       b->cheb.release();
+      b->wb.release();
+      b->wcb.release();
       return rc;
     }
     b->D.release();  // the full-precision history is not kept in this mode
@@ -1939,6 +2028,8 @@ int fh_h_batch_set_mode(fh_h_batch *b, int mode) {
     b->ring.release();
     b->far.release();
     b->cheb.release();
+    b->wb.release();
+    b->wcb.release();
     if ((rc = fh_alloc(ctx, b->D, sizeof(double) * (size_t)b->Ptot * (size_t)b->max_steps))) return rc;
   }
   b->mode = mode;

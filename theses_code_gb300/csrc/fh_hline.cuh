@@ -54,6 +54,8 @@ struct fh_h_dev_inst {
   // spg, spA = 1 - spg (0: classical second derivative), kbf = the
   // mt_psi_caputo factor kb(gamma, i-1, i, i) of A, B, R
   double spg, spA, kbf;
+  // row scale of fh_hline_df.cuh: Da / (Dg kc / c) and 1 / (dL Dg / c)
+  double dq, gq;
 };
 
 __device__ __forceinline__ double fh_h_K(const fh_h_dev_inst &I, double u) {
