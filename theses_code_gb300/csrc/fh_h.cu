@@ -985,14 +985,16 @@ static void hb_cheb_table(std::vector<double> &t) {
 // each of the m points X_j (h_psi_node_at; psi = t: (1 - x/X)^(1 - alpha)),
 // the 128 slot weights at each X_j, then per step r of the block the
 // interpolated weights sum_j L[r][j] w_j, sliced into W3/Ew as k_hb_weights
-// does.  Rows past the last step are zero.
+// does.  Rows past the last step are zero.  The 64 x 128 interpolated weights
+// and their slices are formed in double-float (2^-45; the slices hold 2^-32):
+// in FP64 they were 84 % of the kernel's FP64 work.
 __global__ void __launch_bounds__(256) k_hb_wcheb(const fh_h_dev_inst *__restrict__ inst, int K, int max_steps,
                                                   const double *__restrict__ ibt, const double2 *__restrict__ lgt,
                                                   const double *__restrict__ cheb, long long R, int Kcap,
                                                   __nv_bfloat16 *__restrict__ W3, int8_t *__restrict__ Ew) {
   __shared__ double sv[kHbChebMax][kHbGroupSlots + 1];
-  __shared__ double sw[kHbChebMax][kHbGroupSlots];
-  __shared__ double sL[kSlcK * kHbChebMax];
+  __shared__ float2 sw[kHbChebMax][kHbGroupSlots];
+  __shared__ float2 sL[kSlcK * kHbChebMax];
   __shared__ double sX[kHbChebMax][3];  // log X_j, 1/X_j, scale of X_j
   __shared__ double sn[kHbChebMax][kHbChebMax];  // 2D path: weights at the (slot, step) points
   __shared__ unsigned char slo[kHbChebMax][kHbGroupSlots + 1];
@@ -1002,7 +1004,7 @@ __global__ void __launch_bounds__(256) k_hb_wcheb(const fh_h_dev_inst *__restric
   const int x0 = G * kHbGroupSlots;
   const int m = min(hb_cheb_order(K + 2 - (x0 + kHbGroupSlots - 1)), kHbChebMax);
   const double *tab = cheb + (size_t)m * kHbChebBlock;
-  for (int i = threadIdx.x; i < kSlcK * kHbChebMax; i += blockDim.x) sL[i] = tab[i];
+  for (int i = threadIdx.x; i < kSlcK * kHbChebMax; i += blockDim.x) sL[i] = fh_df_pair(fh_df_bits(tab[i]));
   const double *Lc = ibt + (long long)b * kIbStride;
   const bool psi_t = I.beta == 1.0;
   if (threadIdx.x < m) {
@@ -1061,7 +1063,7 @@ __global__ void __launch_bounds__(256) k_hb_wcheb(const fh_h_dev_inst *__restric
       const double *Lk = sLt + k * kHbChebMax;
       double acc = 0.0;
       for (int ti = 0; ti < mt; ++ti) acc = fma(Lk[ti], sn[ti][j], acc);
-      sw[j][k] = acc;
+      sw[j][k] = fh_df_pair(fh_df_bits(acc));
     }
     __syncthreads();
   } else {
@@ -1094,23 +1096,24 @@ __global__ void __launch_bounds__(256) k_hb_wcheb(const fh_h_dev_inst *__restric
       diff = v0 - v1;
     else
       diff = (Lc[2 * kIbTerms] - v1) - v0;
-    sw[j][k] = x0 + k >= 1 ? sX[j][2] * diff : 0.0;  // slot 0 weighs nothing
+    sw[j][k] = fh_df_pair(fh_df_bits(x0 + k >= 1 ? sX[j][2] * diff : 0.0));  // slot 0 weighs nothing
   }
   __syncthreads();
   }
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int nchunks = K / kSlcK;
   for (int r = warp; r < kSlcK; r += blockDim.x >> 5) {
-    double w[4] = {0.0, 0.0, 0.0, 0.0};
+    float2 w[4] = {};
     if (K + r + 2 <= max_steps) {
-      const double *Lr = sL + r * kHbChebMax;
+      const float2 *Lr = sL + r * kHbChebMax;
       for (int j = 0; j < m; ++j) {
-        const double l = Lr[j];
+        const fh_df l = fh_df_from_pair(Lr[j]);
 #pragma unroll
-        for (int h = 0; h < 4; ++h) w[h] = fma(l, sw[j][lane + 32 * h], w[h]);
+        for (int h = 0; h < 4; ++h)
+          w[h] = fh_df_pair(fh_df_fma(l, fh_df_from_pair(sw[j][lane + 32 * h]), fh_df_from_pair(w[h])));
       }
     }
-    fh_slice_group_values(w, G, nchunks, (long long)b * kSlcK + r, R, Kcap, W3, Ew);
+    fh_slice_group_pairs(w, G, nchunks, (long long)b * kSlcK + r, R, Kcap, W3, Ew);
   }
 }
 
@@ -1188,7 +1191,10 @@ __global__ void k_hb_weights(const fh_h_dev_inst *__restrict__ inst, int K, int 
       w[h] = (live && k >= 1 && k < K) ? sc * diff : 0.0;
     }
   }
-  fh_slice_group_values(w, G, nchunks, m, R, Kcap, W3, Ew);
+  float2 wp[4];
+#pragma unroll
+  for (int h = 0; h < 4; ++h) wp[h] = fh_df_pair(fh_df_bits(w[h]));
+  fh_slice_group_pairs(wp, G, nchunks, m, R, Kcap, W3, Ew);
 }
 
 // History sum of the blocked mode at one step: part[p] = far[p] + sum over

@@ -114,6 +114,34 @@ __device__ __forceinline__ void fh_slice_group_values(const double (&w)[4], int 
   }
 }
 
+// The same for weights as double-float pairs, on the FP32 pipe (the FP64 form
+// takes ~20 instructions of that pipe per weight).
+__device__ __forceinline__ void fh_slice_group_pairs(const float2 (&w)[4], int G, int nchunks, long long m,
+                                                     long long nrows, int Kcap, __nv_bfloat16 *__restrict__ A3,
+                                                     int8_t *__restrict__ Ew) {
+  const int lane = threadIdx.x & 31;
+  const int c0 = 2 * G, nc = min(2, nchunks - c0);
+  float mx = 0.f;
+#pragma unroll
+  for (int h = 0; h < 4; ++h) mx = fmaxf(mx, fabsf(w[h].x));
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+  const int E = fh_point_exp(mx);
+  if (lane == 0)
+    for (int c = c0; c < c0 + nc; ++c) Ew[(long long)c * nrows + m] = (int8_t)E;
+  const float scale = fh_exp2f_int(-E);
+  const long long plane = nrows * (long long)Kcap;
+#pragma unroll
+  for (int h = 0; h < 4; ++h) {
+    if (h >= 2 * nc) break;
+    __nv_bfloat16 bs[kSlcN];
+    fh_slice_pair(w[h].x, w[h].y, scale, bs);
+    const long long o = m * Kcap + c0 * kSlcK + lane + 32 * h;
+#pragma unroll
+    for (int i = 0; i < kSlcN; ++i) A3[i * plane + o] = bs[i];
+  }
+}
+
 // One warp slices row m of group G: val(k) is the weight of layer k.
 template <class Val>
 __device__ __forceinline__ void fh_slice_row_group(const Val &val, int G, int nchunks, long long m, long long nrows,
