@@ -11,6 +11,7 @@
 // stores layer differences d_t = layer[t+1] - layer[t] at slot t for the
 // concatenated state (layer-major), so the history loads coalesce across
 // neighbouring nodes and instances.
+#include <algorithm>
 #include <cooperative_groups.h>
 
 #include <utility>
@@ -83,6 +84,7 @@ struct fh_h_batch {
   // ring (slot t in row t mod 128)
   fh_hblk *hb = nullptr;
   fh_dbuf ring, far, cheb;  // cheb: interpolation tables of k_hb_wcheb
+  fh_dbuf ord;              // instances by falling N
   fh_dbuf wb, wcb;          // the block's near and current weights (k_h_weights_block)
   int max_n = 0;            // the longest instance's N
   bool has_l1 = false;      // some instance has L1 weights (k_hb_weights covers every group)
@@ -405,23 +407,25 @@ __global__ void __launch_bounds__(256) k_h_space_v(const fh_h_dev_inst *__restri
 // The line solves of one step (fh_hline), one CTA of NW warps per instance.
 // Four warps at 152 instances or more, where the FP64 pipe is shared by
 // several CTAs per SM and fewer, longer chunks cost less in scans; eight
-// below, where each instance has an SM to itself.
+// below, where each instance has an SM to itself.  CTA x solves instance
+// ord[x], the longest first, so that no long line starts in the last wave.
 template <int NW, bool SPACE>
 __global__ void __launch_bounds__(32 * NW, NW == 4 ? 3 : 1) k_h_line(
     const fh_h_dev_inst *__restrict__ inst, double *__restrict__ U, const double *__restrict__ wc,
     const double *__restrict__ part, long long ldpart, int splits, double *__restrict__ Al, double *__restrict__ Bt,
     double *__restrict__ fF, double *__restrict__ fG, double *__restrict__ Dnew, int os, int dfstore,
-    const double *__restrict__ sV) {
+    const double *__restrict__ sV, const int *__restrict__ ord) {
   extern __shared__ double hsm[];
   __shared__ fh_hline_scan<NW> sc;
-  const fh_h_dev_inst I = inst[blockIdx.x];
+  const int b = ord[blockIdx.x];
+  const fh_h_dev_inst I = inst[b];
   const double *pp = part + I.off;
   auto ts = [&](int i) {  // split order
     double a = 0.0;
     for (int s = 0; s < splits; ++s) a += pp[(long long)s * ldpart + i];
     return a;
   };
-  fh_hline<NW, SPACE, false>(I, I.Da * wc[blockIdx.x], ts, U, Al, Bt, fF, fG, Dnew, os == I.ob, dfstore, sV, hsm, sc,
+  fh_hline<NW, SPACE, false>(I, I.Da * wc[b], ts, U, Al, Bt, fF, fG, Dnew, os == I.ob, dfstore, sV, hsm, sc,
                              fh_hline_keep{});
 }
 static constexpr int kLineWarps = 4, kLineWarpsSmall = 8;
@@ -433,17 +437,18 @@ template <int NW>
 __global__ void __launch_bounds__(32 * NW, NW == 4 ? 4 : 2) k_h_line_df(
     const fh_h_dev_inst *__restrict__ inst, double *__restrict__ U, const double *__restrict__ wc,
     const float2 *__restrict__ part, double *__restrict__ Al, double *__restrict__ Bt, double *__restrict__ fF,
-    double *__restrict__ fG, float2 *__restrict__ Dnew) {
+    double *__restrict__ fG, float2 *__restrict__ Dnew, const int *__restrict__ ord) {
   extern __shared__ double hsm[];
   __shared__ union {
     fh_hline_df_scan<NW> d;
     fh_hline_scan<NW> f;
   } sc;
-  const fh_h_dev_inst I = inst[blockIdx.x];
-  if (fh_hline_df<NW>(I, wc[blockIdx.x], part, U, Dnew, reinterpret_cast<float2 *>(hsm), sc.d)) return;
+  const int b = ord[blockIdx.x];
+  const fh_h_dev_inst I = inst[b];
+  if (fh_hline_df<NW>(I, wc[b], part, U, Dnew, reinterpret_cast<float2 *>(hsm), sc.d)) return;
   __syncthreads();
   const float2 *pp = part + I.off;
-  fh_hline<NW, false, false>(I, I.Da * wc[blockIdx.x], [&](int i) { return fh_df_to_double(fh_df_from_pair(pp[i])); }, U,
+  fh_hline<NW, false, false>(I, I.Da * wc[b], [&](int i) { return fh_df_to_double(fh_df_from_pair(pp[i])); }, U,
                              Al, Bt, fF, fG, reinterpret_cast<double *>(Dnew), true, 1, nullptr, hsm, sc.f,
                              fh_hline_keep{});
 }
@@ -1401,12 +1406,13 @@ static int h_one_step(fh_h_batch *B, bool next) {
       kern<<<(unsigned)B->n, 32 * nw, fh_hline_smem(32 * nw), ctx->stream>>>(
           B->inst.as<fh_h_dev_inst>(), B->U.as<double>(), wcur, B->part.as<double>(), B->Ptot, splits,
           B->Al.as<double>(), B->Bt.as<double>(), B->fF.as<double>(), B->fG.as<double>(), Dnew, os, dfs,
-          B->sV.as<double>());
+          B->sV.as<double>(), B->ord.as<int>());
     };
     auto line_df = [&](auto kern, int nw) {
       kern<<<(unsigned)B->n, 32 * nw, fh_hline_smem(32 * nw), ctx->stream>>>(
           B->inst.as<fh_h_dev_inst>(), B->U.as<double>(), wcur, B->part.as<float2>(), B->Al.as<double>(),
-          B->Bt.as<double>(), B->fF.as<double>(), B->fG.as<double>(), reinterpret_cast<float2 *>(Dnew));
+          B->Bt.as<double>(), B->fF.as<double>(), B->fG.as<double>(), reinterpret_cast<float2 *>(Dnew),
+          B->ord.as<int>());
     };
     if (h_line_in_df(B))
       B->n < kLineCtaMaxInst ? line_df(k_h_line_df<kLineWarpsSmall>, kLineWarpsSmall)
@@ -1564,6 +1570,7 @@ int fh_h_batch_create(fh_ctx *ctx, int ninst, const fh_h_params *params_host, in
   }
   const size_t st = sizeof(double) * (size_t)B->Ptot;
   if ((rc = fh_alloc(ctx, B->inst, sizeof(fh_h_dev_inst) * ninst, false)) ||
+      (rc = fh_alloc(ctx, B->ord, sizeof(int) * ninst, false)) ||
       (rc = fh_alloc(ctx, B->tl_by[0], sizeof(fh_h_tile) * B->tiles_by[0].size(), false)) ||
       (rc = fh_alloc(ctx, B->tl_by[1], sizeof(fh_h_tile) * B->tiles_by[1].size(), false)) ||
       (rc = fh_alloc(ctx, B->tl_by[2], sizeof(fh_h_tile) * B->tiles_by[2].size(), false)) || (rc = fh_alloc(ctx, B->U, st)) ||
@@ -1600,10 +1607,13 @@ int fh_h_batch_create(fh_ctx *ctx, int ninst, const fh_h_params *params_host, in
     lg[x] = make_double2(h, (double)(l - (long double)h));
   }
   B->di = di;
+  std::vector<int> ord(ninst);
+  for (int b = 0; b < ninst; ++b) ord[b] = b;
+  std::stable_sort(ord.begin(), ord.end(), [&](int x, int y) { return di[x].N > di[y].N; });
   cudaError_t e1 = cudaMemcpyAsync(B->inst.p, di.data(), sizeof(fh_h_dev_inst) * ninst, cudaMemcpyHostToDevice, ctx->stream);
   if (e1 == cudaSuccess)
     e1 = cudaMemcpyAsync(B->lgt.p, lg.data(), sizeof(double2) * lg.size(), cudaMemcpyHostToDevice, ctx->stream);
-  cudaError_t e2 = cudaSuccess;
+  cudaError_t e2 = cudaMemcpyAsync(B->ord.p, ord.data(), sizeof(int) * ninst, cudaMemcpyHostToDevice, ctx->stream);
   for (int k = 0; k < 3 && e2 == cudaSuccess; ++k)
     e2 = cudaMemcpyAsync(B->tl_by[k].p, B->tiles_by[k].data(), sizeof(fh_h_tile) * B->tiles_by[k].size(),
                          cudaMemcpyHostToDevice, ctx->stream);
@@ -1638,7 +1648,7 @@ int fh_h_batch_destroy(fh_h_batch *b) {
 long long fh_h_batch_device_bytes(const fh_h_batch *b) {
   if (!b) return -1;
   const fh_dbuf *bufs[] = {&b->inst, &b->U, &b->D, &b->W, &b->Lb, &b->ibt, &b->lgt, &b->wc, &b->part, &b->Al,
-                           &b->Bt, &b->fF, &b->fG, &b->wsp, &b->sV, &b->ring, &b->far, &b->cheb, &b->wb, &b->wcb,
+                           &b->Bt, &b->fF, &b->fG, &b->wsp, &b->sV, &b->ring, &b->far, &b->cheb, &b->wb, &b->wcb, &b->ord,
                            &b->tl_by[0], &b->tl_by[1], &b->tl_by[2]};
   size_t s = 0;
   for (const fh_dbuf *d : bufs) s += d->bytes;
