@@ -176,3 +176,22 @@ int fh_launch_hist_sum_df_partials(fh_ctx *ctx, int M, int K, long long P, const
                                    long long ldpart, const float2 *far, long long ldfar, int pair_out);
 // Chooses the split count for a K x P history sum given a partial-buffer capacity.
 void fh_hist_plan(long long P, int K, int max_splits, int *splits, int *kchunk);
+
+// Launch of k; dep: it may start when the kernel before it in the stream has
+// called fh_grid_start_next in every CTA (fh_common.cuh), and waits for that
+// kernel's end itself.
+template <class... P, class... A>
+cudaError_t fh_launch_after(bool dep, void (*k)(P...), unsigned grid, unsigned threads, size_t smem, cudaStream_t st,
+                            A &&...args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = dep ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, k, static_cast<A &&>(args)...);
+}

@@ -105,6 +105,7 @@ struct fh_tg_solver {
   // FP64 and DF64 modes: the layers before the current 32-step block at FP64
   // accuracy on the tensor cores (null: every layer summed every step)
   fh_far64 *f64 = nullptr;
+  long long swept = -1;   // ctx->launches after the last y sweep of this call
   int ahead = -1;         // step whose sums the last sweeps have prepared (tg_ahead)
   int j0 = 0;             // first step of the current block (far rows valid when j0 > 0)
   long long ldfar = 0;
@@ -493,6 +494,12 @@ static constexpr int kUnroll = 4;      // equations staged per thread per round
 // 10.2 -> 9.4, y 10.8 -> 9.7 us with two instead of four, 500 steps 14.0 -> 12.9 ms.
 static inline int tg_lines(int lines) { return lines <= 152 ? 1 : lines <= 2 * 152 ? 2 : 4; }
 
+// Shared memory of a sweep's CTA at least: one CTA per SM.  CTAs that start
+// before the sweep ahead of them has ended would otherwise take the SMs that are
+// free then two by two and share their FP64 pipes (251 x 187, 500 steps: 17.2 ms
+// against 11.9).
+static constexpr size_t kSweepSmem = 116 * 1024;
+
 // CTAs of a sweep: the lines', and beside sums ahead of four lines per CTA the
 // SMs those leave idle (512 x 512, DF64, 500 steps: 25.9 -> 25.1 ms; two lines per
 // CTA leave their own threads enough: 251 x 187 11.8 against 11.9 ms).
@@ -674,19 +681,25 @@ __device__ __forceinline__ void tg_ahead_sums(const tg_ahead &a, int half, int n
 // solves run in parallel), then the groups write the half-step field Ch.  The
 // boundary nodes i = 0, N, N+1 are also written into C, which otherwise keeps
 // the full-step field.
+// Each sweep starts while the one before it ends (fh_launch_after) and loads its
+// factors, which do not change; fields, sums and layers are read after
+// fh_grid_wait_prev, through pointers without __restrict__: loads declared
+// read-only could be moved above the wait.  251 x 187 FP64, 500 steps: 12.17 ->
+// 11.87 ms; 512 x 512 DF64: 25.2 -> 24.3 ms.
 template <int LINES>
 __global__ void __launch_bounds__(kXGroup *LINES) k_tg_xsweep(fh_tg_dev g, double *C, double *__restrict__ Ch,
-                                                        const double *__restrict__ part, long long ldp, int splits,
+                                                        const double *part, long long ldp, int splits,
                                                         const double *__restrict__ fax,
                                                         const double *__restrict__ gx,
                                                         const double *__restrict__ alx,
                                                         const double *__restrict__ pfx,
                                                         const double *__restrict__ pbx,
                                                         const double *__restrict__ cw,
-                                                        const float2 *__restrict__ far,
-                                                        const double *__restrict__ dN, const tg_ahead ah) {
+                                                        const float2 *far,
+                                                        const double *dN, const tg_ahead ah) {
   extern __shared__ double sbuf[];
   __shared__ double wsm[2 * kAheadMax];
+  fh_grid_start_next();
   const int warp = threadIdx.x >> 5;
   const int line0 = 1 + blockIdx.x * LINES;
   const int N = g.sN;
@@ -697,6 +710,7 @@ __global__ void __launch_bounds__(kXGroup *LINES) k_tg_xsweep(fh_tg_dev g, doubl
   tg_ahead_stage(ah, wsm);
   const int nline = (g.M - 2 + LINES) / LINES;
   if ((int)blockIdx.x >= nline) {
+    fh_grid_wait_prev();
     __syncthreads();
     tg_ahead_sums<LINES>(ah, 0, nline, wsm);
     return;
@@ -706,18 +720,29 @@ __global__ void __launch_bounds__(kXGroup *LINES) k_tg_xsweep(fh_tg_dev g, doubl
     const int line = line0 + ln;
     double *fa = sbuf + (size_t)ln * 5 * L, *fb = fa + L, *al = fb + L, *pf = al + L, *pb = pf + L;
     const long long base = (long long)line * g.ld;
-    for (int r0 = 1; line < g.M && r0 < N; r0 += kXGroup * kUnroll) {
-      double ts[kUnroll], c[kUnroll], a[kUnroll], gi[kUnroll], l[kUnroll], qf[kUnroll], qb[kUnroll], nv[kUnroll];
+    double a[kUnroll], gi[kUnroll], l[kUnroll], qf[kUnroll], qb[kUnroll];
+    auto tables = [&](int r0) {
 #pragma unroll
       for (int e = 0; e < kUnroll; ++e) {
         const int i = r0 + tg + e * kXGroup;
         const long long id = base + (i < N ? i : 1);
-        c[e] = C[id];
         a[e] = fax[id];
         gi[e] = gx[id];
         l[e] = alx[id];
         qf[e] = pfx[id];
         qb[e] = pbx[id];
+      }
+    };
+    if (line < g.M) tables(1);
+    fh_grid_wait_prev();
+    for (int r0 = 1; line < g.M && r0 < N; r0 += kXGroup * kUnroll) {
+      double ts[kUnroll], c[kUnroll], nv[kUnroll];
+      if (r0 > 1) tables(r0);
+#pragma unroll
+      for (int e = 0; e < kUnroll; ++e) {
+        const int i = r0 + tg + e * kXGroup;
+        const long long id = base + (i < N ? i : 1);
+        c[e] = C[id];
         ts[e] = far ? reinterpret_cast<const double *>(far)[id] : 0.0;  // a pair where there are far rows
         nv[e] = ah.dn ? ah.dn[id] : 0.0;
       }
@@ -789,18 +814,19 @@ __global__ void __launch_bounds__(kXGroup *LINES) k_tg_xsweep(fh_tg_dev g, doubl
 // half-step field Ch and the full-step field C, writes the new full-step field
 // into C and appends the difference D_j = C^{j+1} - C^j.
 template <int LINES>
-__global__ void __launch_bounds__(kXGroup *LINES) k_tg_ysweep(fh_tg_dev g, double *C, const double *__restrict__ Ch,
-                                                        double *__restrict__ Dj, const double *__restrict__ part,
+__global__ void __launch_bounds__(kXGroup *LINES) k_tg_ysweep(fh_tg_dev g, double *C, const double *Ch,
+                                                        double *__restrict__ Dj, const double *part,
                                                         long long ldp, int splits, const double *__restrict__ fay,
                                                         const double *__restrict__ gy,
                                                         const double *__restrict__ aly,
                                                         const double *__restrict__ pfy,
                                                         const double *__restrict__ pby,
                                                         const double *__restrict__ cw,
-                                                        const float2 *__restrict__ far, int dfstore,
-                                                        const double *__restrict__ dN, const tg_ahead ah) {
+                                                        const float2 *far, int dfstore,
+                                                        const double *dN, const tg_ahead ah) {
   extern __shared__ double sbuf[];
   __shared__ double wsm[2 * kAheadMax];
+  fh_grid_start_next();
   const int warp = threadIdx.x >> 5;
   const int N = g.M;
   const int L = tg_line_stride(N);
@@ -811,6 +837,7 @@ __global__ void __launch_bounds__(kXGroup *LINES) k_tg_ysweep(fh_tg_dev g, doubl
   tg_ahead_stage(ah, wsm);
   const int nline = (g.sN - 2 + LINES) / LINES;
   if ((int)blockIdx.x >= nline) {
+    fh_grid_wait_prev();
     __syncthreads();
     tg_ahead_sums<LINES>(ah, 1, nline, wsm);
     return;
@@ -821,19 +848,30 @@ __global__ void __launch_bounds__(kXGroup *LINES) k_tg_ysweep(fh_tg_dev g, doubl
   const int line = i0 + col;
   const bool live = line < g.sN;
   double *fa = sbuf + (size_t)col * 6 * L, *fb = fa + L, *al = fb + L, *pf = al + L, *pb = pf + L, *cf = pb + L;
+  double a[kUnroll], gi[kUnroll], l[kUnroll], qf[kUnroll], qb[kUnroll];
+  auto tables = [&](int r0) {
+#pragma unroll
+    for (int e = 0; e < kUnroll; ++e) {
+      const int q = r0 + rg + e * kRows;
+      const long long id = (live ? line : 1) + (long long)(q < N ? q : 1) * g.ld;
+      a[e] = fay[id];
+      gi[e] = gy[id];
+      l[e] = aly[id];
+      qf[e] = pfy[id];
+      qb[e] = pby[id];
+    }
+  };
+  tables(1);
+  fh_grid_wait_prev();
   for (int r0 = 1; r0 < N; r0 += kRows * kUnroll) {
-    double ts[kUnroll], c[kUnroll], f[kUnroll], a[kUnroll], gi[kUnroll], l[kUnroll], qf[kUnroll], qb[kUnroll], nv[kUnroll];
+    double ts[kUnroll], c[kUnroll], f[kUnroll], nv[kUnroll];
+    if (r0 > 1) tables(r0);
 #pragma unroll
     for (int e = 0; e < kUnroll; ++e) {
       const int q = r0 + rg + e * kRows;
       const long long id = (live ? line : 1) + (long long)(q < N ? q : 1) * g.ld;
       c[e] = Ch[id];
       f[e] = C[id];
-      a[e] = fay[id];
-      gi[e] = gy[id];
-      l[e] = aly[id];
-      qf[e] = pfy[id];
-      qb[e] = pby[id];
       ts[e] = far ? reinterpret_cast<const double *>(far)[id] : 0.0;  // a pair where there are far rows
       nv[e] = ah.dn ? ah.dn[id] : 0.0;
     }
@@ -2297,22 +2335,25 @@ static int tg_one_step(fh_tg_solver *s, int max_n, int *done) {
   const double *dNp = s->massN ? s->dN.as<double>() : nullptr;
   if (s->massN && (rc = n1(0))) return rc;
   const int lx = tg_lines(g.M - 1), ly = tg_lines(g.sN - 1);
-  const size_t smx = sizeof(double) * lx * 5 * (size_t)tg_line_stride(g.sN);
+  const size_t smx = std::max(kSweepSmem, sizeof(double) * lx * 5 * (size_t)tg_line_stride(g.sN));
   auto kx = lx == 1 ? k_tg_xsweep<1> : lx == 2 ? k_tg_xsweep<2> : k_tg_xsweep<4>;
-  kx<<<tg_sweep_ctas(g.M - 1, lx, ah.K > 0), kXGroup * lx, smx, ctx->stream>>>(
+  // each sweep loads its factors while the one before it ends, where nothing was
+  // launched between them
+  fh_launch_after(ctx->launches == s->swept, kx, tg_sweep_ctas(g.M - 1, lx, ah.K > 0), kXGroup * lx, smx, ctx->stream,
       g, s->C.as<double>(), s->Ch.as<double>(), sums, ldsums, splits, s->fax.as<double>(),
       s->gx.as<double>(), s->alx.as<double>(), s->pfx.as<double>(), s->pbx.as<double>(), cwj, farx, dNp, ah);
   if ((rc = fh_after_launch(ctx, "k_tg_xsweep"))) return rc;
   if (s->massN && (rc = n1(1))) return rc;
-  const size_t smy = sizeof(double) * ly * 6 * (size_t)tg_line_stride(g.M);
+  const size_t smy = std::max(kSweepSmem, sizeof(double) * ly * 6 * (size_t)tg_line_stride(g.M));
   auto ky = ly == 1 ? k_tg_ysweep<1> : ly == 2 ? k_tg_ysweep<2> : k_tg_ysweep<4>;
-  ky<<<tg_sweep_ctas(g.sN - 1, ly, ah.K > 0), kXGroup * ly, smy, ctx->stream>>>(
+  fh_launch_after(!s->massN, ky, tg_sweep_ctas(g.sN - 1, ly, ah.K > 0), kXGroup * ly, smy, ctx->stream,
       g, s->C.as<double>(), s->Ch.as<double>(), s->D.as<double>() + (s->one_layer() ? 0LL : (long long)j * g.P),
       sums, ldsums,
       splits, s->fay.as<double>(), s->gy.as<double>(), s->aly.as<double>(), s->pfy.as<double>(),
       s->pby.as<double>(), cwj, fary, s->df ? 1 : 0, dNp, ah);
   fh_prof_mark(ctx, FH_PROF_SWEEP, true);
   if ((rc = fh_after_launch(ctx, "k_tg_ysweep"))) return rc;
+  s->swept = ctx->launches;
   s->tstep++;
   return FH_OK;
 }
@@ -2334,8 +2375,8 @@ static int tg_publish(fh_tg_solver *s) {
 static int tg_set_smem_attrs(fh_ctx *ctx, int sN, int M) {
   static std::mutex mu;
   static int cur_x[64], cur_y[64];
-  const int smx = (int)(sizeof(double) * kXLines * 5 * (size_t)tg_line_stride(sN));
-  const int smy = (int)(sizeof(double) * 4 * 6 * (size_t)tg_line_stride(M));
+  const int smx = std::max((int)kSweepSmem, (int)(sizeof(double) * kXLines * 5 * (size_t)tg_line_stride(sN)));
+  const int smy = std::max((int)kSweepSmem, (int)(sizeof(double) * 4 * 6 * (size_t)tg_line_stride(M)));
   FH_REQUIRE(ctx, smx <= 200 * 1024 && smy <= 200 * 1024, FH_EINVAL,
              "fh_tg_create: grid too large for the sweeps (sN <= 1170, M <= 970)");
   FH_REQUIRE(ctx, ctx->device >= 0 && ctx->device < 64, FH_EINVAL, "fh_tg_create: device index");
@@ -2735,6 +2776,7 @@ int fh_tg_step(fh_tg_solver *s, int nsteps) {
   FH_REQUIRE(ctx, s->tstep + nsteps <= s->max_steps, FH_ENOMEM, "fh_tg_step: history full (%d + %d > %d)", s->tstep,
              nsteps, s->max_steps);
   s->ahead = -1;
+  s->swept = -1;
   if (ctx->graphs && s->tstep == 0 && nsteps > 1) {
     int rc = fh_graph_run(ctx, s->graph, nsteps, [&]() {
       for (int n = 0, d = 1; n < nsteps; n += d) {
