@@ -144,8 +144,8 @@ __device__ __forceinline__ fh_df fh_hl_scan_df(fh_daff G, fh_df v, fh_daff *tot)
 // fh_hline_smem(32 NW) bytes.  False, with nothing written, where the line is
 // left to the FP64 solve.
 template <int NW>
-__device__ __forceinline__ bool fh_hline_df(const fh_h_dev_inst &I, double wc, const float2 *__restrict__ part,
-                                            double *__restrict__ U, float2 *__restrict__ Dnew, float2 *sm,
+__device__ __forceinline__ bool fh_hline_df(const fh_h_dev_inst &I, double wc, const float2 *part, double *U,
+                                            float2 *__restrict__ Dnew, float2 *sm,
                                             fh_hline_df_scan<NW> &sc) {
   constexpr int T = 32 * NW;
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
