@@ -80,3 +80,40 @@ def test_not_finite():
     _check(W, D, live=np.r_[0:5, 8:64])
     got = _sum(W, D)
     assert np.all(np.isnan(got[:, 6])) and np.all(got[:, 5] == np.inf) and np.all(got[:, 7] == -np.inf)
+
+
+def test_batch_tiles():
+    """k_hist_tiles_dp: instances at the edges of its 128-node CTAs against the oracle, and a slot
+    whose earlier occupant left layers that are not finite (tolerance of the plain path, or twice the
+    distance by which the oracle moves under perturbations of 2^-53)."""
+    from oracle import oracle as O
+    from theses_code_gb300 import workloads
+    from theses_code_gb300._lib import Context
+    from theses_code_gb300.solvers import HSolverBatch
+    sizes = (2, 125, 126, 127, 128, 254, 255, 256, 513)
+    params, U0 = [], []
+    for k, N in enumerate(sizes):
+        p = dict(workloads.psi_batch(n=1, seed=40 + k)[0][0], N=N)
+        x = np.arange(N + 2) / N
+        u = 0.3 + 0.1 * np.cos(3 * x)
+        u[N:] = 0.0
+        params.append(p)
+        U0.append(u)
+    ctx = Context(0)
+    ctx.set_graphs(False)
+    s = HSolverBatch(ctx, params, 200)
+    s.set_persistent(False)
+    bad = [u.copy() for u in U0]
+    bad[4][3] = np.inf
+    s.set_u(bad)
+    s.calc_step(30)
+    s.restart(4, params[4], U0[4])
+    s.calc_step(100)
+    got = s.get_u()
+    s.close()
+    ctx.close()
+    for k, (p, u) in enumerate(zip(params, U0)):
+        n = 100 if k == 4 else 130
+        ref = O.h_solve(p, u, n)[0]
+        sens = np.max(np.abs(O.h_solve(dict(p, pert=2.0 ** -53), u, n)[0] - ref)) / np.max(np.abs(ref))
+        assert np.max(np.abs(got[k] - ref)) <= max(1e-12, 2.0 * sens) * np.max(np.abs(ref)), p["N"]

@@ -25,6 +25,7 @@
 #include "fh_weights.cuh"
 #include "fh_hline.cuh"
 #include "fh_hline_df.cuh"
+#include "fh_dp.cuh"
 #include "fh_cluster.cuh"
 
 // batched far contraction on the tensor cores (fh_blocked.cu)
@@ -307,6 +308,23 @@ __global__ void __launch_bounds__(kTileThreads) k_hist_tiles(const fh_h_tile *__
   o.x = a0;
   o.y = a1;
   *reinterpret_cast<double2 *>(part + (long long)s * ldpart + p) = o;
+}
+
+// The same for kDpMin layers and more (fh_dp.cuh): half a 256-node tile per CTA.
+__global__ void __launch_bounds__(kDpThreads, 6) k_hist_tiles_dp(const fh_h_tile *__restrict__ tiles,
+                                                                 const fh_h_dev_inst *__restrict__ inst,
+                                                                 const double *__restrict__ D, long long ldd, int K,
+                                                                 const double *__restrict__ W, int ldw, int kchunk,
+                                                                 double *__restrict__ part, long long ldpart) {
+  const fh_h_tile T = tiles[blockIdx.x >> 1];
+  const int q = ((int)blockIdx.x & 1) * kDpThreads + threadIdx.x, s = blockIdx.y, k0 = s * kchunk;
+  if (((int)blockIdx.x & 1) * kDpThreads >= T.len) return;  // whole CTA
+  const fh_h_dev_inst &I = inst[T.inst];
+  const long long p = I.off + T.start + q;
+  double acc[1] = {};
+  dp_sum<1>(D + (long long)k0 * ldd + p, ldd, max(0, I.ob - k0), min(K, k0 + kchunk) - k0,
+            W + (long long)T.inst * ldw + k0, ldw, q < T.len, acc);
+  if (q < T.len) part[(long long)s * ldpart + p] = acc[0];
 }
 
 // Double-float history ((hi, lo) FP32 pairs): the same tile sum with the
@@ -1273,7 +1291,18 @@ __global__ void __launch_bounds__(kTileThreads) k_h_near_df(const fh_h_tile *__r
 // K = 5000 without splits: 40 KB per CTA, 5 CTAs per SM, 71 % of HBM).
 static constexpr int kHistMaxChunk = 512;
 static constexpr int kHistMaxSplits = 64;  // partial-sum buffers of a batch
-static void h_plan(size_t ntiles, int K, int cap, int *splits, int *kchunk) {
+// FP64 sums of kDpMin layers and more: enough CTAs for ~4 waves of 6, chunks of
+// whole groups (1000 psi instances at 250 layers: one split instead of three).
+static bool h_dp(const fh_h_batch *B, int K) { return B->mode == FH_H_FP64 && K >= kDpMin; }
+static void h_plan(const fh_h_batch *B, int ti, int K, int cap, int *splits, int *kchunk) {
+  if (h_dp(B, K)) {
+    const long long ctas = 2LL * (long long)B->tiles_by[0].size();
+    const int s = (int)std::max(1LL, std::min((long long)std::min(cap, K / 32), (long long)fh_ceil_div(4LL * 152 * 6, ctas)));
+    *kchunk = (int)fh_ceil_div((int)fh_ceil_div(K, s), kDpGroup) * kDpGroup;
+    *splits = (int)fh_ceil_div(K, *kchunk);
+    return;
+  }
+  const size_t ntiles = B->tiles_by[ti].size();
   const long long target = 3LL * 152 * 8;
   int s = (int)fh_ceil_div(target, (long long)(ntiles > 0 ? ntiles : 1));
   if (s > cap) s = cap;
@@ -1290,6 +1319,12 @@ static void h_plan(size_t ntiles, int K, int cap, int *splits, int *kchunk) {
 // History sum over K layers with the weights W into part (tile shape ti).
 static int h_hist(fh_h_batch *B, int ti, int K, int splits, int kchunk, const double *W, cudaStream_t st) {
   fh_ctx *ctx = B->ctx;
+  if (h_dp(B, K)) {
+    k_hist_tiles_dp<<<dim3(2 * (unsigned)B->tiles_by[0].size(), (unsigned)splits), kDpThreads, 0, st>>>(
+        B->tl_by[0].as<fh_h_tile>(), B->inst.as<fh_h_dev_inst>(), B->D.as<double>(), B->Ptot, K, W, B->max_weights, kchunk,
+        B->part.as<double>(), B->Ptot);
+    return fh_after_launch(ctx, "k_hist_tiles_dp");
+  }
   const dim3 g((unsigned)B->tiles_by[ti].size(), (unsigned)splits);
   const size_t smem = sizeof(double) * (size_t)kchunk;
   FH_REQUIRE(ctx, smem <= 48 * 1024, FH_EINVAL, "history chunk too large");
@@ -1405,7 +1440,7 @@ static int h_one_step(fh_h_batch *B, bool next) {
     splits = 1;
   } else if (K > 0) {
     const int ti = tile_shape_index(B->tile_threads);
-    h_plan(B->tiles_by[ti].size(), K, B->split_cap, &splits, &kchunk);
+    h_plan(B, ti, K, B->split_cap, &splits, &kchunk);
     fh_prof_mark(ctx, FH_PROF_HISTORY, false);
     rc = h_hist(B, ti, K, splits, kchunk, B->Wp(par), ctx->stream);
     fh_prof_mark(ctx, FH_PROF_HISTORY, true);
@@ -1969,8 +2004,8 @@ int fh_h_batch_autotune(fh_h_batch *b, float *best_ms) {
   for (int ti = 0; ti < 3; ++ti)
     for (int ci = 0; ci < 3; ++ci) {
       int splits, kchunk;
-      h_plan(b->tiles_by[ti].size(), K, caps[ci] < b->max_splits ? caps[ci] : b->max_splits, &splits, &kchunk);
-      if ((size_t)kchunk * sizeof(double) > 48 * 1024) continue;
+      h_plan(b, ti, K, caps[ci] < b->max_splits ? caps[ci] : b->max_splits, &splits, &kchunk);
+      if (!h_dp(b, K) && (size_t)kchunk * sizeof(double) > 48 * 1024) continue;
       float ms = 0.f;
       for (int rep = 0; rep < 3; ++rep) {  // first repetition warms up
         cudaEventRecord(e0, ctx->stream);
