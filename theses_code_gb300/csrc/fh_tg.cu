@@ -1948,6 +1948,10 @@ __global__ void __launch_bounds__(kFuseThreads, 1) k_tg_sweeps_fused(const tg_fu
     }
     TG_STAMP(6);
   }
+  // the last CTA to leave, past every wait, clears the barrier's counts for the
+  // next launch (a memset between the launches took ~2 us of the stream each:
+  // 512 x 512, 2000 steps 67.4 -> 66.3 ms)
+  if (tid == 0 && atomicAdd(a.bar + 1, 1u) == nblk - 1) a.bar[0] = a.bar[1] = 0;
 }
 
 __global__ void k_to_pairs(const double *__restrict__ x, float2 *__restrict__ y, long long n) {
@@ -2114,7 +2118,6 @@ static int tg_step_df(fh_tg_solver *s, const double *Wj, const double *cwj, int 
         fa.rb0 = nullptr;
         fa.rb_step = fa.rb_xy = 0;
       }
-      FH_CUDA_TRY(ctx, cudaMemsetAsync(s->bar.p, 0, sizeof(unsigned), ctx->stream));
       cudaLaunchConfig_t cfg = {};
       cfg.gridDim = dim3((unsigned)s->fuse_blocks);
       cfg.blockDim = dim3(kFuseThreads);
@@ -2500,7 +2503,7 @@ int fh_tg_create(fh_ctx *ctx, const fh_tg_params *p, int max_steps, int mode, fh
         cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, ctx->device) == cudaSuccess &&
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_tg_sweeps_fused, kFuseThreads, smf) == cudaSuccess &&
         nblk <= nsm * per_sm) {
-      if ((rc = fh_alloc(ctx, s->bar, sizeof(unsigned))) || (rc = fh_alloc(ctx, s->derr, sizeof(int)))) {
+      if ((rc = fh_alloc(ctx, s->bar, 2 * sizeof(unsigned))) || (rc = fh_alloc(ctx, s->derr, sizeof(int)))) {
         delete s;
         return rc;
       }
@@ -2777,6 +2780,8 @@ int fh_tg_step(fh_tg_solver *s, int nsteps) {
              nsteps, s->max_steps);
   s->ahead = -1;
   s->swept = -1;
+  if (s->fused)  // the grid barrier's counts: zero after every launch that did not time out
+    FH_CUDA_TRY(ctx, cudaMemsetAsync(s->bar.p, 0, 2 * sizeof(unsigned), ctx->stream));
   if (ctx->graphs && s->tstep == 0 && nsteps > 1) {
     int rc = fh_graph_run(ctx, s->graph, nsteps, [&]() {
       for (int n = 0, d = 1; n < nsteps; n += d) {
