@@ -677,52 +677,6 @@ static int ab_one_step(fh_ab_solver *s, int max_n, int *done) {
   return FH_OK;
 }
 
-template <class A, int NW, int EM>
-static int ab_res_launch(fh_ab_solver *s, const fh_ab_res_args &a) {
-  fh_ctx *ctx = s->ctx;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(kAbResMaxCtas);
-  cfg.blockDim = dim3(kAbResThreads);
-  cfg.dynamicSmemBytes = ab_res_smem(NW, (s->m - 1 + 32 * NW - 1) / (32 * NW), kAbResMaxCtas);
-  cfg.stream = ctx->stream;
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeClusterDimension;
-  at[0].val.clusterDim.x = kAbResMaxCtas;
-  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
-  cfg.attrs = at;
-  cfg.numAttrs = 1;
-  fh_prof_mark(ctx, FH_PROF_SWEEP, false);
-  FH_CUDA_TRY(ctx, cudaLaunchKernelEx(&cfg, k_ab_resident<A, NW, EM>, a));
-  fh_prof_mark(ctx, FH_PROF_SWEEP, true);
-  return fh_after_launch(ctx, "k_ab_resident");
-}
-
-// Whether the device takes the resident solve's clusters (sixteen CTAs with
-// this much shared memory); sets the kernel's attributes.
-template <class A, int NW, int EM>
-static bool ab_res_ok(int m) {
-  const int E = (m - 1 + 32 * NW - 1) / (32 * NW);
-  if (E > EM) return false;
-  auto kern = k_ab_resident<A, NW, EM>;
-  const int smem = (int)ab_res_smem(NW, EM, kAbResMaxCtas);  // the largest size: solvers share the attribute
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(kAbResMaxCtas);
-  cfg.blockDim = dim3(kAbResThreads);
-  cfg.dynamicSmemBytes = (size_t)smem;
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeClusterDimension;
-  at[0].val.clusterDim.x = kAbResMaxCtas;
-  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
-  cfg.attrs = at;
-  cfg.numAttrs = 1;
-  int active = 0;
-  const bool ok = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) == cudaSuccess &&
-                  cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
-                  cudaOccupancyMaxActiveClusters(&active, kern, &cfg) == cudaSuccess && active >= 1;
-  cudaGetLastError();
-  return ok;
-}
-
 // The block-start work of step K is already enqueued; runs up to max_n steps, to
 // the end of the block at most.  Solving warps, double-float: the fewest that
 // take the line at four equations a thread, sixteen (five) for the longest.
