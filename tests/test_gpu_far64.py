@@ -68,3 +68,24 @@ def test_sweep_lines_vs_oracle(sN, M, mode):
     got, (p, V2, C0) = _solve(sN, M, 36, mode)
     ref = np.asarray(O.tg_solve(p, V2, C0, 36)[0]).ravel()
     assert float(np.max(np.abs(got - ref)) / np.max(np.abs(ref))) <= 1e-12
+
+
+@pytest.mark.parametrize("seed", [2, 3])
+def test_pair_rows_keep_their_precision(seed):
+    """DF64 against FP64 where a group's level sums cancel: a far row's pair holds 2^-48 of its sum,
+    and the steps add such errors with random signs (2-norm; bound 2^-47)."""
+    from theses_code_gb300 import _lib, workloads
+    from theses_code_gb300._lib import Context
+    from theses_code_gb300.solvers import TGSolver
+    alpha = float(np.random.default_rng(seed).uniform(0.5, 0.95))
+    p, V2, C0 = workloads.convection_2d(150, 90, alpha=alpha, tau=5e-4, d=0.1, seed=seed)
+    got = []
+    for mode in (_lib.FH_TG_DF64, _lib.FH_TG_FP64):
+        ctx = Context(0)
+        s = TGSolver(ctx, p, 300, mode)
+        s.set_state(V2, C0)
+        s.calc_step(300)
+        got.append(np.array(s.get_c()))
+        s.close()
+        ctx.close()
+    assert np.linalg.norm(got[0] - got[1]) <= 2.0 ** -47 * np.linalg.norm(got[1])

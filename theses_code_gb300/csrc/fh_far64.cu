@@ -198,8 +198,10 @@ __device__ __forceinline__ float f64_scalef(float x, int e) {  // |e| up to ~2^1
   return x * fh_exp2f_int(a) * fh_exp2f_int(b);
 }
 __device__ __forceinline__ void f64_store(float2 *o, float s0, float s1, float s2, int e, bool bad) {
-  const float t = s1 + s2, h = s0 + t;
-  float2 v = make_float2(f64_scalef(h, e), f64_scalef(t - (h - s0), e));
+  float h0, l0;  // s1 may be far above the last place of s0 (cancelling level sums)
+  f64_two_sum(s0, s1, h0, l0);
+  const float t = l0 + s2, h = h0 + t;
+  float2 v = make_float2(f64_scalef(h, e), f64_scalef(t - (h - h0), e));
   if (bad) v = make_float2(__int_as_float(0x7fc00000), 0.f);
   *o = v;
 }
