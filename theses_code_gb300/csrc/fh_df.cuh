@@ -76,6 +76,25 @@ __device__ __forceinline__ fh_df fh_df_div(fh_df a, fh_df b) {
   return fh_df_renorm(q1, q2);
 }
 
+// A double as a pair, by its bits (conversions run on the FP64 pipe); exact to
+// 2^-48.  Outside the range where both parts are normal: by conversion.
+__device__ __forceinline__ fh_df fh_df_bits(double x) {
+  const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x);
+  const int e = (hi >> 20) & 0x7ff;
+  if (e < 960 || e > 1140) return x == 0.0 ? fh_df{0.f, 0.f} : fh_df_from_double(x);
+  const unsigned sg = hi & 0x80000000u;
+  const float h = __uint_as_float(sg | (unsigned)(e - 896) << 23 | (hi & 0xfffffu) << 3 | lo >> 29);
+  const float l = (float)(int)(lo & 0x1fffffffu) * __uint_as_float(sg | (unsigned)(e - 948) << 23);  // 2^(e - 1075)
+  return fh_df_renorm(h, l);
+}
+// A pair as a double: one FP64 addition.
+__device__ __forceinline__ double fh_f2d_bits(float x) {
+  const unsigned b = __float_as_uint(x), e = b & 0x7f800000u;
+  if (e == 0 || e == 0x7f800000u) return (double)x;
+  return __hiloint2double((int)(((b & 0x7fffffffu) >> 3) + 0x38000000u | (b & 0x80000000u)), (int)(b << 29));
+}
+__device__ __forceinline__ double fh_df_to_double_bits(fh_df a) { return fh_f2d_bits(a.h) + fh_f2d_bits(a.l); }
+
 // Affine map x -> a x + b with double-float coefficients; compose(f2, f1) = f2 o f1.
 struct fh_daff {
   fh_df a, b;

@@ -33,25 +33,6 @@ __device__ const float2 kHdfTab[16] = {  // 2^(j/16)
     {0x1.ae89fap+0f, -0x1.a94b14p-26f}, {0x1.c199bep+0f, -0x1.3d56b2p-27f}, {0x1.d5818ep+0f, -0x1.822dbcp-27f},
     {0x1.ea4afap+0f, 0x1.52486cp-27f}};
 
-// A double as a pair, by its bits (conversions run on the FP64 pipe); exact to
-// 2^-48.  Outside the range where both parts are normal: by conversion.
-__device__ __forceinline__ fh_df fh_df_bits(double x) {
-  const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x);
-  const int e = (hi >> 20) & 0x7ff;
-  if (e < 960 || e > 1140) return x == 0.0 ? fh_df{0.f, 0.f} : fh_df_from_double(x);
-  const unsigned sg = hi & 0x80000000u;
-  const float h = __uint_as_float(sg | (unsigned)(e - 896) << 23 | (hi & 0xfffffu) << 3 | lo >> 29);
-  const float l = (float)(int)(lo & 0x1fffffffu) * __uint_as_float(sg | (unsigned)(e - 948) << 23);  // 2^(e - 1075)
-  return fh_df_renorm(h, l);
-}
-// A pair as a double: one FP64 addition.
-__device__ __forceinline__ double fh_f2d_bits(float x) {
-  const unsigned b = __float_as_uint(x), e = b & 0x7f800000u;
-  if (e == 0 || e == 0x7f800000u) return (double)x;
-  return __hiloint2double((int)(((b & 0x7fffffffu) >> 3) + 0x38000000u | (b & 0x80000000u)), (int)(b << 29));
-}
-__device__ __forceinline__ double fh_df_to_double_bits(fh_df a) { return fh_f2d_bits(a.h) + fh_f2d_bits(a.l); }
-
 // exp(x), |x| <= kHdfExp
 __device__ __forceinline__ fh_df fh_df_exp(fh_df x, const float2 *tab) {
   const float n = rintf(x.h * 0x1.715476p+4f);  // 16 / ln 2
