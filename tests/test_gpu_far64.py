@@ -89,3 +89,11 @@ def test_pair_rows_keep_their_precision(seed):
         s.close()
         ctx.close()
     assert np.linalg.norm(got[0] - got[1]) <= 2.0 ** -47 * np.linalg.norm(got[1])
+
+
+@pytest.mark.parametrize("steps", [1, 2, 3, 128, 129, 256, 257])
+def test_lag_weights_vs_oracle(steps):
+    """psi = t: the weight table from its lags, at the edges of the CTAs that make and copy it."""
+    got, (p, V2, C0) = _solve(12, 9, steps, "FH_TG_FP64")
+    ref = np.asarray(O.tg_solve(p, V2, C0, steps)[0]).ravel()
+    assert float(np.max(np.abs(got - ref)) / np.max(np.abs(ref))) <= 1e-12
