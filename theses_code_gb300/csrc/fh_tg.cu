@@ -263,16 +263,27 @@ __global__ void k_tg_factor_ratio(fh_tg_dev g, int dir, double *__restrict__ al,
 }
 
 // The whole factorization of one line per warp, for lines whose five
-// per-node arrays fit in shared memory: the coefficients A, B (lanes over the
+// per-node arrays fit in shared memory: the coefficients A, B, R (lanes over the
 // nodes, as k_tg_factor_coef), the continuant chain (lane 0, as k_tg_factor,
 // from shared memory instead of global loads on the serial path), the ratios
 // (lanes, as k_tg_factor_ratio) and the chunk prefix products (lane c its
 // chunk c, as k_tg_factor_prefix); the same operations, so the same values.
+// Both directions in one launch (blockIdx.y).  The chain is bound by its FP64
+// instructions, one per 67 cycles: three per node, with R made by the lanes and
+// the range looked up in the exponent field (512 x 512: 444 us in two launches
+// of seven per node -> 152 us).
 constexpr int kFactorLineArrays = 5;
-__global__ void __launch_bounds__(32) k_tg_factor_line(fh_tg_dev g, int dir, const double *__restrict__ V2,
-                                                       const double *__restrict__ cw, double *__restrict__ al,
-                                                       double *__restrict__ gg, double *__restrict__ fa,
-                                                       double *__restrict__ pf, double *__restrict__ pb) {
+struct tg_factor_out {
+  double *al, *gg, *fa, *pf, *pb;
+};
+__global__ void __launch_bounds__(32) k_tg_factor_line(fh_tg_dev g, const double *__restrict__ V2,
+                                                       const double *__restrict__ cw, tg_factor_out ox,
+                                                       tg_factor_out oy) {
+  const int dir = blockIdx.y;
+  if (1 + (int)blockIdx.x >= (dir == 0 ? g.M : g.sN)) return;
+  double *__restrict__ al = dir == 0 ? ox.al : oy.al, *__restrict__ gg = dir == 0 ? ox.gg : oy.gg;
+  double *__restrict__ fa = dir == 0 ? ox.fa : oy.fa, *__restrict__ pf = dir == 0 ? ox.pf : oy.pf;
+  double *__restrict__ pb = dir == 0 ? ox.pb : oy.pb;
   extern __shared__ double fsm[];
   const int line = 1 + blockIdx.x, lane = threadIdx.x;
   const int N = dir == 0 ? g.sN : g.M;
@@ -280,6 +291,7 @@ __global__ void __launch_bounds__(32) k_tg_factor_line(fh_tg_dev g, int dir, con
   const long long stride = dir == 0 ? 1 : g.ld;
   double *sA = fsm, *sB = sA + N, *sP = sB + N, *sQn = sP + N, *sQ = sQn + N;
   const double dl = dir == 0 ? g.dL : g.dLx;
+  const double kcur = dir == 0 ? cw[0] : cw[1];
   for (int i = 1 + lane; i < N; i += 32) {
     const long long id = base + i * stride;
     const double v2 = V2[id];
@@ -294,25 +306,32 @@ __global__ void __launch_bounds__(32) k_tg_factor_line(fh_tg_dev g, int dir, con
     }
     sA[i] = A;
     sB[i] = B;
+    sQn[i] = g.st * (kcur + 0.0) + A + B;  // R, until the chain has passed
   }
   __syncwarp();
   if (lane == 0) {
-    const double kcur = dir == 0 ? cw[0] : cw[1];
     double P = dir == 0 ? 0.0 : 1.0, Q = 1.0;
+    double A = sA[1], B = sB[1], R = sQn[1];
     for (int i = 1; i < N; ++i) {
-      const double A = sA[i], B = sB[i];
-      const double R = g.st * (kcur + 0.0) + A + B;
+      const int in = min(i + 1, N - 1);
+      const double An = sA[in], Bn = sB[in], Rn = sQn[in];
       const double Pn = B * Q, Qn = R * Q - A * P;
       sP[i] = Pn;
       sQn[i] = Qn;
       sQ[i] = Q;
       P = Pn;
       Q = Qn;
-      const double m = fabs(Q);
-      if (m > 0x1p400 || m < 0x1p-400) {
-        const int e = ilogb(Q);
-        P = scalbn(P, -e);
-        Q = scalbn(Q, -e);
+      A = An;
+      B = Bn;
+      R = Rn;
+      const int ex = (__double2hiint(Q) >> 20) & 0x7ff;
+      if (ex >= 1423 || ex < 623) {
+        const double m = fabs(Q);
+        if (m > 0x1p400 || m < 0x1p-400) {
+          const int e = ilogb(Q);
+          P = scalbn(P, -e);
+          Q = scalbn(Q, -e);
+        }
       }
     }
   }
@@ -2013,16 +2032,13 @@ static int tg_factor(fh_tg_solver *s, const double *cwj) {
   const size_t lsm = sizeof(double) * kFactorLineArrays * (size_t)std::max(g.sN, g.M);
   if (lsm <= 48 * 1024) {
     // one warp per line
-    k_tg_factor_line<<<(unsigned)(g.M - 1), 32, lsm, ctx->stream>>>(g, 0, s->V2.as<double>(), cwj,
-                                                                   s->alx.as<double>(), s->gx.as<double>(),
-                                                                   s->fax.as<double>(), s->pfx.as<double>(),
-                                                                   s->pbx.as<double>());
-    if ((rc = fh_after_launch(ctx, "k_tg_factor_line(x)"))) return rc;
-    k_tg_factor_line<<<(unsigned)(g.sN - 1), 32, lsm, ctx->stream>>>(g, 1, s->V2.as<double>(), cwj,
-                                                                    s->aly.as<double>(), s->gy.as<double>(),
-                                                                    s->fay.as<double>(), s->pfy.as<double>(),
-                                                                    s->pby.as<double>());
-    if ((rc = fh_after_launch(ctx, "k_tg_factor_line(y)"))) return rc;
+    const tg_factor_out ox{s->alx.as<double>(), s->gx.as<double>(), s->fax.as<double>(), s->pfx.as<double>(),
+                           s->pbx.as<double>()};
+    const tg_factor_out oy{s->aly.as<double>(), s->gy.as<double>(), s->fay.as<double>(), s->pfy.as<double>(),
+                           s->pby.as<double>()};
+    k_tg_factor_line<<<dim3((unsigned)std::max(g.M - 1, g.sN - 1), 2), 32, lsm, ctx->stream>>>(
+        g, s->V2.as<double>(), cwj, ox, oy);
+    if ((rc = fh_after_launch(ctx, "k_tg_factor_line"))) return rc;
   } else {
     // longer lines: the same passes as separate launches over global memory
     const unsigned cgrid = (unsigned)fh_ceil_div(g.P, 256);
