@@ -42,10 +42,11 @@
 // instructions per cycle and scheduler).
 // Waits are bounded; on expiry *err is set and nothing is stored.
 //
-// Measured, whole solves: 2D 251 x 187, 500 steps, FP64 34.9 -> 14.3 ms (the
-// sums of a step 49 -> ~9 us); 512 x 512, 500 steps, DF64 65.1 -> 28.3 ms; one
-// line of 1024 nodes, 2500 steps, FP64 55.2 -> 12.3 ms with the resident solve
-// of fh_ab.cu.  The results differ from the FP64 sums' by 1e-16 (relative).
+// Measured, whole solves, before and now (with the sweeps' changes since): 2D 251 x
+// 187, 500 steps, FP64 34.9 -> 11.7 ms (the sums of a step 49 -> ~9 us); 512 x
+// 512, 500 steps, DF64 65.1 -> 24.2 ms; one line of 1024 nodes, 2500 steps, FP64
+// 55.2 -> 12.0 ms with the resident solve of fh_ab.cu.  The results differ from the
+// FP64 sums' by 1e-16 (relative).
 #include <cuda_bf16.h>
 
 #include <algorithm>

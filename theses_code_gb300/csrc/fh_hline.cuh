@@ -23,7 +23,8 @@
 // FP64 warp instruction per ~67 cycles and sub-partition, and the same again
 // as latency).  Measured, 1000 psi instances of 64..1024 nodes: coefficients,
 // serial factors and sweeps took 94 + 432 + 148 us per step in three launches;
-// one launch of this form takes ~190 us (250-step solve 215.5 -> 97 ms).  The
+// one launch of this form takes 114 us, the longest lines first (250-step solve
+// 215 -> 79 ms with the history sums of fh_dp.cuh).  The
 // FP64 pipe bounds it: ~70 FP64 instructions per equation, of which the
 // exponential of K(u) and the division take half, and ~75 per warp for the
 // scans.
