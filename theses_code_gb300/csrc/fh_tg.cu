@@ -2411,7 +2411,9 @@ static int tg_one_step(fh_tg_solver *s, int max_n, int *done) {
   if (s->massN && (rc = n1(1))) return rc;
   const size_t smy = std::max(kSweepSmem, sizeof(double) * ly * 6 * (size_t)tg_line_stride(g.M));
   auto ky = ly == 1 ? k_tg_ysweep<1> : ly == 2 ? k_tg_ysweep<2> : k_tg_ysweep<4>;
-  fh_launch_after(!s->massN, ky, tg_sweep_ctas(g.sN - 1, ly, ah.K > 0), kXGroup * ly, smy, ctx->stream,
+  // (the y sweep's factors and weights must be older than the x sweep's launch too:
+  // not where a step makes them)
+  fh_launch_after(!s->massN && s->factor_fixed && s->wtab && j > 0, ky, tg_sweep_ctas(g.sN - 1, ly, ah.K > 0), kXGroup * ly, smy, ctx->stream,
       g, s->C.as<double>(), s->Ch.as<double>(), s->D.as<double>() + (s->one_layer() ? 0LL : (long long)j * g.P),
       sums, ldsums,
       splits, s->fay.as<double>(), s->gy.as<double>(), s->aly.as<double>(), s->pfy.as<double>(),
