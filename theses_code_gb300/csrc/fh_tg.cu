@@ -394,41 +394,6 @@ __global__ void k_tg_factor_prefix(fh_tg_dev g, int dir, const double *__restric
   }
 }
 
-// psi = t without a cut: the weights depend on the lag j - k only,
-//   Da tau^b / b ((l + h)^b - (l + h - 1)^b), b = 1 - alpha, h = 1/2 (x), 1 (y),
-// formed without cancellation.  k_tg_weights_lag computes the last row, which
-// holds every lag, and each step's three current weights; k_tg_weights_shift
-// copies it along the diagonals into the rows before it.  One power pair per
-// lag instead of per slot: 2000 steps 1365 -> 58 us
-// (512 x 512 blocked 66.4 -> 65.3 ms).
-__global__ void __launch_bounds__(128) k_tg_weights_lag(fh_tg_dev g, int nsteps, double *__restrict__ Wall, int ldw,
-                                                        double *__restrict__ cwall) {
-  const int i = blockIdx.x * 128 + threadIdx.x;
-  if (i >= nsteps) return;
-  double *W = Wall + (long long)(nsteps - 1) * 2 * ldw;
-  const double b = 1.0 - g.alpha;
-  if (i > 0) {
-    const double sc = g.Da * pow(g.tau, b) / b;
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const double x = (double)i + (h ? 1.0 : 0.5);
-      W[(long long)h * ldw + nsteps - 1 - i] = -sc * pow(x, b) * expm1(b * log1p(-1.0 / x));
-    }
-  }
-  const double jj = (double)i;
-  cwall[4 * i + 0] = g.Da * fh_psi_int_t(jj + 0.0, jj + 0.0 + 0.5, jj + 0.5, g.tau, g.alpha);
-  cwall[4 * i + 1] = g.Da * fh_psi_int_t(jj + 0.5, jj + 0.5 + 0.5, jj + 1.0, g.tau, g.alpha);
-  cwall[4 * i + 2] = g.Da * fh_psi_int_t(jj + 0.0, jj + 0.0 + 0.5, jj + 1.0, g.tau, g.alpha);
-}
-__global__ void __launch_bounds__(256) k_tg_weights_shift(int nsteps, double *__restrict__ Wall, int ldw) {
-  const int k = blockIdx.x * 256 + threadIdx.x, j = blockIdx.y;
-  if (k >= j) return;
-  const double *last = Wall + (long long)(nsteps - 1) * 2 * ldw + (nsteps - 1 - j);
-  double *W = Wall + (long long)j * 2 * ldw;
-  W[k] = last[k];
-  W[ldw + k] = last[ldw + k];
-}
-
 // All step weights of a solve in one launch: row j of Wall holds
 // [kb(k,0.5,0,1) for k < j | kb(k,1,0,1) for k < j] (x and y rows, pitch ldw),
 // cwall[4j..4j+2] the three current weights of step j.
@@ -2271,21 +2236,10 @@ static int tg_one_step(fh_tg_solver *s, int max_n, int *done) {
   if (s->wtab) {
     if (j == 0) {
       fh_prof_mark(ctx, FH_PROF_WEIGHTS, false);
-      const int ns = s->max_steps;
-      if (g.beta == 1.0 && !(g.hcut > 0.0)) {
-        k_tg_weights_lag<<<(unsigned)fh_ceil_div(ns, 128), 128, 0, ctx->stream>>>(g, ns, s->W.as<double>(), ldw,
-                                                                                 s->cw.as<double>());
-        if ((rc = fh_after_launch(ctx, "k_tg_weights_lag"))) return rc;
-        if (ns > 1) {
-          k_tg_weights_shift<<<dim3((unsigned)fh_ceil_div(ns, 256), (unsigned)(ns - 1)), 256, 0, ctx->stream>>>(
-              ns, s->W.as<double>(), ldw);
-          if ((rc = fh_after_launch(ctx, "k_tg_weights_shift"))) return rc;
-        }
-      } else {
-        dim3 gw((unsigned)fh_ceil_div(ns, kWallThreads), (unsigned)ns);
-        k_tg_weights_all<<<gw, kWallThreads, 0, ctx->stream>>>(g, ns, s->W.as<double>(), ldw, s->cw.as<double>());
-        if ((rc = fh_after_launch(ctx, "k_tg_weights_all"))) return rc;
-      }
+      dim3 gw((unsigned)fh_ceil_div(s->max_steps, kWallThreads), (unsigned)s->max_steps);
+      k_tg_weights_all<<<gw, kWallThreads, 0, ctx->stream>>>(g, s->max_steps, s->W.as<double>(), ldw,
+                                                            s->cw.as<double>());
+      if ((rc = fh_after_launch(ctx, "k_tg_weights_all"))) return rc;
       if (s->mid_tc) {
         k_tg_mid_wslice<<<(unsigned)fh_ceil_div(s->max_steps, kSub), 128, 0, ctx->stream>>>(
             s->W.as<double>(), ldw, s->max_steps, s->mws.as<uint8_t>(), s->mwe.as<int8_t>());
