@@ -32,6 +32,7 @@
 #include "fh_internal.h"
 #include "fh_common.cuh"
 #include "fh_linescan.cuh"
+#include "fh_quot.cuh"
 #include "fh_sm100.cuh"
 #include "fh_slices.cuh"
 #include "fh_weights.cuh"
@@ -1579,21 +1580,16 @@ __device__ __forceinline__ fh_daff tg_group_scan(fh_daff f, fh_daff *sm, int bar
 
 // The end condition u_N = bt_{N-1} / (1 - al_{N-1}): x = 1 - al_{N-1} and the
 // reciprocal of its head, once per launch.  tg_div_end is fh_df_div with its two
-// FP32 quotients from the reciprocal, each corrected by its exact remainders
-// (Markstein, IBM J. Res. Dev. 34, 1990): the correctly rounded quotients
-// without two divisions (590 cycles) on the critical path of every solve.
+// FP32 quotients from the reciprocal (fh_quot.cuh): the same bits without two
+// divisions (590 cycles) on the critical path of every solve.
 struct tg_end {
   fh_df x;
   float r;
 };
-__device__ __forceinline__ float tg_quot(float a, float b, float r) {
-  const float q0 = a * r, q = fmaf(fmaf(-q0, b, a), r, q0);  // faithful
-  return fmaf(fmaf(-q, b, a), r, q);                         // correctly rounded
-}
 __device__ __forceinline__ fh_df tg_div_end(fh_df a, const tg_end &d) {
-  const float q1 = tg_quot(a.h, d.x.h, d.r);
+  const float q1 = fh_quot(a.h, d.x.h, d.r);
   const fh_df r = fh_df_sub(a, fh_df_mul(fh_df{q1, 0.f}, d.x));
-  return fh_df_renorm(q1, tg_quot(r.h, d.x.h, d.r));
+  return fh_df_renorm(q1, fh_quot(r.h, d.x.h, d.r));
 }
 
 // One line of N nodes by the 128 threads of its group: Thomas in the
