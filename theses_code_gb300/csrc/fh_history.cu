@@ -10,6 +10,8 @@
 // Cost model: every element of D is read once per step and used in M FMAs.
 // On GB300 the FP64 pipe, not HBM, bounds this loop once M >= 1; from kDpMin
 // layers on the products therefore move to the integer pipe (k_hist_dp).
+#include <algorithm>
+
 #include "fh_internal.h"
 #include "fh_common.cuh"
 #include "fh_dp.cuh"
@@ -199,6 +201,8 @@ __global__ void __launch_bounds__(kHistThreads) k_hist_sum_df(const float2 *__re
   }
 }
 
+constexpr int kDfMaxChunk = 48 * 1024 / (2 * (int)sizeof(float2));  // layers, two rows of weights
+
 int fh_launch_hist_sum_df_partials(fh_ctx *ctx, int M, int K, long long P, const double *W, int ldw,
                                    const float2 *D, long long ldd, int splits, int kchunk, double *part,
                                    long long ldpart, const float2 *far, long long ldfar, int pair_out) {
@@ -280,6 +284,17 @@ int fh_launch_reduce_splits(fh_ctx *ctx, int splits, long long P, const double *
   k_reduce_splits<<<(unsigned)fh_ceil_div(P, 32), 256, 0, ctx->stream>>>(splits, P, part, ldpart, S);
   fh_prof_mark(ctx, FH_PROF_HISTORY, true);
   return fh_after_launch(ctx, "k_reduce_splits");
+}
+
+// K splits of a double-float sum: enough CTAs for ~3 waves of 8 resident
+// 256-thread CTAs on 152 SMs, at least 32 layers per split, and chunks whose two
+// rows of weights fit in a CTA's shared memory (kDfMaxChunk).
+void fh_hist_plan_df(long long P, int K, int max_splits, int *splits, int *kchunk) {
+  long long s = fh_ceil_div(3LL * 152 * 8, fh_ceil_div(P, 2LL * kHistThreads));
+  s = std::max(1LL, std::min(s, (long long)K / 32));
+  s = std::min((long long)max_splits, std::max(s, (long long)fh_ceil_div(K, kDfMaxChunk)));
+  *kchunk = (int)fh_ceil_div(fh_ceil_div(K, s), 4) * 4;
+  *splits = (int)fh_ceil_div(K, *kchunk);
 }
 
 void fh_hist_plan(long long P, int K, int max_splits, int *splits, int *kchunk) {

@@ -176,6 +176,8 @@ int fh_launch_hist_sum_df_partials(fh_ctx *ctx, int M, int K, long long P, const
                                    long long ldpart, const float2 *far, long long ldfar, int pair_out);
 // Chooses the split count for a K x P history sum given a partial-buffer capacity.
 void fh_hist_plan(long long P, int K, int max_splits, int *splits, int *kchunk);
+// The same for fh_launch_hist_sum_df_partials.
+void fh_hist_plan_df(long long P, int K, int max_splits, int *splits, int *kchunk);
 
 // Launch of k; dep: it may start when the kernel before it in the stream has
 // called fh_grid_start_next in every CTA (fh_common.cuh), and waits for that

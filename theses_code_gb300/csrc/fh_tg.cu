@@ -2328,7 +2328,7 @@ static int tg_one_step(fh_tg_solver *s, int max_n, int *done) {
       s->ahead = j + 1;
     }
   } else if (knear >= 1) {
-    fh_hist_plan(g.P, knear, s->max_splits, &splits, &kchunk);
+    (s->df ? fh_hist_plan_df : fh_hist_plan)(g.P, knear, s->max_splits, &splits, &kchunk);
     if (s->df)
       rc = fh_launch_hist_sum_df_partials(ctx, 2, knear, g.P, Wj + kstart, ldw,
                                           reinterpret_cast<const float2 *>(s->D.as<double>()) + (long long)kstart * g.P,
