@@ -285,9 +285,13 @@ typedef struct {
 /* FH_TG_FP64 and FH_TG_DF64, full history, up to 4096 steps: the layers before
  * the current 32-step block are contracted for the whole block on the tensor
  * cores in exact base-256 digits (seven per value, 2^-55 of a 128-layer group's
- * largest; results as near to a 64-bit sum as the FP64 pipe's); the rest of the
- * sums and all line solves as named.  64 rows of the field more memory; without
- * it every layer is summed every step. */
+ * largest; weights more than 2^3 above the least of their group by FP64
+ * multiply-adds).  A sum is as near to its exact value as in FP64 arithmetic
+ * where the layers of a group are of one size, and within ~1e-15 (6e-15) of the
+ * sum of its terms' magnitudes where they fall like k^-1 (k^-2); whole solves
+ * differ by ~1e-16.  The rest of the sums and all line solves as named.  64 rows
+ * of the field more memory; without it every layer is summed every step, which
+ * rounds otherwise. */
 
 typedef struct fh_tg_solver fh_tg_solver;
 

@@ -12,7 +12,13 @@
 // value is cut into seven balanced base-256 digits, x = 2^E sum_i a_i 256^-i
 // with integers |a_i| <= 128, which bf16 holds exactly; weights per row and
 // group likewise.  The cut is at 2^-55 of the group's largest value, half the
-// last place of an FP64 number of that size.  Every product a_i b_j is an
+// last place of an FP64 number of that size; the error of a group's sum is
+// relative to its largest value times its largest weight.  Weights of the newest
+// lags are up to 2^11 times those 128 layers back (alpha 0.95), so in each row and
+// group those above 2^kSpread times the least take FP64 FMAs instead
+// (k_far64_fix), as in fh_dp.cuh: a group whose values fall like k^-1 then comes
+// out within ~1e-15 of the sum of its terms' magnitudes (k^-2: ~6e-15; FMAs 5e-16;
+// without the rule 1e-13 and 8e-13 at alpha 0.95).  Every product a_i b_j is an
 // integer <= 2^14 and a level sum (i + j = l, at most seven products a layer,
 // 128 layers) stays below 2^24: exact in the FP32 accumulators.  Levels 0..6
 // are kept (28 of 49 products; level 7 starts at 2^-56 of the largest
@@ -74,6 +80,9 @@ constexpr uint32_t kBBytes = 2 * kBGroup;      // a chunk's weight image (56 KiB
 constexpr uint32_t kLevCols = kSl * kBRows;    // TMEM columns of a row group
 constexpr size_t kSmem = 1024 + kABytes + 2 * kBBytes + 64;
 constexpr int kNonFinite = 0x7ff;
+constexpr int kSpread = 3;                     // exponents of a row's weights in a group: the rest by FMAs
+constexpr int kRowBlock = 8;                   // rows of a CTA that cuts weights
+constexpr int kFixRows = 16;                   // rows of a CTA of k_far64_fix
 static_assert(kLay == 8 && kRows == 16, "one 16-byte digit store per thread and half, two threads per row group");
 }  // namespace
 
@@ -131,24 +140,56 @@ __global__ void __launch_bounds__(256) k_far64_exp(const S *__restrict__ D, long
   *q = (int16_t)e;
 }
 
+// Where row n, layer k of the weights stands: as fh_far64_weights and
+// fh_far64_weights_lag take them.
+struct f64_src {
+  const double *w;
+  long long row_step, ldw;
+  int base, nrows;
+  bool lag;
+  __device__ __forceinline__ double at(int n, int k) const {
+    if (n >= nrows) return 0.0;
+    return lag ? w[base + n - k] : w[(long long)(n >> 1) * row_step + (long long)(n & 1) * ldw + k];
+  }
+};
+
 // Weight digits of row n (one warp) in group G: image byte of (row group g,
 // digit i, row r of the group, layer k of the chunk) at
-// chunk * kBBytes + g * kBGroup + i * kBTile + fh_sw128_off(r, k).
-template <class Val>
-__device__ __forceinline__ void far64_wrow(const Val &val, int n, int G, int K, uint8_t *__restrict__ img,
-                                           int16_t *__restrict__ ew) {
-  const int lane = threadIdx.x & 31;
+// chunk * kBBytes + g * kBGroup + i * kBTile + fh_sw128_off(r, k).  Weights above
+// 2^kSpread times the row's least are left out of the digits: bit `lane` of word
+// h of hv[G][n] is layer 4 lane + h; hany[G][n / kRowBlock]: any in those rows.
+__global__ void __launch_bounds__(32 * kRowBlock) k_far64_wrows(int K, const f64_src src, uint8_t *__restrict__ img,
+                                                                int16_t *__restrict__ ew, uint4 *__restrict__ hv,
+                                                                int *__restrict__ hany) {
+  const int n = blockIdx.y * kRowBlock + (threadIdx.x >> 5), G = blockIdx.x, lane = threadIdx.x & 31;
   double w[4];
-  int e = 0;
+  int lo = kNonFinite;
 #pragma unroll
   for (int h = 0; h < 4; ++h) {
     const int k = G * kGroup + 4 * lane + h;
-    w[h] = k < K ? val(k) : 0.0;
+    w[h] = k < K ? src.at(n, k) : 0.0;
+    if (w[h] != 0.0) lo = min(lo, f64_exp(w[h]));
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) lo = min(lo, __shfl_xor_sync(0xffffffffu, lo, o));
+  int e = 0;
+  uint32_t hm[4];
+#pragma unroll
+  for (int h = 0; h < 4; ++h) {
+    const bool heavy = f64_exp(w[h]) > lo + kSpread;
+    hm[h] = __ballot_sync(0xffffffffu, heavy);
+    if (heavy) w[h] = 0.0;
     e = max(e, f64_exp(w[h]));
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) e = max(e, __shfl_xor_sync(0xffffffffu, e, o));
-  if (lane == 0) ew[(long long)G * kF64Rows + n] = (int16_t)e;
+  const uint32_t any = hm[0] | hm[1] | hm[2] | hm[3];
+  if (lane == 0) {
+    ew[(long long)G * kF64Rows + n] = (int16_t)e;
+    hv[(long long)G * kF64Rows + n] = make_uint4(hm[0], hm[1], hm[2], hm[3]);
+  }
+  const int blk = __syncthreads_or(any != 0);
+  if (threadIdx.x == 0) hany[G * (kF64Rows / kRowBlock) + blockIdx.y] = blk;
   unsigned long long q[4];
 #pragma unroll
   for (int h = 0; h < 4; ++h) q[h] = f64_word(w[h], e);
@@ -158,18 +199,6 @@ __device__ __forceinline__ void far64_wrow(const Val &val, int n, int G, int K, 
 #pragma unroll
   for (int i = 0; i < kSl; ++i)
     *reinterpret_cast<uint2 *>(dst + i * kBTile) = make_uint2(f64_digits(q[0], q[1], i), f64_digits(q[2], q[3], i));
-}
-__global__ void __launch_bounds__(256) k_far64_wrows(int K, const double *__restrict__ W, long long row_step,
-                                                     long long ldw, int nrows, uint8_t *__restrict__ img,
-                                                     int16_t *__restrict__ ew) {
-  const int n = blockIdx.y * 8 + (threadIdx.x >> 5);
-  const double *row = W + (long long)(n >> 1) * row_step + (long long)(n & 1) * ldw;
-  far64_wrow([&](int k) { return n < nrows ? row[k] : 0.0; }, n, blockIdx.x, K, img, ew);
-}
-__global__ void __launch_bounds__(256) k_far64_wlag(int K, const double *__restrict__ lag, int base, int nrows,
-                                                    uint8_t *__restrict__ img, int16_t *__restrict__ ew) {
-  const int n = blockIdx.y * 8 + (threadIdx.x >> 5);
-  far64_wrow([&](int k) { return n < nrows ? lag[base + n - k] : 0.0; }, n, blockIdx.x, K, img, ew);
 }
 
 // --------------------------------------------------------------- contraction
@@ -395,13 +424,69 @@ __global__ void __launch_bounds__(256) k_far64_reduce(const float2 *__restrict__
   out[i] = fh_df_pair(a);
 }
 
+// Adds the layers that a row's digits leave out (hv), in FP64: thread = one
+// point, rows [16 y, 16 y + 16).  psi = t, alpha 0.7: 4 layers of the first row, none
+// from the fifth step on; alpha 0.95: 7 to 11 layers of the first sixteen steps.
+__device__ __forceinline__ double f64_value(double x) { return x; }
+__device__ __forceinline__ double f64_value(float2 x) { return (double)x.x + (double)x.y; }
+__device__ __forceinline__ void f64_add(double *o, double x) { *o += x; }
+__device__ __forceinline__ void f64_add(float2 *o, double x) {
+  *o = fh_df_pair(fh_df_add(fh_df_from_pair(*o), fh_df_from_double(x)));
+}
+template <class S>
+__global__ void __launch_bounds__(256) k_far64_fix(const S *__restrict__ D, long long ldd, long long P, int K,
+                                                   const f64_src src, const uint4 *__restrict__ hv,
+                                                   const int *__restrict__ hany, S *__restrict__ out, long long ldo) {
+  __shared__ double sw[kGroup][kFixRows];
+  __shared__ uint32_t un[4];
+  const int n0 = blockIdx.y * kFixRows, ng = (K + kGroup - 1) / kGroup, t = threadIdx.x;
+  const long long p = (long long)blockIdx.x * blockDim.x + t;
+  double acc[kFixRows] = {};
+  bool any = false;
+  for (int G = 0; G < ng; ++G) {
+    const int *ha = hany + G * (kF64Rows / kRowBlock) + n0 / kRowBlock;
+    if (!(ha[0] | ha[1])) continue;  // every thread of the CTA
+    any = true;
+    __syncthreads();
+    if (t < 4) un[t] = 0;
+    __syncthreads();
+    for (int i = t; i < kFixRows * kGroup; i += blockDim.x) {
+      const int n = i / kGroup, k = i % kGroup;
+      const uint4 m = hv[(long long)G * kF64Rows + n0 + n];
+      const uint32_t mh = (k & 3) == 0 ? m.x : (k & 3) == 1 ? m.y : (k & 3) == 2 ? m.z : m.w;
+      const bool heavy = mh >> (k >> 2) & 1u;
+      sw[k][n] = heavy ? src.at(n0 + n, G * kGroup + k) : 0.0;
+      if (heavy) atomicOr(&un[k >> 5], 1u << (k & 31));
+    }
+    __syncthreads();
+    if (p < P) {
+      const S *d = D + (long long)G * kGroup * ldd + p;
+      for (int q = 0; q < 4; ++q)
+        for (uint32_t m = un[q]; m; m &= m - 1) {
+          const int k = 32 * q + __ffs(m) - 1;
+          const double x = f64_value(__ldcs(d + k * ldd));
+#pragma unroll
+          for (int n = 0; n < kFixRows; ++n) {
+            const double w = sw[k][n];
+            if (w != 0.0) acc[n] = fma(w, x, acc[n]);
+          }
+        }
+    }
+  }
+  if (!any || p >= P) return;
+#pragma unroll
+  for (int n = 0; n < kFixRows; ++n)
+    if (acc[n] != 0.0) f64_add(out + (long long)(n0 + n) * ldo + p, acc[n]);
+}
+
 // -------------------------------------------------------------------- host
 struct fh_far64 {
   long long P = 0, ld = 0;  // ld: points rounded up to whole tiles
   int Kcap = 0;
   bool df = false;
   int nsm = 1, max_splits = 1;
-  fh_dbuf img, ew, ed, rows, part, err;
+  fh_dbuf img, ew, ed, rows, part, hv, hany, err;
+  f64_src src = {};  // of the weights in img
 };
 
 namespace {
@@ -411,7 +496,7 @@ int splits_for(long long P, int nsm) {
   const long long tiles = fh_ceil_div(P, kPts);
   return (int)std::max(1LL, std::min((long long)kMaxSplits, nsm / tiles));
 }
-size_t sizes(long long P, int Kcap, int splits, size_t (&b)[5]) {
+void sizes(long long P, int Kcap, int splits, size_t (&b)[7]) {
   const long long ld = fh_ceil_div(P, kPts) * kPts;
   const size_t ng = (size_t)fh_ceil_div(Kcap, kGroup);
   b[0] = ng * 2 * kBBytes;
@@ -419,14 +504,10 @@ size_t sizes(long long P, int Kcap, int splits, size_t (&b)[5]) {
   b[2] = ng * (size_t)ld * 2;
   b[3] = 8 * kF64Rows * (size_t)ld;
   b[4] = splits > 1 ? splits * b[3] : 0;
-  return b[0] + b[1] + b[2] + b[3] + b[4];
+  b[5] = ng * kF64Rows * sizeof(uint4);
+  b[6] = ng * (kF64Rows / kRowBlock) * sizeof(int);
 }
 }  // namespace
-
-size_t fh_far64_bytes_of(long long P, int Kcap, bool) {
-  size_t b[5];
-  return sizes(P, Kcap, splits_for(P, 160), b) + 64;
-}
 
 int fh_far64_create(fh_ctx *ctx, long long P, int Kcap, bool df, fh_far64 **out) {
   *out = nullptr;
@@ -438,11 +519,12 @@ int fh_far64_create(fh_ctx *ctx, long long P, int Kcap, bool df, fh_far64 **out)
   int nsm = 0;
   if (cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, ctx->device) == cudaSuccess && nsm > 0) f->nsm = nsm;
   f->max_splits = splits_for(P, f->nsm);
-  size_t b[5];
+  size_t b[7];
   sizes(P, Kcap, f->max_splits, b);
   int rc;
   if ((rc = fh_alloc(ctx, f->img, b[0])) || (rc = fh_alloc(ctx, f->ew, b[1])) || (rc = fh_alloc(ctx, f->ed, b[2])) ||
       (rc = fh_alloc(ctx, f->rows, b[3], false)) || (b[4] && (rc = fh_alloc(ctx, f->part, b[4], false))) ||
+      (rc = fh_alloc(ctx, f->hv, b[5], false)) || (rc = fh_alloc(ctx, f->hany, b[6], false)) ||
       (rc = fh_alloc(ctx, f->err, sizeof(int)))) {
     delete f;
     return rc;
@@ -459,7 +541,8 @@ int fh_far64_create(fh_ctx *ctx, long long P, int Kcap, bool df, fh_far64 **out)
 }
 void fh_far64_delete(fh_far64 *f) { delete f; }
 size_t fh_far64_bytes(const fh_far64 &f) {
-  return f.img.bytes + f.ew.bytes + f.ed.bytes + f.rows.bytes + f.part.bytes + f.err.bytes;
+  return f.img.bytes + f.ew.bytes + f.ed.bytes + f.rows.bytes + f.part.bytes + f.hv.bytes + f.hany.bytes +
+         f.err.bytes;
 }
 long long fh_far64_pitch(const fh_far64 &f) { return f.ld; }
 const void *fh_far64_rows(const fh_far64 &f) { return f.rows.p; }
@@ -474,15 +557,17 @@ int fh_far64_append(fh_ctx *ctx, fh_far64 &f, const void *D, long long ldd, int 
   return fh_after_launch(ctx, "k_far64_exp");
 }
 
-int fh_far64_weights(fh_ctx *ctx, fh_far64 &f, int K, const double *W, long long row_step, long long ldw, int nrows) {
-  k_far64_wrows<<<dim3((unsigned)fh_ceil_div(K, kGroup), kF64Rows / 8), 256, 0, ctx->stream>>>(
-      K, W, row_step, ldw, nrows, f.img.as<uint8_t>(), f.ew.as<int16_t>());
+static int far64_wrows(fh_ctx *ctx, fh_far64 &f, int K, const f64_src &src) {
+  f.src = src;
+  k_far64_wrows<<<dim3((unsigned)fh_ceil_div(K, kGroup), kF64Rows / kRowBlock), 32 * kRowBlock, 0, ctx->stream>>>(
+      K, src, f.img.as<uint8_t>(), f.ew.as<int16_t>(), f.hv.as<uint4>(), f.hany.as<int>());
   return fh_after_launch(ctx, "k_far64_wrows");
 }
+int fh_far64_weights(fh_ctx *ctx, fh_far64 &f, int K, const double *W, long long row_step, long long ldw, int nrows) {
+  return far64_wrows(ctx, f, K, f64_src{W, row_step, ldw, 0, nrows, false});
+}
 int fh_far64_weights_lag(fh_ctx *ctx, fh_far64 &f, int K, const double *lag, int base, int nrows) {
-  k_far64_wlag<<<dim3((unsigned)fh_ceil_div(K, kGroup), kF64Rows / 8), 256, 0, ctx->stream>>>(
-      K, lag, base, nrows, f.img.as<uint8_t>(), f.ew.as<int16_t>());
-  return fh_after_launch(ctx, "k_far64_wlag");
+  return far64_wrows(ctx, f, K, f64_src{lag, 0, 0, base, nrows, true});
 }
 
 int fh_far64_run(fh_ctx *ctx, fh_far64 &f, const void *D, long long ldd, int K) {
@@ -497,9 +582,14 @@ int fh_far64_run(fh_ctx *ctx, fh_far64 &f, const void *D, long long ldd, int K) 
     k_far64<S><<<grid, kThr, kSmem, ctx->stream>>>(d, ldd, f.P, K, f.img.as<uint8_t>(), f.ew.as<int16_t>(),
                                                    f.ed.as<int16_t>(), f.ld, gps, o, f.ld, f.err.as<int>());
     int rc = fh_after_launch(ctx, "k_far64");
-    if (rc || splits == 1) return rc;
-    k_far64_reduce<<<(unsigned)fh_ceil_div(n, 256), 256, 0, ctx->stream>>>(f.part.as<S>(), splits, n, f.rows.as<S>());
-    return fh_after_launch(ctx, "k_far64_reduce");
+    if (rc) return rc;
+    if (splits > 1) {
+      k_far64_reduce<<<(unsigned)fh_ceil_div(n, 256), 256, 0, ctx->stream>>>(f.part.as<S>(), splits, n, f.rows.as<S>());
+      if ((rc = fh_after_launch(ctx, "k_far64_reduce"))) return rc;
+    }
+    k_far64_fix<S><<<dim3((unsigned)fh_ceil_div(f.P, 256), kF64Rows / kFixRows), 256, 0, ctx->stream>>>(
+        d, ldd, f.P, K, f.src, f.hv.as<uint4>(), f.hany.as<int>(), f.rows.as<S>(), f.ld);
+    return fh_after_launch(ctx, "k_far64_fix");
   };
   fh_prof_mark(ctx, FH_PROF_GEMM, false);
   const int rc = f.df ? go(static_cast<const float2 *>(D)) : go(static_cast<const double *>(D));

@@ -72,11 +72,11 @@ def tg_bytes(sN: int, M: int, steps: int, mode: int) -> int:
             if ntiles < 160:
                 b += 8 * min(8, 160 // ntiles) * 128 * Ppad
     elif 32 < steps <= 4096:
-        # 64 rows of the older layers, their weight images and exponents, and
-        # partial rows when the 128-point tiles are fewer than the SMs
+        # 64 rows of the older layers, their weight images, exponents and
+        # masks, and partial rows when the 128-point tiles are fewer than the SMs
         ld = -(-P // 128) * 128
         ng = -(-steps // 128)
-        b += ng * (2 * 57344 + 128 + 2 * ld) + 512 * ld
+        b += ng * (2 * 57344 + 128 + 1056 + 2 * ld) + 512 * ld
         if ld // 128 <= 80:
             b += 512 * ld * min(8, 160 // (ld // 128))
     return int(b) + 2 * _MIB
