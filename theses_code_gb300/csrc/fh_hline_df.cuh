@@ -12,8 +12,10 @@
 // Everything is divided by Dg kc / c (the row scale of A, B, R): A_i and B_i
 // are then exp(gam u) of the neighbours, the row sum s is (Da c / (Dg kc)) wc,
 // and the FP32 exponent range holds them.  Lines out of that range
-// (kHdfExp, kHdfRow), with states that FP32 pairs do not hold, or too long for
-// one panel are left to the FP64 solve (the function returns false).
+// (kHdfExp, kHdfRow), with states or boundary values that FP32 pairs do not hold
+// (above kHdfState, or all below kHdfFloor: a product of one with a row sum
+// would lose its low word), with al_left outside [0, 1], or too long for one
+// panel are left to the FP64 solve (the function returns false).
 //
 // exp: 2^(j/16) from a table times a Taylor polynomial of degree 6 on
 // |r| <= ln 2 / 32 (next term 2^-51), its terms above the third power in FP32.
@@ -24,6 +26,7 @@
 constexpr float kHdfExp = 11.0f;             // |gam u| at most: exp within 2^+-16
 constexpr float kHdfRow = 0x1p16f;           // row sum at most, 2^-40 at least
 constexpr float kHdfState = 0x1p60f;
+constexpr float kHdfFloor = 0x1p-54f;        // the largest state or boundary value at least
 
 __device__ const float2 kHdfTab[16] = {  // 2^(j/16)
     {0x1.000000p+0f, 0.0f},           {0x1.0b5586p+0f, 0x1.9f3122p-25f},  {0x1.172b84p+0f, -0x1.c15742p-27f},
@@ -140,11 +143,14 @@ __device__ __forceinline__ bool fh_hline_df(const fh_h_dev_inst &I, double wc, c
   __syncthreads();
   // ---- state and exp(gam u)
   const fh_df s = fh_df_bits(I.dq * wc), gam = fh_df_bits(I.kgam);
-  bool ok = s.h >= 0x1p-40f && s.h <= kHdfRow;
+  const fh_df al0 = fh_df_bits(I.al_left), b0 = fh_df_bits(I.bt_left), uN = fh_df_bits(I.u_right);
+  float big = fmaxf(fabsf(b0.h), fabsf(uN.h));
+  bool ok = s.h >= 0x1p-40f && s.h <= kHdfRow && big <= kHdfState && I.al_left >= 0.0 && I.al_left <= 1.0;
   for (int k = t; k <= N + 1; k += T) {
     const fh_df x = fh_df_bits(U[o + k]);
     sU[fh_hsk(k)] = fh_df_pair(x);
     ok = ok && fabsf(x.h) <= kHdfState;
+    big = fmaxf(big, fabsf(x.h));
     if (k <= N) {
       fh_df e = one;
       if (I.kmodel != FH_K_CONST) {
@@ -155,8 +161,7 @@ __device__ __forceinline__ bool fh_hline_df(const fh_h_dev_inst &I, double wc, c
       sE[fh_hsk(k)] = fh_df_pair(e);
     }
   }
-  const fh_df al0 = fh_df_bits(I.al_left), b0 = fh_df_bits(I.bt_left), uN = fh_df_bits(I.u_right);
-  if (!__syncthreads_and(ok)) return false;
+  if (!__syncthreads_and(ok) || !__syncthreads_or(big >= kHdfFloor)) return false;
   // ---- right parts
   {
     const fh_df q = fh_df_bits(I.dq), gq = fh_df_bits(I.gq);
