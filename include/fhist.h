@@ -256,10 +256,13 @@ int fh_h_batch_tstep(const fh_h_batch *b);
  * cores (exact bf16 slices with per-point and per-row power-of-two scales,
  * tcgen05, one 128-point tile of one instance against that instance's 64
  * weight rows), the block's own slots are summed per step in double-float
- * from a 128-layer ring; line solves and weights stay FP64; the history costs
- * 8 bytes per value (slice planes) and the full FP64 history is not kept.
- * Bound 1e-9 relative against the FP64 oracle.  No counterpart in the
- * reference. */
+ * from a 128-layer ring; the history costs 8 bytes per value (slice planes) and
+ * the full FP64 history is not kept.  Line solves are FP64, but in double-float
+ * (2^-47 per operation, the state rounded to 2^-48) on lines of 768 to 1025
+ * intervals, where that is no further from 64-bit results than the reference's
+ * order in FP64; weights of older slots are formed in FP64 and interpolated in
+ * double-float (their slices keep 2^-32).  Bound 1e-9 relative against the FP64
+ * oracle.  No counterpart in the reference. */
 #define FH_H_FP64 0
 #define FH_H_DF64 1
 #define FH_H_BLOCKED 2

@@ -1,10 +1,11 @@
 """Which lines of the mixed-precision mode the double-float solve may take
-(fh_hline_df.cuh): none whose states or boundary values pairs do not hold.
+(fh_hline_df.cuh): none so short that pairs cost accuracy, none whose states or
+boundary values pairs do not hold.
 
-Tolerances.  Scaled states: the mode's own 1e-9 (a line is linear for constant K;
-before the fourth step no history counts).  Otherwise against the FP64 mode within
-one history block: the plain path's 1e-12 and, for the sums in pairs, 2^-47 of the
-solution per step."""
+Tolerances.  Short lines against the FP64 mode within one history block: the plain
+path's 1e-12 and, for the sums in pairs, 2^-47 of the solution per step.  Scaled
+states: the mode's own 1e-9 (a line is linear for constant K; before the fourth
+step no history counts)."""
 import numpy as np
 import pytest
 
@@ -22,6 +23,19 @@ def _run(params, U0, steps, mode):
     s.close()
     ctx.close()
     return u
+
+
+@pytest.mark.parametrize("N,seed", [(256, 2), (512, 1), (640, 2), (640, 3), (767, 3)])
+def test_short_lines_keep_fp64(N, seed):
+    from theses_code_gb300 import _lib, workloads
+    steps = 60
+    params = [dict(p, N=N) for p in workloads.psi_batch(8, seed=seed)[0]]
+    u = 0.25 * (1 + np.cos(np.pi * np.arange(N + 2) / N))
+    u[N:] = 0.0
+    a = _run(params, [u] * 8, steps, _lib.FH_H_BLOCKED)
+    b = _run(params, [u] * 8, steps, _lib.FH_H_FP64)
+    for x, y in zip(a, b):
+        assert np.max(np.abs(x - y)) <= (1e-12 + steps * 2.0 ** -47) * np.max(np.abs(y))
 
 
 @pytest.mark.parametrize("what,k,steps", [("state", -60, 3), ("state", -120, 3), ("state", -200, 3), ("right", -200, 3),

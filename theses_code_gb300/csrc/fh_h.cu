@@ -1354,10 +1354,10 @@ static int h_weights(fh_h_batch *B, int tstep, int os, int par, cudaStream_t st)
   return fh_after_launch(ctx, "k_h_weights");
 }
 
-// Whether the lines are solved in double-float: the blocked mode, classical
-// derivative, lines of one panel.
+// Whether the long lines are solved in double-float (fh_hline_df.cuh): the
+// blocked mode, classical derivative, lines of one panel, some long enough.
 static bool h_line_in_df(const fh_h_batch *B) {
-  return B->mode == FH_H_BLOCKED && !B->space && B->max_n - 1 <= 32 * kLineWarps * kHLineEq;
+  return B->mode == FH_H_BLOCKED && !B->space && B->max_n >= kHdfMinN && B->max_n - 1 <= 32 * kLineWarps * kHLineEq;
 }
 
 // One step.  The weights depend on the step number only, so with `next` (and

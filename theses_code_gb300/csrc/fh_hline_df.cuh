@@ -9,6 +9,17 @@
 // are sums and products of non-negative terms, so an error of 2^-47 per
 // operation stays that of the result relative to its size.
 //
+// Only lines of kHdfMinN intervals and more.  A line's coefficients carry the
+// pairs' 2^-47 into the solution times ~N; the reference's order in FP64 loses
+// ~N^2 2^-53 to cancellation.  Error of psi solves against 64 bits, reference
+// order / pairs / the FP64 form of fh_hline.cuh: N = 256, 600 steps 1.4e-12 /
+// 3.0e-12 / 1.4e-12; 512, 800 steps 4.1e-12 / 5.7e-12 / 0.9e-12; 640: 9.7e-12 /
+// 7.8e-12 / 1.2e-12, single batches 5.9e-12 / 1.0e-11; 768: 2.2e-11 / 1.0e-11 /
+// 1.3e-12; 1024: 3.2e-11 / 1.3e-11 / 1.0e-12 (1500 steps: 768 3.7e-11 / 1.5e-11).
+// So pairs are no further off than the reference's order from 768 on, and shorter
+// lines run in FP64: 512 psi instances of 64..1024 nodes, 1500 steps 111 -> 148 ms,
+// 1.3e-11 -> 1.1e-11.
+//
 // Everything is divided by Dg kc / c (the row scale of A, B, R): A_i and B_i
 // are then exp(gam u) of the neighbours, the row sum s is (Da c / (Dg kc)) wc,
 // and the FP32 exponent range holds them.  Lines out of that range
@@ -27,6 +38,7 @@ constexpr float kHdfExp = 11.0f;             // |gam u| at most: exp within 2^+-
 constexpr float kHdfRow = 0x1p16f;           // row sum at most, 2^-40 at least
 constexpr float kHdfState = 0x1p60f;
 constexpr float kHdfFloor = 0x1p-54f;        // the largest state or boundary value at least
+constexpr int kHdfMinN = 768;                // intervals of a line at least
 
 __device__ const float2 kHdfTab[16] = {  // 2^(j/16)
     {0x1.000000p+0f, 0.0f},           {0x1.0b5586p+0f, 0x1.9f3122p-25f},  {0x1.172b84p+0f, -0x1.c15742p-27f},
@@ -137,7 +149,7 @@ __device__ __forceinline__ bool fh_hline_df(const fh_h_dev_inst &I, double wc, c
   float2 *sE = sm, *sO = sE + fh_hline_len(T), *sU = sO + fh_hline_len(T);
   const long long o = I.off;
   const int N = I.N, n = N - 1;
-  if (n > T * kHLineEq) return false;
+  if (N < kHdfMinN || n > T * kHLineEq) return false;
   const fh_df zero{0.f, 0.f}, one{1.f, 0.f};
   if (t < 16) tab[t] = kHdfTab[t];
   __syncthreads();
