@@ -800,7 +800,16 @@ static int ab_res_setup(fh_ab_solver *s) {
   return ab_src_pairs(s);
 }
 
+// The error flags of the solver's device waits: cleared when a solve starts (set:
+// as an expired wait leaves them, for tests).
+static int ab_mark(fh_ab_solver *s, int expired) {
+  if (s->derr.p) FH_CUDA_TRY(s->ctx, cudaMemsetAsync(s->derr.p, expired, sizeof(int), s->ctx->stream));
+  return s->f64 ? fh_far64_mark(s->ctx, *s->f64, expired) : (int)FH_OK;
+}
+
 extern "C" {
+
+int fh_ab_test_expire(fh_ab_solver *s) { return ab_mark(s, 1); }
 
 int fh_ab_create(fh_ctx *ctx, int m, int max_steps, double tau, double alpha, fh_ab_solver **out) {
   FH_REQUIRE(ctx, ctx && out, FH_EINVAL, "fh_ab_create: null argument");
@@ -889,6 +898,7 @@ int fh_ab_set_c_host(fh_ab_solver *s, const double *C_host) {
   fh_ctx *ctx = s->ctx;
   FH_REQUIRE(ctx, C_host, FH_EINVAL, "fh_ab_set_c_host: null pointer");
   FH_CUDA_TRY(ctx, cudaMemcpyAsync(s->C.p, C_host, sizeof(double) * (s->m + 1), cudaMemcpyHostToDevice, ctx->stream));
+  if (int rc = ab_mark(s, 0)) return rc;
   FH_CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));
   s->step = 0;
   s->T0 = 0;
@@ -900,6 +910,7 @@ int fh_ab_set_c(fh_ab_solver *s, const double *C) {
   fh_ctx *ctx = s->ctx;
   FH_REQUIRE(ctx, C, FH_EINVAL, "fh_ab_set_c: null pointer");
   FH_CUDA_TRY(ctx, cudaMemcpyAsync(s->C.p, C, sizeof(double) * (s->m + 1), cudaMemcpyDeviceToDevice, ctx->stream));
+  if (int rc = ab_mark(s, 0)) return rc;
   s->step = 0;
   s->T0 = 0;
   return FH_OK;

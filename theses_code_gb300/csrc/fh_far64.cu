@@ -604,3 +604,7 @@ int fh_far64_check(fh_ctx *ctx, const fh_far64 &f) {
   FH_REQUIRE(ctx, h == 0, FH_ETIMEOUT, "history contraction: a device wait ran out");
   return FH_OK;
 }
+int fh_far64_mark(fh_ctx *ctx, const fh_far64 &f, int expired) {
+  FH_CUDA_TRY(ctx, cudaMemsetAsync(f.err.p, expired, sizeof(int), ctx->stream));
+  return FH_OK;
+}

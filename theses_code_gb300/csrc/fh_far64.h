@@ -25,3 +25,4 @@ int fh_far64_weights_lag(fh_ctx *ctx, fh_far64 &f, int K, const double *lag, int
 int fh_far64_run(fh_ctx *ctx, fh_far64 &f, const void *D, long long ldd, int K);
 const void *fh_far64_rows(const fh_far64 &f);  // double or float2, row n at n pitch
 int fh_far64_check(fh_ctx *ctx, const fh_far64 &f);  // FH_ETIMEOUT once a device wait ran out (synchronises)
+int fh_far64_mark(fh_ctx *ctx, const fh_far64 &f, int expired);  // 0 at the start of a solve; 1 as an expired wait does

@@ -1728,6 +1728,19 @@ static int h_sync_check(fh_h_batch *b) {
   return FH_OK;
 }
 
+// The flag of an expired wait, in stream order: cleared when a solve starts (set:
+// as an expired wait leaves it, for tests).
+static __global__ void k_h_mark(volatile int *err, int expired) {
+  *err = expired;
+  __threadfence_system();
+}
+static int h_mark(fh_h_batch *b, int expired) {
+  if (!b->perr) return FH_OK;
+  k_h_mark<<<1, 1, 0, b->ctx->stream>>>(b->perr, expired);
+  return fh_after_launch(b->ctx, "k_h_mark");
+}
+int fh_h_batch_test_expire(fh_h_batch *b) { return h_mark(b, 1); }
+
 // The states of instances first .. first + count - 1 between the host's packed
 // order and the device's segments: from kHPackMin instances on one copy and a
 // gather or scatter, below a copy per instance.
@@ -1766,6 +1779,7 @@ int fh_h_batch_set_u_host(fh_h_batch *b, const double *U_host) {
   const int rc = h_copy_u(b, 0, b->n, const_cast<double *>(U_host), false);
   if (rc) return rc;
   FH_CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));
+  if (b->perr) *(volatile int *)b->perr = 0;
   b->tstep = 1;
   b->nsaved = 0;
   return h_reset_clocks(b);
@@ -1818,6 +1832,7 @@ int fh_h_batch_set_u(fh_h_batch *b, const double *U) {
                                      cudaMemcpyDeviceToDevice, ctx->stream));
     src += (long long)cnt;
   }
+  if (int rc = h_mark(b, 0)) return rc;
   b->tstep = 1;
   b->nsaved = 0;
   return h_reset_clocks(b);

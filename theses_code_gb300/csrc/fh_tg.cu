@@ -2745,6 +2745,14 @@ int fh_tg_set_diffusion(fh_tg_solver *s, int fixed_d, double lambda, double ka0,
   return FH_OK;
 }
 
+// The error flags of the solver's device waits: cleared when a solve starts (set:
+// as an expired wait leaves them, for tests).
+static int tg_mark(fh_tg_solver *s, int expired) {
+  if (s->derr.p) FH_CUDA_TRY(s->ctx, cudaMemsetAsync(s->derr.p, expired, sizeof(int), s->ctx->stream));
+  return s->f64 ? fh_far64_mark(s->ctx, *s->f64, expired) : (int)FH_OK;
+}
+int fh_tg_test_expire(fh_tg_solver *s) { return tg_mark(s, 1); }
+
 // Zero series accumulators at the start of a solve.
 static int tg_series_reset(fh_tg_solver *s) {
   if (!s->ser_J) return FH_OK;
@@ -2759,7 +2767,7 @@ int fh_tg_set_state(fh_tg_solver *s, const double *V2, const double *C) {
   const size_t n = sizeof(double) * (size_t)(s->p.sN + 2) * (s->p.M + 2);
   FH_CUDA_TRY(ctx, cudaMemcpyAsync(s->V2.p, V2, n, cudaMemcpyDeviceToDevice, ctx->stream));
   FH_CUDA_TRY(ctx, cudaMemcpyAsync(s->C.p, C, n, cudaMemcpyDeviceToDevice, ctx->stream));
-  if (s->derr.p) FH_CUDA_TRY(ctx, cudaMemsetAsync(s->derr.p, 0, sizeof(int), ctx->stream));
+  if (int rc = tg_mark(s, 0)) return rc;
   if (s->massN) FH_CUDA_TRY(ctx, cudaMemsetAsync(s->Nn.p, 0, s->Nn.bytes, ctx->stream));  // N starts at 0
   if (int rc = tg_series_reset(s)) return rc;
   s->tstep = 0;
@@ -2775,7 +2783,7 @@ int fh_tg_set_state_host(fh_tg_solver *s, const double *V2_host, const double *C
   const size_t n = sizeof(double) * (size_t)(s->p.sN + 2) * (s->p.M + 2);
   FH_CUDA_TRY(ctx, cudaMemcpyAsync(s->V2.p, V2_host, n, cudaMemcpyHostToDevice, ctx->stream));
   FH_CUDA_TRY(ctx, cudaMemcpyAsync(s->C.p, C_host, n, cudaMemcpyHostToDevice, ctx->stream));
-  if (s->derr.p) FH_CUDA_TRY(ctx, cudaMemsetAsync(s->derr.p, 0, sizeof(int), ctx->stream));
+  if (int rc = tg_mark(s, 0)) return rc;
   if (s->massN) FH_CUDA_TRY(ctx, cudaMemsetAsync(s->Nn.p, 0, s->Nn.bytes, ctx->stream));  // N starts at 0
   if (int rc = tg_series_reset(s)) return rc;
   FH_CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));
