@@ -733,6 +733,7 @@ static int ab_res_steps(fh_ab_solver *s, int max_n, int *done) {
   const bool df = s->mode == FH_AB_BLOCKED;
   const int K = s->step, T0 = s->T0, ns = std::min(max_n, T0 + ab_block(s) - K);
   FH_REQUIRE(ctx, K >= T0 && ns >= 1, FH_EINVAL, "fh_ab_step: step %d outside its block at %d", K, T0);
+  FH_REQUIRE(ctx, !df || s->src2.p, FH_ENOMEM, "fh_ab_step: the last source rows found no memory");
   fh_ab_res_args a;
   a.m = s->m;
   a.nrows = s->nrows;
@@ -773,9 +774,21 @@ static int ab_res_steps(fh_ab_solver *s, int max_n, int *done) {
   return FH_OK;
 }
 
+static int ab_res_buffers(fh_ab_solver *s);
+
 // The resident solve's buffers and, in the FP64 mode, the contraction of older
-// entries (without memory for it every step sums every entry).
+// entries (without memory for it every step sums every entry).  Where a buffer
+// fails, the solver is left to step by step solves.
 static int ab_res_setup(fh_ab_solver *s) {
+  const int rc = ab_res_buffers(s);
+  if (rc) {
+    if (s->f64) fh_far64_delete(s->f64);
+    s->f64 = nullptr;
+    s->resident = false;
+  }
+  return rc;
+}
+static int ab_res_buffers(fh_ab_solver *s) {
   fh_ctx *ctx = s->ctx;
   int rc;
   s->graph.reset();
@@ -954,21 +967,19 @@ int fh_ab_set_mode(fh_ab_solver *s, int mode) {
   fh_ctx *ctx = s->ctx;
   FH_REQUIRE(ctx, mode == FH_AB_FP64 || mode == FH_AB_BLOCKED, FH_EINVAL, "fh_ab_set_mode: unknown mode %d", mode);
   FH_REQUIRE(ctx, s->step == 0, FH_EINVAL, "fh_ab_set_mode: only before the first step");
-  s->mode = mode;
   if (mode == FH_AB_BLOCKED && !s->blk && s->max_steps > kAbBlock) {
-    s->blk = fh_blk_new();
+    // on failure the solver keeps its previous mode
+    fh_blk *blk = fh_blk_new();
     const int kcap = (int)fh_ceil_div(s->max_steps, kAbBlock) * kAbBlock;
-    int rc = fh_blk_init(ctx, *s->blk, s->P, kcap);
-    if (!rc) {
-      s->ldfar = fh_blk_ppad(*s->blk);
-      rc = fh_alloc(ctx, s->far, sizeof(float2) * kAbBlock * (size_t)s->ldfar, false);
-    }
-    if (rc) {
-      fh_blk_delete(s->blk);
-      s->blk = nullptr;
+    int rc = fh_blk_init(ctx, *blk, s->P, kcap);
+    if (rc || (rc = fh_alloc(ctx, s->far, sizeof(float2) * kAbBlock * (size_t)fh_blk_ppad(*blk), false))) {
+      fh_blk_delete(blk);
       return rc;
     }
+    s->ldfar = fh_blk_ppad(*blk);
+    s->blk = blk;
   }
+  s->mode = mode;
   if (mode == FH_AB_FP64 && s->blk) {
     fh_blk_delete(s->blk);
     s->blk = nullptr;
