@@ -540,13 +540,13 @@ __global__ void k_blk_toeplitz_rows(const double *__restrict__ w, int base, int 
   const int m = blockIdx.y * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (m >= kBM) return;
   const int k0 = 2 * kBK * blockIdx.x + (threadIdx.x & 31);
-  float2 wp[4];
+  double wd[4];
 #pragma unroll
   for (int h = 0; h < 4; ++h) {
     const int k = k0 + 32 * h;
-    wp[h] = fh_df_pair(fh_df_bits(k < K && m < mrows ? w[base + m - k] : 0.0));
+    wd[h] = k < K && m < mrows ? w[base + m - k] : 0.0;
   }
-  fh_slice_group_pairs(wp, blockIdx.x, K / kBK, m, kBM, Kcap, A3, Ew);
+  fh_slice_group_doubles(wd, blockIdx.x, K / kBK, m, kBM, Kcap, A3, Ew);
 }
 
 // Weight rows W[m*ldw + k], k < K, rows m >= mrows are zero (standalone

@@ -12,6 +12,7 @@
 #include <stdint.h>
 
 #include "fh_common.cuh"
+#include "fh_df.cuh"
 
 constexpr int kSlcK = 64;  // layers per chunk (one 128-byte K-major row of bf16)
 constexpr int kSlcN = 4;   // bf16 slices per value
@@ -136,6 +137,36 @@ __device__ __forceinline__ void fh_slice_group_pairs(const float2 (&w)[4], int G
     if (h >= 2 * nc) break;
     __nv_bfloat16 bs[kSlcN];
     fh_slice_pair(w[h].x, w[h].y, scale, bs);
+    const long long o = m * Kcap + c0 * kSlcK + lane + 32 * h;
+#pragma unroll
+    for (int i = 0; i < kSlcN; ++i) A3[i * plane + o] = bs[i];
+  }
+}
+
+// The same for FP64 weights: scaled by the group's exponent on their bits, then cut
+// as pairs on the FP32 pipe, so that weights of any size keep their slices.
+__device__ __forceinline__ void fh_slice_group_doubles(const double (&w)[4], int G, int nchunks, long long m,
+                                                       long long nrows, int Kcap, __nv_bfloat16 *__restrict__ A3,
+                                                       int8_t *__restrict__ Ew) {
+  const int lane = threadIdx.x & 31;
+  const int c0 = 2 * G, nc = min(2, nchunks - c0);
+  int mx = 0;
+#pragma unroll
+  for (int h = 0; h < 4; ++h) mx = max(mx, (__double2hiint(w[h]) >> 20) & 0x7ff);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+  const int E = mx ? mx - 1029 : 0;  // |w| < 2^(E + 7)
+  if (lane == 0)
+    for (int c = c0; c < c0 + nc; ++c) Ew[(long long)c * nrows + m] = (int8_t)E;
+  const long long plane = nrows * (long long)Kcap;
+#pragma unroll
+  for (int h = 0; h < 4; ++h) {
+    if (h >= 2 * nc) break;
+    const int hi = __double2hiint(w[h]), ex = (hi >> 20) & 0x7ff;
+    const fh_df x = ex > 0 && ex - E > 0 ? fh_df_bits(__hiloint2double(hi - E * (1 << 20), __double2loint(w[h])))
+                                         : fh_df{0.f, 0.f};
+    __nv_bfloat16 bs[kSlcN];
+    fh_slice_pair(x.h, x.l, 1.0f, bs);
     const long long o = m * Kcap + c0 * kSlcK + lane + 32 * h;
 #pragma unroll
     for (int i = 0; i < kSlcN; ++i) A3[i * plane + o] = bs[i];
