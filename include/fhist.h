@@ -269,7 +269,9 @@ int fh_h_batch_tstep(const fh_h_batch *b);
 int fh_h_batch_set_mode(fh_h_batch *b, int mode);
 /* Launch-shape autotuner for the batch history sum: times the candidate tile
  * CTAs (128/256/512 threads) x K-split caps (1/8/64) on the batch's buffers
- * and keeps the fastest; *best_ms (optional) receives its time per launch.
+ * and keeps the fastest; *best_ms (optional) receives its time per launch.  FP64
+ * sums of 64 layers and more have no tile shape: the shape is chosen by the
+ * longest sums that have one.
  * Not during a stream capture.  No counterpart in the reference. */
 int fh_h_batch_autotune(fh_h_batch *b, float *best_ms);
 int fh_h_batch_launch_shape(const fh_h_batch *b, int *tile_threads, int *split_cap);

@@ -1999,10 +1999,34 @@ int fh_h_batch_set_space_order(fh_h_batch *b, const double *gamma_host) {
   return FH_OK;
 }
 
-// Times the batch history sum for every candidate launch shape (tile CTA of
+// Mean time of two launches of the batch history sum over K layers (after one
+// that warms up); history contents do not change it.
+static int h_time_hist(fh_h_batch *b, int ti, int K, int cap, cudaEvent_t e0, cudaEvent_t e1, float *ms) {
+  fh_ctx *ctx = b->ctx;
+  int splits, kchunk;
+  h_plan(b, ti, K, cap < b->max_splits ? cap : b->max_splits, &splits, &kchunk);
+  *ms = 1e30f;
+  if (!h_dp(b, K) && (size_t)kchunk * sizeof(double) > 48 * 1024) return FH_OK;
+  float sum = 0.f;
+  for (int rep = 0; rep < 3; ++rep) {
+    cudaEventRecord(e0, ctx->stream);
+    const int rc = h_hist(b, ti, K, splits, kchunk, b->W.as<double>(), ctx->stream);
+    if (rc) return rc;
+    cudaEventRecord(e1, ctx->stream);
+    FH_CUDA_TRY(ctx, cudaEventSynchronize(e1));
+    float t = 0.f;
+    if (rep > 0) FH_CUDA_TRY(ctx, cudaEventElapsedTime(&t, e0, e1));
+    sum += t;
+  }
+  *ms = sum / 2;
+  return FH_OK;
+}
+
+// Times the batch history sum for the candidate launch shapes (tile CTA of
 // 128/256/512 threads, K split cap 1/8/64) at a probe depth of
-// min(max_steps - 1, 512) layers on the batch's own buffers (history contents
-// do not change the timing) and keeps the fastest.
+// min(max_steps - 1, 512) layers on the batch's own buffers and keeps the fastest.
+// FP64 sums of kDpMin layers and more have no tile shape: theirs is chosen at the
+// deepest sum that has one, the cap at the probe depth.
 int fh_h_batch_autotune(fh_h_batch *b, float *best_ms) {
   FH_REQUIRE(nullptr, b, FH_EINVAL, "null batch");
   fh_ctx *ctx = b->ctx;
@@ -2013,48 +2037,35 @@ int fh_h_batch_autotune(fh_h_batch *b, float *best_ms) {
   static const int caps[3] = {1, 8, 64};
   cudaEvent_t e0, e1;
   FH_CUDA_TRY(ctx, cudaEventCreate(&e0));
-  FH_CUDA_TRY(ctx, cudaEventCreate(&e1));
-  float best = 1e30f;
-  int bt = b->tile_threads, bc = b->split_cap;
-  for (int ti = 0; ti < 3; ++ti)
-    for (int ci = 0; ci < 3; ++ci) {
-      int splits, kchunk;
-      h_plan(b, ti, K, caps[ci] < b->max_splits ? caps[ci] : b->max_splits, &splits, &kchunk);
-      if (!h_dp(b, K) && (size_t)kchunk * sizeof(double) > 48 * 1024) continue;
-      float ms = 0.f;
-      for (int rep = 0; rep < 3; ++rep) {  // first repetition warms up
-        cudaEventRecord(e0, ctx->stream);
-        int rc = h_hist(b, ti, K, splits, kchunk, b->W.as<double>(), ctx->stream);
-        if (rc) {
-          cudaEventDestroy(e0);
-          cudaEventDestroy(e1);
-          return rc;
+  if (cudaEventCreate(&e1) != cudaSuccess) {
+    cudaEventDestroy(e0);
+    return fh_set_error(ctx, FH_ECUDA, "fh_h_batch_autotune: no event");
+  }
+  float best = 1e30f, ms;
+  int rc = FH_OK, shape = tile_shape_index(b->tile_threads), cap = b->split_cap;
+  auto search = [&](int depth, int t0, int t1, int c0, int c1) {
+    best = 1e30f;
+    for (int ti = t0; ti < t1 && !rc; ++ti)
+      for (int ci = c0; ci < c1 && !rc; ++ci)
+        if (!(rc = h_time_hist(b, ti, depth, caps[ci], e0, e1, &ms)) && ms < best) {
+          best = ms;
+          shape = ti;
+          cap = caps[ci];
         }
-        cudaEventRecord(e1, ctx->stream);
-        cudaError_t e = cudaEventSynchronize(e1);
-        if (e != cudaSuccess) {
-          cudaEventDestroy(e0);
-          cudaEventDestroy(e1);
-          return fh_set_error(ctx, FH_ECUDA, "fh_h_batch_autotune: %s", cudaGetErrorString(e));
-        }
-        if (rep > 0) {
-          float t = 0.f;
-          cudaEventElapsedTime(&t, e0, e1);
-          ms += t;
-        }
-      }
-      if (ms < best) {
-        best = ms;
-        bt = kTileShapes[ti];
-        bc = caps[ci];
-      }
-    }
+  };
+  if (h_dp(b, K)) {
+    search(kDpMin - 1, 0, 3, 2, 3);
+    search(K, shape, shape + 1, 0, 3);
+  } else {
+    search(K, 0, 3, 0, 3);
+  }
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
-  b->tile_threads = bt;
-  b->split_cap = bc;
+  if (rc) return rc;
+  b->tile_threads = kTileShapes[shape];
+  b->split_cap = cap;
   b->graph.reset();
-  if (best_ms) *best_ms = best / 2;
+  if (best_ms) *best_ms = best;
   return FH_OK;
 }
 
