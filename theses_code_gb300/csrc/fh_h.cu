@@ -64,7 +64,7 @@ struct fh_h_batch {
   bool use_graph = true;
   int mode = FH_H_FP64;  // FH_H_DF64: history as (hi, lo) FP32 pairs; FH_H_BLOCKED: below
   bool persistent = true;  // small FP64 batches: one launch per call (k_h_persistent)
-  int pers_ctas = 4;       // CTAs per instance there
+  int pers_ctas[2] = {4, 4};  // CTAs per instance there (k_h_persistent, k_h_pers_own)
   int *perr = nullptr;     // pinned: set when a wait of the persistent solve ran out
   std::vector<fh_h_dev_inst> di;  // host copy of inst
   std::vector<int> cap;           // nodes a restarted occupant of each instance may have (segment - 2)
@@ -1558,12 +1558,13 @@ static int h_set_smem_attrs(fh_ctx *ctx) {
 // CTAs per instance of the persistent solve: the largest cluster of which the
 // device holds all n at once (a second wave would double the step time; with
 // few instances more CTAs share the history sums), at least four.
-static int h_pers_ctas(int n) {
+template <class K>
+static int h_pers_ctas(int n, K kern, int threads, size_t smem) {
   for (int c = kPersMaxCtas; c > 4; c /= 2) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(n * c));
-    cfg.blockDim = dim3(kPersThreads);
-    cfg.dynamicSmemBytes = kPersSmem;
+    cfg.blockDim = dim3((unsigned)threads);
+    cfg.dynamicSmemBytes = smem;
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeClusterDimension;
     at[0].val.clusterDim.x = (unsigned)c;
@@ -1571,7 +1572,7 @@ static int h_pers_ctas(int n) {
     cfg.attrs = at;
     cfg.numAttrs = 1;
     int active = 0;
-    if (cudaOccupancyMaxActiveClusters(&active, k_h_persistent, &cfg) == cudaSuccess && active >= n) return c;
+    if (cudaOccupancyMaxActiveClusters(&active, kern, &cfg) == cudaSuccess && active >= n) return c;
     cudaGetLastError();
   }
   return 4;
@@ -1617,7 +1618,8 @@ int fh_h_batch_create(fh_ctx *ctx, int ninst, const fh_h_params *params_host, in
   B->Ptot = off;
   int rc;
   if (ninst <= kPersMaxInst) {
-    B->pers_ctas = h_pers_ctas(ninst);
+    B->pers_ctas[0] = h_pers_ctas(ninst, k_h_persistent, kPersThreads, kPersSmem);
+    B->pers_ctas[1] = h_pers_ctas(ninst, k_h_pers_own, kOwnThreads, kOwnSmem);
     if (cudaHostAlloc(&B->perr, sizeof(int), cudaHostAllocMapped) != cudaSuccess) {
       cudaGetLastError();
       delete B;
@@ -1866,24 +1868,21 @@ static bool h_persistent_ok(const fh_h_batch *b) {
 static int h_persistent_run(fh_h_batch *b, int nsteps) {
   fh_ctx *ctx = b->ctx;
   b->w_ready = -1;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)(b->n * b->pers_ctas));
-  cfg.blockDim = dim3(kPersThreads);
-  cfg.dynamicSmemBytes = kPersSmem;
-  cfg.stream = ctx->stream;
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeClusterDimension;
-  at[0].val.clusterDim.x = (unsigned)b->pers_ctas;
-  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
-  cfg.attrs = at;
-  cfg.numAttrs = 1;
   // nodes or slots shared out (see the kernels)
   bool own = b->max_steps <= kOwnMaxSteps;
   for (const auto &p : b->hp) own = own && p.N <= kOwnMaxN;
-  if (own) {
-    cfg.blockDim = dim3(kOwnThreads);
-    cfg.dynamicSmemBytes = kOwnSmem;
-  }
+  const int ctas = b->pers_ctas[own];
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(b->n * ctas));
+  cfg.blockDim = dim3(own ? kOwnThreads : kPersThreads);
+  cfg.dynamicSmemBytes = own ? kOwnSmem : kPersSmem;
+  cfg.stream = ctx->stream;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = (unsigned)ctas;
+  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
   fh_prof_mark(ctx, FH_PROF_HISTORY, false);
   auto launch = [&](auto kern, auto... last) {
     return cudaLaunchKernelEx(&cfg, kern, (const fh_h_dev_inst *)b->inst.as<fh_h_dev_inst>(), b->tstep, b->nsaved,
