@@ -28,8 +28,9 @@
 // would lose its low word), with al_left outside [0, 1], or too long for one
 // panel are left to the FP64 solve (the function returns false).
 //
-// exp: 2^(j/16) from a table times a Taylor polynomial of degree 6 on
-// |r| <= ln 2 / 32 (next term 2^-51), its terms above the third power in FP32.
+// exp: table and polynomial (Tang, ACM TOMS 15, 1989, here in pairs): 2^(j/16) from
+// a table times a Taylor polynomial of degree 6 on |r| <= ln 2 / 32 (next term
+// 2^-51), its terms above the third power in FP32.
 #pragma once
 #include "fh_df.cuh"
 #include "fh_hline.cuh"
@@ -68,15 +69,18 @@ __device__ __forceinline__ fh_df fh_df_exp(fh_df x, const float2 *tab) {
   return fh_df{t.h * sc, t.l * sc};
 }
 
-// a / b for normal a, b: the FP32 reciprocal's quotient, corrected twice by its remainder.
+// a / b for normal a, b and quotients that a pair holds (2^-78 and more): the FP32
+// reciprocal's quotient, corrected twice by its remainder.
 __device__ __forceinline__ fh_df fh_df_quot(fh_df a, fh_df b) {
   float r;
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(b.h));
   const float q1 = a.h * r;
-  const float m = fmaf(-q1, b.h, a.h) + fmaf(-q1, b.l, a.l);
+  float m, e;
+  fh_two_sum(fmaf(-q1, b.h, a.h), fmaf(-q1, b.l, a.l), m, e);
   const float q2 = m * r;
-  const float q3 = fmaf(-q2, b.h, m) * r;
-  return fh_df_renorm(q1, q2 + q3);
+  const float q3 = (fmaf(-q2, b.h, m) + e) * r;
+  const fh_df q = fh_df_renorm(q1, q2);
+  return fh_df_renorm(q.h, q.l + q3);
 }
 
 struct fh_dmob {
