@@ -79,7 +79,7 @@ int main(int argc, char **argv) {
 """
 
 
-@pytest.mark.parametrize("what", ["quotient"])
+@pytest.mark.parametrize("what", ["quotient", "exp"])
 def test_accuracy(what, tmp_path):
     if shutil.which("nvcc") is None:
         pytest.skip("nvcc not available")

@@ -35,7 +35,9 @@
 #include "fh_df.cuh"
 #include "fh_hline.cuh"
 
-constexpr float kHdfExp = 11.0f;             // |gam u| at most: exp within 2^+-16
+// |gam u| at most: a pair near 8 ends at 2^-44, and exp turns that into a relative
+// error of K (2^-43.9 measured for 11, 2^-46 for 2)
+constexpr float kHdfExp = 2.0f;
 constexpr float kHdfRow = 0x1p16f;           // row sum at most, 2^-40 at least
 constexpr float kHdfState = 0x1p60f;
 constexpr float kHdfFloor = 0x1p-54f;        // the largest state or boundary value at least
