@@ -767,7 +767,9 @@ __global__ void __launch_bounds__(kOwnThreads, 1)
   double *dxb = psm, *pt = dxb + 2 * PW, *wb = pt + kOwnSum, *hist = wb + (psi ? 3 : 1) * (size_t)kw;
   const int cap = (int)((kOwnSmem / sizeof(double) - (size_t)(hist - psm)) / PW);
   double *Dn = D + I.off + n0;
-  const int parts = max(1, kOwnSum / PW), rows = min(PW, kOwnSum);
+  // (at most 64 runs, which one thread adds: of 256, on a line of 8 nodes, the
+  // additions alone took 7 of a step's 11.7 us)
+  const int parts = min(max(1, kOwnSum / PW), 64), rows = min(PW, kOwnSum);
   const int i = t % rows, p = t / rows;  // node and run of a summing thread (nodes i, i + 256, ... when PW > 256)
   // layers of the occupant before the call
   const int have = max(os0 - I.ob - 1, 0);
