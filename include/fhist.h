@@ -304,7 +304,11 @@ typedef struct fh_tg_solver fh_tg_solver;
  * diffusion coefficient d, psi(t) = t^beta, full history. */
 int fh_tg_create(fh_ctx *ctx, const fh_tg_params *p, int max_steps, int mode, fh_tg_solver **out);
 int fh_tg_destroy(fh_tg_solver *s);
-/* V2 = |v|^2 per node and the initial field, (sN+2)*(M+2) each. */
+/* V2 = |v|^2 per node and the initial field, (sN+2)*(M+2) each.  The reference's
+ * half-step scheme is unstable for small alpha on fine grids, in any precision
+ * (512 x 512, tau = 5e-4, smooth |v|^2 up to 1, 2000 steps: alpha 0.51 grows to
+ * 1e31..1e35 and 0.5225 to 2e8, 0.538 and above stay bounded): such a field turns
+ * the last bit of a weight into 1e-6 of itself and more. */
 int fh_tg_set_state_host(fh_tg_solver *s, const double *V2_host, const double *C_host);
 /* Device-pointer variant (inputs already resident in HBM). */
 int fh_tg_set_state(fh_tg_solver *s, const double *V2, const double *C);
@@ -405,7 +409,9 @@ int fh_ab_set_lag_weights_host(fh_ab_solver *s, int n, const double *w_host);
  * the tensor cores with exact bf16 slices, the rest in double-float; ~2x the
  * history memory).  FH_AB_FP64 contracts the entries before the current
  * 64-step block in exact digits at FP64 accuracy (as FH_TG_FP64) on lines of at
- * most 2049 nodes.  No counterpart in the reference. */
+ * most 2049 nodes; without the memory for that (64 rows of the line) it sums every
+ * entry every step, which rounds otherwise.  Where the call fails the solver keeps
+ * its mode.  No counterpart in the reference. */
 #define FH_AB_FP64 0
 #define FH_AB_BLOCKED 1
 int fh_ab_set_mode(fh_ab_solver *s, int mode);

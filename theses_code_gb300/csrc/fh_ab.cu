@@ -680,7 +680,7 @@ static int ab_one_step(fh_ab_solver *s, int max_n, int *done) {
 // The block-start work of step K is already enqueued; runs up to max_n steps, to
 // the end of the block at most.  Solving warps, double-float: the fewest that
 // take the line at four equations a thread, sixteen (five) for the longest.
-// FP64 (one warp instruction per 19 cycles and SM: fewer warps, fewer scans):
+// FP64 (one warp instruction per 17 cycles and SM: fewer warps, fewer scans):
 // eight equations a thread, up to 2049 nodes.
 template <class F>
 static auto ab_res_pick(const fh_ab_solver *s, F f) {

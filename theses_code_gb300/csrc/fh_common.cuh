@@ -8,14 +8,14 @@
 #define FH_WARP 32
 
 // ---------------------------------------------------------------- loads
-// History layers are read once per step and are far larger than L2 in the
-// large configurations: stream them past L1.
 // Programmatic dependent launch (fh_launch_after, fh_internal.h): wait until the
 // grid before this one has completed and its writes are visible; let the grid
 // after this one start.  A grid launched without the attribute returns at once.
 __device__ __forceinline__ void fh_grid_wait_prev() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void fh_grid_start_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
+// History layers are read once per step and are far larger than L2 in the
+// large configurations: stream them past L1.
 __device__ __forceinline__ double2 fh_ld_stream2(const double *p) {
   return __ldcs(reinterpret_cast<const double2 *>(p));
 }

@@ -2,7 +2,7 @@
 // accuracy on the tensor cores: the layers before a block of future steps,
 // contracted once for all its steps instead of once per step.
 //
-// Why: one FP64 warp instruction takes an SM 19 cycles on GB300, so a history
+// Why: one FP64 warp instruction takes an SM 17 cycles on GB300, so a history
 // sum on the FP64 pipe stops at 2.4 TB/s (two sums per 8-byte difference), and
 // in double-float at HBM speed it still reads every layer every step.  A block
 // of 32 steps x 2 half-step rows reads each layer once.
@@ -49,10 +49,11 @@
 // Waits are bounded; on expiry *err is set and nothing is stored.
 //
 // Measured, whole solves, before and now (with the sweeps' changes since): 2D 251 x
-// 187, 500 steps, FP64 34.9 -> 11.7 ms (the sums of a step 49 -> ~9 us); 512 x
-// 512, 500 steps, DF64 65.1 -> 24.2 ms; one line of 1024 nodes, 2500 steps, FP64
-// 55.2 -> 12.0 ms with the resident solve of fh_ab.cu.  The results differ from the
-// FP64 sums' by 1e-16 (relative).
+// 187, 500 steps, FP64 34.9 -> 12.1 ms (the sums of a step 49 -> ~9 us); 512 x
+// 512, 500 steps, DF64 65.1 -> 25.4 ms; one line of 1024 nodes, 2500 steps, FP64
+// 55.0 -> 12.1 ms with the resident solve of fh_ab.cu.  The results differ from the
+// FP64 sums' by 1e-16 (relative).  A layer that is not finite makes its point's rows
+// NaN, as it makes the point's own field one step later.
 #include <cuda_bf16.h>
 
 #include <algorithm>

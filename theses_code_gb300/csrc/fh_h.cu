@@ -670,7 +670,7 @@ __global__ void __launch_bounds__(kPersThreads, 1)
 // solves one after the other and serial factors, 6.6 ms with the solve beside the
 // next step's sums behind one cluster barrier a step, 4.5 ms in this form; 40
 // steps of N = 64 404, 266, 189 us; 32 psi instances of N = 512 over 250 steps
-// 60.6, 8.3, 6.6 ms.
+// 60.6, 8.3, 6.3 ms.
 constexpr int kOwnLine = 32 * kLineWarps;     // threads of the line solve
 constexpr int kOwnSum = 256;                  // threads of the sums
 constexpr int kOwnThreads = kOwnSum + 128;    // and of the weights
@@ -1233,7 +1233,8 @@ __global__ void k_hb_weights(const fh_h_dev_inst *__restrict__ inst, int K, int 
 // Launched beside the line solves of the step before (fh_launch_after): all
 // layers but the newest, the one those solves make, are summed meanwhile.  They
 // are complete, as k_h_line_df lets this kernel start only after its own wait.
-// 512 psi instances of 64..1024 nodes, 1500 steps: 116.5 -> 110.6 ms.
+// 512 psi instances of 64..1024 nodes, 1500 steps: 116.5 -> 110.6 ms (with every
+// line in double-float).
 __global__ void __launch_bounds__(kTileThreads) k_h_near_df(const fh_h_tile *__restrict__ tiles,
                                                             const fh_h_dev_inst *__restrict__ inst,
                                                             const float2 *ring, long long ldr, int t_lo,

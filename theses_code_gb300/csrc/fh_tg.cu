@@ -509,7 +509,7 @@ static constexpr int kYThreads = 512;  // four adjacent y lines per CTA
 static constexpr int kUnroll = 4;      // equations staged per thread per round
 
 // Lines per CTA of the FP64 sweeps: four fill an SM's sub-partitions, but FP64
-// instructions of all of them share one pipe (19 cycles each), so where the lines
+// instructions of all of them share one pipe (17 cycles each), so where the lines
 // leave SMs idle fewer per CTA finish sooner.  251 x 187 (186 and 250 lines): x
 // 10.2 -> 9.4, y 10.8 -> 9.7 us with two instead of four, 500 steps 14.0 -> 12.9 ms.
 static inline int tg_lines(int lines) { return lines <= 152 ? 1 : lines <= 2 * 152 ? 2 : 4; }
@@ -564,7 +564,7 @@ __device__ __forceinline__ float2 tg_wpair(double w) {
   const float h = __double2float_rn(w);
   return make_float2(h, __double2float_rn(w - (double)h));
 }
-// (double)x on the integer pipe (a conversion takes the FP64 pipe 19 cycles).
+// (double)x on the integer pipe (a conversion takes the FP64 pipe 17 cycles).
 __device__ __forceinline__ double tg_f2d(float x) {
   const unsigned b = __float_as_uint(x), e = b & 0x7f800000u;
   if (e == 0 && (b << 1) != 0) return (double)x;  // below the normal range
