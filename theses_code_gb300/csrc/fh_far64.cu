@@ -444,9 +444,14 @@ __global__ void __launch_bounds__(256) k_far64_fix(const S *__restrict__ D, long
   const long long p = (long long)blockIdx.x * blockDim.x + t;
   double acc[kFixRows] = {};
   bool any = false;
+  uint32_t gm = 0;  // groups with such layers among 32
   for (int G = 0; G < ng; ++G) {
-    const int *ha = hany + G * (kF64Rows / kRowBlock) + n0 / kRowBlock;
-    if (!(ha[0] | ha[1])) continue;  // every thread of the CTA
+    if (G % 32 == 0) {
+      const int g = G + (t & 31);
+      const int *ha = hany + g * (kF64Rows / kRowBlock) + n0 / kRowBlock;
+      gm = __ballot_sync(0xffffffffu, g < ng && (ha[0] | ha[1]));
+    }
+    if (!(gm >> (G % 32) & 1u)) continue;  // every thread of the CTA
     any = true;
     __syncthreads();
     if (t < 4) un[t] = 0;
